@@ -628,12 +628,12 @@ __device__ __forceinline__ void plm_array(int lmax, T x, T sq, T (&p)[(LC + 1) *
 // appears so that only the last two terms of each recursion are live in FP64.
 // The amplitude rcut_max^2 / sigma_t^2 is folded into i_l and its derivative:
 //   out[o_il + l] = amp i_l, out[o_ild + l] = amp d i_l / dr (DER),
-//   out[o_er + m], out[o_ei + m], out[o_amp] = amp, out[o_sf];
+//   out[o_e + 2 m], out[o_e + 2 m + 1] = cos(m phi), -sin(m phi), out[o_sf];
 // cos(theta) and sqrt(1 - cos^2) are returned in x, sq.
 template <int LC, bool DER>
 __device__ __forceinline__ void angular_stage(const DevParams &P, int i_sp, double rj, double theta,
-                                              double phi, float *out, int o_il, int o_ild, int o_er,
-                                              int o_ei, int o_amp, int o_sf, double &x, double &sq) {
+                                              double phi, float *out, int o_il, int o_ild, int o_e,
+                                              int o_sf, double &x, double &sq) {
   // The pair kernel rounds everything below to FP32, so the quotients of the
   // reference's expressions are taken as products with one reciprocal each of
   // sigma, x^2 and r (an FP64 division is a long dependent sequence; these are
@@ -642,7 +642,6 @@ __device__ __forceinline__ void angular_stage(const DevParams &P, int i_sp, doub
   const double sig = P.sig_t[i_sp] + P.sig_t_c[i_sp] * rj;               // :579-580
   const double isig = 1.0 / sig;
   const double amp = P.rcut2 * (isig * isig);
-  out[o_amp] = (float)amp;
   x = cos(theta);
   sq = sqrt(1.0 - x * x);
   // i_l(x^2) exp(-x^2) (src/soap_turbo_angular.f90:361-422) and its radial
@@ -704,8 +703,8 @@ __device__ __forceinline__ void angular_stage(const DevParams &P, int i_sp, doub
   double cosm2 = cphi, sinm2 = -sphi;
   const double cosphi2 = 2.0 * cosm2;
   double cosm1 = 1.0, sinm1 = 0.0;
-  out[o_er] = 1.f;
-  out[o_ei] = 0.f;
+  out[o_e] = 1.f;
+  out[o_e + 1] = 0.f;
 #pragma unroll
   for (int l = 1; l <= LC; ++l) {
     const double cos0 = cosphi2 * cosm1 - cosm2, sin0 = cosphi2 * sinm1 - sinm2;
@@ -713,8 +712,8 @@ __device__ __forceinline__ void angular_stage(const DevParams &P, int i_sp, doub
     sinm2 = sinm1;
     cosm1 = cos0;
     sinm1 = sin0;
-    out[o_er + l] = (float)cos0;
-    out[o_ei + l] = (float)(-sin0);
+    out[o_e + 2 * l] = (float)cos0;
+    out[o_e + 2 * l + 1] = (float)(-sin0);
   }
 }
 

@@ -713,6 +713,15 @@ int build_tables(soapb_context *c) {
   };
   const size_t iW = add(Wblk.data(), Wblk.size() * 8), iC = add(central.data(), central.size() * 8);
   const size_t iK = add(kept_nnl.data(), kept_nnl.size() * 4);
+  // the kept components by descending l: the descriptor's dot products over m
+  std::vector<int4> ps_order(nk);
+  for (int q = 0; q < nk; ++q) {
+    const int n = kept_nnl[q] & 0xff, np = (kept_nnl[q] >> 8) & 0xff, l = kept_nnl[q] >> 16, kb = l * (l + 1) / 2;
+    ps_order[q] = make_int4(n * (K | 1) + kb, np * (K | 1) + kb, q, (int)((unsigned)l | (n != np ? 0x80000000u : 0u)));
+  }
+  std::stable_sort(ps_order.begin(), ps_order.end(),
+                   [](const int4 &x, const int4 &y) { return (x.w & 0xff) > (y.w & 0xff); });
+  const size_t iPs = add(ps_order.data(), ps_order.size() * sizeof(int4));
   const size_t iPo = add(pi_off.data(), pi_off.size() * 4), iPq = add(pi_q.data(), pi_q.size() * 4);
   const size_t iPe = add(pi_el.data(), pi_el.size() * 4), iPe64 = add(pi_el64.data(), pi_el64.size() * 8);
   const size_t iJo = add(pj_off.data(), pj_off.size() * 4), iJq = add(pj_o.data(), pj_o.size() * 4);
@@ -792,13 +801,6 @@ int build_tables(soapb_context *c) {
     for (int s = 0; s < c->n_species; ++s)
       for (int n = 0; n < c->alpha[s]; ++n) nmap[P.rad[s].nbeg + n] = s | (n << 8);
     P.off_nmap = put_c(nmap.data(), nmap.size() * 4);
-    std::vector<int> citem;
-    for (int s = 0; s < c->n_species; ++s)
-      for (int kk = 0; kk < K; ++kk)
-        for (int half = 0; half < 2; ++half)
-          if (half * (amax_t / 2) < c->alpha[s]) citem.push_back(s | (kk << 4) | (half << 12));
-    P.n_citem = (int)citem.size();
-    P.off_citem = put(citem.data(), citem.size() * 4);
     // H items (n, l, m0): m = m0 .. m0 + 2 (the contract kernel's kHM) of one
     // (n, l) Y list, which costs the list's length per m; empty lists give no
     // item.  Heaviest first, so that a strided assignment over the CTA's
@@ -940,6 +942,7 @@ int build_tables(soapb_context *c) {
   P.wstride = wstride;
   P.central = (const double *)at(iC);
   P.kept_nnl = (const int *)at(iK);
+  P.ps_order = (const int4 *)at(iPs);
   P.pi_off = (const int *)at(iPo);
   P.pi_q = (const int *)at(iPq);
   P.pi_el = (const float *)at(iPe);

@@ -62,6 +62,8 @@ struct DevParams {
   int wstride;            // doubles between species blocks
   const double *central;  // n_max: poly3gauss central-atom term per radial index
   const int *kept_nnl;    // n_kept: n | np << 8 | l << 16 of the kept components
+  const int4 *ps_order;   // n_kept components by descending l: where their c_nl0 and c_n'l0 stand in
+                          // (n, k_max | 1), their position, and l | (n != n') << 31
   const int *pi_off;      // n_soap + 1: CSR over outputs of the compression map
   const int *pi_q;        //   kept position feeding each entry
   const float *pi_el;
@@ -90,7 +92,6 @@ struct DevParams {
   int off_kpx;            // (l_max+2)(l_max+3)/2 float: preflm to l_max + 1 (pair kernel)
   int off_rad;            // n_species RadSp
   int off_klm;            // KS int: l | m << 8
-  int off_citem;          // n_citem int: c_nlm items species | k << 4 | half << 12
   int off_kept;           // n_kept int: kept_nnl
   int off_central;        // n_max double: poly3gauss central-atom term
   // in blob_c (n_species RadSp at 0):
@@ -101,7 +102,7 @@ struct DevParams {
   int off_hitem;          // n_hitem int: H items n | l << 8
   int off_hloff;          // (l_max+1)*n_max + 1 int: per (l, n) list offsets
   int off_hl;             // packed Y-list entries np | q << 8 | (n == np) << 31, when hl_in_blob
-  int n_citem, n_hitem;
+  int n_hitem;
   int hl_in_blob;         // the packed Y lists fit in the blob (else read from hl_packed)
   const int *hl_packed;   // global copy of the packed Y lists
   int cmap_identity;      // the compression map sends kept component q to output q, weight 1
@@ -181,7 +182,6 @@ cudaError_t launch_descriptor(const DevParams &P, const DevBatch &B, const Launc
 cudaError_t launch_contract(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
                             const double *soap, const double *G, int g_layout, double sgn,
                             const float *keep_c, const double *keep_norm, double *pair);
-size_t descriptor_smem(const DevParams &P, int threads);
 // Device address and size of the static scratch array (soapb_noalloc.cu);
 // `device` must be current.
 cudaError_t noalloc_scratch(int device, unsigned char **addr, size_t *bytes);

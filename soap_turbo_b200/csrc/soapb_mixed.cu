@@ -202,27 +202,29 @@ __device__ __forceinline__ int first_species(unsigned bits) { return __ffs(bits)
 
 // ------------------------------------------------------------ pair rows
 // The angular row of a pair (floats), written by k_pair and read by the site
-// kernels: amp i_l, amp di_l/dr, cos(m phi), -sin(m phi) for l, m <= LC, the
-// amplitude amp = rcut_max^2 / sigma_t^2, 2 sigma_t_scaling / sigma_t,
-// cos(theta), sqrt(1 - cos^2(theta)), then preflm_k P_l^m for l <= l_max (+1
-// with derivatives), k = l(l+1)/2 + m.  So u_k = amp preflm_k P_k i_l of
-// src/soap_turbo_angular.f90:590-594 is one product of two row values.
+// kernels; the descriptor reads its first part alone:
+//   amp i_l for l <= LC (amp = rcut_max^2 / sigma_t^2), a pad, and
+//   (cos(m phi), -sin(m phi)) for m <= LC;
+//   preflm_k P_l^m for l <= l_max (+1 with derivatives), k = l(l+1)/2 + m;
+//   amp di_l/dr, 2 sigma_t_scaling / sigma_t, cos(theta), sqrt(1 - cos^2(theta)).
+// So u_k = amp preflm_k P_k i_l of src/soap_turbo_angular.f90:590-594 is one
+// product of two row values.  LC is even: every part is a multiple of 16 bytes.
 __host__ __device__ constexpr int row_il(int) { return 0; }
-__host__ __device__ constexpr int row_ild(int LC) { return LC + 1; }
-__host__ __device__ constexpr int row_er(int LC) { return 2 * (LC + 1); }
-__host__ __device__ constexpr int row_ei(int LC) { return 3 * (LC + 1); }
-__host__ __device__ constexpr int row_amp(int LC) { return 4 * (LC + 1); }
-__host__ __device__ constexpr int row_sf(int LC) { return 4 * (LC + 1) + 1; }
-__host__ __device__ constexpr int row_x(int LC) { return 4 * (LC + 1) + 2; }
-__host__ __device__ constexpr int row_sq(int LC) { return 4 * (LC + 1) + 3; }
-__host__ __device__ constexpr int row_p(int LC) { return 4 * (LC + 1) + 4; }
-__host__ __device__ constexpr int row_len(int LC) { return (row_p(LC) + (LC + 2) * (LC + 3) / 2 + 3) / 4 * 4; }
+__host__ __device__ constexpr int row_e(int LC) { return LC + 2; }
+__host__ __device__ constexpr int row_p(int LC) { return 3 * LC + 4; }
+__host__ __device__ constexpr int row_tail(int LC) { return (row_p(LC) + (LC + 2) * (LC + 3) / 2 + 3) / 4 * 4; }
+__host__ __device__ constexpr int row_ild(int LC) { return row_tail(LC); }
+__host__ __device__ constexpr int row_sf(int LC) { return row_tail(LC) + LC + 1; }
+__host__ __device__ constexpr int row_x(int LC) { return row_tail(LC) + LC + 2; }
+__host__ __device__ constexpr int row_sq(int LC) { return row_tail(LC) + LC + 3; }
+__host__ __device__ constexpr int row_len(int LC) { return row_tail(LC) + LC + 4; }
 
 int ang_row_floats(const DevParams &P) { return row_len(P.amax_t == 8 ? 8 : 12); }
 // the pair kernel's staging stride in floats (odd): the whole row, or with TAB
-// the larger of its two halves
+// the larger of its P_l^m values and the rest
 __host__ __device__ constexpr int pair_stage_stride(int LC, bool TAB) {
-  return TAB ? (row_p(LC) > row_len(LC) - row_p(LC) ? row_p(LC) : row_len(LC) - row_p(LC)) + 1 : row_len(LC) + 1;
+  const int np = row_tail(LC) - row_p(LC), rest = row_len(LC) - np;
+  return TAB ? (np > rest ? np : rest) + 1 : row_len(LC) + 1;
 }
 
 // ------------------------------------------------------------ pair kernel
@@ -262,9 +264,10 @@ __global__ void __launch_bounds__(kPairThreads)
   }
   constexpr int AW = row_len(LC);
   // odd stride in shared memory: each thread fills its own row, so lanes must
-  // not all map to one bank.  TAB stages the row in two halves (the scalars,
-  // then the P_l^m values) through half the buffer, for more CTAs per SM.
+  // not all map to one bank.  TAB stages the row in two halves (all but the
+  // P_l^m values, then those) through half the buffer, for more CTAs per SM.
   constexpr int AWS = pair_stage_stride(LC, TAB);
+  constexpr int TO = TAB ? row_tail(LC) - row_p(LC) : 0;  // the row's tail follows its head there
   const int head = (P.off_rad + P.n_species * SOAPB_RADSP_BYTES) / 16;
   for (int t = threadIdx.x; t < head; t += NT) ((uint4 *)smem)[t] = ((const uint4 *)P.blob)[t];
   float *rows = (float *)(smem + (size_t)head * 16);
@@ -283,13 +286,13 @@ __global__ void __launch_bounds__(kPairThreads)
       active = true;
       const int isp = __ffs(bits) - 1;
       if (do_der)
-        angular_stage<LC, true>(P, isp, r, B.thetas[k], B.phis[k], row, row_il(LC), row_ild(LC),
-                                row_er(LC), row_ei(LC), row_amp(LC), row_sf(LC), x, sq);
+        angular_stage<LC, true>(P, isp, r, B.thetas[k], B.phis[k], row, row_il(LC), row_ild(LC) - TO,
+                                row_e(LC), row_sf(LC) - TO, x, sq);
       else
-        angular_stage<LC, false>(P, isp, r, B.thetas[k], B.phis[k], row, row_il(LC), row_ild(LC),
-                                 row_er(LC), row_ei(LC), row_amp(LC), row_sf(LC), x, sq);
-      row[row_x(LC)] = (float)x;
-      row[row_sq(LC)] = (float)sq;
+        angular_stage<LC, false>(P, isp, r, B.thetas[k], B.phis[k], row, row_il(LC), row_ild(LC) - TO,
+                                 row_e(LC), row_sf(LC) - TO, x, sq);
+      row[row_x(LC) - TO] = (float)x;
+      row[row_sq(LC) - TO] = (float)sq;
       if constexpr (!TAB) {
         float *Pr = row + row_p(LC);
         const float *kpx = (const float *)(smem + P.off_kpx);
@@ -378,13 +381,14 @@ __global__ void __launch_bounds__(kPairThreads)
   __syncthreads();
   const int nrow = min(NT, pair_hi - k0);
   if constexpr (TAB) {
-    // coalesced 16-byte stores of the rows' first parts, then the P_l^m values
-    // through the same buffer
-    constexpr int P1 = row_p(LC) / 4, P2 = (AW - row_p(LC)) / 4;
+    // coalesced 16-byte stores of the rows' heads and tails, then the P_l^m
+    // values through the same buffer
+    constexpr int H4 = row_p(LC) / 4, T4 = row_tail(LC) / 4, P1 = H4 + (AW / 4 - T4), P2 = T4 - H4;
     for (int t = threadIdx.x; t < nrow * P1; t += NT) {
       const int i = t / P1, j = t - i * P1;
       const float *src = rows + i * AWS + 4 * j;
-      *(float4 *)(B.ang + (size_t)(k0 + i) * AW + 4 * j) = make_float4(src[0], src[1], src[2], src[3]);
+      *(float4 *)(B.ang + (size_t)(k0 + i) * AW + 4 * (j < H4 ? j : j - H4 + T4)) =
+          make_float4(src[0], src[1], src[2], src[3]);
     }
     __syncthreads();
     if (active) {
@@ -746,146 +750,374 @@ __device__ __forceinline__ void site_output(const DevParams &P, unsigned char *s
     }
 }
 
+// ------------------------------------------------------------ entries of a warp
+// The species the radial expansion of each pair of [c0, c1) applies to, for the
+// calling warp: byte c of the result is pair c0 + 32 c + lane, bit s species s
+// (mask set, inside the species' rcut_hard and rcut_max, the self pair only when
+// its expansion is used, and not for the force contraction, vjp).
+__device__ __forceinline__ unsigned long long valid_species(const DevParams &P, const DevBatch &B, int p_begin,
+                                                            int c0, int c1, bool vjp) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long v = 0ull;
+#pragma unroll 4
+  for (int c = 0; c0 + 32 * c < c1; ++c) {
+    const int k = c0 + 32 * c + lane;
+    if (k >= c1) continue;
+    const double r = B.rjs[k];
+    const unsigned bits = B.bits[k];
+    unsigned ok = 0u;
+    // a pair at or beyond rcut_max has no angular row (the reference zeroes its
+    // angular coefficients, src/soap_turbo_angular.f90:549-574); it only matters
+    // for poly3operator, whose radial part has no rcut_hard cut
+    if (r < P.rcut_max)
+      for (int s = 0; s < P.n_species; ++s)
+        if (((bits >> s) & 1u) && r < P.rad[s].rcut_hard && (k > p_begin || (!vjp && P.rad[s].do_central)))
+          ok |= 1u << s;
+    v |= (unsigned long long)ok << (8 * c);
+  }
+  return v;
+}
+
+// Appends species s's entries of a chunk of n_chunk pairs, in order, as chunk-local
+// pair | s << 8 from list[e] on; returns the end.  Every warp of a CTA may write
+// the same list: it writes the same values.
+__device__ __forceinline__ int list_species(unsigned long long valid, int s, int n_chunk, int e, unsigned short *list) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  for (int c = 0; 32 * c < n_chunk; ++c) {
+    const bool on = (valid >> (8 * c + s)) & 1ull;
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (on) list[e + __popc(m & lt)] = (unsigned short)((32 * c + lane) | (s << 8));
+    e += __popc(m);
+  }
+  return e;
+}
+
+// Two FP32 values in a 64-bit register pair, and two fused multiply-adds in one
+// instruction, each rounded as fmaf's.  Kept as 64-bit values from the load to
+// the last use: a float2 would be taken apart and put together around each one.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+  return d;
+}
+__device__ __forceinline__ f32x2 ffma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+__device__ __forceinline__ f32x2 fmul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // ------------------------------------------------------------ descriptor
-template <int NT, int AMAX, int LC>
-__global__ void __launch_bounds__(NT, 640 / NT) k_descriptor(const DevParams P, const DevBatch B,
-                                                      double *__restrict__ soap_out,
-                                                      float *__restrict__ keep_c,
-                                                      double *__restrict__ keep_norm, int keep) {
+// One CTA of a few warps per site; a thread owns one k = (l, m) and NH of the
+// radial indices of every species block (warp w: k = 32 (w % kw) + lane, radial
+// indices from NH (w / kw)).
+//  entries    the (pair, species) entries the expansion applies to, by species,
+//             then in CSR order, found with ballots by every warp for itself
+//  staging    a round of at most 64 entries: the rows' first part and R_n, a
+//             warp per row, with 16-byte asynchronous copies
+//  c_nlm      FP32 partial sums over groups of four entries flushed into FP64;
+//             two radial indices per fma.rn.f32x2.  A species' sums stay in
+//             registers from its first entry to its last.  Rounds are those of
+//             `chunk` pairs' entries cut at multiples of min(chunk / 2, 64): the
+//             groups do not depend on the launch shape.
+//  spectrum   one dot product per kept component, the components ordered by
+//             l (P.ps_order) so that a warp's dot products are equally long
+// What bounds it: instructions (8.3 k per site of 52 pairs and three species, of
+// which the products are a tenth) issued at 43 % of the rate with 14 warps per SM,
+// by the latency of a warp's chain.  One CTA of 128 threads that staged, sorted and
+// summed behind barriers took 15 k: 338 against 251 us at 13092 sites of three
+// species, 55 against 43 us at 1679.
+struct DescLayout {
+  size_t list, base, X, P, S, total;
+};
+__host__ __device__ constexpr int desc_head(int LC) { return (row_p(LC) + (LC + 1) * (LC + 2) / 2 + 3) / 4 * 4; }
+// a staged entry: the row's first part, then its species' R_n
+__host__ __device__ constexpr int desc_stride(int AMAX, int LC) { return desc_head(LC) + AMAX; }
+__host__ __device__ inline DescLayout desc_layout(const DevParams &P, int chunk, int AMAX, int LC) {
+  DescLayout L{};
+  size_t o = align_up((size_t)P.n_max * (size_t)(P.k_max | 1) * sizeof(float2), 16);  // c_nlm, (n, KS), at 0
+  L.base = o; o += 16 * sizeof(int);
+  L.list = o; o = align_up(o + (size_t)chunk * P.n_species * sizeof(unsigned short), 16);
+  // the staged round; after c_nlm the components and the compressed descriptor
+  L.X = L.P = o;
+  const size_t x = o + (size_t)(chunk / 2 < 64 ? chunk / 2 : 64) * desc_stride(AMAX, LC) * sizeof(float);
+  L.S = o + (P.cmap_identity ? 0 : (size_t)P.n_kept * sizeof(float));
+  const size_t y = L.S + (size_t)P.n_soap * sizeof(float);
+  L.total = align_up(x > y ? x : y, 16);
+  return L;
+}
+
+// resident CTAs the register count is held to (the staged round allows seven)
+__host__ __device__ constexpr int desc_min_ctas(int AMAX, int NH) {
+  return AMAX == 8 ? (NH == 8 ? 7 : NH == 4 ? 6 : 3) : 3;
+}
+
+template <int AMAX, int LC, int NH>
+__global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AMAX / NH), desc_min_ctas(AMAX, NH))
+    k_descriptor(const DevParams P, const DevBatch B, int chunk, int kw, double *__restrict__ soap_out,
+                 float *__restrict__ keep_c, double *__restrict__ keep_norm, int keep) {
   // keep: bit 0 keeps c_nlm and the norm for the contract, bit 1 accumulates
   // into soap_out
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr int CH = stage_entries_per_round(NT, 0);
-  constexpr int NH = AMAX / 2;  // radial indices per c_nlm item
-  const int AS = stage_stride(LC, 0);
-  const Layout Ly = make_layout(P, NT, AMAX, LC, 0);
-  const int *klm = (const int *)SBLOB(off_klm);
-  const int *citem = (const int *)SBLOB(off_citem);
-  const int *kept = (const int *)SBLOB(off_kept);
-  const double *central = (const double *)SBLOB(off_central);
-  double *sRed = (double *)(smem + Ly.red);
-  double *sC64 = (double *)(smem + Ly.C64);
-  float *sR = (float *)(smem + Ly.R);
-  float *sA = (float *)(smem + Ly.A);
-  float *sC = (float *)(smem + Ly.C);
-  float *sP = (float *)(smem + Ly.P);
-  float *sS = (float *)(smem + Ly.S);
-  int *sEnt = (int *)(smem + Ly.ent);
-  int *sW_cnt = (int *)(smem + Ly.wcnt);
-  int *sMisc = (int *)(smem + Ly.misc);
-  int *sBase = sMisc, *sCnt = sMisc + SOAPB_MAX_SPECIES, *sNent = sMisc + 2 * SOAPB_MAX_SPECIES;
-  int *sSite = sMisc + 3 * SOAPB_MAX_SPECIES;
-
-  const int tid = threadIdx.x;
-  const int KS = P.k_max | 1;
-  const int n_max = P.n_max, nsp = P.n_species;
-
-  copy_site_blob<NT>(P, smem, 0);
-  first_site(B, B.ticket, sSite);
-  for (;;) {
-    const int site = sSite[0];
-    if (site >= B.site_hi) break;
-    const int p_begin = sSite[1];
-    const int p_end = min(sSite[2], B.n_pairs);
-    int nx = 0, nx0 = 0, nx1 = 0;
-    if (tid == 0) nx = take_ticket(B, B.ticket);  // the next site, fetched ahead
-    for (int t = tid; t < 2 * n_max * KS; t += NT) sC64[t] = 0.0;
-    __syncthreads();
-
-    for (int chunk = p_begin; chunk < p_end; chunk += NT) {
-      int slot[SOAPB_MAX_SPECIES];
-      unsigned my_bits;
-      double my_r;
-      const int n_ent = build_entries<NT>(P, B, p_begin, chunk, p_end, false, sEnt, sW_cnt, sBase,
-                                          sCnt, sNent, slot, my_bits, my_r);
-      for (int ebase = 0; ebase < n_ent; ebase += CH) {
-        const int n_round = min(CH, n_ent - ebase);
-        // ---- A. the entries' rows
-        stage_entries<NT, AMAX, LC, false>(P, B, sEnt, chunk, ebase, n_round, sA, sR, nullptr);
-        __syncthreads();
-        // the central pair's entries carry central_weight (:638-646); the pair
-        // kernel expanded every pair as a neighbour
-        if (chunk == p_begin) {
-          for (int el = tid; el < n_round; el += NT) {
-            const int code = sEnt[ebase + el];
-            const double cw = rad_of(smem, P, code >> 24).cw;
-            if ((code & 0xffffff) == 0 && cw != 1.0)
+  constexpr int AW = row_len(LC), ST = desc_stride(AMAX, LC), HD = desc_head(LC);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+  const DescLayout Ly = desc_layout(P, chunk, AMAX, LC);
+  float2 *sC = (float2 *)smem;
+  float *sX = (float *)(smem + Ly.X), *sP = (float *)(smem + Ly.P), *sS = (float *)(smem + Ly.S);
+  int *sBase = (int *)(smem + Ly.base);
+  unsigned short *list = (unsigned short *)(smem + Ly.list);
+  const int KS = P.k_max | 1, n_max = P.n_max, nsp = P.n_species;
+  const int k_of = 32 * (warp % kw) + lane, n0 = NH * (warp / kw);
+  const bool own = k_of < P.k_max;
+  const int kk = own ? k_of : P.k_max - 1;  // the last lanes repeat the last k and store nothing
+  const int lm = __ldg((const int *)(P.blob + P.off_klm) + kk), l = lm & 0xff, m = lm >> 8;
+  const int rounds = min(chunk / 2, 64);
+  const int n_run = B.site_hi - B.site_lo;
+  const int4 it0 = tid < P.n_kept ? __ldg(P.ps_order + tid) : make_int4(0, 0, 0, 0);
+  // the 16-byte pieces of an entry that the lane stages: of the row's head, then of R_n
+  constexpr int NC = (HD / 4 + AMAX / 4 + 31) / 32;
+  const int n_head = (row_p(LC) + P.k_max + 3) / 4;
+  struct {
+    bool on, rad;
+    int first, dst;
+    unsigned per_pair, per_species;
+  } piece[NC];
 #pragma unroll
-              for (int n = 0; n < AMAX; ++n) sR[(size_t)el * AMAX + n] *= (float)cw;
-          }
-          __syncthreads();
+  for (int c = 0; c < NC; ++c) {
+    const int t = lane + 32 * c, r = t - n_head;
+    piece[c].on = r < AMAX / 4;
+    piece[c].rad = r >= 0;
+    piece[c].first = 4 * (r >= 0 ? r : t);
+    piece[c].dst = r >= 0 ? HD + 4 * r : 4 * t;
+    piece[c].per_pair = r >= 0 ? nsp * 2 * AMAX : AW;
+    piece[c].per_species = r >= 0 ? 2 * AMAX : 0;
+  }
+
+  for (int b = blockIdx.x; b < n_run; b += gridDim.x) {
+    const int site = B.order ? B.order[b] : B.site_lo + b;
+    const int p_begin = B.off[site], p_end = min(B.off[site + 1], B.n_pairs);
+    // the species whose sums the thread holds, its rounds so far, their sums but
+    // for the last, and that of the last
+    int cs = 0, n_rounds = 0;
+    double tr[NH], ti[NH], dr[NH], di[NH];
+    float *kc = keep_c + ((keep & 1) ? (size_t)site * keep_stride(P) + kk : 0);
+    auto finish = [&]() {  // species cs is complete
+      const int a = P.rad[cs].alpha, nb = P.rad[cs].nbeg;
+      if (n_rounds != 1)
+#pragma unroll
+        for (int n = 0; n < NH; ++n) {
+          dr[n] = n_rounds ? tr[n] + dr[n] : 0.0;
+          di[n] = n_rounds ? ti[n] + di[n] : 0.0;
         }
-        // ---- B. c_nlm: item = (species, k, half of the species' radial block);
-        // FP32 partial sums over groups of 4 entries, flushed into FP64
-        const int e_hi = ebase + n_round;
-        for (int it = tid; it < P.n_citem; it += NT) {
-          const int code = citem[it];
-          const int s = code & 15, kk = (code >> 4) & 0xff, half = code >> 12;
-          const int lo = max(sBase[s], ebase), hi = min(sBase[s] + sCnt[s], e_hi);
-          if (lo >= hi) continue;
-          const RadSp &RS = rad_of(smem, P, s);
-          const int nb = RS.nbeg, a = RS.alpha, n0 = half * NH;
-          const int l = klm[kk] & 0xff, m = klm[kk] >> 8;
-          double dr[NH], di[NH];
-          float pr[NH], pi[NH];
+      // poly3gauss central-atom term (src/soap_turbo.f90:646-662)
+      if (P.basis == 1 && kk == 0) {
+        const int mult = B.species_mult[site];
+        for (int mm = 0; mm < mult; ++mm)
+          if (B.species[(size_t)site * B.max_mult + mm] - 1 == cs)
 #pragma unroll
-          for (int n = 0; n < NH; ++n) {
-            dr[n] = di[n] = 0.0;
-            pr[n] = pi[n] = 0.f;
+            for (int n = 0; n < NH; ++n)
+              if (n0 + n < a) dr[n] += P.central[nb + n0 + n];
+      }
+      float2 *cc = sC + (nb + n0) * KS + kk;
+      if (own)
+#pragma unroll
+        for (int n = 0; n < NH; ++n)
+          if (n0 + n < a) cc[n * KS] = make_float2((float)dr[n], (float)di[n]);
+      if (own && (keep & 1)) {
+        float *kr = kc + (nb + n0) * KS, *ki = kr + n_max * KS;
+#pragma unroll
+        for (int n = 0; n < NH; ++n)
+          if (n0 + n < a) {
+            kr[n * KS] = (float)dr[n];
+            ki[n * KS] = (float)di[n];
           }
-          int cnt = 0;
-          for (int e2 = lo; e2 < hi; ++e2) {
-            const int el = e2 - ebase;
-            const float *Ae = sA + (size_t)el * AS;
-            // u_k = (preflm_k P_k) (amp i_l) (src/soap_turbo_angular.f90:590-594)
-            const float u = Ae[row_p(LC) + kk] * Ae[row_il(LC) + l];
-            const float ar = u * Ae[row_er(LC) + m], ai = u * Ae[row_ei(LC) + m];
-            const float *Re = sR + (size_t)el * AMAX + n0;
+      }
+      ++cs;
+      n_rounds = 0;
+    };
+    // a site of one chunk takes all its species at once; else a species at a time
+    const bool multi = p_end - p_begin > chunk;
+    for (int s_lo = 0; s_lo < nsp; s_lo += multi ? 1 : nsp) {
+      const int s_hi = multi ? s_lo + 1 : nsp;
+      for (int c0 = p_begin; c0 < p_end; c0 += chunk) {
+        const int c1 = min(p_end, c0 + chunk);
+        const unsigned long long valid = valid_species(P, B, p_begin, c0, c1, false);
+        // the place of species s_lo among the chunk's entries, which fixes the rounds
+        const int e0 = __reduce_add_sync(0xffffffffu, __popcll(valid & (0x0101010101010101ull * ((1u << s_lo) - 1u))));
+        if (multi) __syncthreads();  // the previous chunk's list is read
+        int e = e0;
+        for (int s = s_lo; s < s_hi; ++s) {
+          if (lane == 0) sBase[s] = e;
+          e = list_species(valid, s, c1 - c0, e, list - e0);
+        }
+        if (lane == 0) sBase[s_hi] = e;
+        __syncwarp();
+        const int e1 = e;
+        const float *src[NC];
 #pragma unroll
-            for (int n = 0; n < NH; ++n) {
-              pr[n] = fmaf(Re[n], ar, pr[n]);
-              pi[n] = fmaf(Re[n], ai, pi[n]);
-            }
-            if (++cnt == 4) {
-              cnt = 0;
+        for (int c = 0; c < NC; ++c)
+          src[c] = piece[c].rad ? B.rad + (size_t)c0 * nsp * 2 * AMAX + piece[c].first
+                                : B.ang + (size_t)c0 * AW + piece[c].first;
+        for (int w0 = e0, w1; w0 < e1; w0 = w1) {
+          w1 = min(e1, w0 + rounds - (w0 & (rounds - 1)));
+          float *dst = sX + warp * ST;
+#pragma unroll 4
+          for (int q = w0 + warp; q < w1; q += nw, dst += nw * ST) {
+            const unsigned code = list[q - e0], j = code & 0xffu, sp = code >> 8;
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+              if (piece[c].on)
+                cp_async16(dst + piece[c].dst, src[c] + (j * piece[c].per_pair + sp * piece[c].per_species));
+          }
+          cp_async_wait_all();
+          __syncthreads();
+          for (int s = s_lo; s < s_hi; ++s) {
+            const int lo = max(w0, sBase[s]), hi = min(w1, sBase[s + 1]);
+            if (lo >= hi) continue;
+            while (cs < s) finish();
+            if (n0 >= P.rad[s].alpha) continue;
+            // the central pair carries central_weight (:638-646): the pair kernel
+            // expanded every pair as a neighbour
+            const bool weighted = P.rad[s].cw != 1.0 && c0 == p_begin && lo == sBase[s] && (list[lo - e0] & 0xff) == 0;
+            const float cw = (float)P.rad[s].cw;
+            if (n_rounds > 0)
 #pragma unroll
               for (int n = 0; n < NH; ++n) {
-                dr[n] += (double)pr[n];
-                di[n] += (double)pi[n];
-                pr[n] = pi[n] = 0.f;
+                tr[n] = n_rounds > 1 ? tr[n] + dr[n] : dr[n];
+                ti[n] = n_rounds > 1 ? ti[n] + di[n] : di[n];
               }
-            }
-          }
+            ++n_rounds;
+            f32x2 pr[NH / 2], pi[NH / 2];
+            const float *A = sX + (lo - w0) * ST;
+            const float *aP = A + row_p(LC) + kk, *aL = A + row_il(LC) + l, *aE = A + row_e(LC) + 2 * m,
+                        *aR = A + HD + n0;
+            auto add = [&](int o, bool first, bool opens) {  // the round's first entry, its group's first
+              // u_k = (preflm_k P_k) (amp i_l) (src/soap_turbo_angular.f90:590-594)
+              const float u = aP[o] * aL[o];
+              const float2 e2 = *(const float2 *)(aE + o);
+              const float ar = u * e2.x, ai = u * e2.y;
+              const f32x2 ar2 = pack2(ar, ar), ai2 = pack2(ai, ai);
+              f32x2 r[NH / 2];
+              if constexpr (NH % 4 == 0) {
 #pragma unroll
-          for (int n = 0; n < NH; ++n) {
-            if (n0 + n < a) {
-              sC64[(size_t)(nb + n0 + n) * KS + kk] += dr[n] + (double)pr[n];
-              sC64[(size_t)(n_max + nb + n0 + n) * KS + kk] += di[n] + (double)pi[n];
+                for (int n = 0; n < NH / 4; ++n) {
+                  const ulonglong2 v = *(const ulonglong2 *)(aR + o + 4 * n);
+                  r[2 * n] = v.x;
+                  r[2 * n + 1] = v.y;
+                }
+              } else {
+#pragma unroll
+                for (int n = 0; n < NH / 2; ++n) r[n] = *(const f32x2 *)(aR + o + 2 * n);
+              }
+              if (first && weighted)
+#pragma unroll
+                for (int n = 0; n < NH / 2; ++n) {
+                  const float2 v = unpack2(r[n]);
+                  r[n] = pack2(v.x * cw, v.y * cw);
+                }
+#pragma unroll
+              for (int n = 0; n < NH / 2; ++n) {
+                pr[n] = opens ? fmul2(r[n], ar2) : ffma2(r[n], ar2, pr[n]);
+                pi[n] = opens ? fmul2(r[n], ai2) : ffma2(r[n], ai2, pi[n]);
+              }
+            };
+            auto flush = [&](bool first) {  // the round's first group
+#pragma unroll
+              for (int n = 0; n < NH / 2; ++n) {
+                const float2 vr = unpack2(pr[n]), vi = unpack2(pi[n]);
+                dr[2 * n] = first ? (double)vr.x : dr[2 * n] + (double)vr.x;
+                dr[2 * n + 1] = first ? (double)vr.y : dr[2 * n + 1] + (double)vr.y;
+                di[2 * n] = first ? (double)vi.x : di[2 * n] + (double)vi.x;
+                di[2 * n + 1] = first ? (double)vi.y : di[2 * n + 1] + (double)vi.y;
+              }
+            };
+            int i = lo;
+            for (; i + 4 <= hi; i += 4) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) add(q * ST, q == 0 && i == lo, q == 0);
+              if (i == lo) flush(true);
+              else flush(false);
+              aP += 4 * ST;
+              aL += 4 * ST;
+              aE += 4 * ST;
+              aR += 4 * ST;
+            }
+            if (i < hi) {
+              const int n_last = hi - i;
+              add(0, i == lo, true);
+              if (n_last > 1) add(ST, false, false);
+              if (n_last > 2) add(2 * ST, false, false);
+              if (i == lo) flush(true);
+              else flush(false);
             }
           }
+          __syncthreads();  // the round's rows are read
         }
-        __syncthreads();
       }
     }
-
-    ahead_bounds(B, nx, nx0, nx1);
-    // ---- poly3gauss central-atom term (src/soap_turbo.f90:646-662)
-    if (P.basis == 1) {
-      const int mult = B.species_mult[site];
-      for (int mm = 0; mm < mult; ++mm) {
-        const int s = B.species[(size_t)site * B.max_mult + mm] - 1;
-        if (s < 0 || s >= nsp) continue;
-        const RadSp &RS = rad_of(smem, P, s);
-        for (int n = tid; n < RS.alpha; n += NT) sC64[(size_t)(RS.nbeg + n) * KS] += central[RS.nbeg + n];
-        __syncthreads();
-      }
+    while (cs < nsp) finish();
+    __syncthreads();
+    // power spectrum of the kept components (src/soap_turbo.f90:750-795)
+    float *pout = P.cmap_identity ? sS : sP;
+    int4 it = it0;
+    for (int t = tid; t < P.n_kept; t += nt) {
+      const int4 nx = t + nt < P.n_kept ? __ldg(P.ps_order + t + nt) : it;  // a round trip ahead
+      const float2 *cn = sC + it.x, *cp = sC + it.y;
+      const int lq = it.w & 0xff;
+      const float acc0 = cn[0].x * cp[0].x + cn[0].y * cp[0].y;
+      float acc = 0.f;
+#pragma unroll 4
+      for (int q = 1; q <= lq; ++q) acc += cn[q].x * cp[q].x + cn[q].y * cp[q].y;
+      const float base = it.w < 0 ? 1.41421356237309504880f : 1.f;
+      const float v = base * (acc0 + 2.f * acc);
+      pout[it.z] = v;
+      it = nx;
     }
     __syncthreads();
-    for (int t = tid; t < 2 * n_max * KS; t += NT) sC[t] = (float)sC64[t];
-    __syncthreads();
-
-    site_output<NT>(P, smem, sC, sP, sS, nullptr, kept, sRed, site, soap_out, keep_c, keep_norm, keep, false);
-    ahead_publish(sSite, nx, nx0, nx1);
+    if (!P.cmap_identity) {
+      // compression through the map (:798-802)
+      for (int o = tid; o < P.n_soap; o += nt) {
+        float v = 0.f;
+        for (int t = P.pi_off[o]; t < P.pi_off[o + 1]; ++t) v += P.pi_el[t] * sP[P.pi_q[t]];
+        sS[o] = v;
+      }
+      __syncthreads();
+    }
+    // the norm (:805-809), by every warp for itself: its order then does not
+    // depend on the number of warps.  accumulate: the caller's soap row is added
+    // before the norm is taken, as the reference adds the compressed descriptor
+    // into soap (:798-802)
+    double *out = soap_out + (size_t)site * P.n_soap;
+    const bool acc = (keep & 2) != 0;
+    double nrm2 = 0.0;
+    for (int o = lane; o < P.n_soap; o += 32) {
+      const double v = acc ? (double)sS[o] + out[o] : (double)sS[o];
+      nrm2 += v * v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nrm2 += __shfl_xor_sync(0xffffffffu, nrm2, o);
+    if (acc) __syncthreads();  // every warp has read the caller's row
+    double norm = sqrt(nrm2);
+    if (norm < 1.0e-5) norm = 1.0;
+    const double inv = 1.0 / norm;
+    if (acc)
+      for (int o = tid; o < P.n_soap; o += nt) out[o] = ((double)sS[o] + out[o]) * inv;
+    else
+      for (int o = tid; o < P.n_soap; o += nt) out[o] = (double)sS[o] * inv;
+    if ((keep & 1) && tid == 0) keep_norm[site] = norm;
+    __syncthreads();  // sC and sS are free for the next site
   }
 }
 
@@ -1045,7 +1277,7 @@ __global__ void __launch_bounds__(NT) k_descriptor_tc(const DevParams P, const D
               const float *Ae = sA + (size_t)e * AS;
               // u_k = (preflm_k P_k)(amp i_l) (src/soap_turbo_angular.f90:590-594)
               const float u = Ae[row_p(LC) + my_k] * Ae[row_il(LC) + my_l];
-              v[e] = u * Ae[(my_ri ? row_ei(LC) : row_er(LC)) + my_m];
+              v[e] = u * Ae[row_e(LC) + 2 * my_m + my_ri];
             }
           }
 #pragma unroll
@@ -1234,7 +1466,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_contract(const DevParams P, co
   constexpr int GPT = 8;  // G values a thread holds while the norm dot product is reduced
   static_assert(AMAX % 4 == 0, "vector loads of H need AMAX % 4 == 0");
   const int AS = stage_stride(LC, 1);
-  constexpr int O_IL = row_il(LC), O_ILD = row_ild(LC), O_ER = row_er(LC), O_EI = row_ei(LC),
+  constexpr int O_IL = row_il(LC), O_ILD = row_ild(LC), O_E = row_e(LC),
                 O_SF = row_sf(LC), O_X = row_x(LC), O_SQ = row_sq(LC),
                 O_P = row_p(LC);
   const Layout Ly = make_layout(P, NT, AMAX, LC, 1);
@@ -1409,8 +1641,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_contract(const DevParams P, co
               float *rot = sRot + 4 * (code & 0xffffff);
               rot[0] = Ae[O_X];
               rot[1] = Ae[O_SQ];
-              rot[2] = Ae[O_ER + 1];
-              rot[3] = -Ae[O_EI + 1];
+              rot[2] = Ae[O_E + 2];
+              rot[3] = -Ae[O_E + 3];
             }
             float R[AMAX], Rd[AMAX];
 #pragma unroll
@@ -1433,7 +1665,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_contract(const DevParams P, co
               // rows hold amp i_l, amp di_l/dr and preflm_k P_k; kcoef carries the
               // preflm ratios of the derivative combinations
               const float il = Ae[O_IL + l], ild = Ae[O_ILD + l];
-              const float er = Ae[O_ER + m], ei = Ae[O_EI + m];
+              const float er = Ae[O_E + 2 * m], ei = Ae[O_E + 2 * m + 1];
               const float u = Pk * il;
               const float ur = Pk * ild - sfac * u;
               const float ua = dvs * il;
@@ -1596,7 +1828,7 @@ __global__ void __launch_bounds__(NT) k_contract_tc(const DevParams P, const Dev
   static_assert(KC <= 2 * kTcCols / 4 && 2 * KC <= kTcCols, "U/V columns");
   constexpr int GPT = 8;
   constexpr int AW = row_len(LC);
-  constexpr int O_IL = row_il(LC), O_ILD = row_ild(LC), O_ER = row_er(LC), O_EI = row_ei(LC),
+  constexpr int O_IL = row_il(LC), O_ILD = row_ild(LC), O_E = row_e(LC),
                 O_SF = row_sf(LC), O_X = row_x(LC), O_SQ = row_sq(LC), O_P = row_p(LC);
   extern __shared__ __align__(16) unsigned char smem[];  // no-swizzle operand tiles need 16-byte alignment
   const TcLayout Ly = make_tc_layout(P, NT, AMAX);
@@ -1846,8 +2078,8 @@ __global__ void __launch_bounds__(NT) k_contract_tc(const DevParams P, const Dev
 #pragma unroll
         for (int l = 0; l <= LC; ++l) {
           il[l] = act ? Ae[(O_IL + l) * kTcEntries] : 0.f;
-          er[l] = act ? Ae[(O_ER + l) * kTcEntries] : 0.f;
-          ei[l] = act ? Ae[(O_EI + l) * kTcEntries] : 0.f;
+          er[l] = act ? Ae[(O_E + 2 * l) * kTcEntries] : 0.f;
+          ei[l] = act ? Ae[(O_E + 2 * l + 1) * kTcEntries] : 0.f;
           ild[l] = (act && vrole) ? Ae[(O_ILD + l) * kTcEntries] : 0.f;
         }
         if (act && vrole) sfac = Ae[O_SF * kTcEntries];
@@ -2073,20 +2305,46 @@ static cudaError_t run_descriptor_tc(const DevParams &P, const DevBatch &B, cons
   return cudaGetLastError();
 }
 
-template <int NT, int AMAX, int LC>
-static cudaError_t run_descriptor(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
-                                  double *soap, float *keep_c, double *keep_norm, int keep) {
-  if (AMAX == 8 && LC == 8 && descriptor_tc_fits(P))
-    return run_descriptor_tc(P, B, cfg, soap, keep_c, keep_norm, keep);
-  const size_t sm = make_layout(P, NT, AMAX, LC, 0).total;
-  auto kern = k_descriptor<NT, AMAX, LC>;
+// Radial indices per thread: the fewer, the more warps share a site and the more
+// loads a product takes.  Two where the sites are at most two per SM and a site's
+// latency is all; four below kDescWideSites sites, and where every k fits one
+// warp; eight from there on.  Steps of descriptor and contract with 2, 4 and 8:
+// 64 sites of one species 42.8, 45.1 and 48.7 us; with 4 and 8: 1679 sites of three
+// 127.5 and 135, 16384 of one 835 and 817; the descriptor alone at 13092 sites of
+// three 385 and 383.
+constexpr int kDescFewSites = 2 * 148, kDescWideSites = 4096;
+
+template <int AMAX, int LC, int NH>
+static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg, int max_alpha,
+                                     double *soap, float *keep_c, double *keep_norm, int keep) {
+  const int kw = (P.k_max + 31) / 32, threads = 32 * kw * ((max_alpha + NH - 1) / NH);
+  const size_t sm = desc_layout(P, cfg.threads, AMAX, LC).total;
+  auto kern = k_descriptor<AMAX, LC, NH>;
   cudaError_t e = ensure_smem_limit(kern, sm);
   if (e != cudaSuccess) return e;
-  if (B.site_hi > B.site_lo) {
-    const int grid = persistent_grid(kern, NT, sm, B.site_hi - B.site_lo, cfg.max_ctas);
-    kern<<<grid, NT, sm, cfg.stream>>>(P, B, soap, keep_c, keep_norm, keep);
+  const int n = B.site_hi - B.site_lo;
+  if (n > 0) {
+    const int grid = cfg.max_ctas > 0 && cfg.max_ctas < n ? cfg.max_ctas : n;
+    kern<<<grid, threads, sm, cfg.stream>>>(P, B, cfg.threads, kw, soap, keep_c, keep_norm, keep);
   }
   return cudaGetLastError();
+}
+
+template <int AMAX, int LC>
+static cudaError_t run_descriptor(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg, double *soap,
+                                  float *keep_c, double *keep_norm, int keep) {
+  if (AMAX == 8 && LC == 8 && descriptor_tc_fits(P))
+    return run_descriptor_tc(P, B, cfg, soap, keep_c, keep_norm, keep);
+  int max_alpha = 1;
+  for (int s = 0; s < P.n_species; ++s) max_alpha = P.rad[s].alpha > max_alpha ? P.rad[s].alpha : max_alpha;
+  if constexpr (AMAX == 8) {
+    const int n = B.site_hi - B.site_lo;
+    if (n <= kDescFewSites)
+      return run_descriptor_as<AMAX, LC, 2>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
+    if (n < kDescWideSites || P.k_max <= 32)
+      return run_descriptor_as<AMAX, LC, 4>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
+  }
+  return run_descriptor_as<AMAX, LC, 8>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
 }
 
 // The tensor-core contract for the alpha <= 8, l_max <= 8 instantiation: a
@@ -2192,7 +2450,8 @@ cudaError_t launch_pair(const DevParams &P, const DevBatch &B, cudaStream_t s, i
 
 cudaError_t launch_descriptor(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
                               double *soap, float *keep_c, double *keep_norm, int keep) {
-  SOAPB_DISPATCH(run_descriptor, P, B, cfg, soap, keep_c, keep_norm, keep);
+  if (P.amax_t == 8) return run_descriptor<8, 8>(P, B, cfg, soap, keep_c, keep_norm, keep);
+  return run_descriptor<16, 12>(P, B, cfg, soap, keep_c, keep_norm, keep);
 }
 
 cudaError_t launch_contract(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
@@ -2203,9 +2462,6 @@ cudaError_t launch_contract(const DevParams &P, const DevBatch &B, const LaunchC
 
 size_t keep_floats_per_site(const DevParams &P) { return keep_stride(P); }
 
-size_t descriptor_smem(const DevParams &P, int threads) {
-  return make_layout(P, threads, P.amax_t, P.amax_t == 8 ? 8 : 12, 0).total;
-}
 size_t contract_smem(const DevParams &P, int threads) {
   return make_layout(P, threads, P.amax_t, P.amax_t == 8 ? 8 : 12, 1).total;
 }
