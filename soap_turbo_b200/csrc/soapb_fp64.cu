@@ -994,6 +994,7 @@ cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaSt
                                    const Fp64Work &w, int do_der, double *soap, double *cart,
                                    int *launches, const double *soap_acc, const double *self_init) {
   const int np = B.n_pairs, nsites = B.n_sites;
+  const int ang_der = do_der && cart;  // only soap_cart_der reads the angular planes' derivatives
   int nl = 0;
   if (np > 0) {
     const int blocks = (np + 127) / 128;
@@ -1005,8 +1006,8 @@ cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaSt
       if (op) k64_radial<16, true><<<blocks, 128, 0, s>>>(P, B, do_der, w.rad, w.rad_der);
       else k64_radial<16, false><<<blocks, 128, 0, s>>>(P, B, do_der, w.rad, w.rad_der);
     }
-    if (P.l_max <= 8) k64_angular2<8><<<(np + 31) / 32, do_der ? 128 : 32, 0, s>>>(P, B, do_der, (double2 *)w.ang);
-    else k64_angular<12><<<blocks, 128, 0, s>>>(P, B, do_der, (double2 *)w.ang);
+    if (P.l_max <= 8) k64_angular2<8><<<(np + 31) / 32, ang_der ? 128 : 32, 0, s>>>(P, B, ang_der, (double2 *)w.ang);
+    else k64_angular<12><<<blocks, 128, 0, s>>>(P, B, ang_der, (double2 *)w.ang);
     nl += 2;
   }
   if (nsites > 0) {

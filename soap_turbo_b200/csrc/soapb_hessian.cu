@@ -12,9 +12,9 @@
 // src/soap_turbo.f90:1537-1652); k64_hess is persistent, one CTA per site at a
 // time, and follows the reference's two passes around the weight vectors' S
 // matrices (see the kernel).  The angular factor Omega = C_k Q_l^m(t) w^m and
-// its Cartesian gradient and Hessian are rebuilt from the record where needed
-// (Q_l^m = d^m P_l / dt^m, w = (x - iy)/r), as the reference does.  Every sum
-// runs in a fixed order, so results repeat bit for bit.
+// its derivatives are rebuilt from the record where needed (Q_l^m = d^m P_l /
+// dt^m, w = (x - iy)/r), as the reference does.  Every sum runs in a fixed order,
+// so results repeat bit for bit.
 #include "soapb_device.cuh"
 
 namespace soapb {
@@ -22,10 +22,11 @@ namespace soapb {
 namespace {
 
 constexpr double kPi = 3.14159265358979323846;
-constexpr int kHessThreads = 128;
-constexpr int kHessS = 26;  // k-sums per weight vector in pass B
-constexpr int kHessPC = 8;  // pairs per chunk of pass A
-constexpr int kHessRed = kHessS + 1;  // row stride of the per-warp transpose buffer
+constexpr int kHessThreads = 256;
+constexpr int kHessPC = 8;      // pairs per chunk of pass A
+constexpr int kHessCols = 13;   // k-sums of a unit of pass B at most (odd: the transpose buffer's row stride)
+constexpr int kHessChunk = 256; // pairs whose entries are listed at a time
+constexpr size_t kHessSmemPair = 113 * 1024;  // shared memory of a CTA of which an SM holds two
 
 #define CU_RET(x)                         \
   do {                                    \
@@ -239,12 +240,6 @@ __device__ __forceinline__ void stc(double *p, dcx v) {
   p[1] = v.im;
 }
 
-__device__ __forceinline__ int l_of_k(int k) {
-  int l = 0;
-  while ((l + 1) * (l + 2) / 2 <= k) ++l;
-  return l;
-}
-
 // get_ilexp (src/soap_turbo_angular.f90:361-422) to lmax, for the F_l of the Hessian
 __device__ void ilexp_to(int lmax, double x, double *out) {
   const double xcut = 1.0e-7, x2 = x * x, x4 = x2 * x2, inv_x2 = (x2 > 0.0) ? 1.0 / x2 : 0.0;
@@ -364,57 +359,49 @@ __global__ void k64_hgeo(const DevParams P, const DevBatch B, double *geo, int *
   }
 }
 
-// Omega, dOmega and (want2) d2Omega of component kq from a pair record
-// (:1620-1650); Ck the signed prefactor (-1)^m preflm.
-__device__ __forceinline__ void omega_k(const double *g, const GeoLayout &Lg, int kq, int ll, int mm, double Ck,
-                                        bool want2, dcx &Om, dcx *dOm, dcx *d2Om) {
-  const double *Qt = g + Lg.Q;
-  const double q0 = Qt[kq], q1 = (mm + 1 <= ll) ? Qt[kq + 1] : 0.0, q2 = (mm + 2 <= ll) ? Qt[kq + 2] : 0.0;
-  const dcx w0 = ldc(g + Lg.wp + 2 * (mm + 2)), w1 = ldc(g + Lg.wp + 2 * (mm + 1)), w2 = ldc(g + Lg.wp + 2 * mm);
-  const double *tv = g + Lg.t;
-  dcx wv[3];
-  for (int aa = 0; aa < 3; ++aa) wv[aa] = ldc(g + Lg.w + 2 * aa);
-  Om = (Ck * q0) * w0;
-  for (int aa = 0; aa < 3; ++aa) dOm[aa] = Ck * ((q1 * tv[aa]) * w0 + (q0 * (double)mm) * (w1 * wv[aa]));
-  if (want2)
-    for (int bb = 0; bb < 3; ++bb)
-      for (int aa = 0; aa < 3; ++aa)
-        d2Om[bb * 3 + aa] =
-            Ck * ((q2 * tv[aa] * tv[bb]) * w0 + (q1 * g[Lg.th + bb * 3 + aa]) * w0 +
-                  (q1 * (double)mm) * (w1 * (tv[aa] * wv[bb] + tv[bb] * wv[aa])) +
-                  (q0 * (double)(mm * (mm - 1))) * (w2 * (wv[aa] * wv[bb])) +
-                  (q0 * (double)mm) * (w1 * ldc(g + Lg.wh + 2 * (bb * 3 + aa))));
-}
-
-// One (b, a) element of the second-derivative block from the k-sums S of a
-// weight vector (layout: S1, S2, S3[3], S4 upper triangle[6], S5[3], S6[3][3], S7[3]).
-__device__ __forceinline__ double hv_block(const double *S, const double *nh, double invr, int aa, int bb) {
-  const int lo = aa < bb ? aa : bb, hi = aa < bb ? bb : aa;
-  const int tri = lo == 0 ? hi : (lo == 1 ? 2 + hi : 5);
-  return -(nh[aa] * nh[bb] * S[0] + (aa == bb ? invr * S[1] : 0.0) + nh[aa] * S[2 + bb] + nh[bb] * S[2 + aa] +
-           S[5 + tri] + nh[bb] * S[11 + aa] + S[14 + aa * 3 + bb]);
-}
-
 // Per-CTA global scratch of the Hessian kernel (hess_scratch_doubles)
 struct HessScratch {
-  double *Gacc;   // (n_max, k_max, 3) complex: G = sum_j d c_nlm / d r_j
-  double *Zv;     // (n_vec + 4, n_max, k_max) complex: S_v c for every weight vector
-  double *ZGv;    // (n_vec + 1, n_max, k_max, 3) complex: S_v G for the Hessian's vectors
+  double *G;      // (n_max, k_max, 3) complex: sum_j d c_nlm / d r_j, when it is not in shared memory
   double *dp1;    // (n_soap, 3): d p / d r_i, unnormalised
   double *kept3;  // (3, n_kept)
-  double *vk;     // (n_kept): a weight vector spread through the compression
+  double *vk;     // (n_kept): a weight vector spread through the compression, when not in shared memory
 };
 
-__device__ HessScratch carve(double *base, const DevParams &P, int n_vec) {
-  const size_t nk = (size_t)P.n_max * P.k_max;
+__device__ HessScratch carve(double *base, const DevParams &P) {
   HessScratch h;
-  h.Gacc = base;
-  h.Zv = h.Gacc + 6 * nk;
-  h.ZGv = h.Zv + 2 * (size_t)(n_vec + 4) * nk;
-  h.dp1 = h.ZGv + 6 * (size_t)(n_vec + 1) * nk;
+  h.G = base;
+  h.dp1 = h.G + 6 * (size_t)P.n_max * P.k_max;
   h.kept3 = h.dp1 + 3 * (size_t)P.n_soap;
   h.vk = h.kept3 + 3 * (size_t)P.n_kept;
   return h;
+}
+
+// Shared memory of k64_hess, in doubles.
+struct HessSmem {
+  int G, Z, red, vk, rad, dot, list, total;
+  bool g_shared, vk_shared;
+};
+__host__ __device__ inline HessSmem hess_smem(const DevParams &P, int n_vec) {
+  HessSmem S;
+  const int N = P.n_max, K = P.k_max, AB = P.amax_t;
+  S.vk_shared = P.n_kept <= 2048;
+  // pass B: a species' tables of one weight vector and the warps' transpose
+  // buffers; pass A: a chunk of pairs' angular factors and radial rows
+  const int b = 8 * AB * K + (kHessThreads / 32) * 32 * kHessCols, a = kHessPC * (12 * K + 2 * AB);
+  int o = 0;
+  S.Z = o;
+  S.red = o + 8 * AB * K;
+  o += a > b ? a : b;
+  S.vk = o;   o += S.vk_shared ? P.n_kept : 0;
+  S.rad = o;  o += (kHessThreads / 16) * 3 * AB;
+  S.dot = o;  o += 4 + 4 * n_vec;
+  S.list = o; o += (kHessChunk * P.n_species + 3) / 4;
+  o = (o + 1) & ~1;
+  // G last: in shared memory when two CTAs still fit an SM
+  S.G = o;
+  S.g_shared = (size_t)(o + 6 * N * K) * sizeof(double) <= kHessSmemPair;
+  S.total = o + (S.g_shared ? 6 * N * K : 0);
+  return S;
 }
 
 // Warp-wise dot product over fixed lane strides and a fixed shuffle tree.
@@ -436,49 +423,95 @@ __device__ __forceinline__ double weight(const double *vecs, const double *soap_
   return dp1[3 * o + (v - n_vec - 1)];
 }
 
+// Whether pair k takes part for species s: its radial row is not zero and it has a record.
+__device__ __forceinline__ unsigned hess_species(const DevParams &P, const DevBatch &B, const int *good, int k) {
+  if (!good[k]) return 0u;
+  const double r = B.rjs[k];
+  const unsigned bits = B.bits[k];
+  unsigned ok = 0u;
+  for (int s = 0; s < P.n_species; ++s)
+    if (((bits >> s) & 1u) && r < P.rad[s].rcut_hard) ok |= 1u << s;
+  return ok;
+}
+
+// The k-sums of a (pair, weight vector), from Omega = C Q_l^m(t) w^m and its
+// derivatives in t and w (d Omega_a = Omega_t t_a + Omega_w w_a and so on, so that
+// the Cartesian tensors t_a, w_a, t_ab, w_ab enter once per pair, not per k):
+//   0  Re[(z2 - z1/r) Om]   1 Re[z1 Om]   2 Re[z1 Om_t]   3,4 z1 Om_w
+//   5  Re[z0 Om_t]  6,7 z0 Om_w  8 Re[z0 Om_tt]  9,10 z0 Om_tw  11,12 z0 Om_ww
+//   13 + 4 q: Re[gg1_q Om], Re[gg0_q Om_t], gg0_q Om_w (two)
+// with z_i the radial contractions of Z_v and gg_q those of ZG_v's component q
+// (:1378-1412, reassociated over k); a vector of which only v . dp_j is needed has
+// four: Re[z1 Om], Re[z0 Om_t], z0 Om_w.
+constexpr int kSumsFull = 25, kSumsLight = 4;
+
+// The sums of pair records read at one Cartesian element.
+__device__ __forceinline__ double re_prod(const double *s, const double *w) { return s[0] * w[0] - s[1] * w[1]; }
+// v . dp_j (b) = n_b S2 + Re sum z0 dOm_b
+__device__ __forceinline__ double first_der(double s_om, double s_t, const double *s_w, const double *g,
+                                            const GeoLayout &Lg, int b) {
+  return g[Lg.nh + b] * s_om + s_t * g[Lg.t + b] + re_prod(s_w, g + Lg.w + 2 * b);
+}
+__device__ __forceinline__ double second_der(const double *S, const double *g, const GeoLayout &Lg, int aa, int bb) {
+  const double *t = g + Lg.t, *wa = g + Lg.w + 2 * aa, *wb = g + Lg.w + 2 * bb, *wh = g + Lg.wh + 2 * (bb * 3 + aa);
+  const double na = g[Lg.nh + aa], nb = g[Lg.nh + bb];
+  const double s3a = S[2] * t[aa] + re_prod(S + 3, wa), s3b = S[2] * t[bb] + re_prod(S + 3, wb);
+  const double tw[2] = {t[aa] * wb[0] + t[bb] * wa[0], t[aa] * wb[1] + t[bb] * wa[1]};
+  const double ww[2] = {wa[0] * wb[0] - wa[1] * wb[1], wa[0] * wb[1] + wa[1] * wb[0]};
+  const double s4 = S[8] * t[aa] * t[bb] + S[5] * g[Lg.th + bb * 3 + aa] + re_prod(S + 9, tw) + re_prod(S + 11, ww) +
+                    re_prod(S + 6, wh);
+  const double *Sq = S + 13 + 4 * aa;
+  const double s6 = Sq[1] * t[bb] + re_prod(Sq + 2, wb);
+  return -(na * nb * S[0] + (aa == bb ? g[Lg.invr] * S[1] : 0.0) + na * s3b + nb * s3a + s4 + nb * Sq[0] + s6);
+}
+
 // ---- the Hessian, persistent, one CTA per site at a time.  Per site:
-//  A  G(n,k) = sum_j d/dr_j [4 pi R_n F_l Omega_k] (:1305-1334), a fixed-order
-//     sum over the site's pairs of R'_n A_j + R_n B_j, with the pairs' angular
-//     factors A_j, B_j built in shared memory chunk by chunk; then
-//     dp1 = d p / d r_i = -(d p / d c) G component by component of p (the
-//     reference sums -dp_j over the pairs; the two agree to rounding, since
-//     sum_j d c / d r_j = G);
-//  Z  every weight vector v spread back through the compression into its
-//     S_v(n, n', l) and applied to c_nlm (Z_v) and to G (ZG_v) (:1336-1376);
-//  B  one half-warp per pair, lanes over k: Z_v and ZG_v contracted with the pair's
-//     R_n, R'_n, R''_n and Omega, dOmega, d2Omega (:1378-1412) give the second
-//     derivative hv and the first derivative v . dp_j (what the reference's
-//     self-test rebuilds, here the value used), and from them the
+//  A  G(n,k) = sum_j d/dr_j [4 pi R_n F_l Omega_k] (:1305-1334), a species'
+//     pairs in CSR order and its radial indices only (the others' R_n are
+//     zero), with the pairs' angular factors A_j, B_j built in shared memory
+//     chunk by chunk; then dp1 = d p / d r_i = -(d p / d c) G component by
+//     component of p (the reference sums -dp_j over the pairs; the two agree to
+//     rounding, since sum_j d c / d r_j = G);
+//  B  per weight vector and species: the vector spread back through the
+//     compression into its S_v(n, n', l) and applied to c_nlm (Z_v) and to G (ZG_v)
+//     (:1336-1376), the species' tables in shared memory; then a half-warp per
+//     pair of the species, lanes over k, contracts them with the pair's R_n, R'_n,
+//     R''_n and Omega into the k-sums above.  Z_v and the three components of
+//     ZG_v are units of their own, so that a species of some twenty pairs still
+//     fills the warps;
+//  C  per pair: the second derivative hv and the first derivatives v . dp_j (what
+//     the reference's self-test rebuilds, here the value used), and from them the
 //     normalisation (:1414-1484).
-// Sums run in a fixed order (pairs to half-warps by index, k within a round by
-// lane order through shared memory, k rounds in order, half-warps in order).
-__global__ void __launch_bounds__(kHessThreads, 4) k64_hess(const DevParams P, const DevBatch B, const double *rad,
+// Sums run in a fixed order (pairs in CSR order, k within a lane, lanes through
+// shared memory).  Read from L2 for every pair, whole Z_v and ZG_v rows had bound
+// the kernel (a pair of three species' definition took 190 KB).
+template <bool GS>
+__global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, const DevBatch B, const double *rad,
                                                          const double *rad_der, const double *rad_der2,
                                                          const double *geo, const int *good, const double2 *cnk,
                                                          const double *norm, const double *soap, int n_vec,
-                                                         const double *vecs, double *hess, double *scratch,
-                                                         size_t scratch_per_cta, int *ticket) {
+                                                         const double *vecs, double *hess, double *sums,
+                                                         double *scratch, size_t scratch_per_cta, int *ticket) {
   extern __shared__ __align__(16) double sm[];
   __shared__ int s_site;
-  const int N = P.n_max, K = P.k_max, ns = P.n_soap, nk = P.n_kept;
+  __shared__ int s_base[SOAPB_MAX_SPECIES + 1];
+  const int N = P.n_max, K = P.k_max, ns = P.n_soap, nk = P.n_kept, AB = P.amax_t, nsp = P.n_species;
   const int nvh = n_vec + 1, nva = n_vec + 4;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_warps = kHessThreads / 32;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = lane >> 4, hl = lane & 15;
+  constexpr int NT = kHessThreads, NW = NT / 32;
+  const size_t sp_sums = (size_t)kSumsFull * nvh + 3 * kSumsLight;
   const GeoLayout Lg(P.l_max);
-  // shared: the site's dot products (3 + 4 n_vec), then a region used by pass
-  // A (a chunk of kHessPC pairs: their A, B factors (K, 12) and R, R' rows) and
-  // by pass B (per half-warp: the k-sums of its pair (n_vec + 4, kHessS), its
-  // radial rows (3 n_max), its running hsum (n_vec, 9) and its transpose buffer)
-  const int sd = 3 + 4 * n_vec + ((3 + 4 * n_vec) & 1);
-  const int per_half = kHessS * nva + 3 * N + 9 * n_vec + 16 * kHessRed;  // per half-warp, pass B
-  double *sdot = sm;
-  double *cab = sm + sd;
-  double *crr = cab + (size_t)kHessPC * K * 12;
-  const int half = lane >> 4, hl = lane & 15, n_halves = 2 * n_warps;
-  double *wsum = sm + sd + (size_t)(2 * warp + half) * per_half;
-  double *wrad = wsum + kHessS * nva;
-  double *whs = wrad + 3 * N;
-  double *red = whs + 9 * n_vec;  // (16 lanes, kHessRed): the k-sums before their column sums
-  const HessScratch h = carve(scratch + scratch_per_cta * blockIdx.x, P, n_vec);
+  const HessSmem Ly = hess_smem(P, n_vec);
+  const HessScratch h = carve(scratch + scratch_per_cta * blockIdx.x, P);
+  double *G = GS ? sm + Ly.G : h.G;
+  double *vk = Ly.vk_shared ? sm + Ly.vk : h.vk;
+  double *cab = sm + Ly.Z, *crr = cab + (size_t)kHessPC * K * 12;
+  double2 *sZ = (double2 *)(sm + Ly.Z), *sZG = sZ + (size_t)AB * K;  // (n, K); (q, n, K)
+  double *red = sm + Ly.red + (size_t)warp * 32 * kHessCols;
+  double *wrad = sm + Ly.rad + (size_t)(2 * warp + half) * 3 * AB;
+  double *sdot = sm + Ly.dot;
+  unsigned short *list = (unsigned short *)(sm + Ly.list);
+  const int *klm = (const int *)(P.blob + P.off_klm);
   const double fourpi = 4.0 * kPi;
 
   for (;;) {
@@ -491,71 +524,100 @@ __global__ void __launch_bounds__(kHessThreads, 4) k64_hess(const DevParams P, c
     const double sv = norm[site], invs = 1.0 / sv, invs3 = invs / (sv * sv), invs5 = invs3 / (sv * sv);
     const double2 *c = cnk + (size_t)site * N * K;
     const double *soap_i = soap + (size_t)site * ns;
-    // ---- A: G, threads over (n, k), the pairs in CSR order in chunks of kHessPC:
-    // A(j, k, q) = 4 pi F_l nh_q Omega_k, B = 4 pi (F'_l nh_q Omega_k + F_l dOmega_kq),
-    // G(n, k, q) = sum_j R'_n(j) A(j, k, q) + R_n(j) B(j, k, q) (:1320-1331)
-    for (int t = tid; t < 6 * N * K; t += kHessThreads) h.Gacc[t] = 0.0;
-    for (int jc = p0 + 1; jc < p1; jc += kHessPC) {
-      const int nc = min(kHessPC, p1 - jc);
-      __syncthreads();
-      for (int t = tid; t < nc * 2 * N; t += kHessThreads) {
-        const int pp = t / (2 * N), r = t - pp * 2 * N;
-        crr[t] = (r < N ? rad : rad_der)[(size_t)(jc + pp) * N + (r < N ? r : r - N)];
+    // the entries of species [s_lo, s_hi) among the pairs [c0, c1), pair - c0, from
+    // list[s_base[s]] on (every warp writes the same list)
+    auto build = [&](int s_lo, int s_hi, int c0, int c1) {
+      __syncthreads();  // the list before is read
+      unsigned long long v = 0ull;
+      for (int t = 0; c0 + 32 * t < c1; ++t) {
+        const int k = c0 + 32 * t + lane;
+        if (k < c1) v |= (unsigned long long)hess_species(P, B, good, k) << (8 * t);
       }
-      for (int t = tid; t < nc * K; t += kHessThreads) {
-        const int pp = t / K, k = t - pp * K, j = jc + pp;
-        double *o = cab + (size_t)t * 12;
-        if (!good[j]) {
-          for (int e = 0; e < 12; ++e) o[e] = 0.0;
-          continue;
-        }
-        const double *g = geo + (size_t)j * Lg.size;
-        const int l = l_of_k(k), m = k - l * (l + 1) / 2;
-        dcx Om, dOm[3];
-        omega_k(g, Lg, k, l, m, (m & 1) ? -P.preflm64[k] : P.preflm64[k], false, Om, dOm, nullptr);
-        const double f0 = fourpi * g[Lg.F + l], f1 = fourpi * g[Lg.F1 + l];
-        for (int q = 0; q < 3; ++q) {
-          const double nq = g[Lg.nh + q];
-          stc(o + 4 * q, (f0 * nq) * Om);
-          stc(o + 4 * q + 2, (f1 * nq) * Om + f0 * dOm[q]);
+      int e = 0;
+      for (int s = s_lo; s < s_hi; ++s) {
+        if (lane == 0) s_base[s] = e;
+        for (int t = 0; c0 + 32 * t < c1; ++t) {
+          const bool on = (v >> (8 * t + s)) & 1ull;
+          const unsigned m = __ballot_sync(0xffffffffu, on);
+          // bit 15: no earlier species of the pair
+          if (on)
+            list[e + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(
+                (32 * t + lane) | ((((v >> (8 * t)) & ((1ull << s) - 1ull)) & 0xffull) ? 0 : 0x8000));
+          e += __popc(m);
         }
       }
+      if (lane == 0) s_base[s_hi] = e;
       __syncthreads();
-      // threads over (k, four radial indices): each pair's A, B are loaded once for four n
-      for (int it = tid; it < ((N + 3) >> 2) * K; it += kHessThreads) {
-        const int nb = it / K, k = it - nb * K, n0 = 4 * nb;
-        dcx gq[4][3];
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-#pragma unroll
-          for (int q = 0; q < 3; ++q)
-            gq[t][q] = (n0 + t < N) ? ldc(h.Gacc + ((size_t)(n0 + t) * K + k) * 6 + 2 * q) : cx(0.0, 0.0);
-        for (int pp = 0; pp < nc; ++pp) {
-          const double *a = cab + ((size_t)pp * K + k) * 12;
-          dcx Aq[3], Bq[3];
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            Aq[q] = ldc(a + 4 * q);
-            Bq[q] = ldc(a + 4 * q + 2);
+    };
+    const bool multi = p1 - p0 - 1 > kHessChunk;
+    if (!multi) build(0, nsp, p0 + 1, p1);
+    // ---- A
+    for (int t = tid; t < 6 * N * K; t += NT) G[t] = 0.0;
+    for (int s = 0; s < nsp; ++s) {
+      const int a = P.rad[s].alpha, nb = P.rad[s].nbeg;
+      for (int c0 = p0 + 1; c0 < p1; c0 += kHessChunk) {
+        if (multi) build(s, s + 1, c0, min(p1, c0 + kHessChunk));
+        const int e0 = s_base[s], e1 = s_base[s + 1];
+        for (int eb = e0; eb < e1; eb += kHessPC) {
+          const int nc = min(kHessPC, e1 - eb);
+          __syncthreads();  // the chunk before is read (and G is cleared)
+          for (int t = tid; t < nc * 2 * a; t += NT) {
+            const int pp = t / (2 * a), r = t - pp * 2 * a;
+            const size_t j = c0 + (list[eb + pp] & 0x7fff);
+            crr[pp * 2 * AB + (r < a ? r : AB + r - a)] = (r < a ? rad : rad_der)[j * N + nb + (r < a ? r : r - a)];
           }
+          for (int t = tid; t < nc * K; t += NT) {
+            const int pp = t / K, k = t - pp * K, lm = klm[k], l = lm & 0xff, m = lm >> 8;
+            const double *g = geo + (size_t)(c0 + (list[eb + pp] & 0x7fff)) * Lg.size;
+            const double C = (m & 1) ? -P.preflm64[k] : P.preflm64[k];
+            const double q0 = C * g[Lg.Q + k], q1 = (m < l) ? C * g[Lg.Q + k + 1] : 0.0;
+            const dcx w0 = ldc(g + Lg.wp + 2 * (m + 2)), w1 = ldc(g + Lg.wp + 2 * (m + 1));
+            const dcx Om = q0 * w0, Ot = q1 * w0, Ow = (q0 * (double)m) * w1;
+            const double f0 = fourpi * g[Lg.F + l], f1 = fourpi * g[Lg.F1 + l];
+            double *o = cab + (size_t)t * 12;
+            for (int q = 0; q < 3; ++q) {
+              const double nq = g[Lg.nh + q];
+              stc(o + 4 * q, (f0 * nq) * Om);
+              stc(o + 4 * q + 2, (f1 * nq) * Om + f0 * (g[Lg.t + q] * Ot + Ow * ldc(g + Lg.w + 2 * q)));
+            }
+          }
+          __syncthreads();
+          // threads over (k, two radial indices)
+          for (int it = tid; it < ((a + 1) >> 1) * K; it += NT) {
+            const int n2 = it / K, k = it - n2 * K, n0 = 2 * n2, n1 = min(n0 + 1, a - 1);
+            double2 *g0 = (double2 *)(G + ((size_t)(nb + n0) * K + k) * 6);
+            double2 *g1 = (double2 *)(G + ((size_t)(nb + n1) * K + k) * 6);
+            double2 x[3], y[3];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const int n = min(n0 + t, N - 1);  // the tail's extra rows are not stored
-            const double r0 = crr[pp * 2 * N + n], r1 = crr[pp * 2 * N + N + n];
+            for (int q = 0; q < 3; ++q) {
+              x[q] = g0[q];
+              y[q] = g1[q];
+            }
+            for (int pp = 0; pp < nc; ++pp) {
+              const double2 *f = (const double2 *)(cab + ((size_t)pp * K + k) * 12);
+              const double *R = crr + pp * 2 * AB;
+              const double r0 = R[n0], d0 = R[AB + n0], r1 = R[n1], d1 = R[AB + n1];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) gq[t][q] = gq[t][q] + r1 * Aq[q] + r0 * Bq[q];
+              for (int q = 0; q < 3; ++q) {
+                const double2 A = f[2 * q], D = f[2 * q + 1];
+                x[q].x = x[q].x + d0 * A.x + r0 * D.x;
+                x[q].y = x[q].y + d0 * A.y + r0 * D.y;
+                y[q].x = y[q].x + d1 * A.x + r1 * D.x;
+                y[q].y = y[q].y + d1 * A.y + r1 * D.y;
+              }
+            }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+              g0[q] = x[q];
+              if (n0 + 1 < a) g1[q] = y[q];
+            }
           }
         }
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-          if (n0 + t < N)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) stc(h.Gacc + ((size_t)(n0 + t) * K + k) * 6 + 2 * q, gq[t][q]);
       }
     }
     __syncthreads();
     // dp1 in the kept components, then through the compression map
-    for (int q = tid; q < nk; q += kHessThreads) {
+    for (int q = tid; q < nk; q += NT) {
       const int code = P.kept_nnl[q];
       const int n = code & 0xff, np = (code >> 8) & 0xff, l = code >> 16;
       const double base = (n == np) ? 1.0 : sqrt(2.0);
@@ -564,14 +626,15 @@ __global__ void __launch_bounds__(kHessThreads, 4) k64_hess(const DevParams P, c
         const int k = l * (l + 1) / 2 + m;
         const double w = base * ((m > 0) ? 2.0 : 1.0);
         const double2 a = c[(size_t)n * K + k], b = c[(size_t)np * K + k];
-        const double *ga = h.Gacc + ((size_t)n * K + k) * 6, *gb = h.Gacc + ((size_t)np * K + k) * 6;
+        const double *ga = G + ((size_t)n * K + k) * 6, *gb = G + ((size_t)np * K + k) * 6;
+#pragma unroll
         for (int e = 0; e < 3; ++e)
           d[e] = d[e] - w * (ga[2 * e] * b.x + ga[2 * e + 1] * b.y + a.x * gb[2 * e] + a.y * gb[2 * e + 1]);
       }
       for (int e = 0; e < 3; ++e) h.kept3[(size_t)e * nk + q] = d[e];
     }
     __syncthreads();
-    for (int o = tid; o < ns; o += kHessThreads) {
+    for (int o = tid; o < ns; o += NT) {
       double d0 = 0.0, d1 = 0.0, d2 = 0.0;
       for (int t = P.pi_off[o]; t < P.pi_off[o + 1]; ++t) {
         const double e = P.pi_el64[t];
@@ -586,7 +649,7 @@ __global__ void __launch_bounds__(kHessThreads, 4) k64_hess(const DevParams P, c
     }
     __syncthreads();
     // the site's dot products: t1 (3), then per v wp, u1 (3)
-    for (int d = warp; d < 3 + 4 * n_vec; d += n_warps) {
+    for (int d = warp; d < 3 + 4 * n_vec; d += NW) {
       double r;
       if (d < 3) r = sv * warp_dot(soap_i, 1, h.dp1 + d, 3, ns);
       else {
@@ -596,210 +659,208 @@ __global__ void __launch_bounds__(kHessThreads, 4) k64_hess(const DevParams P, c
       }
       if (lane == 0) sdot[d] = r;
     }
-    // ---- Z: S_v applied to c and G through the per-(l, n) lists of the kept
-    // components (2 v on the diagonal, sqrt 2 v off it, np ascending)
+    // ---- B
     for (int v = 0; v < nva; ++v) {
-      for (int q = tid; q < nk; q += kHessThreads) {
-        double s = 0.0;
+      const bool full = v < nvh;
+      const size_t off = full ? (size_t)v * kSumsFull : (size_t)nvh * kSumsFull + (v - nvh) * kSumsLight;
+      for (int q = tid; q < nk; q += NT) {
+        double x = 0.0;
         for (int t = P.pj_off[q]; t < P.pj_off[q + 1]; ++t)
-          s = s + P.pj_el64[t] * weight(vecs, soap_i, sv, h.dp1, n_vec, ns, site, v, P.pj_o[t]);
-        h.vk[q] = s;
+          x = x + P.pj_el64[t] * weight(vecs, soap_i, sv, h.dp1, n_vec, ns, site, v, P.pj_o[t]);
+        vk[q] = x;
       }
-      __syncthreads();
-      for (int it = tid; it < N * K; it += kHessThreads) {
-        const int n = it / K, k = it - n * K, l = l_of_k(k);
-        dcx zc = cx(0.0, 0.0), b0[3] = {cx(0.0, 0.0), cx(0.0, 0.0), cx(0.0, 0.0)};
-        for (int t = P.hl_off[l * N + n]; t < P.hl_off[l * N + n + 1]; ++t) {
-          const int np = P.hl_np[t];
-          const double smv = P.hl_fac64[t] * h.vk[P.hl_q[t]];
-          const double2 cc = c[(size_t)np * K + k];
-          zc = zc + cx(smv * cc.x, smv * cc.y);
-          if (v < nvh)
-            for (int q = 0; q < 3; ++q) b0[q] = b0[q] + smv * ldc(h.Gacc + ((size_t)np * K + k) * 6 + 2 * q);
-        }
-        stc(h.Zv + (((size_t)v * N + n) * K + k) * 2, zc);
-        if (v < nvh)
-          for (int q = 0; q < 3; ++q) stc(h.ZGv + ((((size_t)v * N + n) * K + k) * 3 + q) * 2, b0[q]);
-      }
-      __syncthreads();
-    }
-    // ---- B: one half-warp per pair, lanes over k (rounds of 16).  Per weight
-    // vector the k-sums below give the block (:1378-1412, reassociated over k):
-    //   S1 = sum w Re[(z2 - z1/r) Om]   S2 = sum w Re[z1 Om]    S3_b = sum w Re[z1 dOm_b]
-    //   S4_ab = sum w Re[z0 d2Om_ab]    S5_a = sum w Re[gg1_a Om]
-    //   S6_ab = sum w Re[gg0_a dOm_b]   S7_b = sum w Re[z0 dOm_b]
-    //   hv(b, a) = -(n_a n_b S1 + [a = b] S2 / r + n_a S3_b + n_b S3_a + S4_ab + n_b S5_a + S6_ab)
-    //   v . dp_j (b) = n_b S2 + S7_b
-    // The two halves of a warp read the same Z rows (same k), for two pairs.
-    for (int t = hl; t < 9 * n_vec; t += 16) whs[t] = 0.0;
-    for (int jb = p0 + 1 + 2 * warp; jb < p1; jb += 2 * n_warps) {  // the same trip count for both halves
-      const int j = jb + half;
-      const bool pv = j < p1 && good[j];  // this half has a pair
-      const double *g = geo + (size_t)(pv ? j : 0) * Lg.size;
-      for (int t = hl; t < 3 * N; t += 16) {
-        const int w = t / N, n = t - w * N;
-        wrad[t] = pv ? (w == 0 ? rad : (w == 1 ? rad_der : rad_der2))[(size_t)j * N + n] : 0.0;
-      }
-      for (int t = hl; t < kHessS * nva; t += 16) wsum[t] = 0.0;
-      __syncwarp();
-      for (int k0 = 0; k0 < K; k0 += 16) {
-        const int k = k0 + hl;
-        const bool act = pv && k < K;
-        const int kc = act ? k : 0;
-        const int l = l_of_k(kc), m = kc - l * (l + 1) / 2;
-        dcx Om = cx(0.0, 0.0), dOm[3], d2Om[9];
-        for (int e = 0; e < 3; ++e) dOm[e] = Om;
-        for (int e = 0; e < 9; ++e) d2Om[e] = Om;
-        double wmk = 0.0, f0 = 0.0, f1 = 0.0, f2 = 0.0, invr = 0.0;
-        if (act) {
-          omega_k(g, Lg, kc, l, m, (m & 1) ? -P.preflm64[kc] : P.preflm64[kc], true, Om, dOm, d2Om);
-          wmk = (m > 0) ? 2.0 : 1.0;
-          f0 = fourpi * g[Lg.F + l];
-          f1 = fourpi * g[Lg.F1 + l];
-          f2 = fourpi * g[Lg.F2 + l];
-          invr = g[Lg.invr];
-        }
-        for (int v = 0; v < nva; ++v) {
-          const bool full = v < nvh;
-          double *ws = wsum + v * kHessS;
-          double *my = red + hl * kHessRed;
-          // a-pass: R, R', R'' against Z_v
-          dcx a0 = cx(0.0, 0.0), a1 = a0, a2 = a0;
-          if (act) {
-            const double2 *zv = (const double2 *)h.Zv + (size_t)v * N * K + k;
-#pragma unroll 8
-            for (int n = 0; n < N; ++n) {
-              const double2 zz = zv[(size_t)n * K];
-              const dcx zc = cx(zz.x, -zz.y);
-              a0 = a0 + wrad[n] * zc;
-              a1 = a1 + wrad[N + n] * zc;
-              if (full) a2 = a2 + wrad[2 * N + n] * zc;
-            }
-          }
-          const dcx z0 = f0 * a0, z1 = f0 * a1 + f1 * a0;
-          my[1] = wmk * (z1 * Om).re;
+      for (int s = 0; s < nsp; ++s) {
+        const int a = P.rad[s].alpha, nb = P.rad[s].nbeg;
+        if (!multi && s_base[s] == s_base[s + 1]) continue;
+        __syncthreads();  // vk is complete, the tables before are read
+        // S_v through the per-(l, n) lists of the kept components (2 v on the
+        // diagonal, sqrt 2 v off it, np ascending)
+        for (int it = tid; it < a * K; it += NT) {
+          const int n = it / K, k = it - n * K, l = klm[k] & 0xff;
+          double2 z = make_double2(0.0, 0.0), b[3];
 #pragma unroll
-          for (int bb = 0; bb < 3; ++bb) my[23 + bb] = wmk * (z0 * dOm[bb]).re;
-          if (!full) {  // the four first-derivative sums: lanes 0..3 of each half add its 16 rows
-            __syncwarp();
-            if (hl < 4) {
-              const int e = hl == 0 ? 1 : 22 + hl;
-              double acc = 0.0;
-              for (int r = 0; r < 16; ++r) acc += red[r * kHessRed + e];
-              ws[e] += acc;
-            }
-            __syncwarp();
-            continue;
-          }
-          {
-            const dcx z2 = f0 * a2 + (2.0 * f1) * a1 + f2 * a0;
-            my[0] = wmk * ((z2 - invr * z1) * Om).re;
+          for (int q = 0; q < 3; ++q) b[q] = z;
+          const int li = l * N + nb + n;
+          for (int t = P.hl_off[li]; t < P.hl_off[li + 1]; ++t) {
+            const int np = P.hl_np[t];
+            const double y = P.hl_fac64[t] * vk[P.hl_q[t]];
+            const double2 cc = c[(size_t)np * K + k];
+            z.x += y * cc.x;
+            z.y += y * cc.y;
+            if (full) {
+              const double2 *gg = (const double2 *)(G + ((size_t)np * K + k) * 6);
 #pragma unroll
-            for (int bb = 0; bb < 3; ++bb) my[2 + bb] = wmk * (z1 * dOm[bb]).re;
-            int e = 5;
-#pragma unroll
-            for (int aa = 0; aa < 3; ++aa)
-#pragma unroll
-              for (int bb = aa; bb < 3; ++bb) my[e++] = wmk * (z0 * d2Om[bb * 3 + aa]).re;
-          }
-          // b-pass: R, R' against ZG_v, one Cartesian component at a time
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            dcx b0 = cx(0.0, 0.0), b1 = b0;
-            if (act) {
-              const double2 *zg = (const double2 *)h.ZGv + ((size_t)v * N * K + k) * 3 + q;
-#pragma unroll 8
-              for (int n = 0; n < N; ++n) {
-                const double2 gz = zg[(size_t)n * K * 3];
-                const dcx gc = cx(gz.x, -gz.y);
-                b0 = b0 + wrad[n] * gc;
-                b1 = b1 + wrad[N + n] * gc;
+              for (int q = 0; q < 3; ++q) {
+                const double2 gv = gg[q];
+                b[q].x += y * gv.x;
+                b[q].y += y * gv.y;
               }
             }
-            const dcx gg0 = f0 * b0, gg1 = f0 * b1 + f1 * b0;
-            my[11 + q] = wmk * (gg1 * Om).re;
+          }
+          sZ[n * K + k] = z;
+          if (full)
 #pragma unroll
-            for (int bb = 0; bb < 3; ++bb) my[14 + q * 3 + bb] = wmk * (gg0 * dOm[bb]).re;
+            for (int q = 0; q < 3; ++q) sZG[(q * AB + n) * K + k] = b[q];
+        }
+        __syncthreads();
+        for (int c0 = p0 + 1; c0 < p1; c0 += kHessChunk) {
+          if (multi) build(s, s + 1, c0, min(p1, c0 + kHessChunk));
+          const int e0 = s_base[s], n_two = (s_base[s + 1] - e0 + 1) >> 1;
+          // units: two pairs (one per half-warp) and Z_v (part 0) or a component of ZG_v
+          for (int u = warp; u < n_two * (full ? 4 : 1); u += NW) {
+            const int part = u / n_two, e = e0 + 2 * (u - part * n_two) + half;
+            const bool pv = e < s_base[s + 1];
+            const int code = list[pv ? e : e0], j = c0 + (code & 0x7fff);
+            const double *g = geo + (size_t)j * Lg.size;
+            for (int t = hl; t < 3 * a; t += 16) {
+              const int w = t / a, n = t - w * a;
+              wrad[w * AB + n] = (w == 0 ? rad : (w == 1 ? rad_der : rad_der2))[(size_t)j * N + nb + n];
+            }
+            __syncwarp();
+            double acc[kHessCols];
+#pragma unroll
+            for (int t = 0; t < kHessCols; ++t) acc[t] = 0.0;
+            const double invr = g[Lg.invr];
+            const double2 *tab = part == 0 ? sZ : sZG + (size_t)(part - 1) * AB * K;
+            for (int k = hl; k < K; k += 16) {
+              const int lm = klm[k], l = lm & 0xff, m = lm >> 8;
+              double2 a0 = make_double2(0.0, 0.0), a1 = a0, a2 = a0;
+              const double2 *z = tab + k;
+              if (full && part == 0) {
+#pragma unroll 4
+                for (int n = 0; n < a; ++n) {
+                  const double2 zz = z[n * K];
+                  const double r0 = wrad[n], r1 = wrad[AB + n], r2 = wrad[2 * AB + n];
+                  a0.x += r0 * zz.x;
+                  a0.y -= r0 * zz.y;
+                  a1.x += r1 * zz.x;
+                  a1.y -= r1 * zz.y;
+                  a2.x += r2 * zz.x;
+                  a2.y -= r2 * zz.y;
+                }
+              } else {
+#pragma unroll 4
+                for (int n = 0; n < a; ++n) {
+                  const double2 zz = z[n * K];
+                  const double r0 = wrad[n], r1 = wrad[AB + n];
+                  a0.x += r0 * zz.x;
+                  a0.y -= r0 * zz.y;
+                  a1.x += r1 * zz.x;
+                  a1.y -= r1 * zz.y;
+                }
+              }
+              const double C = ((m > 0) ? 2.0 : 1.0) * ((m & 1) ? -P.preflm64[k] : P.preflm64[k]);
+              const double q0 = C * g[Lg.Q + k], q1 = (m < l) ? C * g[Lg.Q + k + 1] : 0.0;
+              const dcx w0 = ldc(g + Lg.wp + 2 * (m + 2)), w1 = (double)m * ldc(g + Lg.wp + 2 * (m + 1));
+              const dcx Om = q0 * w0, Ot = q1 * w0, Ow = q0 * w1;
+              const double f0 = fourpi * g[Lg.F + l], f1 = fourpi * g[Lg.F1 + l];
+              const dcx z0 = cx(f0 * a0.x, f0 * a0.y), z1 = cx(f0 * a1.x + f1 * a0.x, f0 * a1.y + f1 * a0.y);
+              if (full && part == 0) {
+                const double q2 = (m + 1 < l) ? C * g[Lg.Q + k + 2] : 0.0;
+                const dcx w2 = (double)(m * (m - 1)) * ldc(g + Lg.wp + 2 * m);
+                const double f2 = fourpi * g[Lg.F2 + l];
+                const dcx y = cx(f0 * a2.x + 2.0 * f1 * a1.x + f2 * a0.x - invr * z1.re,
+                                 f0 * a2.y + 2.0 * f1 * a1.y + f2 * a0.y - invr * z1.im);
+                acc[0] += y.re * Om.re - y.im * Om.im;
+                acc[1] += z1.re * Om.re - z1.im * Om.im;
+                acc[2] += z1.re * Ot.re - z1.im * Ot.im;
+                acc[3] += z1.re * Ow.re - z1.im * Ow.im;
+                acc[4] += z1.re * Ow.im + z1.im * Ow.re;
+                acc[5] += z0.re * Ot.re - z0.im * Ot.im;
+                acc[6] += z0.re * Ow.re - z0.im * Ow.im;
+                acc[7] += z0.re * Ow.im + z0.im * Ow.re;
+                const dcx Ott = q2 * w0, Otw = q1 * w1, Oww = q0 * w2;
+                acc[8] += z0.re * Ott.re - z0.im * Ott.im;
+                acc[9] += z0.re * Otw.re - z0.im * Otw.im;
+                acc[10] += z0.re * Otw.im + z0.im * Otw.re;
+                acc[11] += z0.re * Oww.re - z0.im * Oww.im;
+                acc[12] += z0.re * Oww.im + z0.im * Oww.re;
+              } else {
+                acc[0] += z1.re * Om.re - z1.im * Om.im;
+                acc[1] += z0.re * Ot.re - z0.im * Ot.im;
+                acc[2] += z0.re * Ow.re - z0.im * Ow.im;
+                acc[3] += z0.re * Ow.im + z0.im * Ow.re;
+              }
+            }
+            // the lanes' sums: lane t of a half adds column t of its half's 16 rows
+            const bool wide = full && part == 0;
+            const int cols = wide ? kHessCols : 4;
+#pragma unroll
+            for (int t = 0; t < kHessCols; ++t)
+              if (t < 4 || wide) red[lane * kHessCols + t] = acc[t];
+            __syncwarp();
+            if (pv && hl < cols) {
+              double x = 0.0;
+#pragma unroll
+              for (int r = 0; r < 16; ++r) x += red[(16 * half + r) * kHessCols + hl];
+              double *o = sums + (size_t)j * sp_sums + off + (part > 0 ? 13 + 4 * (part - 1) : 0) + hl;
+              *o = (code & 0x8000) ? x : *o + x;
+            }
+            __syncwarp();
           }
-          // the 26 sums over the half's k: lane e adds the 16 rows of column e in order
-          __syncwarp();
-          for (int e = hl; e < kHessS; e += 16) {
-            double acc = 0.0;
-            for (int r = 0; r < 16; ++r) acc += red[r * kHessRed + e];
-            ws[e] += acc;
-          }
-          __syncwarp();
         }
       }
-      __syncwarp();
-      // the normalisation (:1414-1484): t2 = p . dp_j, c12(b, a) = dp1(:, a) . dp_j(:, b),
-      // u2 = w . dp_j
-      if (pv) {
-        const double invr = g[Lg.invr];
-        const double nh[3] = {g[Lg.nh], g[Lg.nh + 1], g[Lg.nh + 2]};
-        for (int t = hl; t < 9 * n_vec; t += 16) {
-          const int v = t / 9, e = t - v * 9, bb = e / 3, aa = e - bb * 3;
-          const double *t1 = sdot, *dv = sdot + 3 + 4 * v;
-          const double wp = dv[0], *u1 = dv + 1;
-          const double *Sp = wsum + n_vec * kHessS, *Sv = wsum + v * kHessS;
-          const double t2b = nh[bb] * Sp[1] + Sp[23 + bb], u2b = nh[bb] * Sv[1] + Sv[23 + bb];
-          const double *Sc = wsum + (n_vec + 1 + aa) * kHessS;
-          const double c12 = nh[bb] * Sc[1] + Sc[23 + bb];
-          const double hvv = hv_block(Sv, nh, invr, aa, bb), hvp = hv_block(Sp, nh, invr, aa, bb);
-          const double hval = hvv * invs - (u1[aa] * t2b + u2b * t1[aa]) * invs3 - wp * (c12 + hvp) * invs3 +
-                              3.0 * wp * t1[aa] * t2b * invs5;
-          hess[((size_t)j * n_vec + v) * 9 + e] = hval;
-          whs[t] += hval;
-        }
-      }
-      __syncwarp();
+      __syncthreads();  // vk is read
+    }
+    // ---- C: the normalisation (:1414-1484): t2 = p . dp_j, c12(b, a) = dp1(:, a) .
+    // dp_j(:, b), u2 = w . dp_j.  Pairs the Hessian skips keep the zero blocks the
+    // launcher cleared.
+    for (int it = tid; it < (p1 - p0 - 1) * 9 * n_vec; it += NT) {
+      const int jj = it / (9 * n_vec), t = it - jj * 9 * n_vec, v = t / 9, e = t - v * 9, bb = e / 3, aa = e - bb * 3;
+      const int j = p0 + 1 + jj;
+      if (!hess_species(P, B, good, j)) continue;
+      const double *g = geo + (size_t)j * Lg.size, *S = sums + (size_t)j * sp_sums;
+      const double *Sv = S + v * kSumsFull, *Sp = S + n_vec * kSumsFull, *Sc = S + nvh * kSumsFull + aa * kSumsLight;
+      const double *t1 = sdot, *dv = sdot + 3 + 4 * v;
+      const double wp = dv[0], *u1 = dv + 1;
+      const double t2b = first_der(Sp[1], Sp[5], Sp + 6, g, Lg, bb), u2b = first_der(Sv[1], Sv[5], Sv + 6, g, Lg, bb);
+      const double c12 = first_der(Sc[0], Sc[1], Sc + 2, g, Lg, bb);
+      const double hvv = second_der(Sv, g, Lg, aa, bb), hvp = second_der(Sp, g, Lg, aa, bb);
+      hess[((size_t)j * n_vec + v) * 9 + e] = hvv * invs - (u1[aa] * t2b + u2b * t1[aa]) * invs3 -
+                                              wp * (c12 + hvp) * invs3 + 3.0 * wp * t1[aa] * t2b * invs5;
     }
     __syncthreads();
-    // the self pair: minus the sum of the others (:1488-1495), half-warps in
-    // order; pairs the Hessian skips keep the zero blocks the launcher cleared
+    // the self pair: minus the sum of the others (:1488-1495)
     if (p1 > p0)
-      for (int t = tid; t < 9 * n_vec; t += kHessThreads) {
-        double s = 0.0;
-        for (int w = 0; w < n_halves; ++w) s += sm[sd + (size_t)w * per_half + kHessS * nva + 3 * N + t];
-        hess[((size_t)p0 * n_vec) * 9 + t] = -s;
+      for (int t = warp; t < 9 * n_vec; t += NW) {
+        double x = 0.0;
+        for (int j = p0 + 1 + lane; j < p1; j += 32) x += hess[(size_t)j * n_vec * 9 + t];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) hess[(size_t)p0 * n_vec * 9 + t] = -x;
       }
   }
 }
 
 }  // namespace
 
-// Doubles per CTA, a multiple of 32 so that every CTA's region (and the
-// complex tables in it, read with 16-byte loads) starts on a 256-byte boundary.
-size_t hess_scratch_doubles(const DevParams &P, int n_vec) {
-  const size_t nk = (size_t)P.n_max * P.k_max;
-  const size_t n = 6 * nk + 2 * (size_t)(n_vec + 4) * nk + 6 * (size_t)(n_vec + 1) * nk + 3 * (size_t)P.n_soap +
-                   4 * (size_t)P.n_kept;
+// Doubles per CTA, a multiple of 32 so that every CTA's region starts on a
+// 256-byte boundary.
+size_t hess_scratch_doubles(const DevParams &P) {
+  const size_t n = 6 * (size_t)P.n_max * P.k_max + 3 * (size_t)P.n_soap + 4 * (size_t)P.n_kept;
   return (n + 31) / 32 * 32;
 }
 
+size_t hess_sums_doubles(int n_vec) { return (size_t)kSumsFull * (n_vec + 1) + 3 * kSumsLight; }
+
 size_t hess_geo_doubles(const DevParams &P) { return (size_t)GeoLayout(P.l_max).size; }
 
-size_t hess_smem_bytes(const DevParams &P, int n_vec) {
-  const size_t nw = kHessThreads / 32, sd = 3 + 4 * (size_t)n_vec;
-  const size_t pass_a = (size_t)kHessPC * (12 * (size_t)P.k_max + 2 * (size_t)P.n_max);
-  const size_t pass_b =
-      2 * nw * (kHessS * (size_t)(n_vec + 4) + 3 * (size_t)P.n_max + 9 * (size_t)n_vec + 16 * (size_t)kHessRed);
-  return sizeof(double) * (sd + (sd & 1) + (pass_a > pass_b ? pass_a : pass_b));
-}
+size_t hess_smem_bytes(const DevParams &P, int n_vec) { return sizeof(double) * (size_t)hess_smem(P, n_vec).total; }
 
 int hess_grid(const DevParams &P, int n_vec) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t sm = hess_smem_bytes(P, n_vec);
-  if (cudaFuncSetAttribute(k64_hess, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return sms;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k64_hess, kHessThreads, sm);
+  auto kern = hess_smem(P, n_vec).g_shared ? k64_hess<true> : k64_hess<false>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return sms;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kHessThreads, sm);
   return sms * (per_sm > 0 ? per_sm : 1);
 }
 
 cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s, const Fp64Work &w,
                            double *rad_der2, double *geo, int *good, const double *soap, int n_vec,
-                           const double *vecs, double *hess, double *scratch, int grid, int *ticket, int *launches) {
+                           const double *vecs, double *hess, double *sums, double *scratch, int grid, int *ticket, int *launches) {
   CU_RET(cudaMemsetAsync(hess, 0, sizeof(double) * 9 * (size_t)n_vec * B.n_pairs, s));
   CU_RET(cudaMemsetAsync(ticket, 0, sizeof(int), s));
   if (B.n_pairs > 0) {
@@ -813,11 +874,11 @@ cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s
   }
   if (B.n_sites > 0) {
     const size_t sm = hess_smem_bytes(P, n_vec);
-    CU_RET(cudaFuncSetAttribute(k64_hess, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    auto kern = hess_smem(P, n_vec).g_shared ? k64_hess<true> : k64_hess<false>;
+    CU_RET(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int g = grid < B.n_sites ? grid : B.n_sites;
-    k64_hess<<<g, kHessThreads, sm, s>>>(P, B, w.rad, w.rad_der, rad_der2, geo, good, (const double2 *)w.cnk,
-                                        w.norm, soap, n_vec, vecs, hess, scratch, hess_scratch_doubles(P, n_vec),
-                                        ticket);
+    kern<<<g, kHessThreads, sm, s>>>(P, B, w.rad, w.rad_der, rad_der2, geo, good, (const double2 *)w.cnk, w.norm, soap,
+                                     n_vec, vecs, hess, sums, scratch, hess_scratch_doubles(P), ticket);
     if (launches) *launches += 1;
   }
   return cudaGetLastError();

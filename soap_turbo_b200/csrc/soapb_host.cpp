@@ -305,7 +305,7 @@ struct soapb_context {
   DBuf f64_rad, f64_rad_der, f64_ang, f64_cnk, f64_soap_un, f64_norm;
   // central-atom Hessian: second radial derivatives, pair geometry records and
   // flags, per-CTA scratch, the descriptor it recomputes, its work counter
-  DBuf hs_rad_der2, hs_geo, hs_good, hs_scratch, hs_soap, hs_ticket, hs_vchunk, hs_hchunk;
+  DBuf hs_rad_der2, hs_geo, hs_good, hs_scratch, hs_sums, hs_soap, hs_ticket, hs_vchunk, hs_hchunk;
   // neighbour-list builder: cell list, counts and the batch it hands out
   DBuf nb_acell, nb_ccount, nb_cstart, nb_cfill, nb_catoms, nb_counts, nb_off, nb_state;
   DBuf nb_rjs, nb_th, nb_ph, nb_mask, nb_natom, nb_nneigh, nb_species, nb_smult;
@@ -346,7 +346,7 @@ struct soapb_context {
   ~soapb_context() {
     timing_release();
     for (DBuf *b : {&tables, &off, &bits, &err, &keep_c, &keep_norm, &order, &rad, &ang, &f64_rad, &f64_rad_der,
-                    &f64_ang, &f64_cnk, &f64_soap_un, &f64_norm, &hs_rad_der2, &hs_geo, &hs_good, &hs_scratch, &hs_soap,
+                    &f64_ang, &f64_cnk, &f64_soap_un, &f64_norm, &hs_rad_der2, &hs_geo, &hs_good, &hs_scratch, &hs_sums, &hs_soap,
                     &hs_ticket, &hs_vchunk, &hs_hchunk, &nb_acell, &nb_ccount, &nb_cstart,
                     &nb_cfill, &nb_catoms, &nb_counts, &nb_off, &nb_state, &nb_rjs, &nb_th, &nb_ph,
                     &nb_mask, &nb_natom, &nb_nneigh, &nb_species, &nb_smult})
@@ -1301,10 +1301,10 @@ int ctx_hessian(soapb_context *c, const soapb_batch *b, const double *d_soap, in
   if (rc) return rc;
   if (n_vec == 0) return SOAPB_OK;
   if (b->n_sites > 0 && !d_vecs) return fail(SOAPB_ERR_ARGUMENT, "null vecs");
-  // The kernel keeps per-warp k-sums for every weight vector in shared memory:
-  // more vectors than fit are done in chunks (each vector's block depends on
-  // that vector alone, so the chunking changes no bits).
-  int chunk = n_vec;
+  // The kernel keeps the pairs' k-sums for every weight vector of a launch: more
+  // than kHessVecs are done in chunks (each vector's block depends on that vector
+  // alone, so the chunking changes no bits).
+  int chunk = std::min(n_vec, kHessVecs);
   {
     int dev = 0, smem_max = 0;
     CU(cudaGetDevice(&dev));
@@ -1321,7 +1321,7 @@ int ctx_hessian(soapb_context *c, const soapb_batch *b, const double *d_soap, in
   const size_t np = (size_t)b->n_atom_pairs + 1, ns = (size_t)b->n_sites + 1;
   if ((rc = c->f64_rad.ensure(8 * np * c->n_max))) return rc;
   if ((rc = c->f64_rad_der.ensure(8 * np * c->n_max))) return rc;
-  if ((rc = c->f64_ang.ensure(16 * np * P.k_max * 4))) return rc;
+  if ((rc = c->f64_ang.ensure(16 * np * P.k_max))) return rc;
   if ((rc = c->f64_cnk.ensure(16 * ns * c->n_max * P.k_max))) return rc;
   if ((rc = c->f64_soap_un.ensure(8 * ns * c->n_soap))) return rc;
   if ((rc = c->f64_norm.ensure(8 * ns))) return rc;
@@ -1331,7 +1331,8 @@ int ctx_hessian(soapb_context *c, const soapb_batch *b, const double *d_soap, in
   if ((rc = c->hs_soap.ensure(8 * ns * c->n_soap))) return rc;
   if ((rc = c->hs_ticket.ensure(16))) return rc;
   const int grid = std::max(1, std::min(hess_grid(P, chunk), b->n_sites));
-  if ((rc = c->hs_scratch.ensure(8 * (size_t)grid * hess_scratch_doubles(P, chunk)))) return rc;
+  if ((rc = c->hs_scratch.ensure(8 * (size_t)grid * hess_scratch_doubles(P)))) return rc;
+  if ((rc = c->hs_sums.ensure(8 * np * hess_sums_doubles(chunk)))) return rc;
   const size_t nsv = (size_t)c->n_soap, npair = (size_t)b->n_atom_pairs, nsite = (size_t)b->n_sites;
   if (chunk < n_vec) {
     if ((rc = c->hs_vchunk.ensure(8 * (nsite * chunk * nsv + 1)))) return rc;
@@ -1354,7 +1355,7 @@ int ctx_hessian(soapb_context *c, const soapb_batch *b, const double *d_soap, in
     }
     CU(launch_hessian(P, B, c->stream, w, c->hs_rad_der2.as<double>(), c->hs_geo.as<double>(),
                       c->hs_good.as<int>(), d_soap ? d_soap : c->hs_soap.as<double>(), nc, vecs, hess,
-                      c->hs_scratch.as<double>(), grid, c->hs_ticket.as<int>(), &nl));
+                      c->hs_sums.as<double>(), c->hs_scratch.as<double>(), grid, c->hs_ticket.as<int>(), &nl));
     if (chunk < n_vec && npair > 0)
       CU(cudaMemcpy2DAsync(d_hess + (size_t)v0 * 9, 72 * (size_t)n_vec, c->hs_hchunk.p, 72 * (size_t)nc,
                            72 * (size_t)nc, npair, cudaMemcpyDeviceToDevice, c->stream));

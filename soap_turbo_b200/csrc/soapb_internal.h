@@ -254,12 +254,16 @@ cudaError_t launch_fp64_contract(const DevParams &P, const DevBatch &B, cudaStre
 // left with do_der: second radial derivatives into rad_der2 (n_pairs, n_max),
 // per-pair geometry records into geo (n_pairs * hess_geo_doubles) and good
 // (n_pairs ints), then hess (n_pairs, n_vec, 3, 3) = 9 n_vec doubles per pair,
-// cleared first.  scratch: grid * hess_scratch_doubles doubles; ticket: one int.
-size_t hess_scratch_doubles(const DevParams &P, int n_vec);
+// cleared first.  sums: n_pairs * hess_sums_doubles doubles; scratch: grid *
+// hess_scratch_doubles doubles; ticket: one int.
+size_t hess_scratch_doubles(const DevParams &P);
+size_t hess_sums_doubles(int n_vec);                   // per pair, of k64_hess's k-sums
+constexpr int kHessVecs = 16;                          // weight vectors of one launch at most
 size_t hess_geo_doubles(const DevParams &P);
 size_t hess_smem_bytes(const DevParams &P, int n_vec);  // dynamic shared memory of k64_hess
 int hess_grid(const DevParams &P, int n_vec);
 cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s, const Fp64Work &w,
                            double *rad_der2, double *geo, int *good, const double *soap, int n_vec,
-                           const double *vecs, double *hess, double *scratch, int grid, int *ticket, int *launches);
+                           const double *vecs, double *hess, double *sums, double *scratch, int grid, int *ticket,
+                           int *launches);
 }  // namespace soapb
