@@ -195,61 +195,157 @@ __global__ void __launch_bounds__(128, 4) k64_angular2(const DevParams P, const 
   }
 }
 
-// ---- c_nlm, one CTA per site, threads over (n, k) (src/soap_turbo.f90:626-664).
-// The site's pairs go in chunks of kCnkChunk whose radial values and angular
-// plane are staged in shared memory with coalesced loads; each thread then sums
-// its (n, k) items over the chunk's pairs in CSR order.
-constexpr int kCnkChunk = 32;
-__global__ void __launch_bounds__(256) k64_cnk(const DevParams P, const DevBatch B, const double *rad,
-                                               const double2 *ang, double2 *cnk) {
-  extern __shared__ double csm[];
-  const int site = blockIdx.x;
-  const int K = P.k_max, N = P.n_max;
-  const int p0 = B.off[site], p1 = min(B.off[site + 1], B.n_pairs);
-  double *sR = csm;                          // kCnkChunk x N
-  double2 *sA = (double2 *)(csm + kCnkChunk * N);  // kCnkChunk x K
-  constexpr int IT = 8;                      // items per thread (N K <= 8 * 256)
-  double cr[IT], ci[IT];
-#pragma unroll
-  for (int j = 0; j < IT; ++j) cr[j] = ci[j] = 0.0;
-  for (int c0 = p0; c0 < p1; c0 += kCnkChunk) {
-    const int np_ = min(kCnkChunk, p1 - c0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < np_ * N; t += blockDim.x) sR[t] = rad[(size_t)c0 * N + t];
-    for (int t = threadIdx.x; t < np_ * K; t += blockDim.x) sA[t] = ang[(size_t)c0 * K + t];
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < IT; ++j) {
-      const int it = threadIdx.x + j * blockDim.x;
-      if (it >= N * K) break;
-      const int n = it / K, kk = it - n * K;
-      for (int q = 0; q < np_; ++q) {
-        const double fr = kFourPi64 * sR[q * N + n];
-        const double2 a = sA[q * K + kk];
-        cr[j] = cr[j] + fr * a.x;
-        ci[j] = ci[j] + fr * a.y;
-      }
-    }
-  }
-  double2 *c = cnk + (size_t)site * N * K;
-#pragma unroll
-  for (int j = 0; j < IT; ++j) {
-    const int it = threadIdx.x + j * blockDim.x;
-    if (it >= N * K) break;
-    const int n = it / K, kk = it - n * K;
-    double r = cr[j];
-    if (P.basis == 1 && kk == 0) {
-      for (int mm = 0; mm < B.species_mult[site]; ++mm) {
-        const int s = B.species[(size_t)site * B.max_mult + mm] - 1;
-        if (s >= 0 && s < P.n_species && n >= P.rad[s].nbeg && n < P.rad[s].nbeg + P.rad[s].alpha)
-          r += P.central[n];
-      }
-    }
-    c[it] = make_double2(r, ci[j]);
-  }
+// ---- c_nlm, power spectrum, compression and norm, one CTA per site
+// (src/soap_turbo.f90:626-664, 750-813).  c_nlm: the site's pairs in chunks of 32,
+// their radial values and angular plane staged in shared memory with coalesced
+// loads; a thread owns one k and four radial indices of one species and sums the
+// chunk's pairs of that species in CSR order (the other species' R_n are zero:
+// adding them changed nothing and took two thirds of the time with three
+// species).  The coefficients stay in shared memory for the dot products over
+// m, ordered by l so that a warp's are equally long.
+// soap_acc (may be null): the caller's soap, added before the norm is taken, as
+// the reference adds the compressed descriptor into soap (:798-802).
+// IT: items (species, four radial indices, k) per thread.
+constexpr int kSiteChunk = 32, kSiteThreads = 256;
+struct SiteSmem {
+  int C, A, R, p, total;  // in doubles
+};
+__host__ __device__ inline SiteSmem site_smem(const DevParams &P) {
+  SiteSmem L;
+  const int N = P.n_max, K = P.k_max;
+  L.C = 0;  // (N, K | 1) double2
+  int o = 2 * N * (K | 1);
+  L.A = o;
+  L.R = o + 2 * kSiteChunk * K;
+  const int a = L.R + kSiteChunk * (N + 4), b = o + P.n_kept;  // a chunk; then the components
+  L.p = o;
+  L.total = a > b ? a : b;
+  return L;
+}
+__host__ __device__ inline int site_items(const DevParams &P) {
+  int n = 0;
+  for (int s = 0; s < P.n_species; ++s) n += (P.rad[s].alpha + 3) / 4 * P.k_max;
+  return n;
 }
 
-// The CSR-order item loop of the form above for definitions with N K > 8 x 256.
+template <int IT>
+__global__ void __launch_bounds__(kSiteThreads) k64_site(const DevParams P, const DevBatch B, const double *rad,
+                                                         const double2 *ang, double2 *cnk, const double *soap_acc,
+                                                         double *soap_un, double *norm, double *soap) {
+  extern __shared__ __align__(16) double csm[];
+  __shared__ double s_red[kSiteThreads / 32];
+  const int site = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  const int K = P.k_max, N = P.n_max, KS = K | 1;
+  const int p0 = B.off[site], p1 = min(B.off[site + 1], B.n_pairs);
+  const SiteSmem L = site_smem(P);
+  double2 *sC = (double2 *)csm, *sA = (double2 *)(csm + L.A);
+  double *sR = csm + L.R, *sp = csm + L.p;
+  const int RS = (N + 3) / 4 * 4;  // R row (read four at a time; past a species' block its values are not stored)
+  // the thread's items: species, first radial index, k
+  int is[IT], in[IT], ik[IT];
+  double2 c[IT][4];
+#pragma unroll
+  for (int j = 0; j < IT; ++j) {
+    int it = tid + j * kSiteThreads;
+    is[j] = -1;
+    in[j] = ik[j] = 0;
+    for (int s = 0; s < P.n_species; ++s) {
+      const int w = (P.rad[s].alpha + 3) / 4 * K;
+      if (it >= 0 && it < w) {
+        is[j] = s;
+        in[j] = 4 * (it / K);
+        ik[j] = it - it / K * K;
+      }
+      it -= w;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[j][q] = make_double2(0.0, 0.0);
+  }
+  for (int c0 = p0; c0 < p1; c0 += kSiteChunk) {
+    const int nc = min(kSiteChunk, p1 - c0);
+    __syncthreads();
+    for (int t = tid; t < nc * N; t += kSiteThreads) {
+      const int q = t / N;
+      sR[q * RS + t - q * N] = kFourPi64 * rad[(size_t)c0 * N + t];
+    }
+    for (int t = tid; t < nc * K; t += kSiteThreads) sA[t] = ang[(size_t)c0 * K + t];
+    __syncthreads();
+    // the chunk's pairs whose radial rows are not zero, per species
+    const double r = lane < nc ? B.rjs[c0 + lane] : 0.0;
+    const unsigned bits = lane < nc ? B.bits[c0 + lane] : 0u;
+#pragma unroll
+    for (int j = 0; j < IT; ++j) {
+      for (int s = 0; s < P.n_species; ++s) {
+        const unsigned pairs = __ballot_sync(0xffffffffu, ((bits >> s) & 1u) && r < P.rad[s].rcut_hard &&
+                                                              (c0 + lane != p0 || P.rad[s].do_central));
+        if (is[j] != s) continue;
+        const double *R = sR + P.rad[s].nbeg + in[j];
+        const double2 *A = sA + ik[j];
+        for (unsigned m = pairs; m; m &= m - 1u) {
+          const int q = __ffs(m) - 1;
+          const double2 a = A[q * K];
+#pragma unroll
+          for (int n = 0; n < 4; ++n) {
+            const double fr = R[q * RS + n];
+            c[j][n].x = c[j][n].x + fr * a.x;
+            c[j][n].y = c[j][n].y + fr * a.y;
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < IT; ++j) {
+    if (is[j] < 0) continue;
+    const int s = is[j], nb = P.rad[s].nbeg, kk = ik[j];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int n = in[j] + q;
+      if (n >= P.rad[s].alpha) continue;
+      if (P.basis == 1 && kk == 0)
+        for (int mm = 0; mm < B.species_mult[site]; ++mm)
+          if (B.species[(size_t)site * B.max_mult + mm] - 1 == s) c[j][q].x += P.central[nb + n];
+      sC[(nb + n) * KS + kk] = c[j][q];
+      cnk[((size_t)site * N + nb + n) * K + kk] = c[j][q];
+    }
+  }
+  __syncthreads();  // c_nlm is complete, the staged chunk is read
+  for (int t = tid; t < P.n_kept; t += kSiteThreads) {
+    const int4 it = __ldg(P.ps_order + t);
+    const double2 *a = sC + it.x, *b = sC + it.y;
+    const int l = it.w & 0xff;
+    const double base = it.w < 0 ? sqrt(2.0) : 1.0;
+    double acc = 0.0;
+    for (int m = 0; m <= l; ++m) {
+      const double mult = base * ((m > 0) ? 2.0 : 1.0);
+      acc = acc + mult * (a[m].x * b[m].x + a[m].y * b[m].y);
+    }
+    sp[it.z] = acc;
+  }
+  __syncthreads();
+  double part = 0.0;
+  double *un = soap_un + (size_t)site * P.n_soap, *out = soap + (size_t)site * P.n_soap;
+  const double *in_row = soap_acc ? soap_acc + (size_t)site * P.n_soap : nullptr;
+  for (int o = tid; o < P.n_soap; o += kSiteThreads) {
+    double v = in_row ? in_row[o] : 0.0;
+    for (int t = P.pi_off[o]; t < P.pi_off[o + 1]; ++t) v = v + P.pi_el64[t] * sp[P.pi_q[t]];
+    un[o] = v;
+    part += v * v;
+  }
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  if (lane == 0) s_red[tid >> 5] = part;
+  __syncthreads();
+  double t = 0.0;
+  for (int w = 0; w < kSiteThreads / 32; ++w) t += s_red[w];
+  double nr = sqrt(t);
+  if (nr < 1.0e-5) nr = 1.0;
+  if (tid == 0) norm[site] = nr;
+  // each thread normalises the components it wrote
+  for (int o = tid; o < P.n_soap; o += kSiteThreads) out[o] = un[o] / nr;
+}
+
+// The same in two kernels for definitions whose items or shared memory the one
+// above does not hold: c_nlm, threads over (n, k) ...
 __global__ void k64_cnk_wide(const DevParams P, const DevBatch B, const double *rad, const double2 *ang,
                              double2 *cnk) {
   const int site = blockIdx.x;
@@ -276,9 +372,7 @@ __global__ void k64_cnk_wide(const DevParams P, const DevBatch B, const double *
   }
 }
 
-// ---- power spectrum + compression + norm, one CTA per site (:750-813).
-// soap_acc (may be null): the caller's soap, added before the norm is taken, as
-// the reference adds the compressed descriptor into soap (:798-802).
+// ... and power spectrum + compression + norm, one CTA per site.
 __global__ void k64_soap(const DevParams P, const DevBatch B, const double2 *cnk, const double *soap_acc,
                          double *soap_un, double *norm) {
   extern __shared__ double sp[];  // n_kept
@@ -1010,14 +1104,18 @@ cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaSt
     else k64_angular<12><<<blocks, 128, 0, s>>>(P, B, ang_der, (double2 *)w.ang);
     nl += 2;
   }
-  if (nsites > 0) {
-    if (P.n_max * P.k_max <= 8 * 256) {
-      const size_t smc = (size_t)kCnkChunk * (P.n_max + 2 * P.k_max) * sizeof(double);
-      cudaFuncSetAttribute(k64_cnk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smc);
-      k64_cnk<<<nsites, 256, smc, s>>>(P, B, w.rad, (const double2 *)w.ang, (double2 *)w.cnk);
-    } else {
-      k64_cnk_wide<<<nsites, 256, 0, s>>>(P, B, w.rad, (const double2 *)w.ang, (double2 *)w.cnk);
-    }
+  const size_t sms = (size_t)site_smem(P).total * sizeof(double);
+  const int items = (site_items(P) + kSiteThreads - 1) / kSiteThreads;
+  const bool one = items <= 2 && sms <= kCartSmemCap;
+  if (nsites > 0 && one) {
+    auto kern = items == 1 ? k64_site<1> : k64_site<2>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms);
+    if (e != cudaSuccess) return e;
+    kern<<<nsites, kSiteThreads, sms, s>>>(P, B, w.rad, (const double2 *)w.ang, (double2 *)w.cnk, soap_acc,
+                                           w.soap_unnorm, w.norm, soap);
+    nl += 1;
+  } else if (nsites > 0) {
+    k64_cnk_wide<<<nsites, 256, 0, s>>>(P, B, w.rad, (const double2 *)w.ang, (double2 *)w.cnk);
     const size_t sm = (size_t)P.n_kept * sizeof(double);
     cudaFuncSetAttribute(k64_soap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k64_soap<<<nsites, 256, sm, s>>>(P, B, (const double2 *)w.cnk, soap_acc, w.soap_unnorm, w.norm);
@@ -1049,7 +1147,7 @@ cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaSt
     }
     nl += 1;
   }
-  if (nsites > 0) {
+  if (nsites > 0 && !one) {
     const size_t n = (size_t)nsites * P.n_soap;
     k64_normalise<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, B, w.soap_unnorm, w.norm, soap);
     nl += 1;

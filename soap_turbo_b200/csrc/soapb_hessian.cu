@@ -23,10 +23,10 @@ namespace {
 
 constexpr double kPi = 3.14159265358979323846;
 constexpr int kHessThreads = 256;
-constexpr int kHessPC = 8;      // pairs per chunk of pass A
+constexpr int kHessPC = 16;     // pairs per chunk of pass A
 constexpr int kHessCols = 13;   // k-sums of a unit of pass B at most (odd: the transpose buffer's row stride)
 constexpr int kHessChunk = 256; // pairs whose entries are listed at a time
-constexpr size_t kHessSmemPair = 113 * 1024;  // shared memory of a CTA of which an SM holds two
+constexpr int kHessSmemPair = 113 * 1024;  // shared memory of a CTA of which an SM holds two
 
 #define CU_RET(x)                         \
   do {                                    \
@@ -199,13 +199,18 @@ __global__ void k64_radial_d2(const DevParams P, const DevBatch B, double *rad_d
   const double r = B.rjs[k];
   const unsigned bits = B.bits[k];
   double *r2o = rad_der2 + (size_t)k * P.n_max;
+  unsigned todo = 0u;
   for (int s = 0; s < P.n_species; ++s) {
     const RadSp &S = P.rad[s];
-    const bool ok = ((bits >> s) & 1u) && r < S.rcut_hard && (!is_self || S.do_central);
-    if (!ok) {
+    if (((bits >> s) & 1u) && r < S.rcut_hard && (!is_self || S.do_central)) todo |= 1u << s;
+    else
       for (int n = 0; n < S.alpha; ++n) r2o[S.nbeg + n] = 0.0;
-      continue;
-    }
+  }
+  // one expansion per valid species; lanes of different species share it
+  while (todo) {
+    const int s = __ffs(todo) - 1;
+    todo &= todo - 1u;
+    const RadSp &S = P.rad[s];
     double val[AMAX], der[AMAX], der2[AMAX];
     radial_pair_d2<AMAX>(P, S, P.Wblk + (size_t)s * P.wstride, r, is_self, val, der, der2);
     for (int n = 0; n < S.alpha; ++n) r2o[S.nbeg + n] = der2[n] * S.gscale;
@@ -215,21 +220,19 @@ __global__ void k64_radial_d2(const DevParams P, const DevBatch B, double *rad_d
 // Per-pair record of the Hessian (pair_geometry, src/soap_turbo.f90:1537-1652),
 // written once by k64_hgeo and read by k64_hess: offsets in doubles.
 struct GeoLayout {
-  int nh, invr, F, F1, F2, t, th, w, wh, Q, wp, size;
+  int nh, invr, F, t, th, w, wh, Q, wp, size;
   __host__ __device__ explicit GeoLayout(int L) {
     const int L1 = L + 1, K = L1 * (L1 + 1) / 2;
     nh = 0;
     invr = 3;
-    F = 4;
-    F1 = F + L1;
-    F2 = F1 + L1;
-    t = F2 + L1;
-    th = t + 3;
-    w = th + 9;   // 3 complex
+    w = 4;        // 3 complex; the complex values at even offsets
     wh = w + 6;   // 9 complex
-    Q = wh + 18;  // K: Q_l^m(t) = d^m P_l / dt^m
-    wp = Q + K;   // L + 3 complex: w^m at m + 2, w^-2 = w^-1 = 0
-    size = wp + 2 * (L + 3);
+    wp = wh + 18; // L + 3 complex: w^m at m + 2, w^-2 = w^-1 = 0
+    t = wp + 2 * (L + 3);
+    th = t + 3;
+    F = th + 9;   // F_l, F'_l, F''_l of each l
+    Q = F + 3 * L1;  // K: Q_l^m(t) = d^m P_l / dt^m, and two pads (Q_l^m+1, Q_l^m+2 of the last k are read)
+    size = Q + K + 2;
     size += size & 1;
   }
 };
@@ -272,13 +275,12 @@ __device__ void ilexp_to(int lmax, double x, double *out) {
 // ---- pair geometry, one thread per pair: F_l and its first two r-derivatives,
 // the unit vector, the gradients and Hessians of t = cos(theta) and
 // w = (x - iy)/r, Q_l^m(t) and w^m.  good[k] = 0 for pairs the Hessian skips
-// (beyond rcut_max, at the origin, or in no species).
-__global__ void k64_hgeo(const DevParams P, const DevBatch B, double *geo, int *good) {
-  const int kk = blockIdx.x * blockDim.x + threadIdx.x;
-  if (kk >= B.n_pairs) return;
+// (beyond rcut_max, at the origin, or in no species).  A warp's records are built
+// in shared memory (rows of odd length) and copied out side by side: written by
+// their threads, a value at a time 1 KB apart, they took 121 us for 88 k pairs.
+__device__ void pair_record(const DevParams &P, const DevBatch &B, int kk, double *g, int *good) {
   const int L = P.l_max;
   const GeoLayout Lg(L);
-  double *g = geo + (size_t)kk * Lg.size;
   const double rr = B.rjs[kk];
   const unsigned bits = B.bits[kk];
   const bool ok = rr < P.rcut_max && rr >= 1.0e-10 && bits != 0u;
@@ -302,9 +304,9 @@ __global__ void k64_hgeo(const DevParams P, const DevBatch B, double *geo, int *
     const double d2il = il[l + 2] + ((double)(2 * l + 1) * invz - 2.0) * il[l + 1] +
                         (rl * (rl - 1.0) * invz * invz - 2.0 * rl * invz + 1.0) * il[l];
     const double f0 = il[l], f1 = dil * zp, f2 = d2il * zp * zp + dil * zp2;
-    g[Lg.F + l] = amp * f0;
-    g[Lg.F1 + l] = ampd * f0 + amp * f1;
-    g[Lg.F2 + l] = ampdd * f0 + 2.0 * ampd * f1 + amp * f2;
+    g[Lg.F + 3 * l] = amp * f0;
+    g[Lg.F + 3 * l + 1] = ampd * f0 + amp * f1;
+    g[Lg.F + 3 * l + 2] = ampdd * f0 + 2.0 * ampd * f1 + amp * f2;
   }
   double nh[3];
   const double sin_t = sin(B.thetas[kk]), cos_t = cos(B.thetas[kk]);
@@ -349,6 +351,7 @@ __global__ void k64_hgeo(const DevParams P, const DevBatch B, double *geo, int *
     Qt[kbb + ll - 1] = (double)(2 * ll - 1) * tt * Qt[kbb - 1];
     Qt[kbb + ll] = (double)(2 * ll - 1) * Qt[kbb - 1];
   }
+  Qt[Lg.size - Lg.Q - 1] = Qt[(L + 1) * (L + 2) / 2] = Qt[(L + 1) * (L + 2) / 2 + 1] = 0.0;
   dcx wpow = cx(1.0, 0.0);
   stc(g + Lg.wp, cx(0.0, 0.0));
   stc(g + Lg.wp + 2, cx(0.0, 0.0));
@@ -358,19 +361,29 @@ __global__ void k64_hgeo(const DevParams P, const DevBatch B, double *geo, int *
     stc(g + Lg.wp + 2 * (mm + 2), wpow);
   }
 }
+__global__ void __launch_bounds__(32) k64_hgeo(const DevParams P, const DevBatch B, double *geo, int *good) {
+  extern __shared__ double srec[];
+  const int k0 = blockIdx.x * 32, lane = threadIdx.x, size = GeoLayout(P.l_max).size, row = size | 1;
+  if (k0 + lane < B.n_pairs) pair_record(P, B, k0 + lane, srec + lane * row, good);
+  __syncwarp();
+  const int n = min(32, B.n_pairs - k0);
+  double *o = geo + (size_t)k0 * size;
+  for (int i = 0; i < n; ++i)
+    for (int t = lane; t < size; t += 32) o[(size_t)i * size + t] = srec[i * row + t];
+}
 
 // Per-CTA global scratch of the Hessian kernel (hess_scratch_doubles)
 struct HessScratch {
-  double *G;      // (n_max, k_max, 3) complex: sum_j d c_nlm / d r_j, when it is not in shared memory
+  double2 *G;     // (3, n_max, k_max) complex: sum_j d c_nlm / d r_j
   double *dp1;    // (n_soap, 3): d p / d r_i, unnormalised
   double *kept3;  // (3, n_kept)
-  double *vk;     // (n_kept): a weight vector spread through the compression, when not in shared memory
+  double *vk;     // (3, n_kept): weight vectors spread through the compression
 };
 
 __device__ HessScratch carve(double *base, const DevParams &P) {
   HessScratch h;
-  h.G = base;
-  h.dp1 = h.G + 6 * (size_t)P.n_max * P.k_max;
+  h.G = (double2 *)base;
+  h.dp1 = base + 6 * (size_t)P.n_max * P.k_max;
   h.kept3 = h.dp1 + 3 * (size_t)P.n_soap;
   h.vk = h.kept3 + 3 * (size_t)P.n_kept;
   return h;
@@ -378,29 +391,29 @@ __device__ HessScratch carve(double *base, const DevParams &P) {
 
 // Shared memory of k64_hess, in doubles.
 struct HessSmem {
-  int G, Z, red, vk, rad, dot, list, total;
-  bool g_shared, vk_shared;
+  int Z, red, ck, rad, dot, list, total;
+  int rows;  // radial indices whose tables it holds
 };
 __host__ __device__ inline HessSmem hess_smem(const DevParams &P, int n_vec) {
   HessSmem S;
   const int N = P.n_max, K = P.k_max, AB = P.amax_t;
-  S.vk_shared = P.n_kept <= 2048;
-  // pass B: a species' tables of one weight vector and the warps' transpose
-  // buffers; pass A: a chunk of pairs' angular factors and radial rows
-  const int b = 8 * AB * K + (kHessThreads / 32) * 32 * kHessCols, a = kHessPC * (12 * K + 2 * AB);
-  int o = 0;
-  S.Z = o;
-  S.red = o + 8 * AB * K;
-  o += a > b ? a : b;
-  S.vk = o;   o += S.vk_shared ? P.n_kept : 0;
-  S.rad = o;  o += (kHessThreads / 16) * 3 * AB;
-  S.dot = o;  o += 4 + 4 * n_vec;
-  S.list = o; o += (kHessChunk * P.n_species + 3) / 4;
-  o = (o + 1) & ~1;
-  // G last: in shared memory when two CTAs still fit an SM
-  S.G = o;
-  S.g_shared = (size_t)(o + 6 * N * K) * sizeof(double) <= kHessSmemPair;
-  S.total = o + (S.g_shared ? 6 * N * K : 0);
+  const int n_red = (kHessThreads / 32) * 32 * kHessCols, n_rad = (kHessThreads / 16) * 4 * AB;
+  const int n_dot = 4 + 4 * n_vec, n_list = (kHessChunk * P.n_species + 3) / 4, n_ck = K + (K + 1) / 2;
+  // pass B: the tables of one weight vector, of every species where two CTAs
+  // then still fit an SM, and the warps' transpose buffers
+  int rows = (kHessSmemPair / 8 - n_red - n_rad - n_dot - n_list - n_ck - 4) / (8 * K);
+  if (rows > N) rows = N;
+  if (rows < AB) rows = AB;
+  S.rows = rows;
+  S.Z = 0;
+  S.red = 8 * rows * K;
+  const int b = S.red + n_red, a = kHessPC * (12 * K + 2 * AB);  // pass A: a chunk's angular factors and radial rows
+  int o = ((a > b ? a : b) + 1) & ~1;
+  S.rad = o;  o += n_rad;
+  S.ck = o;   o += n_ck;
+  S.dot = o;  o += n_dot;
+  S.list = o; o += n_list;
+  S.total = o;
   return S;
 }
 
@@ -472,20 +485,23 @@ __device__ __forceinline__ double second_der(const double *S, const double *g, c
 //     chunk by chunk; then dp1 = d p / d r_i = -(d p / d c) G component by
 //     component of p (the reference sums -dp_j over the pairs; the two agree to
 //     rounding, since sum_j d c / d r_j = G);
-//  B  per weight vector and species: the vector spread back through the
-//     compression into its S_v(n, n', l) and applied to c_nlm (Z_v) and to G (ZG_v)
-//     (:1336-1376), the species' tables in shared memory; then a half-warp per
-//     pair of the species, lanes over k, contracts them with the pair's R_n, R'_n,
-//     R''_n and Omega into the k-sums above.  Z_v and the three components of
-//     ZG_v are units of their own, so that a species of some twenty pairs still
-//     fills the warps;
+//  B  per weight vector: the vector spread back through the compression into its
+//     S_v(n, n', l) and applied to c_nlm (Z_v) and to G (ZG_v) (:1336-1376), the
+//     tables in shared memory; then a half-warp per pair, lanes over k, contracts
+//     its species' rows of them with the pair's R_n, R'_n, R''_n and Omega into the
+//     k-sums above, Z_v and ZG_v as units of their own;
 //  C  per pair: the second derivative hv and the first derivatives v . dp_j (what
 //     the reference's self-test rebuilds, here the value used), and from them the
 //     normalisation (:1414-1484).
 // Sums run in a fixed order (pairs in CSR order, k within a lane, lanes through
-// shared memory).  Read from L2 for every pair, whole Z_v and ZG_v rows had bound
-// the kernel (a pair of three species' definition took 190 KB).
-template <bool GS>
+// shared memory).
+// What bounds it: instructions (280 k per site of 52 pairs, three species, one
+// vector; a third of them FP64), issued at 38 % of the rate by 16 warps per SM that
+// wait for the pair records, G and c_nlm from L1 and L2.  1.16 ms at 1679 such
+// sites.  Against it, 3.07 ms: tables of every radial index read from L2 by every
+// pair (190 KB each) and Cartesian tensors of Omega formed per k; 1.81 ms with the
+// tables of a species and vector at a time in shared memory, and G beside them, the
+// barriers between them taking a quarter of the time.
 __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, const DevBatch B, const double *rad,
                                                          const double *rad_der, const double *rad_der2,
                                                          const double *geo, const int *good, const double2 *cnk,
@@ -496,23 +512,31 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
   __shared__ int s_site;
   __shared__ int s_base[SOAPB_MAX_SPECIES + 1];
   const int N = P.n_max, K = P.k_max, ns = P.n_soap, nk = P.n_kept, AB = P.amax_t, nsp = P.n_species;
-  const int nvh = n_vec + 1, nva = n_vec + 4;
+  const int nvh = n_vec + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = lane >> 4, hl = lane & 15;
   constexpr int NT = kHessThreads, NW = NT / 32;
   const size_t sp_sums = (size_t)kSumsFull * nvh + 3 * kSumsLight;
   const GeoLayout Lg(P.l_max);
   const HessSmem Ly = hess_smem(P, n_vec);
   const HessScratch h = carve(scratch + scratch_per_cta * blockIdx.x, P);
-  double *G = GS ? sm + Ly.G : h.G;
-  double *vk = Ly.vk_shared ? sm + Ly.vk : h.vk;
-  double *cab = sm + Ly.Z, *crr = cab + (size_t)kHessPC * K * 12;
-  double2 *sZ = (double2 *)(sm + Ly.Z), *sZG = sZ + (size_t)AB * K;  // (n, K); (q, n, K)
+  double2 *G = h.G;
+  const int RT = Ly.rows, NK = N * K;
+  double2 *cab = (double2 *)(sm + Ly.Z);  // (pair, A_x, B_x, A_y, .., K): lanes over k side by side
+  double *crr = sm + Ly.Z + (size_t)kHessPC * K * 12;
+  double2 *sZ = (double2 *)(sm + Ly.Z), *sZG = sZ + (size_t)RT * K;  // (row, K); (q, row, K)
   double *red = sm + Ly.red + (size_t)warp * 32 * kHessCols;
-  double *wrad = sm + Ly.rad + (size_t)(2 * warp + half) * 3 * AB;
+  double *wrad = sm + Ly.rad + (size_t)(2 * warp + half) * 4 * AB;
   double *sdot = sm + Ly.dot;
   unsigned short *list = (unsigned short *)(sm + Ly.list);
-  const int *klm = (const int *)(P.blob + P.off_klm);
+  // per k: 4 pi (-1)^m preflm, and l | m << 8
+  double *sck = sm + Ly.ck;
+  int *klm = (int *)(sck + K);
   const double fourpi = 4.0 * kPi;
+  for (int k = tid; k < K; k += NT) {
+    const int lm = ((const int *)(P.blob + P.off_klm))[k];
+    klm[k] = lm;
+    sck[k] = ((lm >> 8) & 1) ? -fourpi * P.preflm64[k] : fourpi * P.preflm64[k];
+  }
 
   for (;;) {
     __syncthreads();
@@ -525,13 +549,16 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
     const double2 *c = cnk + (size_t)site * N * K;
     const double *soap_i = soap + (size_t)site * ns;
     // the entries of species [s_lo, s_hi) among the pairs [c0, c1), pair - c0, from
-    // list[s_base[s]] on (every warp writes the same list)
+    // list[s_base[s]] on (every warp writes the same list); whether a pair has several
     auto build = [&](int s_lo, int s_hi, int c0, int c1) {
       __syncthreads();  // the list before is read
       unsigned long long v = 0ull;
+      bool several = false;
       for (int t = 0; c0 + 32 * t < c1; ++t) {
         const int k = c0 + 32 * t + lane;
-        if (k < c1) v |= (unsigned long long)hess_species(P, B, good, k) << (8 * t);
+        const unsigned ok = k < c1 ? hess_species(P, B, good, k) : 0u;
+        v |= (unsigned long long)ok << (8 * t);
+        several |= (ok & (ok - 1u)) != 0u;
       }
       int e = 0;
       for (int s = s_lo; s < s_hi; ++s) {
@@ -548,11 +575,14 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
       }
       if (lane == 0) s_base[s_hi] = e;
       __syncthreads();
+      return __any_sync(0xffffffffu, several) != 0;
     };
+    // species one at a time where the site takes several chunks, and where a pair's
+    // sums come from several species (they are added in the species' order)
     const bool multi = p1 - p0 - 1 > kHessChunk;
-    if (!multi) build(0, nsp, p0 + 1, p1);
+    const bool apart = multi || build(0, nsp, p0 + 1, p1);
     // ---- A
-    for (int t = tid; t < 6 * N * K; t += NT) G[t] = 0.0;
+    for (int t = tid; t < 3 * NK; t += NT) G[t] = make_double2(0.0, 0.0);
     for (int s = 0; s < nsp; ++s) {
       const int a = P.rad[s].alpha, nb = P.rad[s].nbeg;
       for (int c0 = p0 + 1; c0 < p1; c0 += kHessChunk) {
@@ -569,37 +599,38 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
           for (int t = tid; t < nc * K; t += NT) {
             const int pp = t / K, k = t - pp * K, lm = klm[k], l = lm & 0xff, m = lm >> 8;
             const double *g = geo + (size_t)(c0 + (list[eb + pp] & 0x7fff)) * Lg.size;
-            const double C = (m & 1) ? -P.preflm64[k] : P.preflm64[k];
+            const double C = sck[k];
             const double q0 = C * g[Lg.Q + k], q1 = (m < l) ? C * g[Lg.Q + k + 1] : 0.0;
             const dcx w0 = ldc(g + Lg.wp + 2 * (m + 2)), w1 = ldc(g + Lg.wp + 2 * (m + 1));
             const dcx Om = q0 * w0, Ot = q1 * w0, Ow = (q0 * (double)m) * w1;
-            const double f0 = fourpi * g[Lg.F + l], f1 = fourpi * g[Lg.F1 + l];
-            double *o = cab + (size_t)t * 12;
+            const double f0 = g[Lg.F + 3 * l], f1 = g[Lg.F + 3 * l + 1];
+            double2 *o = cab + pp * 6 * K + k;
+#pragma unroll
             for (int q = 0; q < 3; ++q) {
               const double nq = g[Lg.nh + q];
-              stc(o + 4 * q, (f0 * nq) * Om);
-              stc(o + 4 * q + 2, (f1 * nq) * Om + f0 * (g[Lg.t + q] * Ot + Ow * ldc(g + Lg.w + 2 * q)));
+              const dcx d = (f1 * nq) * Om + f0 * (g[Lg.t + q] * Ot + Ow * ldc(g + Lg.w + 2 * q));
+              o[2 * q * K] = make_double2(f0 * nq * Om.re, f0 * nq * Om.im);
+              o[(2 * q + 1) * K] = make_double2(d.re, d.im);
             }
           }
           __syncthreads();
           // threads over (k, two radial indices)
           for (int it = tid; it < ((a + 1) >> 1) * K; it += NT) {
             const int n2 = it / K, k = it - n2 * K, n0 = 2 * n2, n1 = min(n0 + 1, a - 1);
-            double2 *g0 = (double2 *)(G + ((size_t)(nb + n0) * K + k) * 6);
-            double2 *g1 = (double2 *)(G + ((size_t)(nb + n1) * K + k) * 6);
+            double2 *g0 = G + (nb + n0) * K + k, *g1 = G + (nb + n1) * K + k;
             double2 x[3], y[3];
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-              x[q] = g0[q];
-              y[q] = g1[q];
+              x[q] = g0[q * NK];
+              y[q] = g1[q * NK];
             }
             for (int pp = 0; pp < nc; ++pp) {
-              const double2 *f = (const double2 *)(cab + ((size_t)pp * K + k) * 12);
+              const double2 *f = cab + pp * 6 * K + k;
               const double *R = crr + pp * 2 * AB;
               const double r0 = R[n0], d0 = R[AB + n0], r1 = R[n1], d1 = R[AB + n1];
 #pragma unroll
               for (int q = 0; q < 3; ++q) {
-                const double2 A = f[2 * q], D = f[2 * q + 1];
+                const double2 A = f[2 * q * K], D = f[(2 * q + 1) * K];
                 x[q].x = x[q].x + d0 * A.x + r0 * D.x;
                 x[q].y = x[q].y + d0 * A.y + r0 * D.y;
                 y[q].x = y[q].x + d1 * A.x + r1 * D.x;
@@ -608,8 +639,8 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
             }
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-              g0[q] = x[q];
-              if (n0 + 1 < a) g1[q] = y[q];
+              g0[q * NK] = x[q];
+              if (n0 + 1 < a) g1[q * NK] = y[q];
             }
           }
         }
@@ -626,10 +657,11 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
         const int k = l * (l + 1) / 2 + m;
         const double w = base * ((m > 0) ? 2.0 : 1.0);
         const double2 a = c[(size_t)n * K + k], b = c[(size_t)np * K + k];
-        const double *ga = G + ((size_t)n * K + k) * 6, *gb = G + ((size_t)np * K + k) * 6;
 #pragma unroll
-        for (int e = 0; e < 3; ++e)
-          d[e] = d[e] - w * (ga[2 * e] * b.x + ga[2 * e + 1] * b.y + a.x * gb[2 * e] + a.y * gb[2 * e + 1]);
+        for (int e = 0; e < 3; ++e) {
+          const double2 ga = G[e * NK + n * K + k], gb = G[e * NK + np * K + k];
+          d[e] = d[e] - w * (ga.x * b.x + ga.y * b.y + a.x * gb.x + a.y * gb.y);
+        }
       }
       for (int e = 0; e < 3; ++e) h.kept3[(size_t)e * nk + q] = d[e];
     }
@@ -659,149 +691,183 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
       }
       if (lane == 0) sdot[d] = r;
     }
-    // ---- B
-    for (int v = 0; v < nva; ++v) {
+    // ---- B: a pass per vector of the Hessian, then one for the three columns of
+    // dp1 together (their tables in ZG's place, their sums being the same)
+    for (int v = 0; v <= nvh; ++v) {
       const bool full = v < nvh;
-      const size_t off = full ? (size_t)v * kSumsFull : (size_t)nvh * kSumsFull + (v - nvh) * kSumsLight;
-      for (int q = tid; q < nk; q += NT) {
+      const size_t off = (size_t)v * kSumsFull + (full ? 13 : 0);  // of the ZG sums
+      __syncthreads();  // the vectors before are read
+      for (int t = tid; t < (full ? nk : 3 * nk); t += NT) {
+        const int w = t / nk, q = t - w * nk;
         double x = 0.0;
-        for (int t = P.pj_off[q]; t < P.pj_off[q + 1]; ++t)
-          x = x + P.pj_el64[t] * weight(vecs, soap_i, sv, h.dp1, n_vec, ns, site, v, P.pj_o[t]);
-        vk[q] = x;
+        for (int i = P.pj_off[q]; i < P.pj_off[q + 1]; ++i)
+          x = x + P.pj_el64[i] * weight(vecs, soap_i, sv, h.dp1, n_vec, ns, site, v + w, P.pj_o[i]);
+        h.vk[t] = x;
       }
-      for (int s = 0; s < nsp; ++s) {
-        const int a = P.rad[s].alpha, nb = P.rad[s].nbeg;
-        if (!multi && s_base[s] == s_base[s + 1]) continue;
+      for (int s_lo = 0, s_hi; s_lo < nsp; s_lo = s_hi) {
+        // as many species as the tables hold
+        int n_rows = P.rad[s_lo].alpha;
+        for (s_hi = s_lo + 1; !apart && s_hi < nsp && n_rows + P.rad[s_hi].alpha <= RT; ++s_hi) n_rows += P.rad[s_hi].alpha;
+        const int nb = P.rad[s_lo].nbeg;
         __syncthreads();  // vk is complete, the tables before are read
         // S_v through the per-(l, n) lists of the kept components (2 v on the
         // diagonal, sqrt 2 v off it, np ascending)
-        for (int it = tid; it < a * K; it += NT) {
+        for (int it = tid; it < n_rows * K; it += NT) {
           const int n = it / K, k = it - n * K, l = klm[k] & 0xff;
           double2 z = make_double2(0.0, 0.0), b[3];
 #pragma unroll
           for (int q = 0; q < 3; ++q) b[q] = z;
-          const int li = l * N + nb + n;
-          for (int t = P.hl_off[li]; t < P.hl_off[li + 1]; ++t) {
-            const int np = P.hl_np[t];
-            const double y = P.hl_fac64[t] * vk[P.hl_q[t]];
-            const double2 cc = c[(size_t)np * K + k];
-            z.x += y * cc.x;
-            z.y += y * cc.y;
-            if (full) {
-              const double2 *gg = (const double2 *)(G + ((size_t)np * K + k) * 6);
+          const int li = l * N + nb + n, t1 = P.hl_off[li + 1];
+          if (full) {
+#pragma unroll 4
+            for (int t = P.hl_off[li]; t < t1; ++t) {
+              const int code = __ldg(P.hl_packed + t), np = code & 0xff;
+              const double y = (code < 0 ? 2.0 : sqrt(2.0)) * h.vk[(code >> 8) & 0xffff];
+              const double2 cc = c[np * K + k];
+              const double2 *gg = G + np * K + k;
+              z.x += y * cc.x;
+              z.y += y * cc.y;
 #pragma unroll
               for (int q = 0; q < 3; ++q) {
-                const double2 gv = gg[q];
+                const double2 gv = gg[q * NK];
                 b[q].x += y * gv.x;
                 b[q].y += y * gv.y;
               }
             }
-          }
-          sZ[n * K + k] = z;
-          if (full)
+            sZ[n * K + k] = z;
+          } else {
+#pragma unroll 4
+            for (int t = P.hl_off[li]; t < t1; ++t) {
+              const int code = __ldg(P.hl_packed + t), np = code & 0xff, q0 = (code >> 8) & 0xffff;
+              const double f = code < 0 ? 2.0 : sqrt(2.0);
+              const double2 cc = c[np * K + k];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) sZG[(q * AB + n) * K + k] = b[q];
+              for (int q = 0; q < 3; ++q) {
+                const double y = f * h.vk[q * nk + q0];
+                b[q].x += y * cc.x;
+                b[q].y += y * cc.y;
+              }
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 3; ++q) sZG[(q * RT + n) * K + k] = b[q];
         }
         __syncthreads();
         for (int c0 = p0 + 1; c0 < p1; c0 += kHessChunk) {
-          if (multi) build(s, s + 1, c0, min(p1, c0 + kHessChunk));
-          const int e0 = s_base[s], n_two = (s_base[s + 1] - e0 + 1) >> 1;
-          // units: two pairs (one per half-warp) and Z_v (part 0) or a component of ZG_v
-          for (int u = warp; u < n_two * (full ? 4 : 1); u += NW) {
-            const int part = u / n_two, e = e0 + 2 * (u - part * n_two) + half;
+          if (multi) build(s_lo, s_hi, c0, min(p1, c0 + kHessChunk));
+          int n_two = 0;  // pairs of entries
+          for (int s = s_lo; s < s_hi; ++s) n_two += (s_base[s + 1] - s_base[s] + 1) >> 1;
+          // units: two pairs (one per half-warp), Z_v (all first) or ZG_v
+          for (int u = warp; u < (full ? 2 : 1) * n_two; u += NW) {
+            const bool zg = !full || u >= n_two;
+            int e = u >= n_two ? u - n_two : u, s = s_lo;
+            for (int m2; e >= (m2 = (s_base[s + 1] - s_base[s] + 1) >> 1); ++s) e -= m2;
+            const int e0 = s_base[s], a = P.rad[s].alpha, row = P.rad[s].nbeg - nb;
+            e = e0 + 2 * e + half;
             const bool pv = e < s_base[s + 1];
             const int code = list[pv ? e : e0], j = c0 + (code & 0x7fff);
             const double *g = geo + (size_t)j * Lg.size;
+            // R_n, R'_n, R''_n side by side
             for (int t = hl; t < 3 * a; t += 16) {
               const int w = t / a, n = t - w * a;
-              wrad[w * AB + n] = (w == 0 ? rad : (w == 1 ? rad_der : rad_der2))[(size_t)j * N + nb + n];
+              wrad[4 * n + w] = (w == 0 ? rad : (w == 1 ? rad_der : rad_der2))[(size_t)j * N + nb + row + n];
             }
             __syncwarp();
             double acc[kHessCols];
 #pragma unroll
             for (int t = 0; t < kHessCols; ++t) acc[t] = 0.0;
-            const double invr = g[Lg.invr];
-            const double2 *tab = part == 0 ? sZ : sZG + (size_t)(part - 1) * AB * K;
+            const double *gQ = g + Lg.Q, *gW = g + Lg.wp, *gF = g + Lg.F;
             for (int k = hl; k < K; k += 16) {
               const int lm = klm[k], l = lm & 0xff, m = lm >> 8;
+              // Om = q0 w0, Om_t = q1 w0, Om_w = q0 w1, ...
+              const double C = ((m > 0) ? 2.0 : 1.0) * sck[k];
+              const double q0 = C * gQ[k], q1 = (m < l) ? C * gQ[k + 1] : 0.0;
+              const double2 w0 = *(const double2 *)(gW + 2 * (m + 2)), v1 = *(const double2 *)(gW + 2 * (m + 1));
+              const double f0 = gF[3 * l], f1 = gF[3 * l + 1];
+              const dcx W0 = cx(w0.x, w0.y), W1 = cx((double)m * v1.x, (double)m * v1.y);
+              const dcx Om = q0 * W0, Ot = q1 * W0, Ow = q0 * W1;
+              if (zg) {
+                double2 a0[3], a1[3];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) a0[q] = a1[q] = make_double2(0.0, 0.0);
+                const double2 *z = sZG + row * K + k;
+#pragma unroll 2
+                for (int n = 0; n < a; ++n, z += K) {
+                  const double2 r = *(const double2 *)(wrad + 4 * n);
+#pragma unroll
+                  for (int q = 0; q < 3; ++q) {
+                    const double2 zz = z[q * RT * K];
+                    a0[q].x += r.x * zz.x;
+                    a0[q].y -= r.x * zz.y;
+                    a1[q].x += r.y * zz.x;
+                    a1[q].y -= r.y * zz.y;
+                  }
+                }
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                  const dcx z0 = cx(f0 * a0[q].x, f0 * a0[q].y);
+                  const dcx z1 = cx(f0 * a1[q].x + f1 * a0[q].x, f0 * a1[q].y + f1 * a0[q].y);
+                  acc[4 * q] += z1.re * Om.re - z1.im * Om.im;
+                  acc[4 * q + 1] += z0.re * Ot.re - z0.im * Ot.im;
+                  acc[4 * q + 2] += z0.re * Ow.re - z0.im * Ow.im;
+                  acc[4 * q + 3] += z0.re * Ow.im + z0.im * Ow.re;
+                }
+                continue;
+              }
               double2 a0 = make_double2(0.0, 0.0), a1 = a0, a2 = a0;
-              const double2 *z = tab + k;
-              if (full && part == 0) {
+              const double2 *z = sZ + row * K + k;
 #pragma unroll 4
-                for (int n = 0; n < a; ++n) {
-                  const double2 zz = z[n * K];
-                  const double r0 = wrad[n], r1 = wrad[AB + n], r2 = wrad[2 * AB + n];
-                  a0.x += r0 * zz.x;
-                  a0.y -= r0 * zz.y;
-                  a1.x += r1 * zz.x;
-                  a1.y -= r1 * zz.y;
-                  a2.x += r2 * zz.x;
-                  a2.y -= r2 * zz.y;
-                }
-              } else {
-#pragma unroll 4
-                for (int n = 0; n < a; ++n) {
-                  const double2 zz = z[n * K];
-                  const double r0 = wrad[n], r1 = wrad[AB + n];
-                  a0.x += r0 * zz.x;
-                  a0.y -= r0 * zz.y;
-                  a1.x += r1 * zz.x;
-                  a1.y -= r1 * zz.y;
-                }
+              for (int n = 0; n < a; ++n, z += K) {
+                const double2 zz = *z, r = *(const double2 *)(wrad + 4 * n);
+                const double r2 = wrad[4 * n + 2];
+                a0.x += r.x * zz.x;
+                a0.y -= r.x * zz.y;
+                a1.x += r.y * zz.x;
+                a1.y -= r.y * zz.y;
+                a2.x += r2 * zz.x;
+                a2.y -= r2 * zz.y;
               }
-              const double C = ((m > 0) ? 2.0 : 1.0) * ((m & 1) ? -P.preflm64[k] : P.preflm64[k]);
-              const double q0 = C * g[Lg.Q + k], q1 = (m < l) ? C * g[Lg.Q + k + 1] : 0.0;
-              const dcx w0 = ldc(g + Lg.wp + 2 * (m + 2)), w1 = (double)m * ldc(g + Lg.wp + 2 * (m + 1));
-              const dcx Om = q0 * w0, Ot = q1 * w0, Ow = q0 * w1;
-              const double f0 = fourpi * g[Lg.F + l], f1 = fourpi * g[Lg.F1 + l];
               const dcx z0 = cx(f0 * a0.x, f0 * a0.y), z1 = cx(f0 * a1.x + f1 * a0.x, f0 * a1.y + f1 * a0.y);
-              if (full && part == 0) {
-                const double q2 = (m + 1 < l) ? C * g[Lg.Q + k + 2] : 0.0;
-                const dcx w2 = (double)(m * (m - 1)) * ldc(g + Lg.wp + 2 * m);
-                const double f2 = fourpi * g[Lg.F2 + l];
-                const dcx y = cx(f0 * a2.x + 2.0 * f1 * a1.x + f2 * a0.x - invr * z1.re,
-                                 f0 * a2.y + 2.0 * f1 * a1.y + f2 * a0.y - invr * z1.im);
-                acc[0] += y.re * Om.re - y.im * Om.im;
-                acc[1] += z1.re * Om.re - z1.im * Om.im;
-                acc[2] += z1.re * Ot.re - z1.im * Ot.im;
-                acc[3] += z1.re * Ow.re - z1.im * Ow.im;
-                acc[4] += z1.re * Ow.im + z1.im * Ow.re;
-                acc[5] += z0.re * Ot.re - z0.im * Ot.im;
-                acc[6] += z0.re * Ow.re - z0.im * Ow.im;
-                acc[7] += z0.re * Ow.im + z0.im * Ow.re;
-                const dcx Ott = q2 * w0, Otw = q1 * w1, Oww = q0 * w2;
-                acc[8] += z0.re * Ott.re - z0.im * Ott.im;
-                acc[9] += z0.re * Otw.re - z0.im * Otw.im;
-                acc[10] += z0.re * Otw.im + z0.im * Otw.re;
-                acc[11] += z0.re * Oww.re - z0.im * Oww.im;
-                acc[12] += z0.re * Oww.im + z0.im * Oww.re;
-              } else {
-                acc[0] += z1.re * Om.re - z1.im * Om.im;
-                acc[1] += z0.re * Ot.re - z0.im * Ot.im;
-                acc[2] += z0.re * Ow.re - z0.im * Ow.im;
-                acc[3] += z0.re * Ow.im + z0.im * Ow.re;
-              }
+              const double q2 = (m + 1 < l) ? C * gQ[k + 2] : 0.0, f2 = gF[3 * l + 2];
+              const double2 v2 = *(const double2 *)(gW + 2 * m);
+              const double mm = (double)(m * (m - 1)), invr = g[Lg.invr];
+              const dcx W2 = cx(mm * v2.x, mm * v2.y);
+              const dcx y = cx(f0 * a2.x + 2.0 * f1 * a1.x + f2 * a0.x - invr * z1.re,
+                               f0 * a2.y + 2.0 * f1 * a1.y + f2 * a0.y - invr * z1.im);
+              acc[0] += y.re * Om.re - y.im * Om.im;
+              acc[1] += z1.re * Om.re - z1.im * Om.im;
+              acc[2] += z1.re * Ot.re - z1.im * Ot.im;
+              acc[3] += z1.re * Ow.re - z1.im * Ow.im;
+              acc[4] += z1.re * Ow.im + z1.im * Ow.re;
+              acc[5] += z0.re * Ot.re - z0.im * Ot.im;
+              acc[6] += z0.re * Ow.re - z0.im * Ow.im;
+              acc[7] += z0.re * Ow.im + z0.im * Ow.re;
+              const dcx Ott = q2 * W0, Otw = q1 * W1, Oww = q0 * W2;
+              acc[8] += z0.re * Ott.re - z0.im * Ott.im;
+              acc[9] += z0.re * Otw.re - z0.im * Otw.im;
+              acc[10] += z0.re * Otw.im + z0.im * Otw.re;
+              acc[11] += z0.re * Oww.re - z0.im * Oww.im;
+              acc[12] += z0.re * Oww.im + z0.im * Oww.re;
             }
             // the lanes' sums: lane t of a half adds column t of its half's 16 rows
-            const bool wide = full && part == 0;
-            const int cols = wide ? kHessCols : 4;
+            const int cols = zg ? 12 : 13;
 #pragma unroll
             for (int t = 0; t < kHessCols; ++t)
-              if (t < 4 || wide) red[lane * kHessCols + t] = acc[t];
+              if (t < cols) red[lane * kHessCols + t] = acc[t];
             __syncwarp();
             if (pv && hl < cols) {
               double x = 0.0;
 #pragma unroll
               for (int r = 0; r < 16; ++r) x += red[(16 * half + r) * kHessCols + hl];
-              double *o = sums + (size_t)j * sp_sums + off + (part > 0 ? 13 + 4 * (part - 1) : 0) + hl;
+              double *o = sums + (size_t)j * sp_sums + off - (zg ? 0 : 13) + hl;
               *o = (code & 0x8000) ? x : *o + x;
             }
             __syncwarp();
           }
         }
       }
-      __syncthreads();  // vk is read
     }
+    __syncthreads();
     // ---- C: the normalisation (:1414-1484): t2 = p . dp_j, c12(b, a) = dp1(:, a) .
     // dp_j(:, b), u2 = w . dp_j.  Pairs the Hessian skips keep the zero blocks the
     // launcher cleared.
@@ -837,7 +903,7 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
 // Doubles per CTA, a multiple of 32 so that every CTA's region starts on a
 // 256-byte boundary.
 size_t hess_scratch_doubles(const DevParams &P) {
-  const size_t n = 6 * (size_t)P.n_max * P.k_max + 3 * (size_t)P.n_soap + 4 * (size_t)P.n_kept;
+  const size_t n = 6 * (size_t)P.n_max * P.k_max + 3 * (size_t)P.n_soap + 6 * (size_t)P.n_kept;
   return (n + 31) / 32 * 32;
 }
 
@@ -852,7 +918,7 @@ int hess_grid(const DevParams &P, int n_vec) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t sm = hess_smem_bytes(P, n_vec);
-  auto kern = hess_smem(P, n_vec).g_shared ? k64_hess<true> : k64_hess<false>;
+  auto kern = k64_hess;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return sms;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kHessThreads, sm);
   return sms * (per_sm > 0 ? per_sm : 1);
@@ -869,12 +935,14 @@ cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s
     for (int sp = 0; sp < P.n_species; ++sp) amax = amax > P.rad[sp].alpha ? amax : P.rad[sp].alpha;
     if (amax <= 8) k64_radial_d2<8><<<blocks, 128, 0, s>>>(P, B, rad_der2);
     else k64_radial_d2<16><<<blocks, 128, 0, s>>>(P, B, rad_der2);
-    k64_hgeo<<<blocks, 128, 0, s>>>(P, B, geo, good);
+    const size_t smg = 32 * sizeof(double) * (hess_geo_doubles(P) | 1);
+    CU_RET(cudaFuncSetAttribute(k64_hgeo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smg));
+    k64_hgeo<<<(B.n_pairs + 31) / 32, 32, smg, s>>>(P, B, geo, good);
     if (launches) *launches += 2;
   }
   if (B.n_sites > 0) {
     const size_t sm = hess_smem_bytes(P, n_vec);
-    auto kern = hess_smem(P, n_vec).g_shared ? k64_hess<true> : k64_hess<false>;
+    auto kern = k64_hess;
     CU_RET(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int g = grid < B.n_sites ? grid : B.n_sites;
     kern<<<g, kHessThreads, sm, s>>>(P, B, w.rad, w.rad_der, rad_der2, geo, good, (const double2 *)w.cnk, w.norm, soap,
