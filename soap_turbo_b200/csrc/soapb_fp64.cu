@@ -1023,31 +1023,351 @@ __global__ void __launch_bounds__(256, 2) k64_cart_site3(const DevParams P, cons
   }
 }
 
+// ---- soap_cart_der for a one-to-one compression map, n_max <= 32, l_max <= 8 and
+// n_soap <= 3 x 256.  A component o = (n, n', l) of a pair's column is
+//   x_c = pre [R_n T_c(n', l) + R_n' T_c(n, l) + e_c (R'_n P(n', l) + R'_n' P(n, l))] / |p|
+//         - s_o D_c,
+// with P and T_c the sums over m of c_nlm with the pair's angular expansion and with
+// its derivatives turned to Cartesian axis c (:837-887, 1927-2075), e the unit vector,
+// and D = sum_o s_o x_c / |p|^3 the normalisation's part, which needs no pass over the
+// components: it is the contraction of the pair's expansion with the weights z_nlm =
+// sum_n' Y(n, n', l) c_n'lm that the site's soap row spreads into (as soap_contract's H).
+// Radial values of other species are zero and their terms are skipped.
+// A CTA takes its site's pairs kC4Pairs at a time:
+//  * the next batch's angular planes and radial values are copied asynchronously
+//    into a second buffer, and its rotations formed, while a batch computes;
+//  * the derivative planes are rotated (a thread per pair and k); then two warps per
+//    pair sum P, T over m, lane n (c_nlm rows padded to 49, the (n, l) rows to 9, so
+//    that lanes fall in distinct banks), and form D, lanes over (plane, n);
+//  * the components CTA-wide, thread t owning o = t, t + 256, t + 512, which leave
+//    through a warp's shared buffer as contiguous stores and are summed for the self
+//    column in registers.
+// Few sites: `split` CTAs share a site; their sums for the self column are added in
+// order by the last of them to finish.
+// What bounds it: shared-memory reads and instruction issue beside the column
+// stores (24 n_soap bytes a pair).  Forming every derivative twice (once for D) from
+// spherical sums took 360 us for 22 k pairs of 621 components; see the launcher.
+constexpr int kC4Pairs = 4, kC4Kp = 49, kC4L1 = 9, kC4Threads = 256;
+struct Cart4Smem {
+  int C, Z, A, PT, R, rot, dot, out, total;
+};
+__host__ __device__ inline Cart4Smem cart4_smem(const DevParams &P) {
+  Cart4Smem L;
+  const int N = P.n_max, K = P.k_max;
+  int o = 0;  // the double2 arrays first, at even offsets
+  L.C = o;   o += 2 * N * kC4Kp;
+  L.Z = o;   o += 2 * N * kC4Kp;
+  L.A = o;   o += 2 * kC4Pairs * 8 * K;  // two buffers: this batch, the next
+  L.PT = o;  o += kC4Pairs * 4 * N * kC4L1;
+  L.R = o;   o += 2 * kC4Pairs * 2 * N;  // two buffers
+  L.rot = o; o += 2 * kC4Pairs * 8;      // two buffers
+  L.dot = o; o += kC4Pairs * 2 * 4;
+  L.out = o; o += kC4Threads * 3;
+  L.total = o;
+  return L;
+}
+
+template <int LC>
+__global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams P, const DevBatch B, const double *rad,
+                                                                const double *rad_der, const double2 *ang,
+                                                                const double2 *cnk, const double *soap_un,
+                                                                const double *norm, const double *self_init,
+                                                                double *cart, int split, double *parts, int *done) {
+  static_assert(LC + 1 == kC4L1 && kC4Pairs * 2 == kC4Threads / 32, "row length, two warps per pair");
+  constexpr int NT = kC4Threads, OPT = 3, L1 = LC + 1;
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int s_last;
+  const int site = blockIdx.x / split, part = blockIdx.x - site * split;
+  const int p0 = B.off[site], p1 = min(B.off[site + 1], B.n_pairs);
+  if (p1 <= p0) return;
+  const int N = P.n_max, K = P.k_max, ns = P.n_soap, w3 = 3 * ns, L = P.l_max;
+  // this CTA's pairs: a contiguous run of whole batches
+  const int n_batch = (p1 - p0 - 1 + kC4Pairs - 1) / kC4Pairs, per = (n_batch + split - 1) / split * kC4Pairs;
+  const int q0 = min(p1, p0 + 1 + part * per), q1 = min(p1, q0 + per);
+  const size_t plane = (size_t)B.n_pairs * K;
+  const Cart4Smem Ly = cart4_smem(P);
+  double2 *sC = (double2 *)(sm + Ly.C), *sZ = (double2 *)(sm + Ly.Z), *sA = (double2 *)(sm + Ly.A),
+          *sPT = (double2 *)(sm + Ly.PT);
+  double *sR = sm + Ly.R, *sRot = sm + Ly.rot, *sDot = sm + Ly.dot;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double *sOut = sm + Ly.out + warp * 96;
+  const double2 *c = cnk + (size_t)site * N * K;
+  const double *sv = soap_un + (size_t)site * ns;
+  const int szA = kC4Pairs * 4 * K, szR = kC4Pairs * 2 * N, NL = N * L1;
+
+  auto stage = [&](int b, int kb) {
+    const int nb = min(kC4Pairs, q1 - kb);
+    double2 *dA = sA + b * szA;
+    double *dR = sR + b * szR;
+    for (int t = tid; t < nb * 4 * K; t += NT) {
+      const int q = t / (4 * K), r = t - q * 4 * K, pl = r / K, kk = r - pl * K;
+      cp_async_16(dA + (q * 4 + pl) * K + kk, ang + pl * plane + (size_t)(kb + q) * K + kk);
+    }
+    for (int t = tid; t < nb * 2 * N; t += NT) {
+      const int q = t / (2 * N), r = t - q * 2 * N;
+      cp_async_8(dR + t, r < N ? rad + (size_t)(kb + q) * N + r : rad_der + (size_t)(kb + q) * N + r - N);
+    }
+    cp_async_commit();
+  };
+  auto rotation = [&](int b, int kb) {
+    const int j = tid - (NT - kC4Pairs);
+    if (j >= 0 && j < min(kC4Pairs, q1 - kb)) {
+      const int k = kb + j;
+      double st, ct, sf, cf;
+      sincos(B.thetas[k], &st, &ct);
+      sincos(B.phis[k], &sf, &cf);
+      const double ir = 1.0 / B.rjs[k];
+      double *rt = sRot + b * kC4Pairs * 8 + 8 * j;
+      rt[0] = st * cf; rt[1] = st * sf; rt[2] = ct;
+      rt[3] = -ct * cf * ir; rt[4] = -ct * sf * ir; rt[5] = st * ir;
+      rt[6] = -sf * ir; rt[7] = cf * ir;
+    }
+  };
+  if (q0 < q1) {
+    stage(0, q0);
+    rotation(0, q0);
+  }
+  for (int t = tid; t < N * K; t += NT) {
+    const int n = t / K, kk = t - n * K;
+    sC[n * kC4Kp + kk] = c[t];
+  }
+  __syncthreads();
+  // z_nlm, with the sum over m's factor 2 for m > 0
+  for (int t = tid; t < N * K; t += NT) {
+    const int n = t / K, kk = t - n * K, lm = __ldg((const int *)(P.blob + P.off_klm) + kk), l = lm & 0xff;
+    double2 z = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int i = P.hl_off[l * N + n]; i < P.hl_off[l * N + n + 1]; ++i) {
+      const int code = __ldg(P.hl_packed + i);
+      const double y = (code < 0 ? 2.0 : sqrt(2.0)) * sv[(code >> 8) & 0xffff];
+      const double2 v = sC[(code & 0xff) * kC4Kp + kk];
+      z.x += y * v.x;
+      z.y += y * v.y;
+    }
+    const double w = (lm >> 8) ? 2.0 : 1.0;
+    sZ[n * kC4Kp + kk] = make_double2(w * z.x, w * z.y);
+  }
+  const double nr = norm[site], inv_p = 1.0 / nr, inv_p3 = kFourPi64 / (nr * nr * nr);
+  // this thread's components: (n, l) and (n', l) in a pair's P, T rows and their species
+  int ia[OPT], ib[OPT], sa[OPT], sb[OPT];
+  double pre[OPT], so[OPT], self_[OPT][3];
+#pragma unroll
+  for (int j = 0; j < OPT; ++j) {
+    const int o = tid + j * NT;
+    const int code = o < ns ? P.kept_nnl[o] : 0;
+    const int n = code & 0xff, np = (code >> 8) & 0xff, l = code >> 16;
+    ia[j] = n * L1 + l;
+    ib[j] = np * L1 + l;
+    sa[j] = sb[j] = 0;
+    for (int s = 0; s < P.n_species; ++s) {
+      if (n >= P.rad[s].nbeg) sa[j] = s;
+      if (np >= P.rad[s].nbeg) sb[j] = s;
+    }
+    pre[j] = kFourPi64 * ((n == np) ? 1.0 : sqrt(2.0)) * inv_p;
+    so[j] = o < ns ? sv[o] : 0.0;
+    self_[j][0] = self_[j][1] = self_[j][2] = 0.0;
+  }
+
+  int buf = 0;
+  for (int kb = q0; kb < q1; kb += kC4Pairs, buf ^= 1) {
+    const int nb = min(kC4Pairs, q1 - kb);
+    __syncthreads();  // the previous batch's readers are done, buffer buf ^ 1 is free (and z is complete)
+    const bool more = kb + kC4Pairs < q1;
+    if (more) {
+      stage(buf ^ 1, kb + kC4Pairs);
+      cp_async_wait_1();
+    } else {
+      cp_async_wait_0();
+    }
+    __syncthreads();
+    double2 *cA = sA + buf * szA;
+    const double *cR = sR + buf * szR, *cRot = sRot + buf * kC4Pairs * 8;
+    // ---- radial, azimuthal and polar derivatives to x, y, z, in place
+    for (int t = tid; t < nb * K; t += NT) {
+      const int q = t / K;
+      double2 *A = cA + (q * 4 + 1) * K + t - q * K;
+      const double *rt = cRot + 8 * q;
+      const double2 r = A[0], a = A[K], o = A[2 * K];
+      A[0] = make_double2(rt[0] * r.x + rt[3] * o.x + rt[6] * a.x, rt[0] * r.y + rt[3] * o.y + rt[6] * a.y);
+      A[K] = make_double2(rt[1] * r.x + rt[4] * o.x + rt[7] * a.x, rt[1] * r.y + rt[4] * o.y + rt[7] * a.y);
+      A[2 * K] = make_double2(rt[2] * r.x + rt[5] * o.x, rt[2] * r.y + rt[5] * o.y);
+    }
+    if (more) rotation(buf ^ 1, kb + kC4Pairs);
+    __syncthreads();
+    {
+      const int q = warp >> 1, h = warp & 1;
+      if (q < nb) {
+        // ---- warp 2q + h, lane n: (P, T_x) or (T_y, T_z) of pair q
+        if (lane < N) {
+          const double2 *A0 = cA + (q * 4 + 2 * h) * K, *A1 = A0 + K, *cn = sC + lane * kC4Kp;
+          double2 *o = sPT + (q * 2 + h) * NL + lane * L1;
+#pragma unroll
+          for (int l = 0; l <= LC; ++l) {
+            double s0 = 0.0, s1 = 0.0;
+            if (l <= L) {
+#pragma unroll
+              for (int m = 0; m <= l; ++m) {
+                const int kk = l * (l + 1) / 2 + m;
+                const double w = (m == 0) ? 1.0 : 2.0;
+                const double2 cc = cn[kk], a0 = A0[kk], a1 = A1[kk];
+                s0 = s0 + w * (a0.x * cc.x + a0.y * cc.y);
+                s1 = s1 + w * (a1.x * cc.x + a1.y * cc.y);
+              }
+            }
+            o[l] = make_double2(s0, s1);
+          }
+        }
+        // ---- D's sums: lanes (plane, n), every second k
+        const int pl = lane >> 3;
+        const unsigned bits = B.bits[kb + q];
+        const double *R = cR + q * 2 * N + (pl ? 0 : N);
+        const double2 *A = cA + (q * 4 + pl) * K;
+        double d = 0.0;
+        for (int s = 0; s < P.n_species; ++s) {
+          if (!((bits >> s) & 1u)) continue;
+          const int n_end = P.rad[s].nbeg + P.rad[s].alpha;
+          for (int n = P.rad[s].nbeg + (lane & 7); n < n_end; n += 8) {
+            const double2 *zn = sZ + n * kC4Kp;
+            double t0 = 0.0, t1 = 0.0;
+#pragma unroll 4
+            for (int kk = h; kk < K; kk += 2) {
+              const double2 z = zn[kk], a = A[kk];
+              t0 += a.x * z.x;
+              t1 += a.y * z.y;
+            }
+            d += R[n] * (t0 + t1);
+          }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if ((lane & 7) == 0) sDot[(q * 2 + h) * 4 + pl] = d;
+      }
+    }
+    __syncthreads();
+    // ---- the columns
+#pragma unroll 1
+    for (int q = 0; q < nb; ++q) {
+      const unsigned bits = B.bits[kb + q];
+      const double *rt = cRot + 8 * q, *d0 = sDot + q * 8;
+      const double cx = rt[0], cy = rt[1], cz = rt[2], dA = d0[0] + d0[4];
+      const double dx = inv_p3 * (d0[1] + d0[5] + cx * dA), dy = inv_p3 * (d0[2] + d0[6] + cy * dA),
+                   dz = inv_p3 * (d0[3] + d0[7] + cz * dA);
+      const double2 *t0 = sPT + q * 2 * NL, *t1 = t0 + NL;
+      const double *R = cR + q * 2 * N;
+      double *col = cart + (size_t)(kb + q) * w3;
+#pragma unroll
+      for (int j = 0; j < OPT; ++j) {
+        const int ob = 3 * (j * NT + 32 * warp);  // the warp's first value
+        if (ob >= w3) continue;
+        double x = 0.0, y = 0.0, z = 0.0, e = 0.0;
+        if ((bits >> sa[j]) & 1u) {
+          const int n = ia[j] / L1;
+          const double r = R[n], rd = R[N + n];
+          const double2 u = t0[ib[j]], v = t1[ib[j]];
+          e = rd * u.x;
+          x = r * u.y;
+          y = r * v.x;
+          z = r * v.y;
+        }
+        if ((bits >> sb[j]) & 1u) {
+          const int n = ib[j] / L1;
+          const double r = R[n], rd = R[N + n];
+          const double2 u = t0[ia[j]], v = t1[ia[j]];
+          e += rd * u.x;
+          x += r * u.y;
+          y += r * v.x;
+          z += r * v.y;
+        }
+        x = pre[j] * (x + cx * e) - so[j] * dx;
+        y = pre[j] * (y + cy * e) - so[j] * dy;
+        z = pre[j] * (z + cz * e) - so[j] * dz;
+        self_[j][0] -= x;
+        self_[j][1] -= y;
+        self_[j][2] -= z;
+        __syncwarp();
+        sOut[3 * lane] = x;
+        sOut[3 * lane + 1] = y;
+        sOut[3 * lane + 2] = z;
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const int t = lane + 32 * i;
+          if (ob + t < w3) col[ob + t] = sOut[t];
+        }
+      }
+    }
+  }
+  // ---- the self column, from the caller's values on
+  const double *si = self_init ? self_init + (size_t)site * w3 : nullptr;
+  double *col = cart + (size_t)p0 * w3;
+  if (split > 1) {
+    double *mine = parts + (size_t)blockIdx.x * w3;
+#pragma unroll
+    for (int j = 0; j < OPT; ++j) {
+      const int o = tid + j * NT;
+      if (o < ns)
+        for (int cc = 0; cc < 3; ++cc) mine[3 * o + cc] = self_[j][cc];
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(done + site, 1) == split - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const double *all = parts + (size_t)site * split * w3;
+    for (int t = tid; t < w3; t += NT) {
+      double v = si ? si[t] : 0.0;
+      for (int i = 0; i < split; ++i) v += __ldcg(all + (size_t)i * w3 + t);
+      col[t] = v;
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < OPT; ++j) {
+    const int o = tid + j * NT;
+    if (o < ns)
+      for (int cc = 0; cc < 3; ++cc) col[3 * o + cc] = self_[j][cc] + (si ? si[3 * o + cc] : 0.0);
+  }
+}
+
 // ---- pair = sgn * sum_s G(i,s) soap_cart_der(:, s, k): one CTA per site with
-// the site's G row in shared memory, one warp per pair; lane j takes the
-// components o = j, j + 32, ... (a warp's three loads of a step cover 768
-// contiguous bytes of the column).
+// the site's G row in shared memory, a warp per pair.  The column (3, n_soap) is
+// read as it lies, 32 consecutive values per load: value t is component t % 3 of o =
+// t / 3, and three loads on the same (lane, component) pattern comes back, so each
+// lane keeps one sum per load of a triple.
+// What bounds it: the columns' bytes.  Three loads of every third value each, as
+// before, read every sector three times: 93 us for 22 k columns of 621 (331 MB).
 template <int NT>
 __global__ void __launch_bounds__(NT) k64_contract_site(const DevParams P, const DevBatch B, const double *cart,
-                                                        const double *G, int g_layout, double sgn,
+                                                        const double *G, int g_layout, double sgn, int split,
                                                         double *pair) {
   extern __shared__ double sG[];  // n_soap
-  const int site = blockIdx.x;
+  const int site = blockIdx.x / split, part = blockIdx.x - site * split;
   const int p0 = B.off[site], p1 = min(B.off[site + 1], B.n_pairs);
-  const int ns = P.n_soap;
+  const int ns = P.n_soap, w3 = 3 * ns;
   for (int o = threadIdx.x; o < ns; o += NT)
     sG[o] = g_layout == 0 ? G[(size_t)o * B.n_sites + site] : G[(size_t)site * ns + o];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k = p0 + warp; k < p1; k += NT / 32) {
-    const double *ck = cart + (size_t)k * 3 * ns;
-    double x = 0.0, y = 0.0, z = 0.0;
-    for (int o = lane; o < ns; o += 32) {
-      const double g = sG[o];
-      x += g * ck[3 * o];
-      y += g * ck[3 * o + 1];
-      z += g * ck[3 * o + 2];
+  const int o0 = lane / 3, o1 = (lane + 32) / 3, o2 = (lane + 64) / 3;
+  for (int k = p0 + part * (NT / 32) + warp; k < p1; k += split * (NT / 32)) {
+    const double *ck = cart + (size_t)k * w3 + lane;
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    int t = 0, o = 0;
+#pragma unroll 4
+    for (; t + 96 <= w3; t += 96, o += 32) {
+      a0 += sG[o + o0] * __ldcs(ck + t);
+      a1 += sG[o + o1] * __ldcs(ck + t + 32);
+      a2 += sG[o + o2] * __ldcs(ck + t + 64);
     }
+    if (t + lane < w3) a0 += sG[o + o0] * __ldcs(ck + t);
+    if (t + lane + 32 < w3) a1 += sG[o + o1] * __ldcs(ck + t + 32);
+    if (t + lane + 64 < w3) a2 += sG[o + o2] * __ldcs(ck + t + 64);
+    // load i of a triple holds component (lane + 2 i) % 3
+    const int m = lane % 3;
+    double x = m == 0 ? a0 : (m == 1 ? a1 : a2);
+    double y = m == 0 ? a2 : (m == 1 ? a0 : a1);
+    double z = m == 0 ? a1 : (m == 1 ? a2 : a0);
     for (int s = 16; s > 0; s >>= 1) {
       x += __shfl_xor_sync(0xffffffffu, x, s);
       y += __shfl_xor_sync(0xffffffffu, y, s);
@@ -1082,6 +1402,23 @@ constexpr size_t kCartSmemCap = 227 * 1024;
 size_t fp64_cart_smem(const DevParams &P) {
   const size_t staged = (size_t)cart_smem(P, true).total * sizeof(double);
   return staged <= kCartSmemCap ? staged : (size_t)cart_smem(P, false).total * sizeof(double);
+}
+
+// CTAs per site of k64_cart_site4 (two of which fit an SM): the share that leaves
+// the fewest pairs to the last wave, every further CTA of a site costing it about a
+// twelfth (the site's c_nlm and z again).
+int fp64_cart_split(const DevParams &P, int n_sites) {
+  const int slots = 2 * 148;
+  int best = 1;
+  double cost = 1e30;
+  for (int s = 1; s <= 4; ++s) {
+    const double waves = (double)(((long)n_sites * s + slots - 1) / slots) / s * (1.0 + 0.08 * (s - 1));
+    if (waves < cost) {
+      cost = waves;
+      best = s;
+    }
+  }
+  return P.cmap_identity ? best : 1;
 }
 
 cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaStream_t s,
@@ -1124,7 +1461,16 @@ cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaSt
   if (do_der && cart && np > 0 && nsites > 0) {
     const size_t sm2 = (size_t)cart2_smem(P).total * sizeof(double);
     const size_t sm3 = (size_t)cart3_smem(P).total * sizeof(double);
-    if (P.n_max <= 32 && P.l_max <= 8 && P.n_soap <= 3 * 256 && sm3 <= kCartSmemCap) {
+    const size_t sm4 = (size_t)cart4_smem(P).total * sizeof(double);
+    if (P.cmap_identity && P.n_max <= 32 && P.l_max <= 8 && P.n_soap <= 3 * kC4Threads && sm4 <= kCartSmemCap) {
+      auto kern = k64_cart_site4<8>;
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm4);
+      if (e != cudaSuccess) return e;
+      if (w.split > 1 && (e = cudaMemsetAsync(w.done, 0, sizeof(int) * (size_t)nsites, s)) != cudaSuccess) return e;
+      kern<<<nsites * w.split, kC4Threads, sm4, s>>>(P, B, w.rad, w.rad_der, (const double2 *)w.ang,
+                                                     (const double2 *)w.cnk, w.soap_unnorm, w.norm, self_init, cart,
+                                                     w.split, w.parts, w.done);
+    } else if (P.n_max <= 32 && P.l_max <= 8 && P.n_soap <= 3 * 256 && sm3 <= kCartSmemCap) {
       auto kern = k64_cart_site3<8>;
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
       if (e != cudaSuccess) return e;
@@ -1164,7 +1510,9 @@ cudaError_t launch_fp64_contract(const DevParams &P, const DevBatch &B, cudaStre
   auto kern = k64_contract_site<256>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  kern<<<B.n_sites, 256, sm, s>>>(P, B, cart, G, g_layout, sgn, pair);
+  // CTAs per site: the chip full, at 2048 threads per SM, where the sites are few
+  const int split = B.n_sites >= 148 * 4 ? 1 : (B.n_sites >= 148 * 2 ? 2 : 4);
+  kern<<<B.n_sites * split, 256, sm, s>>>(P, B, cart, G, g_layout, sgn, split, pair);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }

@@ -302,7 +302,7 @@ struct soapb_context {
   DBuf tables;
   // arena
   DBuf off, bits, err, keep_c, keep_norm, rad, ang;
-  DBuf f64_rad, f64_rad_der, f64_ang, f64_cnk, f64_soap_un, f64_norm;
+  DBuf f64_rad, f64_rad_der, f64_ang, f64_cnk, f64_soap_un, f64_norm, f64_parts, f64_done;
   // central-atom Hessian: second radial derivatives, pair geometry records and
   // flags, per-CTA scratch, the descriptor it recomputes, its work counter
   DBuf hs_rad_der2, hs_geo, hs_good, hs_scratch, hs_sums, hs_soap, hs_ticket, hs_vchunk, hs_hchunk;
@@ -346,8 +346,8 @@ struct soapb_context {
   ~soapb_context() {
     timing_release();
     for (DBuf *b : {&tables, &off, &bits, &err, &keep_c, &keep_norm, &order, &rad, &ang, &f64_rad, &f64_rad_der,
-                    &f64_ang, &f64_cnk, &f64_soap_un, &f64_norm, &hs_rad_der2, &hs_geo, &hs_good, &hs_scratch, &hs_sums, &hs_soap,
-                    &hs_ticket, &hs_vchunk, &hs_hchunk, &nb_acell, &nb_ccount, &nb_cstart,
+                    &f64_ang, &f64_cnk, &f64_soap_un, &f64_norm, &f64_parts, &f64_done, &hs_rad_der2, &hs_geo, &hs_good,
+                    &hs_scratch, &hs_sums, &hs_soap, &hs_ticket, &hs_vchunk, &hs_hchunk, &nb_acell, &nb_ccount, &nb_cstart,
                     &nb_cfill, &nb_catoms, &nb_counts, &nb_off, &nb_state, &nb_rjs, &nb_th, &nb_ph,
                     &nb_mask, &nb_natom, &nb_nneigh, &nb_species, &nb_smult})
       b->release();
@@ -1274,6 +1274,11 @@ int ctx_fp64(soapb_context *c, const soapb_batch *b, double *d_soap, double *d_c
   if ((rc = c->f64_norm.ensure(8 * ns))) return rc;
   Fp64Work w{c->f64_rad.as<double>(), c->f64_rad_der.as<double>(), c->f64_ang.as<double>(),
              c->f64_cnk.as<double>(), c->f64_soap_un.as<double>(), c->f64_norm.as<double>()};
+  if (do_der && (w.split = fp64_cart_split(P, b->n_sites)) > 1) {
+    if ((rc = c->f64_parts.ensure(24 * ns * w.split * c->n_soap)) || (rc = c->f64_done.ensure(4 * ns))) return rc;
+    w.parts = c->f64_parts.as<double>();
+    w.done = c->f64_done.as<int>();
+  }
   int nl = 0;
   CU(launch_fp64_descriptor(P, B, c->stream, w, do_der, d_soap, d_cart, &nl, accumulate ? d_soap : nullptr,
                             d_self_init));

@@ -237,7 +237,13 @@ struct Fp64Work {
   double *cnk;             // (n_sites, n_max, k_max) complex
   double *soap_unnorm;     // (n_sites, n_soap)
   double *norm;            // n_sites
+  // soap_cart_der by several CTAs per site (fp64_cart_split): their sums for the
+  // self column, (n_sites, split, 3 n_soap), and how many are done, n_sites
+  int split = 1;
+  double *parts = nullptr;
+  int *done = nullptr;
 };
+int fp64_cart_split(const DevParams &P, int n_sites);
 // soap_acc (may be null): the caller's soap, accumulated into before the norm
 // (compressed get_soap); self_init (may be null, with cart): the caller's self
 // columns of soap_cart_der, (3, n_soap) per site, which the self column
