@@ -1093,19 +1093,21 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
   double *sOut = sm + Ly.out + warp * 96;
   const double2 *c = cnk + (size_t)site * N * K;
   const double *sv = soap_un + (size_t)site * ns;
+  const int *klm = (const int *)(P.blob + P.off_klm);
+  const int PK = kC4Pairs * K, tq = tid / K;
   const int szA = kC4Pairs * 4 * K, szR = kC4Pairs * 2 * N, NL = N * L1;
 
+  // a batch's pairs lie side by side in every plane: a run per plane, no index to take apart
   auto stage = [&](int b, int kb) {
     const int nb = min(kC4Pairs, q1 - kb);
     double2 *dA = sA + b * szA;
     double *dR = sR + b * szR;
-    for (int t = tid; t < nb * 4 * K; t += NT) {
-      const int q = t / (4 * K), r = t - q * 4 * K, pl = r / K, kk = r - pl * K;
-      cp_async_16(dA + (q * 4 + pl) * K + kk, ang + pl * plane + (size_t)(kb + q) * K + kk);
-    }
-    for (int t = tid; t < nb * 2 * N; t += NT) {
-      const int q = t / (2 * N), r = t - q * 2 * N;
-      cp_async_8(dR + t, r < N ? rad + (size_t)(kb + q) * N + r : rad_der + (size_t)(kb + q) * N + r - N);
+    for (int t = tid; t < nb * K; t += NT)
+#pragma unroll
+      for (int pl = 0; pl < 4; ++pl) cp_async_16(dA + pl * kC4Pairs * K + t, ang + pl * plane + (size_t)kb * K + t);
+    for (int t = tid; t < nb * N; t += NT) {
+      cp_async_8(dR + t, rad + (size_t)kb * N + t);
+      cp_async_8(dR + kC4Pairs * N + t, rad_der + (size_t)kb * N + t);
     }
     cp_async_commit();
   };
@@ -1129,12 +1131,13 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
   }
   for (int t = tid; t < N * K; t += NT) {
     const int n = t / K, kk = t - n * K;
-    sC[n * kC4Kp + kk] = c[t];
+    const double2 v = c[t];
+    const double w = (__ldg(klm + kk) >> 8) ? 2.0 : 1.0;  // of m > 0 in the sums over m
+    sC[n * kC4Kp + kk] = make_double2(w * v.x, w * v.y);
   }
   __syncthreads();
-  // z_nlm, with the sum over m's factor 2 for m > 0
   for (int t = tid; t < N * K; t += NT) {
-    const int n = t / K, kk = t - n * K, lm = __ldg((const int *)(P.blob + P.off_klm) + kk), l = lm & 0xff;
+    const int n = t / K, kk = t - n * K, l = __ldg(klm + kk) & 0xff;
     double2 z = make_double2(0.0, 0.0);
 #pragma unroll 4
     for (int i = P.hl_off[l * N + n]; i < P.hl_off[l * N + n + 1]; ++i) {
@@ -1144,8 +1147,7 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
       z.x += y * v.x;
       z.y += y * v.y;
     }
-    const double w = (lm >> 8) ? 2.0 : 1.0;
-    sZ[n * kC4Kp + kk] = make_double2(w * z.x, w * z.y);
+    sZ[n * kC4Kp + kk] = z;
   }
   const double nr = norm[site], inv_p = 1.0 / nr, inv_p3 = kFourPi64 / (nr * nr * nr);
   // this thread's components: (n, l) and (n', l) in a pair's P, T rows and their species
@@ -1183,14 +1185,13 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
     double2 *cA = sA + buf * szA;
     const double *cR = sR + buf * szR, *cRot = sRot + buf * kC4Pairs * 8;
     // ---- radial, azimuthal and polar derivatives to x, y, z, in place
-    for (int t = tid; t < nb * K; t += NT) {
-      const int q = t / K;
-      double2 *A = cA + (q * 4 + 1) * K + t - q * K;
+    for (int t = tid, q = tq; t < nb * K; t += NT, q = t / K) {
+      double2 *A = cA + PK + t;
       const double *rt = cRot + 8 * q;
-      const double2 r = A[0], a = A[K], o = A[2 * K];
+      const double2 r = A[0], a = A[PK], o = A[2 * PK];
       A[0] = make_double2(rt[0] * r.x + rt[3] * o.x + rt[6] * a.x, rt[0] * r.y + rt[3] * o.y + rt[6] * a.y);
-      A[K] = make_double2(rt[1] * r.x + rt[4] * o.x + rt[7] * a.x, rt[1] * r.y + rt[4] * o.y + rt[7] * a.y);
-      A[2 * K] = make_double2(rt[2] * r.x + rt[5] * o.x, rt[2] * r.y + rt[5] * o.y);
+      A[PK] = make_double2(rt[1] * r.x + rt[4] * o.x + rt[7] * a.x, rt[1] * r.y + rt[4] * o.y + rt[7] * a.y);
+      A[2 * PK] = make_double2(rt[2] * r.x + rt[5] * o.x, rt[2] * r.y + rt[5] * o.y);
     }
     if (more) rotation(buf ^ 1, kb + kC4Pairs);
     __syncthreads();
@@ -1199,7 +1200,7 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
       if (q < nb) {
         // ---- warp 2q + h, lane n: (P, T_x) or (T_y, T_z) of pair q
         if (lane < N) {
-          const double2 *A0 = cA + (q * 4 + 2 * h) * K, *A1 = A0 + K, *cn = sC + lane * kC4Kp;
+          const double2 *A0 = cA + 2 * h * PK + q * K, *A1 = A0 + PK, *cn = sC + lane * kC4Kp;
           double2 *o = sPT + (q * 2 + h) * NL + lane * L1;
 #pragma unroll
           for (int l = 0; l <= LC; ++l) {
@@ -1208,10 +1209,11 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
 #pragma unroll
               for (int m = 0; m <= l; ++m) {
                 const int kk = l * (l + 1) / 2 + m;
-                const double w = (m == 0) ? 1.0 : 2.0;
                 const double2 cc = cn[kk], a0 = A0[kk], a1 = A1[kk];
-                s0 = s0 + w * (a0.x * cc.x + a0.y * cc.y);
-                s1 = s1 + w * (a1.x * cc.x + a1.y * cc.y);
+                s0 += a0.x * cc.x;
+                s1 += a1.x * cc.x;
+                s0 += a0.y * cc.y;
+                s1 += a1.y * cc.y;
               }
             }
             o[l] = make_double2(s0, s1);
@@ -1220,8 +1222,8 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
         // ---- D's sums: lanes (plane, n), every second k
         const int pl = lane >> 3;
         const unsigned bits = B.bits[kb + q];
-        const double *R = cR + q * 2 * N + (pl ? 0 : N);
-        const double2 *A = cA + (q * 4 + pl) * K;
+        const double *R = cR + q * N + (pl ? 0 : kC4Pairs * N);
+        const double2 *A = cA + pl * PK + q * K;
         double d = 0.0;
         for (int s = 0; s < P.n_species; ++s) {
           if (!((bits >> s) & 1u)) continue;
@@ -1253,7 +1255,7 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
       const double dx = inv_p3 * (d0[1] + d0[5] + cx * dA), dy = inv_p3 * (d0[2] + d0[6] + cy * dA),
                    dz = inv_p3 * (d0[3] + d0[7] + cz * dA);
       const double2 *t0 = sPT + q * 2 * NL, *t1 = t0 + NL;
-      const double *R = cR + q * 2 * N;
+      const double *R = cR + q * N, *Rd = R + kC4Pairs * N;
       double *col = cart + (size_t)(kb + q) * w3;
 #pragma unroll
       for (int j = 0; j < OPT; ++j) {
@@ -1262,7 +1264,7 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
         double x = 0.0, y = 0.0, z = 0.0, e = 0.0;
         if ((bits >> sa[j]) & 1u) {
           const int n = ia[j] / L1;
-          const double r = R[n], rd = R[N + n];
+          const double r = R[n], rd = Rd[n];
           const double2 u = t0[ib[j]], v = t1[ib[j]];
           e = rd * u.x;
           x = r * u.y;
@@ -1271,7 +1273,7 @@ __global__ void __launch_bounds__(kC4Threads, 2) k64_cart_site4(const DevParams 
         }
         if ((bits >> sb[j]) & 1u) {
           const int n = ib[j] / L1;
-          const double r = R[n], rd = R[N + n];
+          const double r = R[n], rd = Rd[n];
           const double2 u = t0[ia[j]], v = t1[ia[j]];
           e += rd * u.x;
           x += r * u.y;
