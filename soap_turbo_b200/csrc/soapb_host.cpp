@@ -733,6 +733,7 @@ int build_tables(soapb_context *c) {
   const int amax_t = (amax <= 8 && L <= 8) ? 8 : 16;
   const int KS = K | 1;
   std::vector<unsigned char> blob, blob_c;
+  std::vector<int> h_zero;
   auto put_in = [](std::vector<unsigned char> &b, const void *src, size_t bytes) {
     const size_t o = b.size();
     b.resize((o + bytes + 15) / 16 * 16, 0);
@@ -819,6 +820,16 @@ int build_tables(soapb_context *c) {
     for (auto &p : hw) hitem.push_back(p.second);
     P.n_hitem = (int)hitem.size();
     P.off_hitem = put_c(hitem.data(), hitem.size() * 4);
+    // H entries that no item writes: of empty lists, and past a species' alpha
+    for (int l = 0; l <= L; ++l)
+      for (int m = 0; m <= l; ++m)
+        for (int s = 0; s < c->n_species; ++s)
+          for (int n = 0; n < amax_t; ++n) {
+            const int li = l * N + P.rad[s].nbeg + n;
+            if (n >= c->alpha[s] || hl_off[li + 1] == hl_off[li])
+              h_zero.push_back(((l * (l + 1) / 2 + m) << 16) | (s * amax_t + n));
+          }
+    P.n_hzero = (int)h_zero.size();
     P.off_kept = put(kept_nnl.data(), kept_nnl.size() * 4);
     P.off_central = put(central.data(), central.size() * 8);
     P.off_hloff = put_c(hl_off.data(), hl_off.size() * 4);
@@ -931,6 +942,7 @@ int build_tables(soapb_context *c) {
   const size_t iBlob = add(blob.data(), blob.size());
   const size_t iBlobC = add(blob_c.data(), blob_c.size());
   const size_t iHp = add(hl_packed.data(), hl_packed.size() * 4);
+  const size_t iHz = add(h_zero.data(), h_zero.size() * 4);
   int rc = c->tables.ensure(total + 256);
   if (rc) return rc;
   std::vector<unsigned char> host(total + 256, 0);
@@ -959,6 +971,7 @@ int build_tables(soapb_context *c) {
   P.blob = (const unsigned char *)at(iBlob);
   P.blob_c = (const unsigned char *)at(iBlobC);
   P.hl_packed = (const int *)at(iHp);
+  P.h_zero = (const int *)at(iHz);
   P.rtab_coef = (const float *)at(iRt);
   P.n_soap = c->n_soap;
   P.n_kept = c->n_kept;
@@ -1123,12 +1136,12 @@ int pick_threads(const soapb_context *c) {
 }
 
 // Launch configuration of a site kernel: the caller's CTA size if set, else
-// the autotuner's choice for that kernel, else 128 threads on the occupancy grid.
+// the autotuner's choice for that kernel, else 0: the launcher's rule.
 LaunchCfg site_cfg(const soapb_context *c, bool contract) {
   if (c->threads) return LaunchCfg{pick_threads(c), c->stream, c->max_ctas};
   const int t = contract ? c->tune_tc : c->tune_td;
   if (t) return LaunchCfg{t, c->stream, contract ? c->tune_cc : c->tune_cd};
-  return LaunchCfg{128, c->stream, c->max_ctas};
+  return LaunchCfg{0, c->stream, c->max_ctas};
 }
 
 // Status of the inputs from the prep error word a launch left (see soapb_scan.cuh).

@@ -77,6 +77,8 @@ struct DevParams {
   const int *hl_q;
   const float *hl_fac;
   const double *hl_fac64;
+  const int *h_zero;      // n_hzero: the (k << 16 | species amax_t + local index) of H that no H item writes
+  int n_hzero;
   // Per-CTA constants of the mixed kernels: two blobs copied into shared
   // memory with 16-byte loads, one for the pair and descriptor kernels
   // (blob: W blocks, then from off_rad on the descriptor's part) and one for
@@ -158,9 +160,10 @@ struct DevBatch {
 // Kernel launchers (soapb_mixed.cu, soapb_fp64.cu)
 namespace soapb {
 struct LaunchCfg {
-  int threads;           // threads per site CTA
+  int threads;           // 64, 128 or 256: threads per site of the contract, and the pairs whose entries the
+                         // descriptor sorts and groups together; 0: the launcher's rule, and 128 pairs
   cudaStream_t stream;
-  int max_ctas;          // persistent grid cap (0 = from the occupancy)
+  int max_ctas;          // grid cap (0: one CTA per site)
 };
 cudaError_t launch_prep(const DevParams &P, const DevBatch &B, cudaStream_t s);
 // sites per tile of the CSR offset scan (soapb_scan.cuh)
@@ -185,7 +188,6 @@ cudaError_t launch_contract(const DevParams &P, const DevBatch &B, const LaunchC
 // Device address and size of the static scratch array (soapb_noalloc.cu);
 // `device` must be current.
 cudaError_t noalloc_scratch(int device, unsigned char **addr, size_t *bytes);
-size_t contract_smem(const DevParams &P, int threads);
 size_t contract_tc_smem(const DevParams &P);  // dynamic shared memory of the tensor-core contract
 
 // Error codes reported through an error word (kErrTop - code under atomicMax,

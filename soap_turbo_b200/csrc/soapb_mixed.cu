@@ -417,26 +417,7 @@ __global__ void __launch_bounds__(kPairThreads)
 }
 
 // ------------------------------------------------------------ layouts
-// Shared memory of the site kernels (bytes); host and device agree on it.
-// The site part of the constants blob (species constants, per-k tables, item
-// maps, kept components, Y lists) comes first.  Region X holds the per-round
-// entry staging; outside the chunk loop the same bytes hold per-site arrays.
-struct Layout {
-  size_t red, ent, wcnt, misc;
-  size_t C64, H, Rot, F;
-  size_t X;
-  size_t R, Rd, A;       // staging inside X
-  size_t C, P, S;        // per-site arrays inside X
-  size_t total;
-};
-
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-// entries whose rows are staged in shared memory at a time: half the CTA, at
-// most 64 for the descriptor (mode 0) and 32 for the contract (mode 1), whose
-// longer staged rows would otherwise cost it a CTA per SM
-__host__ __device__ constexpr int stage_entries_per_round(int NT, int mode) {
-  return NT / 2 < (mode ? 32 : 64) ? NT / 2 : (mode ? 32 : 64);
-}
 // Staged rows are longer than the global ones and stay 16-byte aligned for the
 // asynchronous copies.  The contract (mode 1) pads by 16 floats so that its two
 // half-warps, which read neighbouring rows at the same offsets, use disjoint
@@ -445,7 +426,7 @@ __host__ __device__ inline int stage_stride(int LC, int mode) { return row_len(L
 // row stride of H: the species blocks padded to AMAX, plus 4 so that 128-bit
 // loads of consecutive k rows fall in distinct banks
 __host__ __device__ inline int h_stride(int n_species, int AMAX) { return n_species * AMAX + 4; }
-// floats per site of the kept c_nlm, padded to a multiple of 4 so that every
+// floats per site of the kept c_nlm, (n, k_max | 1) of (re, im), padded to a multiple of 4 so that every
 // site's block starts 16-byte aligned
 __host__ __device__ inline size_t keep_stride(const DevParams &P) {
   return ((size_t)2 * P.n_max * (size_t)(P.k_max | 1) + 3) / 4 * 4;
@@ -453,41 +434,6 @@ __host__ __device__ inline size_t keep_stride(const DevParams &P) {
 // bytes of constants a site kernel keeps in shared memory (mode 0 descriptor, 1 contract)
 __host__ __device__ inline size_t site_blob_bytes(const DevParams &P, int mode) {
   return mode ? (size_t)P.blob_c_bytes : (size_t)(P.blob_bytes - P.off_rad);
-}
-
-__host__ __device__ inline Layout make_layout(const DevParams &P, int NT, int AMAX, int LC, int mode) {
-  Layout L{};
-  const size_t KS = (size_t)(P.k_max | 1);
-  const size_t nsp = (size_t)P.n_species, CH = (size_t)stage_entries_per_round(NT, mode);
-  const size_t nC = 2 * (size_t)P.n_max * KS;
-  size_t o = site_blob_bytes(P, mode);
-  L.red = o;  o += 40 * sizeof(double);
-  L.ent = o;  o += (size_t)NT * nsp * sizeof(int);
-  L.wcnt = o; o += (size_t)SOAPB_MAX_SPECIES * (NT / 32) * sizeof(int);
-  L.misc = o; o += 64 * sizeof(int);
-  o = align_up(o, 16);
-  if (mode == 0) {
-    L.C64 = o; o += nC * sizeof(double);
-  } else {
-    L.H = o;   o += 2 * KS * (size_t)h_stride(P.n_species, AMAX) * sizeof(float);
-    L.Rot = o; o += (size_t)NT * 4 * sizeof(float);
-    L.F = o;   o += (size_t)NT * nsp * 3 * sizeof(float);
-  }
-  o = align_up(o, 16);
-  L.X = o;
-  size_t x = o;
-  L.R = x; x += CH * AMAX * sizeof(float);
-  if (mode == 1) { L.Rd = x; x += CH * AMAX * sizeof(float); }
-  L.A = x; x += CH * (size_t)stage_stride(LC, mode) * sizeof(float);
-  const size_t end_stage = x;
-  x = o;
-  L.C = x; x += nC * sizeof(float);
-  L.P = x; x += (size_t)P.n_kept * sizeof(float);
-  L.S = x; x += (size_t)P.n_soap * sizeof(float);
-  const size_t end_site = x;
-  o = end_stage > end_site ? end_stage : end_site;
-  L.total = align_up(o, 16);
-  return L;
 }
 
 template <int NT>
@@ -742,10 +688,8 @@ __device__ __forceinline__ void site_output(const DevParams &P, unsigned char *s
     else
       for (int o = tid; o < P.n_soap; o += NT) out[o] = (double)sS[o] * inv;
     if (keep & 1) {
-      float *kc = keep_c + (size_t)site * keep_stride(P);
-      const int n4 = (2 * n_max * KS) / 4;
-      for (int t = tid; t < n4; t += NT) ((float4 *)kc)[t] = ((const float4 *)sC)[t];
-      for (int t = 4 * n4 + tid; t < 2 * n_max * KS; t += NT) kc[t] = sC[t];
+      float2 *kc = (float2 *)(keep_c + (size_t)site * keep_stride(P));
+      for (int t = tid; t < n_max * KS; t += NT) kc[t] = make_float2(sC[t], sC[n_max * KS + t]);
       if (tid == 0) keep_norm[site] = norm;
     }
 }
@@ -878,7 +822,7 @@ __global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AM
   float *sX = (float *)(smem + Ly.X), *sP = (float *)(smem + Ly.P), *sS = (float *)(smem + Ly.S);
   int *sBase = (int *)(smem + Ly.base);
   unsigned short *list = (unsigned short *)(smem + Ly.list);
-  const int KS = P.k_max | 1, n_max = P.n_max, nsp = P.n_species;
+  const int KS = P.k_max | 1, nsp = P.n_species;
   const int k_of = 32 * (warp % kw) + lane, n0 = NH * (warp / kw);
   const bool own = k_of < P.k_max;
   const int kk = own ? k_of : P.k_max - 1;  // the last lanes repeat the last k and store nothing
@@ -912,7 +856,7 @@ __global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AM
     // for the last, and that of the last
     int cs = 0, n_rounds = 0;
     double tr[NH], ti[NH], dr[NH], di[NH];
-    float *kc = keep_c + ((keep & 1) ? (size_t)site * keep_stride(P) + kk : 0);
+    float2 *kc = (float2 *)(keep_c + ((keep & 1) ? (size_t)site * keep_stride(P) : 0)) + kk;
     auto finish = [&]() {  // species cs is complete
       const int a = P.rad[cs].alpha, nb = P.rad[cs].nbeg;
       if (n_rounds != 1)
@@ -936,13 +880,10 @@ __global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AM
         for (int n = 0; n < NH; ++n)
           if (n0 + n < a) cc[n * KS] = make_float2((float)dr[n], (float)di[n]);
       if (own && (keep & 1)) {
-        float *kr = kc + (nb + n0) * KS, *ki = kr + n_max * KS;
+        float2 *kr = kc + (nb + n0) * KS;
 #pragma unroll
         for (int n = 0; n < NH; ++n)
-          if (n0 + n < a) {
-            kr[n * KS] = (float)dr[n];
-            ki[n * KS] = (float)di[n];
-          }
+          if (n0 + n < a) kr[n * KS] = make_float2((float)dr[n], (float)di[n]);
       }
       ++cs;
       n_rounds = 0;
@@ -1450,303 +1391,413 @@ __global__ void __launch_bounds__(NT) k_descriptor_tc(const DevParams P, const D
 }
 
 // ------------------------------------------------------------ contract
+// One CTA of a few warps per site.
+//  G -> Gp -> Gu -> H  as the reference (src/soap_turbo.f90:1783-1835); H(n, k) to
+//             shared memory as (re, im) pairs
+//  entries    (pair, species) by species, two at a time to a warp, a half-warp
+//             each, lane hl over k = hl + 16 j; the rows come two entries ahead
+//             into the warp's own buffer by asynchronous copies, so that no barrier
+//             stands between the entries
+//  contraction  U = sum_n R'_n H(n, k), V = sum_n R_n H(n, k), H in registers from a
+//             species' first entry to its last where they hold it (AMAX 8, three k a
+//             lane); the k summed over the lanes
+//  pairs      their entries added, rotated to Cartesian; the self pair minus their sum
+// What bounds it: instructions (16 k per site of 58 pairs and one species), issued at
+// 59 % of the rate by 16 warps per SM.  The kernel before (one CTA of 128 threads,
+// 32 staged entries behind barriers, H read from shared memory for every entry)
+// took 439 us at 16384 sites of one species and 66 at 1679 of three; this one 313 and 62.
+struct ContractLayout {
+  size_t H, base, list, slot, red, X, C, Gu, Gp, F, stage, total;
+};
+constexpr int kContractChunk = 128;  // pairs whose entries are listed at a time
+// a staged entry: the row, then R_n and dR_n/dr, padded so that the two half-warps'
+// rows lie in disjoint halves of the banks
+__host__ __device__ constexpr int contract_stride(int AMAX, int LC) {
+  return (row_len(LC) + 2 * AMAX + 15) / 32 * 32 + 16;
+}
+// row of H: the species' blocks of AMAX (re, im) and a pad that spreads the k rows over the banks
+__host__ __device__ inline int contract_h_stride(const DevParams &P, int AMAX) { return P.n_species * AMAX + 2; }
+__host__ __device__ inline ContractLayout contract_layout(const DevParams &P, int threads, int AMAX, int LC) {
+  ContractLayout L{};
+  const size_t KS = (size_t)(P.k_max | 1), nsp = (size_t)P.n_species;
+  size_t o = 0;
+  L.H = o;    o += KS * (size_t)contract_h_stride(P, AMAX) * sizeof(float2);
+  o = align_up(o, 16);
+  L.red = o;  o += 40 * sizeof(double);
+  L.base = o; o += 16 * sizeof(int);
+  L.list = o; o += kContractChunk * nsp * sizeof(unsigned short);
+  L.slot = o; o += kContractChunk * nsp * sizeof(short);
+  o = align_up(o, 16);
+  // the site's c_nlm, Gp and Gu; then the entries' rows and sums
+  L.X = L.C = o;
+  size_t x = o + ((size_t)P.n_max * KS + 2) * sizeof(float2);  // H items read up to two values past the end
+  L.Gp = x;   x += (size_t)P.n_soap * sizeof(float);
+  L.Gu = x;   x += (P.cmap_identity ? 0 : (size_t)P.n_kept) * sizeof(float);
+  L.stage = o;
+  size_t y = o + (size_t)(threads / 32) * 4 * contract_stride(AMAX, LC) * sizeof(float);
+  L.F = y;    y += kContractChunk * nsp * 3 * sizeof(float);
+  L.total = align_up(x > y ? x : y, 16);
+  return L;
+}
+
 constexpr int kHM = 3;  // m values per H item (the host's items must agree)
 
-template <int NT, int AMAX, int LC>
-__global__ void __launch_bounds__(NT, 512 / NT) k_contract(const DevParams P, const DevBatch B,
-                                                    const double *__restrict__ soap_in,
-                                                    const double *__restrict__ G, int g_layout,
-                                                    double sgn, const float *__restrict__ keep_c,
-                                                    const double *__restrict__ keep_norm,
-                                                    double *__restrict__ pair_out) {
+template <int AMAX, int LC>
+__global__ void __launch_bounds__(256, 2)
+    k_contract(const DevParams P, const DevBatch B, const double *__restrict__ soap_in, const double *__restrict__ G,
+               int g_layout, double sgn, const float *__restrict__ keep_c, const double *__restrict__ keep_norm,
+               double *__restrict__ pair_out) {
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr int CH = stage_entries_per_round(NT, 1);
-  constexpr int KC = (LC + 1) * (LC + 2) / 2;
-  constexpr int KJ = (KC + 15) / 16;
-  constexpr int GPT = 8;  // G values a thread holds while the norm dot product is reduced
-  static_assert(AMAX % 4 == 0, "vector loads of H need AMAX % 4 == 0");
-  const int AS = stage_stride(LC, 1);
-  constexpr int O_IL = row_il(LC), O_ILD = row_ild(LC), O_E = row_e(LC),
-                O_SF = row_sf(LC), O_X = row_x(LC), O_SQ = row_sq(LC),
-                O_P = row_p(LC);
-  const Layout Ly = make_layout(P, NT, AMAX, LC, 1);
-  const int4 *kidx = (const int4 *)SBLOBC(off_kidx);
-  const float4 *kcoef = (const float4 *)SBLOBC(off_kcoef);
-  const int *klm = (const int *)SBLOBC(off_klm_c);
-  const int *nmap = (const int *)SBLOBC(off_nmap);
-  const int *hitem = (const int *)SBLOBC(off_hitem);
-  const int *hloff = (const int *)SBLOBC(off_hloff);
-  const int *hl = P.hl_in_blob ? (const int *)SBLOBC(off_hl) : P.hl_packed;
+  constexpr int AW = row_len(LC), ST = contract_stride(AMAX, LC);
+  constexpr int KC = (LC + 1) * (LC + 2) / 2, KJ = (KC + 15) / 16;
+  constexpr bool HREG = AMAX * KJ <= 24;  // the lane's H of a species fits its registers
+  constexpr int GPT = 5;  // G values a thread holds while the norm dot product is reduced
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+  const int half = lane >> 4, hl = lane & 15, n_acc = 8 / nw;
+  const ContractLayout Ly = contract_layout(P, nt, AMAX, LC);
+  float2 *sH = (float2 *)(smem + Ly.H);
   double *sRed = (double *)(smem + Ly.red);
-  float *sH = (float *)(smem + Ly.H);
-  float *sRot = (float *)(smem + Ly.Rot);
-  float *sF = (float *)(smem + Ly.F);
-  float *sC = (float *)(smem + Ly.C);
-  float *sGu = (float *)(smem + Ly.P);
-  float *sGp = (float *)(smem + Ly.S);
-  float *sR = (float *)(smem + Ly.R);
-  float *sRd = (float *)(smem + Ly.Rd);
-  float *sA = (float *)(smem + Ly.A);
-  int *sEnt = (int *)(smem + Ly.ent);
-  int *sW_cnt = (int *)(smem + Ly.wcnt);
-  int *sMisc = (int *)(smem + Ly.misc);
-  int *sBase = sMisc, *sCnt = sMisc + SOAPB_MAX_SPECIES, *sNent = sMisc + 2 * SOAPB_MAX_SPECIES;
-  int *sSite = sMisc + 3 * SOAPB_MAX_SPECIES;
+  int *sBase = (int *)(smem + Ly.base);
+  unsigned short *list = (unsigned short *)(smem + Ly.list);
+  short *slot = (short *)(smem + Ly.slot);
+  float2 *sC = (float2 *)(smem + Ly.C);
+  float *sGp = (float *)(smem + Ly.Gp), *sGu = P.cmap_identity ? sGp : (float *)(smem + Ly.Gu);
+  float *sF = (float *)(smem + Ly.F), *stage = (float *)(smem + Ly.stage) + (size_t)warp * 4 * ST;
+  const int KS = P.k_max | 1, HS = contract_h_stride(P, AMAX);
+  const int n_max = P.n_max, k_max = P.k_max, n_soap = P.n_soap, nsp = P.n_species, n_sites = B.n_sites;
+  const int *klm = (const int *)(P.blob + P.off_klm);
+  const int *hitem = (const int *)(P.blob_c + P.off_hitem), *nmap = (const int *)(P.blob_c + P.off_nmap);
+  const int n_run = B.site_hi - B.site_lo;
 
-  const int tid = threadIdx.x;
-  const int KS = P.k_max | 1;
-  const int HS = h_stride(P.n_species, AMAX);
-  const size_t HPL = (size_t)KS * HS;  // H plane (re, then im)
-  const int n_max = P.n_max, k_max = P.k_max, n_soap = P.n_soap, nsp = P.n_species;
-  const int n_sites = B.n_sites;
-  const int hw = tid >> 4, hl16 = tid & 15;
-  float *sGu_eff = P.cmap_identity ? sGp : sGu;
+  // the lane's k: where its values stand in a row, and the derivative forms'
+  // coefficients (src/soap_turbo_angular.f90:194-246; a form that an (l, m) lacks has
+  // coefficient 0 and reads a neighbouring value)
+  int oP[KJ], oX[KJ], oL[KJ], oE[KJ];
+  float4 cf[KJ];
+#pragma unroll
+  for (int j = 0; j < KJ; ++j) {
+    const int k = hl + 16 * j, kk = k < k_max ? k : 0, lm = __ldg(klm + kk), l = lm & 0xff, m = lm >> 8;
+    oP[j] = row_p(LC) + kk;
+    oX[j] = row_p(LC) + kk + (m ? -1 : 1);
+    oL[j] = l;
+    oE[j] = row_e(LC) + 2 * m;
+    cf[j] = k < k_max ? __ldg((const float4 *)(P.blob_c + P.off_kcoef) + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  // the pieces (16 bytes) of two entries' rows that the lane stages
+  constexpr int NPC = (AW + 2 * AMAX) / 4, NC = (2 * NPC + 31) / 32;
+  struct {
+    bool on, rad;
+    int second, first, dst;
+    unsigned per_pair, per_species;
+  } piece[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int t = lane + 32 * c, p = t >= NPC ? t - NPC : t;
+    piece[c].on = t < 2 * NPC;
+    piece[c].second = t >= NPC ? 1 : 0;
+    piece[c].rad = p >= AW / 4;
+    piece[c].first = 4 * (p >= AW / 4 ? p - AW / 4 : p);
+    piece[c].dst = piece[c].second * ST + 4 * p;
+    piece[c].per_pair = p >= AW / 4 ? nsp * 2 * AMAX : AW;
+    piece[c].per_species = p >= AW / 4 ? 2 * AMAX : 0;
+  }
 
-  copy_site_blob<NT>(P, smem, 1);
-  for (int t = tid; t < 2 * (int)HPL; t += NT) sH[t] = 0.f;  // entries no item writes stay 0
-  first_site(B, B.ticket + 1, sSite);
-  for (;;) {
-    const int site = sSite[0];
-    if (site >= B.site_hi) break;
-    const int p_begin = sSite[1];
-    const int p_end = min(sSite[2], B.n_pairs);
-    int nx = 0, nx0 = 0, nx1 = 0;
-    if (tid == 0) nx = take_ticket(B, B.ticket + 1);  // the next site, fetched ahead
-    // ---- every per-site load is issued here, so their latencies overlap
+  for (int b = blockIdx.x; b < n_run; b += gridDim.x) {
+    const int site = B.order ? B.order[b] : B.site_lo + b;
+    const int p_begin = B.off[site], p_end = min(B.off[site + 1], B.n_pairs);
     const double knorm = keep_norm[site];
     const double *q = soap_in + (size_t)site * n_soap;
+    const double *g = g_layout == 0 ? G + site : G + (size_t)site * n_soap;
+    const size_t gs = g_layout == 0 ? (size_t)n_sites : 1;
     double gv[GPT], qv[GPT];
 #pragma unroll
     for (int j = 0; j < GPT; ++j) {
-      const int o = tid + j * NT;
+      const int o = tid + j * nt;
       gv[j] = qv[j] = 0.0;
       if (o < n_soap) {
-        gv[j] = g_layout == 0 ? G[(size_t)o * n_sites + site] : G[(size_t)site * n_soap + o];
+        gv[j] = g[o * gs];
         qv[j] = q[o];
       }
     }
     {
       const float *kc = keep_c + (size_t)site * keep_stride(P);
       const int n4 = (2 * n_max * KS) / 4;
-      for (int t = tid; t < n4; t += NT) cp_async16(sC + 4 * t, kc + 4 * t);
-      for (int t = 4 * n4 + tid; t < 2 * n_max * KS; t += NT) sC[t] = kc[t];
-      cp_async_wait_all();
+      for (int t = tid; t < n4; t += nt) cp_async16((float *)sC + 4 * t, kc + 4 * t);
+      for (int t = 4 * n4 + tid; t < 2 * n_max * KS; t += nt) ((float *)sC)[t] = kc[t];
     }
-    // ---- back through the normalisation (src/soap_turbo.f90:1783-1790)
+    // ---- back through the normalisation (src/soap_turbo.f90:1783-1790): q . G as 256
+    // sums over o = v, v + 256, .., a thread's 256 / nt of them apart, then added in
+    // one order: the result does not depend on the CTA size
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int j = 0; j < GPT; ++j) {
+      const double v = qv[j] * gv[j];
+      if (n_acc == 4) acc[j & 3] += v;
+      else if (n_acc == 2) acc[j & 1] += v;
+      else acc[0] += v;
+    }
+    for (int o = tid + GPT * nt, j = GPT; o < n_soap; o += nt, ++j) {
+      const double v = q[o] * g[o * gs];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i == (j & (n_acc - 1))) acc[i] += v;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i < n_acc) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        if (lane == 0) sRed[warp + i * nw] = acc[i];
+      }
+    __syncthreads();
     double qg = 0.0;
 #pragma unroll
-    for (int j = 0; j < GPT; ++j) qg += qv[j] * gv[j];
-    for (int o = tid + GPT * NT; o < n_soap; o += NT) {
-      const double g = g_layout == 0 ? G[(size_t)o * n_sites + site] : G[(size_t)site * n_soap + o];
-      sGp[o] = (float)g;  // staged raw; finished below
-      qg += q[o] * g;
-    }
-    qg = block_sum<NT>(qg, sRed);
+    for (int w = 0; w < 8; ++w) qg += sRed[w];
     const double inv = 1.0 / knorm;
 #pragma unroll
     for (int j = 0; j < GPT; ++j) {
-      const int o = tid + j * NT;
+      const int o = tid + j * nt;
       if (o < n_soap) sGp[o] = (float)((gv[j] - qv[j] * qg) * inv);
     }
-    for (int o = tid + GPT * NT; o < n_soap; o += NT) sGp[o] = (float)(((double)sGp[o] - q[o] * qg) * inv);
+    for (int o = tid + GPT * nt; o < n_soap; o += nt) sGp[o] = (float)((g[o * gs] - q[o] * qg) * inv);
+    cp_async_wait_all();
     __syncthreads();
     // ---- back through the compression (:1791-1798), unless it is one-to-one
     if (!P.cmap_identity) {
-      for (int t = tid; t < P.n_kept; t += NT) {
+      for (int t = tid; t < P.n_kept; t += nt) {
         float v = 0.f;
         for (int e = P.pj_off[t]; e < P.pj_off[t + 1]; ++e) v += P.pj_el[e] * sGp[P.pj_o[e]];
         sGu[t] = v;
       }
       __syncthreads();
     }
-    // ---- H(k,n) = w(m) sum_np Y(n,np,l) c(k,np) over the non-zero Y (:1800-1835);
-    // one item per (n, l, m0) walks its Y list once for m = m0 .. m0 + kHM - 1
-    // (up to l); the host orders the items heaviest first.  Every H entry an
-    // item writes is rewritten at every site; the others stay 0.
-    for (int it = tid; it < P.n_hitem; it += NT) {
-      const int code = hitem[it];
-      const int n = code & 0xff, l = (code >> 8) & 0xff, m0 = code >> 16;
-      const int kb = l * (l + 1) / 2 + m0, mn = min(kHM, l + 1 - m0);
-      float hr[kHM], hi[kHM];
+    // ---- H(k,n) = w(m) sum_np Y(n,np,l) c(k,np) over the non-zero Y (:1800-1835); an
+    // item per (n, l, m0) walks its Y list once for up to kHM values of m, the
+    // longest lists first
+    for (int it = tid; it < P.n_hitem; it += nt) {
+      const int code = __ldg(hitem + it), n = code & 0xff, l = (code >> 8) & 0xff, m0 = code >> 16;
+      const int kb = l * (l + 1) / 2 + m0, mn = min(kHM, l + 1 - m0), li = l * n_max + n;
+      const int t1 = __ldg(P.hl_off + li + 1);
+      float2 h[kHM];
 #pragma unroll
-      for (int j = 0; j < kHM; ++j) hr[j] = hi[j] = 0.f;
-      const int li = l * n_max + n;
-      for (int t = hloff[li]; t < hloff[li + 1]; ++t) {
-        const int e = hl[t];
-        const int np = e & 0xff, qq = (e >> 8) & 0xffff;
-        const float y = ((e >> 31) ? 2.f : 1.41421356237309504880f) * sGu_eff[qq];
-        const float *cr = sC + (size_t)np * KS + kb;
-        const float *ci = cr + (size_t)n_max * KS;
+      for (int j = 0; j < kHM; ++j) h[j] = make_float2(0.f, 0.f);
+      const float2 *cb = sC + kb;
+#pragma unroll 2
+      for (int t = __ldg(P.hl_off + li); t < t1; ++t) {
+        const int e = __ldg(P.hl_packed + t);
+        const float y = (e < 0 ? 2.f : 1.41421356237309504880f) * sGu[(e >> 8) & 0xffff];
+        // past the last m the values belong to the next l, or to the next array: read, not stored
+        const float2 *c = cb + (e & 0xff) * KS;
 #pragma unroll
         for (int j = 0; j < kHM; ++j) {
-          if (j < mn) {
-            hr[j] = fmaf(y, cr[j], hr[j]);
-            hi[j] = fmaf(y, ci[j], hi[j]);
-          }
+          h[j].x = fmaf(y, c[j].x, h[j].x);
+          h[j].y = fmaf(y, c[j].y, h[j].y);
         }
       }
-      const int nm = nmap[n];
-      const int col = (nm & 0xff) * AMAX + (nm >> 8);
+      const int nm = __ldg(nmap + n);
+      float2 *o = sH + kb * HS + (nm & 0xff) * AMAX + (nm >> 8);
 #pragma unroll
-      for (int j = 0; j < kHM; ++j) {
+      for (int j = 0; j < kHM; ++j)
         if (j < mn) {
           const float w = (m0 + j == 0) ? 1.f : 2.f;
-          sH[(size_t)(kb + j) * HS + col] = w * hr[j];
-          sH[HPL + (size_t)(kb + j) * HS + col] = w * hi[j];
+          o[j * HS] = make_float2(w * h[j].x, w * h[j].y);
         }
-      }
     }
-    __syncthreads();
-    ahead_bounds(B, nx, nx0, nx1);
+    // what no item writes: the columns past a species' alpha, and of empty lists
+    for (int t = tid; t < P.n_hzero; t += nt) {
+      const int code = __ldg(P.h_zero + t);
+      sH[(code >> 16) * HS + (code & 0xffff)] = make_float2(0.f, 0.f);
+    }
 
-    double self_x = 0.0, self_y = 0.0, self_z = 0.0;
-
-    for (int chunk = p_begin; chunk < p_end; chunk += NT) {
-      int slot[SOAPB_MAX_SPECIES];
-      unsigned my_bits;
-      double my_r;
-      const int n_ent = build_entries<NT>(P, B, p_begin, chunk, p_end, true, sEnt, sW_cnt, sBase,
-                                          sCnt, sNent, slot, my_bits, my_r);
-      for (int ebase = 0; ebase < n_ent; ebase += CH) {
-        const int n_round = min(CH, n_ent - ebase);
-        // ---- A. the entries' angular rows and radial rows
-        stage_entries<NT, AMAX, LC, true>(P, B, sEnt, chunk, ebase, n_round, sA, sR, sRd);
-        __syncthreads();
-        // ---- B. contraction against H: a half-warp per entry, lanes over k.
-        // Lane hl16 of a half-warp handles k = hl16 + 16 j.
-        int4 kix[KJ];
-        float4 kcf[KJ];
-        int klmr[KJ];
-#pragma unroll
-        for (int j = 0; j < KJ; ++j) {
-          const int kk = hl16 + 16 * j;
-          const bool v = kk < k_max;
-          kix[j] = v ? kidx[kk] : make_int4(0, 0, 0, 0);
-          kcf[j] = v ? kcoef[kk] : make_float4(0.f, 0.f, 0.f, 0.f);
-          klmr[j] = v ? klm[kk] : -1;
+    double self = 0.0;  // threads 0..2: a component of the central pair
+    for (int c0 = p_begin; c0 < p_end; c0 += kContractChunk) {
+      const int c1 = min(p_end, c0 + kContractChunk);
+      if (c0 > p_begin) __syncthreads();  // the chunk before is read
+      // entries by species, and per (pair, species) its entry or -1, by the last warp
+      // (which has the shortest of H's lists)
+      if (warp == nw - 1) {
+        const unsigned long long valid = valid_species(P, B, p_begin, c0, c1, true);
+        const unsigned lt = (1u << lane) - 1u;
+        int e = 0;
+        for (int s = 0; s < nsp; ++s) {
+          if (lane == 0) sBase[s] = e;
+          for (int c = 0; c0 + 32 * c < c1; ++c) {
+            const bool on = (valid >> (8 * c + s)) & 1ull;
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            const int at = e + __popc(m & lt);
+            if (on) list[at] = (unsigned short)(32 * c + lane);
+            slot[s * kContractChunk + 32 * c + lane] = (short)(on ? at : -1);
+            e += __popc(m);
+          }
         }
-        // The loop bound is uniform per warp (both halves iterate together) so
-        // the full-mask shuffles below always see all 32 lanes.
-        for (int eb = 2 * (tid >> 5); eb < n_round; eb += NT / 16) {
-          const int el = eb + (hw & 1);
-          const bool act = el < n_round;
-          float f_rad = 0.f, f_azi = 0.f, f_pol = 0.f;
-          if (act) {
-            const int code = sEnt[ebase + el];
-            const int s = code >> 24;
-            const float *Ae = sA + (size_t)el * AS;
-            const float *Pe = Ae + O_P;
-            if (hl16 == 0) {
-              // the rotation to Cartesian uses the same angles (:1867-1871)
-              float *rot = sRot + 4 * (code & 0xffffff);
-              rot[0] = Ae[O_X];
-              rot[1] = Ae[O_SQ];
-              rot[2] = Ae[O_E + 2];
-              rot[3] = -Ae[O_E + 3];
-            }
-            float R[AMAX], Rd[AMAX];
+        if (lane == 0) sBase[nsp] = e;
+      }
+      __syncthreads();  // H and the lists are complete; c_nlm and Gp under the rows are read
+      const float *src[NC];
 #pragma unroll
-            for (int n4 = 0; n4 < AMAX / 4; ++n4) {
-              const float4 a = ((const float4 *)(sR + (size_t)el * AMAX))[n4];
-              const float4 d = ((const float4 *)(sRd + (size_t)el * AMAX))[n4];
-              R[4 * n4] = a.x; R[4 * n4 + 1] = a.y; R[4 * n4 + 2] = a.z; R[4 * n4 + 3] = a.w;
-              Rd[4 * n4] = d.x; Rd[4 * n4 + 1] = d.y; Rd[4 * n4 + 2] = d.z; Rd[4 * n4 + 3] = d.w;
-            }
-            const float sfac = Ae[O_SF];
-            const float *Hs = sH + (size_t)s * AMAX;
+      for (int c = 0; c < NC; ++c)
+        src[c] = piece[c].rad ? B.rad + (size_t)c0 * nsp * 2 * AMAX + piece[c].first
+                              : B.ang + (size_t)c0 * AW + piece[c].first;
+      // a unit: two entries of a species.  The units go round the warps, from one
+      // species on to the next; s, e: this warp's next unit, turn: the warp to which
+      // the species' first unit falls
+      int s = 0, turn = 0, e = sBase[0] + 2 * warp;
+      auto settle = [&]() {  // past the species' last unit: on to the next species
+        while (s < nsp && e >= sBase[s + 1]) {
+          turn = (turn + ((sBase[s + 1] - sBase[s] + 1) >> 1)) & (nw - 1);
+          ++s;
+          if (s < nsp) e = sBase[s] + 2 * ((warp - turn) & (nw - 1));
+        }
+      };
+      auto copy = [&](float *dst) {
+        const int last = sBase[s + 1] - 1;
+        const unsigned j0 = list[e], j1 = list[min(e + 1, last)];
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (piece[c].on)
+            cp_async16(dst + piece[c].dst,
+                       src[c] + ((piece[c].second ? j1 : j0) * piece[c].per_pair + s * piece[c].per_species));
+      };
+      float2 H[HREG ? KJ * AMAX : 1];
+      int hs = -1;  // the species H holds
+      settle();
+      if (s < nsp) copy(stage);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+      for (int buf = 0; s < nsp; buf ^= 1) {
+        const int us = s, ue = e, u_end = sBase[s + 1];
+        e += 2 * nw;
+        settle();
+        if (s < nsp) copy(stage + (buf ^ 1) * 2 * ST);
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
+        const float2 *Hs = sH + us * AMAX;
+        if constexpr (HREG)
+          if (us != hs) {
+            hs = us;
 #pragma unroll
             for (int j = 0; j < KJ; ++j) {
-              if (klmr[j] < 0) continue;
-              const int kk = hl16 + 16 * j;
-              const int l = klmr[j] & 0xff, m = klmr[j] >> 8;
-              const float Pk = Pe[kk];
-              const float dms = kcf[j].x * Pe[kix[j].x] + kcf[j].y * Pe[kix[j].y];
-              const float dvs = kcf[j].z * Pe[kix[j].z] + kcf[j].w * Pe[kix[j].w];
-              // rows hold amp i_l, amp di_l/dr and preflm_k P_k; kcoef carries the
-              // preflm ratios of the derivative combinations
-              const float il = Ae[O_IL + l], ild = Ae[O_ILD + l];
-              const float er = Ae[O_E + 2 * m], ei = Ae[O_E + 2 * m + 1];
-              const float u = Pk * il;
-              const float ur = Pk * ild - sfac * u;
-              const float ua = dvs * il;
-              const float up = dms * il;
-              const float4 *hr4 = (const float4 *)(Hs + (size_t)kk * HS);
-              const float4 *hi4 = (const float4 *)(Hs + HPL + (size_t)kk * HS);
-              float Ur = 0.f, Ui = 0.f, Vr = 0.f, Vi = 0.f;
+              const int k = hl + 16 * j;
 #pragma unroll
-              for (int n4 = 0; n4 < AMAX / 4; ++n4) {
-                const float4 hr = hr4[n4], hi = hi4[n4];
-                Ur = fmaf(Rd[4 * n4], hr.x, Ur); Ur = fmaf(Rd[4 * n4 + 1], hr.y, Ur);
-                Ur = fmaf(Rd[4 * n4 + 2], hr.z, Ur); Ur = fmaf(Rd[4 * n4 + 3], hr.w, Ur);
-                Ui = fmaf(Rd[4 * n4], hi.x, Ui); Ui = fmaf(Rd[4 * n4 + 1], hi.y, Ui);
-                Ui = fmaf(Rd[4 * n4 + 2], hi.z, Ui); Ui = fmaf(Rd[4 * n4 + 3], hi.w, Ui);
-                Vr = fmaf(R[4 * n4], hr.x, Vr); Vr = fmaf(R[4 * n4 + 1], hr.y, Vr);
-                Vr = fmaf(R[4 * n4 + 2], hr.z, Vr); Vr = fmaf(R[4 * n4 + 3], hr.w, Vr);
-                Vi = fmaf(R[4 * n4], hi.x, Vi); Vi = fmaf(R[4 * n4 + 1], hi.y, Vi);
-                Vi = fmaf(R[4 * n4 + 2], hi.z, Vi); Vi = fmaf(R[4 * n4 + 3], hi.w, Vi);
+              for (int n = 0; n < AMAX; n += 2) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k < k_max) v = *(const float4 *)(Hs + k * HS + n);
+                H[j * AMAX + n] = make_float2(v.x, v.y);
+                H[j * AMAX + n + 1] = make_float2(v.z, v.w);
               }
-              const float reU = er * Ur + ei * Ui;
-              const float reV = er * Vr + ei * Vi;
-              const float imV = ei * Vr - er * Vi;
-              f_rad = fmaf(u, reU, fmaf(ur, reV, f_rad));
-              f_azi = fmaf(-ua, imV, f_azi);
-              f_pol = fmaf(up, reV, f_pol);
             }
           }
+        __syncwarp();
+        const float *A = stage + (2 * buf + half) * ST;
+        const bool act = ue + half < u_end;
+        float R[AMAX], Rd[AMAX];
 #pragma unroll
-          for (int o = 8; o > 0; o >>= 1) {
-            f_rad += __shfl_xor_sync(0xffffffffu, f_rad, o);
-            f_azi += __shfl_xor_sync(0xffffffffu, f_azi, o);
-            f_pol += __shfl_xor_sync(0xffffffffu, f_pol, o);
-          }
-          if (act && hl16 == 0) {
-            float *Fe = sF + (size_t)(ebase + el) * 3;
-            Fe[0] = f_rad;
-            Fe[1] = f_azi;
-            Fe[2] = f_pol;
-          }
+        for (int n4 = 0; n4 < AMAX / 4; ++n4) {
+          const float4 a = ((const float4 *)(A + AW))[n4], d = ((const float4 *)(A + AW + AMAX))[n4];
+          R[4 * n4] = a.x; R[4 * n4 + 1] = a.y; R[4 * n4 + 2] = a.z; R[4 * n4 + 3] = a.w;
+          Rd[4 * n4] = d.x; Rd[4 * n4 + 1] = d.y; Rd[4 * n4 + 2] = d.z; Rd[4 * n4 + 3] = d.w;
         }
-        __syncthreads();
+        const float sfac = A[row_sf(LC)];
+        float f_rad = 0.f, f_azi = 0.f, f_pol = 0.f;
+#pragma unroll
+        for (int j = 0; j < KJ; ++j) {
+          if (16 * j >= k_max) break;
+          float Ur = 0.f, Ui = 0.f, Vr = 0.f, Vi = 0.f;
+          const int kj = hl + 16 * j;
+          const float2 *h = Hs + (kj < k_max ? kj : 0) * HS;
+#pragma unroll
+          for (int n = 0; n < AMAX; n += 2) {
+            float4 v;
+            if constexpr (HREG)
+              v = make_float4(H[j * AMAX + n].x, H[j * AMAX + n].y, H[j * AMAX + n + 1].x, H[j * AMAX + n + 1].y);
+            else
+              v = *(const float4 *)(h + n);
+            Ur = fmaf(Rd[n], v.x, Ur); Ui = fmaf(Rd[n], v.y, Ui);
+            Vr = fmaf(R[n], v.x, Vr); Vi = fmaf(R[n], v.y, Vi);
+            Ur = fmaf(Rd[n + 1], v.z, Ur); Ui = fmaf(Rd[n + 1], v.w, Ui);
+            Vr = fmaf(R[n + 1], v.z, Vr); Vi = fmaf(R[n + 1], v.w, Vi);
+          }
+          if (!HREG && kj >= k_max) Ur = Ui = Vr = Vi = 0.f;
+          // rows hold amp i_l, amp di_l/dr and preflm_k P_k; cf carries the
+          // preflm ratios of the derivative combinations
+          const float Pk = A[oP[j]], il = A[row_il(LC) + oL[j]], ild = A[row_ild(LC) + oL[j]];
+          const float2 ee = *(const float2 *)(A + oE[j]);
+          const float *Pl = A + oP[j] + oL[j];
+          const float dms = cf[j].x * A[oX[j]] + cf[j].y * A[oP[j] + 1];
+          const float dvs = cf[j].z * Pl[0] + cf[j].w * Pl[2];
+          const float er = ee.x, ei = ee.y;
+          const float uu = Pk * il;
+          const float ur = Pk * ild - sfac * uu;
+          const float ua = dvs * il;
+          const float up = dms * il;
+          const float reU = er * Ur + ei * Ui;
+          const float reV = er * Vr + ei * Vi;
+          const float imV = ei * Vr - er * Vi;
+          f_rad = fmaf(uu, reU, fmaf(ur, reV, f_rad));
+          f_azi = fmaf(-ua, imV, f_azi);
+          f_pol = fmaf(up, reV, f_pol);
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+          f_rad += __shfl_xor_sync(0xffffffffu, f_rad, o);
+          f_azi += __shfl_xor_sync(0xffffffffu, f_azi, o);
+          f_pol += __shfl_xor_sync(0xffffffffu, f_pol, o);
+        }
+        if (act && hl == 0) {
+          float *F = sF + 3 * (ue + half);
+          F[0] = f_rad;
+          F[1] = f_azi;
+          F[2] = f_pol;
+        }
+        __syncwarp();  // the rows are read: the buffer is free for the unit after next
       }
+      __syncthreads();
       // ---- per pair: sum its entries, rotate to Cartesian (:1864-1875)
-      const int k = chunk + tid;
-      if (k < p_end && k > p_begin) {
-        double px = 0.0, py = 0.0, pz = 0.0;
-        if (my_bits != 0u) {
-          double fr = 0.0, fa = 0.0, fp = 0.0;
-#pragma unroll
-          for (int s = 0; s < SOAPB_MAX_SPECIES; ++s) {
-            if (s < nsp && slot[s] >= 0) {
-              fr += sF[3 * slot[s] + 0];
-              fa += sF[3 * slot[s] + 1];
-              fp += sF[3 * slot[s] + 2];
+      // and, 32 pairs at a time, their sums for the central pair
+      for (int k = tid; k < (c1 - c0 + 31) / 32 * 32; k += nt) {
+        double px = 0.0, py = 0.0, pz = 0.0, fr = 0.0, fa = 0.0, fp = 0.0;
+        if (c0 + k < c1 && c0 + k > p_begin) {
+          bool any = false;
+          for (int s = 0; s < nsp; ++s) {
+            const int e = slot[s * kContractChunk + k];
+            if (e >= 0) {
+              any = true;
+              fr += sF[3 * e];
+              fa += sF[3 * e + 1];
+              fp += sF[3 * e + 2];
             }
           }
-          const float *rot = sRot + 4 * tid;
-          const double ct = rot[0], st = rot[1], cf = rot[2], sf = rot[3];
-          const double ir = 1.0 / my_r;
-          px = sgn * (st * cf * fr - ct * cf * ir * fp - sf * ir * fa);
-          py = sgn * (st * sf * fr - ct * sf * ir * fp + cf * ir * fa);
-          pz = sgn * (ct * fr + st * ir * fp);
+          if (any) {
+            const float *A = B.ang + (size_t)(c0 + k) * AW;
+            const double ct = A[row_x(LC)], st = A[row_sq(LC)], cf_ = A[row_e(LC) + 2], sf = -A[row_e(LC) + 3];
+            const double ir = 1.0 / B.rjs[c0 + k];
+            px = sgn * (st * cf_ * fr - ct * cf_ * ir * fp - sf * ir * fa);
+            py = sgn * (st * sf * fr - ct * sf * ir * fp + cf_ * ir * fa);
+            pz = sgn * (ct * fr + st * ir * fp);
+          }
+          double *po = pair_out + (size_t)3 * (c0 + k);
+          po[0] = px;
+          po[1] = py;
+          po[2] = pz;
         }
-        double *po = pair_out + (size_t)3 * k;
-        po[0] = px;
-        po[1] = py;
-        po[2] = pz;
-        self_x -= px;
-        self_y -= py;
-        self_z -= pz;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          px += __shfl_xor_sync(0xffffffffu, px, o);
+          py += __shfl_xor_sync(0xffffffffu, py, o);
+          pz += __shfl_xor_sync(0xffffffffu, pz, o);
+        }
+        if (lane == 0) {
+          double *r = sRed + 8 + 3 * (k >> 5);
+          r[0] = px;
+          r[1] = py;
+          r[2] = pz;
+        }
       }
+      __syncthreads();
+      if (tid < 3)
+        for (int w = 0; c0 + 32 * w < c1; ++w) self -= sRed[8 + 3 * w + tid];
     }
     // the central pair is minus the sum of the others (:1875)
-    block_sum3<NT>(self_x, self_y, self_z, sRed);
-    if (tid == 0 && p_end > p_begin) {
-      double *po = pair_out + (size_t)3 * p_begin;
-      po[0] = self_x;
-      po[1] = self_y;
-      po[2] = self_z;
-    }
-    ahead_publish(sSite, nx, nx0, nx1);
+    if (tid < 3 && p_end > p_begin) pair_out[(size_t)3 * p_begin + tid] = self;
+    __syncthreads();  // shared memory is free for the next site
   }
 }
 
@@ -1945,13 +1996,12 @@ __global__ void __launch_bounds__(NT) k_contract_tc(const DevParams P, const Dev
         const int e = hl[t];
         const int np = e & 0xff, qq = (e >> 8) & 0xffff;
         const float y = ((e >> 31) ? 2.f : 1.41421356237309504880f) * sGu_eff[qq];
-        const float *cr = sC + (size_t)np * KS + kb;
-        const float *ci = cr + (size_t)n_max * KS;
+        const float2 *c = (const float2 *)sC + (size_t)np * KS + kb;
 #pragma unroll
         for (int j = 0; j < kHM; ++j) {
           if (j < mn) {
-            hr[j] = fmaf(y, cr[j], hr[j]);
-            hi[j] = fmaf(y, ci[j], hi[j]);
+            hr[j] = fmaf(y, c[j].x, hr[j]);
+            hi[j] = fmaf(y, c[j].y, hi[j]);
           }
         }
       }
@@ -2318,14 +2368,15 @@ template <int AMAX, int LC, int NH>
 static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg, int max_alpha,
                                      double *soap, float *keep_c, double *keep_norm, int keep) {
   const int kw = (P.k_max + 31) / 32, threads = 32 * kw * ((max_alpha + NH - 1) / NH);
-  const size_t sm = desc_layout(P, cfg.threads, AMAX, LC).total;
+  const int chunk = cfg.threads ? cfg.threads : 128;  // fixes the summation groups
+  const size_t sm = desc_layout(P, chunk, AMAX, LC).total;
   auto kern = k_descriptor<AMAX, LC, NH>;
   cudaError_t e = ensure_smem_limit(kern, sm);
   if (e != cudaSuccess) return e;
   const int n = B.site_hi - B.site_lo;
   if (n > 0) {
     const int grid = cfg.max_ctas > 0 && cfg.max_ctas < n ? cfg.max_ctas : n;
-    kern<<<grid, threads, sm, cfg.stream>>>(P, B, cfg.threads, kw, soap, keep_c, keep_norm, keep);
+    kern<<<grid, threads, sm, cfg.stream>>>(P, B, chunk, kw, soap, keep_c, keep_norm, keep);
   }
   return cudaGetLastError();
 }
@@ -2371,19 +2422,41 @@ static cudaError_t run_contract_tc(const DevParams &P, const DevBatch &B, const 
   return cudaGetLastError();
 }
 
-template <int NT, int AMAX, int LC>
+// Threads per site: with 64 a site costs the least work, with more it is done
+// sooner and the last wave wastes less (of 64, 128 and 256 threads 8, 4 and 2 CTAs
+// fit an SM).  The choice with the cheapest waves, a site at 128 and 256 threads
+// costing 1.2 and 1.6 of its share at 64.  Steps at 64, 128 and 256 threads: 64 sites
+// 47.1, 43.0, 40.8 us; 367 of two species 86, 74, 80; 727 of two 67, 71, 76; 1679 of
+// three 137, 126, 147; 16384 of one 715, 779, 941.
+static int contract_threads(int n_sites) {
+  const int slots[3] = {148 * 8, 148 * 4, 148 * 2};
+  const double cost[3] = {1.0, 1.2, 1.6};
+  int best = 0;
+  double least = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    const double t = (double)((n_sites + slots[i] - 1) / slots[i]) * slots[i] * cost[i];
+    if (i == 0 || t < least) {
+      least = t;
+      best = i;
+    }
+  }
+  return 64 << best;
+}
+
+template <int AMAX, int LC>
 static cudaError_t run_contract(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
                                 const double *soap, const double *G, int g_layout, double sgn,
                                 const float *keep_c, const double *keep_norm, double *pair) {
   if (AMAX == 8 && LC == 8 && P.tc_contract)
     return run_contract_tc(P, B, cfg, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
-  const size_t sm = make_layout(P, NT, AMAX, LC, 1).total;
-  auto kern = k_contract<NT, AMAX, LC>;
+  const int n = B.site_hi - B.site_lo, threads = cfg.threads ? cfg.threads : contract_threads(n);
+  const size_t sm = contract_layout(P, threads, AMAX, LC).total;
+  auto kern = k_contract<AMAX, LC>;
   cudaError_t e = ensure_smem_limit(kern, sm);
   if (e != cudaSuccess) return e;
-  if (B.site_hi > B.site_lo) {
-    const int grid = persistent_grid(kern, NT, sm, B.site_hi - B.site_lo, cfg.max_ctas);
-    kern<<<grid, NT, sm, cfg.stream>>>(P, B, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
+  if (n > 0) {
+    const int grid = cfg.max_ctas > 0 && cfg.max_ctas < n ? cfg.max_ctas : n;
+    kern<<<grid, threads, sm, cfg.stream>>>(P, B, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
   }
   return cudaGetLastError();
 }
@@ -2434,20 +2507,7 @@ cudaError_t launch_pair(const DevParams &P, const DevBatch &B, cudaStream_t s, i
 }
 
 // The radial block is fixed by the definition: the host lays the constants
-// blob out for amax_t (8 when every alpha <= 8 and l_max <= 8, else 16).  The
-// CTA size (threads per site) is a launch choice: 64, 128 or 256.
-#define SOAPB_DISPATCH_NT(FN, NT, ...)                    \
-  do {                                                    \
-    if (P.amax_t == 8) return FN<NT, 8, 8>(__VA_ARGS__);  \
-    return FN<NT, 16, 12>(__VA_ARGS__);                   \
-  } while (0)
-#define SOAPB_DISPATCH(FN, ...)                                             \
-  do {                                                                      \
-    if (cfg.threads == 64) SOAPB_DISPATCH_NT(FN, 64, __VA_ARGS__);          \
-    if (cfg.threads == 256) SOAPB_DISPATCH_NT(FN, 256, __VA_ARGS__);        \
-    SOAPB_DISPATCH_NT(FN, 128, __VA_ARGS__);                                \
-  } while (0)
-
+// blob out for amax_t (8 when every alpha <= 8 and l_max <= 8, else 16).
 cudaError_t launch_descriptor(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
                               double *soap, float *keep_c, double *keep_norm, int keep) {
   if (P.amax_t == 8) return run_descriptor<8, 8>(P, B, cfg, soap, keep_c, keep_norm, keep);
@@ -2457,13 +2517,10 @@ cudaError_t launch_descriptor(const DevParams &P, const DevBatch &B, const Launc
 cudaError_t launch_contract(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
                             const double *soap, const double *G, int g_layout, double sgn,
                             const float *keep_c, const double *keep_norm, double *pair) {
-  SOAPB_DISPATCH(run_contract, P, B, cfg, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
+  if (P.amax_t == 8) return run_contract<8, 8>(P, B, cfg, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
+  return run_contract<16, 12>(P, B, cfg, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
 }
 
 size_t keep_floats_per_site(const DevParams &P) { return keep_stride(P); }
-
-size_t contract_smem(const DevParams &P, int threads) {
-  return make_layout(P, threads, P.amax_t, P.amax_t == 8 ? 8 : 12, 1).total;
-}
 
 }  // namespace soapb
