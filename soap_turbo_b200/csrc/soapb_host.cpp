@@ -307,7 +307,8 @@ struct soapb_context {
   // flags, per-CTA scratch, the descriptor it recomputes, its work counter
   DBuf hs_rad_der2, hs_geo, hs_good, hs_scratch, hs_sums, hs_soap, hs_ticket, hs_vchunk, hs_hchunk;
   // neighbour-list builder: cell list, counts and the batch it hands out
-  DBuf nb_acell, nb_ccount, nb_cstart, nb_cfill, nb_catoms, nb_counts, nb_off, nb_state;
+  DBuf nb_acell, nb_cstart, nb_cells, nb_counts, nb_off, nb_state;
+  unsigned long long *nb_status = nullptr;  // page-locked: a build's pair count and error words
   DBuf nb_rjs, nb_th, nb_ph, nb_mask, nb_natom, nb_nneigh, nb_species, nb_smult;
   cudaStream_t stream = 0;
   int threads = 0;   // threads per site CTA chosen by the caller (0 = tuned or default)
@@ -347,10 +348,10 @@ struct soapb_context {
     timing_release();
     for (DBuf *b : {&tables, &off, &bits, &err, &keep_c, &keep_norm, &order, &rad, &ang, &f64_rad, &f64_rad_der,
                     &f64_ang, &f64_cnk, &f64_soap_un, &f64_norm, &f64_parts, &f64_done, &hs_rad_der2, &hs_geo, &hs_good,
-                    &hs_scratch, &hs_sums, &hs_soap, &hs_ticket, &hs_vchunk, &hs_hchunk, &nb_acell, &nb_ccount, &nb_cstart,
-                    &nb_cfill, &nb_catoms, &nb_counts, &nb_off, &nb_state, &nb_rjs, &nb_th, &nb_ph,
-                    &nb_mask, &nb_natom, &nb_nneigh, &nb_species, &nb_smult})
+                    &hs_scratch, &hs_sums, &hs_soap, &hs_ticket, &hs_vchunk, &hs_hchunk, &nb_acell, &nb_cstart, &nb_cells,
+                    &nb_counts, &nb_off, &nb_state, &nb_rjs, &nb_th, &nb_ph, &nb_mask, &nb_natom, &nb_nneigh, &nb_species, &nb_smult})
       b->release();
+    if (nb_status) cudaFreeHost(nb_status);
   }
 };
 
@@ -1671,68 +1672,71 @@ int soapb_build_neighbors(soapb_context *c, int32_t n_atoms, const double *d_pos
   g.n_species = c->n_species;
   const int n_cells = g.nc[0] * g.nc[1] * g.nc[2];
   const size_t w_cells = (size_t)prep_err_words(n_cells), w_sites = (size_t)prep_err_words(n_sites);
+  // cleared by one memset: the error word, the scans' states, then the cells' counts
+  // and fills and the count pass's counter
+  const size_t words = 1 + w_cells + w_sites, n_clear = 8 * words + 4 * (2 * (size_t)n_cells + 2);
   int rc;
   if ((rc = c->nb_acell.ensure(sizeof(int4) * (size_t)n_atoms)) ||
-      (rc = c->nb_ccount.ensure(sizeof(int) * ((size_t)n_cells + 1))) ||
       (rc = c->nb_cstart.ensure(sizeof(int) * ((size_t)n_cells + 1))) ||
-      (rc = c->nb_cfill.ensure(sizeof(int) * (size_t)n_cells)) ||
-      (rc = c->nb_catoms.ensure(sizeof(int) * (size_t)n_atoms)) ||
+      (rc = c->nb_cells.ensure(sizeof(NbAtom) * (size_t)n_atoms)) ||
       (rc = c->nb_counts.ensure(sizeof(int) * ((size_t)n_sites + 1))) ||
-      (rc = c->nb_off.ensure(sizeof(int) * ((size_t)n_sites + 1))) ||
-      (rc = c->nb_state.ensure(8 * (1 + w_cells + w_sites))))
-    return rc;
-  unsigned long long *st = c->nb_state.as<unsigned long long>();
-  cudaStream_t s = c->stream;
-  CU(cudaMemsetAsync(c->nb_ccount.p, 0, sizeof(int) * ((size_t)n_cells + 1), s));
-  CU(cudaMemsetAsync(c->nb_cfill.p, 0, sizeof(int) * (size_t)n_cells, s));
-  CU(cudaMemsetAsync(st, 0, 8 * (1 + w_cells + w_sites), s));
-  int4 *acell = c->nb_acell.as<int4>();
-  int *cstart = c->nb_cstart.as<int>(), *catoms = c->nb_catoms.as<int>();
-  CU(launch_nb_bin(g, d_positions, acell, c->nb_ccount.as<int>(), st, s));
-  CU(launch_scan(c->nb_ccount.as<int>(), n_cells, cstart, st + 1, s));
-  CU(launch_nb_place(g, acell, cstart, c->nb_cfill.as<int>(), catoms, s));
-  CU(launch_nb_count(g, d_positions, d_sites, acell, cstart, catoms, c->nb_counts.as<int>(), st, s));
-  CU(launch_scan(c->nb_counts.as<int>(), n_sites, c->nb_off.as<int>(), st + 1 + w_cells, s));
-  c->launches += 4 + (n_sites > 0);
-  int total = 0;
-  if (n_sites > 0) CU(cudaMemcpyAsync(&total, c->nb_off.as<int>() + n_sites, sizeof(int), cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
-  if (total < 0) return fail(SOAPB_ERR_ARGUMENT, "more than 2^31 pairs");
-  const size_t np = (size_t)total;
-  if ((rc = c->nb_rjs.ensure(8 * (np + 1))) || (rc = c->nb_th.ensure(8 * (np + 1))) ||
-      (rc = c->nb_ph.ensure(8 * (np + 1))) || (rc = c->nb_mask.ensure((size_t)c->n_species * np + 16)) ||
-      (rc = c->nb_natom.ensure(4 * (np + 1))) || (rc = c->nb_nneigh.ensure(4 * ((size_t)n_sites + 1))) ||
+      (rc = c->nb_off.ensure(sizeof(int) * ((size_t)n_sites + 1))) || (rc = c->nb_state.ensure(n_clear)) ||
+      (rc = c->nb_nneigh.ensure(4 * ((size_t)n_sites + 1))) ||
       (rc = c->nb_species.ensure(4 * ((size_t)max_mult * n_sites + 1))) ||
       (rc = c->nb_smult.ensure(4 * ((size_t)n_sites + 1))))
     return rc;
+  if (!c->nb_status) CU(cudaHostAlloc((void **)&c->nb_status, 4 * sizeof(unsigned long long), cudaHostAllocDefault));
+  unsigned long long *st = c->nb_state.as<unsigned long long>();
+  int *ccount = (int *)(st + words), *cfill = ccount + n_cells + 1, *done = cfill + n_cells;
+  cudaStream_t s = c->stream;
+  CU(cudaMemsetAsync(st, 0, n_clear, s));
+  int4 *acell = c->nb_acell.as<int4>();
+  int *cstart = c->nb_cstart.as<int>();
+  NbAtom *cells = c->nb_cells.as<NbAtom>();
+  int nl = 0;
+  CU(launch_nb_cells(g, n_cells, d_positions, acell, ccount, cstart, cfill, cells, st, st + 1, &nl, s));
+  CU(launch_nb_count(g, d_positions, d_sites, acell, cstart, cells, c->nb_counts.as<int>(), c->nb_off.as<int>(), done,
+                     st, st + 1 + w_cells, &nl, s));
+  // the fill pass into the buffers as the last call left them; where they turn out
+  // too small they grow, with a sixteenth to spare, and it runs again
+  int total = 0;
   NbOut o{};
-  o.n_pairs = total;
-  o.rjs = c->nb_rjs.as<double>();
-  o.thetas = c->nb_th.as<double>();
-  o.phis = c->nb_ph.as<double>();
-  o.mask = c->nb_mask.as<uint8_t>();
-  o.neigh_atom = c->nb_natom.as<int>();
-  o.n_neigh = c->nb_nneigh.as<int>();
-  o.species = c->nb_species.as<int>();
-  o.species_mult = c->nb_smult.as<int>();
-  CU(launch_nb_fill(g, d_positions, d_sites, d_atom_species, d_atom_mult, acell, cstart, catoms,
-                    c->nb_off.as<int>(), o, st, s));
-  c->launches += (n_sites > 0);
-  unsigned long long w[3] = {0, 0, 0};
-  CU(cudaMemcpyAsync(&w[0], st, 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaMemcpyAsync(&w[1], st + 1, 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaMemcpyAsync(&w[2], st + 1 + w_cells, 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
-  if (w[1] || w[2]) return fail(SOAPB_ERR_CUDA, "the neighbour-list scan gave up waiting for a preceding tile");
-  if (w[0]) {
-    const unsigned long long code = kErrTop - w[0];
-    if (code == kErrWrap)
-      return fail(SOAPB_ERR_INPUT, "an atom position is not finite or lies more than %d cells outside the cell",
-                  kNbMaxWrap);
-    if (code < (1ull << 32)) return fail(SOAPB_ERR_INPUT, "sites(%llu) is not an atom index", code + 1);
-    return fail(SOAPB_ERR_ARGUMENT, "site %llu has more than %d neighbours within rcut = %g",
-                code - (1ull << 32) + 1, kNbCap, rcut);
+  for (;;) {
+    const size_t cap = std::min(std::min(std::min(c->nb_rjs.cap, c->nb_th.cap), c->nb_ph.cap) / 8,
+                                std::min(c->nb_natom.cap / 4, c->nb_mask.cap / (size_t)c->n_species));
+    o.n_pairs = (int)std::min(cap, (size_t)INT32_MAX);
+    o.rjs = c->nb_rjs.as<double>();
+    o.thetas = c->nb_th.as<double>();
+    o.phis = c->nb_ph.as<double>();
+    o.mask = c->nb_mask.as<uint8_t>();
+    o.neigh_atom = c->nb_natom.as<int>();
+    o.n_neigh = c->nb_nneigh.as<int>();
+    o.species = c->nb_species.as<int>();
+    o.species_mult = c->nb_smult.as<int>();
+    CU(launch_nb_fill(g, d_positions, d_sites, d_atom_species, d_atom_mult, acell, cstart, cells, c->nb_off.as<int>(),
+                      o, st, (int)w_cells, c->nb_status, s));
+    nl += 1;
+    CU(cudaStreamSynchronize(s));
+    const volatile unsigned long long *w = c->nb_status;
+    if (w[2] || w[3]) return fail(SOAPB_ERR_CUDA, "the neighbour-list scan gave up waiting for a preceding tile");
+    if (w[1]) {
+      const unsigned long long code = kErrTop - w[1];
+      if (code == kErrWrap)
+        return fail(SOAPB_ERR_INPUT, "an atom position is not finite or lies more than %d cells outside the cell",
+                    kNbMaxWrap);
+      if (code < (1ull << 32)) return fail(SOAPB_ERR_INPUT, "sites(%llu) is not an atom index", code + 1);
+      return fail(SOAPB_ERR_ARGUMENT, "site %llu has more than %d neighbours within rcut = %g",
+                  code - (1ull << 32) + 1, kNbCap, rcut);
+    }
+    total = (int)(long long)w[0];
+    if (total < 0) return fail(SOAPB_ERR_ARGUMENT, "more than 2^31 pairs");
+    if (total <= o.n_pairs && c->nb_rjs.p) break;
+    const size_t np = (size_t)total + (size_t)total / 16 + 16;
+    if ((rc = c->nb_rjs.ensure(8 * np)) || (rc = c->nb_th.ensure(8 * np)) || (rc = c->nb_ph.ensure(8 * np)) ||
+        (rc = c->nb_mask.ensure((size_t)c->n_species * np)) || (rc = c->nb_natom.ensure(4 * np)))
+      return rc;
   }
+  c->launches += nl;
   out->n_sites = n_sites;
   out->n_atom_pairs = total;
   out->max_species_multiplicity = max_mult;

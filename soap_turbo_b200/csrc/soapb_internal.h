@@ -216,16 +216,24 @@ struct NbOut {     // get_soap's inputs, plus the atom behind every pair
   uint8_t *mask;   // (n_species, n_pairs)
   int *neigh_atom, *n_neigh, *species, *species_mult;
 };
-cudaError_t launch_nb_bin(const NbGeom &g, const double *pos, int4 *atom_cell, int *cell_count,
-                          unsigned long long *err, cudaStream_t s);
-cudaError_t launch_nb_place(const NbGeom &g, const int4 *atom_cell, const int *cell_start, int *cell_fill,
-                            int *cell_atoms, cudaStream_t s);
+struct alignas(32) NbAtom {  // an atom in cell order: position, index, the translation that wraps it (10 bits each)
+  double x, y, z;
+  int atom, wrap;
+};
+// One CTA makes the cell list up to these sizes, and the last CTA of the count
+// pass scans the counts of up to kNbOneSites sites.
+constexpr int kNbOneAtoms = 8192, kNbOneCells = 8192, kNbOneSites = 4096;
+cudaError_t launch_nb_cells(const NbGeom &g, int n_cells, const double *pos, int4 *atom_cell, int *cell_count,
+                            int *cell_start, int *cell_fill, NbAtom *cells, unsigned long long *err,
+                            unsigned long long *scan_state, int *launches, cudaStream_t s);
 cudaError_t launch_nb_count(const NbGeom &g, const double *pos, const int *sites, const int4 *atom_cell,
-                            const int *cell_start, const int *cell_atoms, int *counts, unsigned long long *err,
-                            cudaStream_t s);
+                            const int *cell_start, const NbAtom *cells, int *counts, int *off, int *done,
+                            unsigned long long *err, unsigned long long *scan_state, int *launches, cudaStream_t s);
+// o.n_pairs: the capacity of its buffers; status (page-locked): see k_nb_fill
 cudaError_t launch_nb_fill(const NbGeom &g, const double *pos, const int *sites, const int *atom_species,
-                           const int *atom_mult, const int4 *atom_cell, const int *cell_start, const int *cell_atoms,
-                           const int *off, const NbOut &o, unsigned long long *err, cudaStream_t s);
+                           const int *atom_mult, const int4 *atom_cell, const int *cell_start, const NbAtom *cells,
+                           const int *off, const NbOut &o, const unsigned long long *err, int w_cells,
+                           unsigned long long *status, cudaStream_t s);
 // Exclusive scan of n counts into off (n + 1 entries); state: prep_err_words(n)
 // words cleared beforehand.  blocks < 0: one block per tile (the scan); fewer
 // blocks and a smaller max_spins serve the self-test of the bounded wait.

@@ -9,10 +9,17 @@
 // are at least rcut wide along each axis, and a site visits the cells within
 // R = ceil(rcut * n_cells / plane_spacing) of its own along each axis, with the
 // lattice translation each wrap implies (so small cells, where R cells reach
-// around the box, visit several images of the same atoms).  Two passes: count,
-// scan the counts into CSR offsets, then fill.  One warp per site; the fill
-// pass gathers the site's row in shared memory and sorts it by (neighbour
-// atom, distance) so the order depends on nothing but the inputs.
+// around the box, visit several images of the same atoms).  The atoms are
+// copied in cell order, so the cells of one (x, y) column of a site's stencil are
+// one run of them, and a warp takes a site's runs end to end, a candidate per lane.
+// Two passes: count (whose last CTA scans the counts into CSR offsets where the
+// sites are few), then fill.  One warp per site; the fill pass gathers the site's
+// row in shared memory and sorts it by (neighbour atom, distance) so the order
+// depends on nothing but the inputs.
+// What bounds it, at some thousand atoms: the launches and each pass's chain of
+// dependent loads.  A cell at a time (27 of some 12 atoms, read through their
+// indices) count and fill took 32 and 57 us for 1679 sites of 4096 atoms; see
+// soapb_build_neighbors for the whole.
 #include "soapb_scan.cuh"
 
 namespace soapb {
@@ -22,30 +29,28 @@ namespace {
 constexpr int kNbWarps = 4;      // warps (sites) per CTA of the count kernel
 constexpr int kNbFillWarps = 2;  // warps (sites) per CTA of the fill kernel (its rows sit in shared memory)
 constexpr int kNbShift = 512;    // image components are stored as n + kNbShift in 10 bits
+constexpr int kNbOneThreads = 1024;
 static_assert(kNbMaxReach + 1 + 2 * kNbMaxWrap < kNbShift, "image translations must fit 10 bits");
 
 __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
 // Displacement of atom j's image n (integer lattice vector) from atom i:
 // (r_j + n . lattice) - r_i.  Both passes call this, so they agree bit for bit.
-__device__ __forceinline__ void image_disp(const NbGeom &g, const double *pos, int i, int j, int nx, int ny,
-                                           int nz, double &dx, double &dy, double &dz) {
+__device__ __forceinline__ void image_disp(const NbGeom &g, double xj, double yj, double zj, double xi, double yi,
+                                           double zi, int nx, int ny, int nz, double &dx, double &dy, double &dz) {
   const double tx = nx * g.lat[0] + ny * g.lat[3] + nz * g.lat[6];
   const double ty = nx * g.lat[1] + ny * g.lat[4] + nz * g.lat[7];
   const double tz = nx * g.lat[2] + ny * g.lat[5] + nz * g.lat[8];
-  dx = (pos[3 * j] + tx) - pos[3 * i];
-  dy = (pos[3 * j + 1] + ty) - pos[3 * i + 1];
-  dz = (pos[3 * j + 2] + tz) - pos[3 * i + 2];
+  dx = (xj + tx) - xi;
+  dy = (yj + ty) - yi;
+  dz = (zj + tz) - zi;
 }
 
-// ---- per atom: its cell and the lattice translation that wraps it into the cell
+// ---- an atom's cell and the lattice translation that wraps it into the cell
 // (image translations then stay within +-(kNbMaxReach + 1 + 2 kNbMaxWrap) <
 // kNbShift, the packing range of the fill pass; farther atoms, and non-finite
 // positions, are reported and put in cell 0)
-__global__ void k_nb_bin(NbGeom g, const double *pos, int4 *atom_cell, int *cell_count,
-                         unsigned long long *err) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= g.n_atoms) return;
+__device__ __forceinline__ int4 bin_atom(const NbGeom &g, const double *pos, int a, unsigned long long *err) {
   const double x = pos[3 * a], y = pos[3 * a + 1], z = pos[3 * a + 2];
   int c[3], w[3];
   bool bad = false;
@@ -63,83 +68,215 @@ __global__ void k_nb_bin(NbGeom g, const double *pos, int4 *atom_cell, int *cell
     }
   }
   if (bad) atomicMax(err, kErrTop - kErrWrap);
-  const int cell = (c[0] * g.nc[1] + c[1]) * g.nc[2] + c[2];
-  atom_cell[a] = make_int4(cell, w[0], w[1], w[2]);
-  atomicAdd(&cell_count[cell], 1);
+  return make_int4((c[0] * g.nc[1] + c[1]) * g.nc[2] + c[2], w[0], w[1], w[2]);
+}
+__device__ __forceinline__ int pack3(int x, int y, int z) {
+  return ((x + kNbShift) << 20) | ((y + kNbShift) << 10) | (z + kNbShift);
+}
+__device__ __forceinline__ NbAtom cell_atom(const double *pos, int a, int4 c) {
+  return NbAtom{pos[3 * a], pos[3 * a + 1], pos[3 * a + 2], a, pack3(c.y, c.z, c.w)};
 }
 
-// ---- per atom: its slot in its cell (the order inside a cell is arbitrary)
-__global__ void k_nb_place(NbGeom g, const int4 *atom_cell, const int *cell_start, int *cell_fill,
-                           int *cell_atoms) {
+// The cell list of few atoms by one CTA: counts in shared memory, scanned, and the
+// atoms copied to their slots (the order inside a cell is arbitrary).
+__global__ void __launch_bounds__(kNbOneThreads) k_nb_cells(NbGeom g, int n_cells, const double *pos, int4 *atom_cell,
+                                                            int *cell_start, NbAtom *cells, unsigned long long *err) {
+  __shared__ int cnt[kNbOneCells];
+  __shared__ int wsum[kNbOneThreads / 32];
+  constexpr int PER = kNbOneAtoms / kNbOneThreads, CPT = kNbOneCells / kNbOneThreads;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < n_cells; i += kNbOneThreads) cnt[i] = 0;
+  __syncthreads();
+  int4 c[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int a = tid + j * kNbOneThreads;
+    if (a < g.n_atoms) {
+      c[j] = bin_atom(g, pos, a, err);
+      atom_cell[a] = c[j];
+      atomicAdd(&cnt[c[j].x], 1);
+    }
+  }
+  __syncthreads();
+  int own[CPT], sum = 0;
+#pragma unroll
+  for (int i = 0; i < CPT; ++i) {
+    const int q = tid * CPT + i;
+    own[i] = q < n_cells ? cnt[q] : 0;
+    sum += own[i];
+  }
+  int x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wsum[warp] = x;
+  __syncthreads();
+  int run = x - sum;
+  for (int w = 0; w < warp; ++w) run += wsum[w];
+#pragma unroll
+  for (int i = 0; i < CPT; ++i) {
+    const int q = tid * CPT + i;
+    if (q < n_cells) {
+      cell_start[q] = run;
+      cnt[q] = run;
+    }
+    run += own[i];
+  }
+  if (tid == 0) cell_start[n_cells] = g.n_atoms;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int a = tid + j * kNbOneThreads;
+    if (a < g.n_atoms) cells[atomicAdd(&cnt[c[j].x], 1)] = cell_atom(pos, a, c[j]);
+  }
+}
+
+// ... and of many, in three launches: bin, the scan, place
+__global__ void k_nb_bin(NbGeom g, const double *pos, int4 *atom_cell, int *cell_count,
+                         unsigned long long *err) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= g.n_atoms) return;
-  const int cell = atom_cell[a].x;
-  cell_atoms[cell_start[cell] + atomicAdd(&cell_fill[cell], 1)] = a;
+  const int4 c = bin_atom(g, pos, a, err);
+  atom_cell[a] = c;
+  atomicAdd(&cell_count[c.x], 1);
+}
+__global__ void k_nb_place(NbGeom g, const double *pos, const int4 *atom_cell, const int *cell_start, int *cell_fill,
+                           NbAtom *cells) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= g.n_atoms) return;
+  const int4 c = atom_cell[a];
+  cells[cell_start[c.x] + atomicAdd(&cell_fill[c.x], 1)] = cell_atom(pos, a, c);
 }
 
-// Visits every candidate image of a site's stencil: visit(j, nx, ny, nz, ok)
+// Visits every candidate image of a site's stencil: visit(j, nx, ny, nz, r2, ok)
 // is called by all lanes of the warp together (ok false on padding lanes), so
-// it may use warp collectives.
+// it may use warp collectives.  A run is the stencil's cells of one x, y and wrap
+// in z, contiguous in the cell order; 32 runs are laid end to end at a time.
 template <typename Visit>
 __device__ __forceinline__ void for_each_neighbour(const NbGeom &g, const double *pos, const int4 *atom_cell,
-                                                   const int *cell_start, const int *cell_atoms, int a,
-                                                   Visit visit) {
+                                                   const int *cell_start, const NbAtom *cells, int a, Visit visit) {
   const int lane = threadIdx.x & 31;
   const int4 ca = atom_cell[a];
-  const int cell = ca.x;
-  const int cz = cell % g.nc[2], cy = (cell / g.nc[2]) % g.nc[1], cx = cell / (g.nc[2] * g.nc[1]);
-  for (int ox = -g.R[0]; ox <= g.R[0]; ++ox) {
-    const int X = cx + ox, wx = floor_div(X, g.nc[0]);
-    const int qx = X - wx * g.nc[0];
-    for (int oy = -g.R[1]; oy <= g.R[1]; ++oy) {
-      const int Y = cy + oy, wy = floor_div(Y, g.nc[1]);
-      const int qy = Y - wy * g.nc[1];
-      for (int oz = -g.R[2]; oz <= g.R[2]; ++oz) {
-        const int Z = cz + oz, wz = floor_div(Z, g.nc[2]);
-        const int qz = Z - wz * g.nc[2];
-        const int q = (qx * g.nc[1] + qy) * g.nc[2] + qz;
-        const int t0 = cell_start[q], t1 = cell_start[q + 1];
-        for (int t = t0; t < t1; t += 32) {
-          const int tt = t + lane;
-          int j = 0, nx = 0, ny = 0, nz = 0;
-          bool ok = false;
-          if (tt < t1) {
-            j = cell_atoms[tt];
-            const int4 cj = atom_cell[j];
-            // the image of j in cell (X, Y, Z): translation (w - w_j + w_a) lattice vectors
-            nx = wx - cj.y + ca.y;
-            ny = wy - cj.z + ca.z;
-            nz = wz - cj.w + ca.w;
-            double dx, dy, dz;
-            image_disp(g, pos, a, j, nx, ny, nz, dx, dy, dz);
-            ok = dx * dx + dy * dy + dz * dz < g.rcut2 && !(j == a && nx == 0 && ny == 0 && nz == 0);
-          }
-          visit(j, nx, ny, nz, ok);
+  const double xi = pos[3 * a], yi = pos[3 * a + 1], zi = pos[3 * a + 2];
+  const int cz = ca.x % g.nc[2], cy = (ca.x / g.nc[2]) % g.nc[1], cx = ca.x / (g.nc[2] * g.nc[1]);
+  const int wz0 = floor_div(cz - g.R[2], g.nc[2]), nz = floor_div(cz + g.R[2], g.nc[2]) - wz0 + 1;
+  const int ny = 2 * g.R[1] + 1, n_run = (2 * g.R[0] + 1) * ny * nz;
+  for (int r0 = 0; r0 < n_run; r0 += 32) {
+    int start = 0, len = 0, tr = 0;  // the lane's run, and the translation of its cells
+    if (r0 + lane < n_run) {
+      const int rr = r0 + lane, iz = rr % nz, t = rr / nz, iy = t % ny, ix = t / ny;
+      const int X = cx + ix - g.R[0], wx = floor_div(X, g.nc[0]), qx = X - wx * g.nc[0];
+      const int Y = cy + iy - g.R[1], wy = floor_div(Y, g.nc[1]), qy = Y - wy * g.nc[1];
+      const int wz = wz0 + iz, lo = max(cz - g.R[2] - wz * g.nc[2], 0),
+                hi = min(cz + g.R[2] - wz * g.nc[2], g.nc[2] - 1);
+      const int q = (qx * g.nc[1] + qy) * g.nc[2];
+      start = cell_start[q + lo];
+      len = cell_start[q + hi + 1] - start;
+      tr = pack3(wx + ca.y, wy + ca.z, wz + ca.w);
+    }
+    int incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    // two candidates a lane at a time, so that their loads overlap
+    for (int c0 = 0; c0 < total; c0 += 64) {
+      NbAtom b[2];
+      int w[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = c0 + 32 * h + lane;
+        int r = 0;  // the run of candidate c: how many end at or before it
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(0xffffffffu, incl, r + step - 1) <= c) r += step;
+        const int at = c - __shfl_sync(0xffffffffu, incl, r) + __shfl_sync(0xffffffffu, len, r) +
+                       __shfl_sync(0xffffffffu, start, r);
+        w[h] = __shfl_sync(0xffffffffu, tr, r);
+        if (c < total) b[h] = cells[at];
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (c0 + 32 * h >= total) break;
+        int j = 0, nx = 0, ny_ = 0, nz_ = 0;
+        double r2 = 0.0;
+        bool ok = false;
+        if (c0 + 32 * h + lane < total) {
+          j = b[h].atom;
+          // the image of j in the run's cells: translation (w - w_j + w_a) lattice vectors
+          nx = (w[h] >> 20) - (b[h].wrap >> 20);
+          ny_ = ((w[h] >> 10) & 1023) - ((b[h].wrap >> 10) & 1023);
+          nz_ = (w[h] & 1023) - (b[h].wrap & 1023);
+          double dx, dy, dz;
+          image_disp(g, b[h].x, b[h].y, b[h].z, xi, yi, zi, nx, ny_, nz_, dx, dy, dz);
+          r2 = dx * dx + dy * dy + dz * dz;
+          ok = r2 < g.rcut2 && !(j == a && nx == 0 && ny_ == 0 && nz_ == 0);
         }
+        visit(j, nx, ny_, nz_, r2, ok);
       }
     }
   }
 }
 
-// ---- pass 1: neighbours of each site (the row length is one more: the site itself)
+// ---- pass 1: neighbours of each site (the row length is one more: the site itself).
+// done (may be null): the CTAs finished; the last one then scans the counts of up to
+// kNbOneSites sites into the CSR offsets.
 __global__ void __launch_bounds__(32 * kNbWarps) k_nb_count(NbGeom g, const double *pos, const int *sites,
                                                             const int4 *atom_cell, const int *cell_start,
-                                                            const int *cell_atoms, int *counts,
+                                                            const NbAtom *cells, int *counts, int *off, int *done,
                                                             unsigned long long *err) {
-  const int w = blockIdx.x * kNbWarps + (threadIdx.x >> 5);
-  if (w >= g.n_sites) return;
-  const int a = sites[w];
-  if (a < 0 || a >= g.n_atoms) {
-    if ((threadIdx.x & 31) == 0) {
-      counts[w] = 1;
-      atomicMax(err, kErrTop - (unsigned long long)w);  // site index out of range
+  constexpr int NT = 32 * kNbWarps;
+  const int w = blockIdx.x * kNbWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (w < g.n_sites) {
+    const int a = sites[w];
+    int cnt = 0;
+    unsigned long long bad = 0ull;
+    if (a < 0 || a >= g.n_atoms) {
+      bad = kErrTop - (unsigned long long)w;  // site index out of range
+    } else {
+      for_each_neighbour(g, pos, atom_cell, cell_start, cells, a, [&](int, int, int, int, double, bool ok) {
+        cnt += __popc(__ballot_sync(0xffffffffu, ok));
+      });
+      if (cnt > kNbCap) bad = kErrTop - ((1ull << 32) + (unsigned long long)w);  // row too long
     }
-    return;
+    if (lane == 0) {
+      counts[w] = 1 + cnt;
+      if (bad) atomicMax(err, bad);
+    }
   }
-  int cnt = 0;
-  for_each_neighbour(g, pos, atom_cell, cell_start, cell_atoms, a,
-                     [&](int, int, int, int, bool ok) { cnt += __popc(__ballot_sync(0xffffffffu, ok)); });
-  if ((threadIdx.x & 31) == 0) counts[w] = 1 + cnt;
+  if (!done) return;
+  __shared__ int s_last;
+  __shared__ int wsum[kNbWarps];
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const int per = (g.n_sites + NT - 1) / NT, i0 = threadIdx.x * per, i1 = min(g.n_sites, i0 + per);
+  int sum = 0;
+#pragma unroll 8
+  for (int i = i0; i < i1; ++i) sum += __ldcg(counts + i);
+  int x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wsum[threadIdx.x >> 5] = x;
+  __syncthreads();
+  int run = x - sum;
+  for (int v = 0; v < (int)(threadIdx.x >> 5); ++v) run += wsum[v];
+#pragma unroll 8
+  for (int i = i0; i < i1; ++i) {
+    off[i] = run;
+    run += __ldcg(counts + i);
+  }
+  if (threadIdx.x == NT - 1) off[g.n_sites] = run;
 }
 
 // The species bits of neighbour j in the row of central atom a, as
@@ -156,73 +293,101 @@ __device__ __forceinline__ unsigned mask_bits(const NbGeom &g, const int *atom_s
   return bits;
 }
 
-// ---- pass 2: each site's row, sorted by (neighbour atom, distance)
+// ---- pass 2: each site's row, sorted by (neighbour atom, distance).  The pair count
+// comes from the offsets; nothing is written where it is above the buffers'
+// capacity, o.n_pairs (the host then makes room and launches again).  status, in
+// page-locked host memory, receives the pair count and the three error words.
 __global__ void __launch_bounds__(32 * kNbFillWarps) k_nb_fill(NbGeom g, const double *pos, const int *sites,
                                                            const int *atom_species, const int *atom_mult,
                                                            const int4 *atom_cell, const int *cell_start,
-                                                           const int *cell_atoms, const int *off,
-                                                           NbOut o, unsigned long long *err) {
+                                                           const NbAtom *cells, const int *off, NbOut o,
+                                                           const unsigned long long *err, int w_cells,
+                                                           volatile unsigned long long *status) {
   __shared__ unsigned long long s_key[kNbFillWarps][kNbCap];
   __shared__ unsigned s_img[kNbFillWarps][kNbCap];
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = blockIdx.x * kNbFillWarps + wl;
-  if (w >= g.n_sites) return;
+  const int n_pairs = g.n_sites > 0 ? off[g.n_sites] : 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    status[0] = (unsigned long long)(long long)n_pairs;
+    status[1] = err[0];
+    status[2] = err[1];
+    status[3] = err[1 + w_cells];
+  }
+  if (w >= g.n_sites || n_pairs < 0 || n_pairs > o.n_pairs) return;
   const int a = sites[w];
   const int base = off[w], cnt = off[w + 1] - base - 1;
-  if (a < 0 || a >= g.n_atoms) return;  // reported by the count pass
-  if (cnt > kNbCap) {
-    if (lane == 0) atomicMax(err, kErrTop - ((1ull << 32) + (unsigned long long)w));  // row too long
-    return;
-  }
+  if (a < 0 || a >= g.n_atoms || cnt > kNbCap) return;  // reported by the count pass
   unsigned long long *key = s_key[wl];
   unsigned *img = s_img[wl];
   int filled = 0;
   const unsigned lt = (1u << lane) - 1u;
-  for_each_neighbour(g, pos, atom_cell, cell_start, cell_atoms, a, [&](int j, int nx, int ny, int nz, bool ok) {
+  for_each_neighbour(g, pos, atom_cell, cell_start, cells, a, [&](int j, int nx, int ny, int nz, double r2, bool ok) {
     const unsigned bal = __ballot_sync(0xffffffffu, ok);
     if (ok) {
       const int slot = filled + __popc(bal & lt);
       if (slot < kNbCap) {
-        double dx, dy, dz;
-        image_disp(g, pos, a, j, nx, ny, nz, dx, dy, dz);
-        const float r = (float)sqrt(dx * dx + dy * dy + dz * dz);
+        const float r = (float)sqrt(r2);
         key[slot] = ((unsigned long long)(unsigned)j << 32) | __float_as_uint(r);
-        img[slot] = ((unsigned)(nx + kNbShift) << 20) | ((unsigned)(ny + kNbShift) << 10) |
-                    (unsigned)(nz + kNbShift);
+        img[slot] = (unsigned)pack3(nx, ny, nz);
       }
     }
     filled += __popc(bal);
   });
+  __syncwarp();
   // bitonic sort of the row by (atom, FP32 distance, image translation in x, y, z
   // order): every candidate differs in that triple, so the row's order does not
   // depend on the order the cell list happened to hold the atoms in (padded with
   // the largest key)
-  int npow = 1;
-  while (npow < cnt) npow <<= 1;
-  for (int t = cnt + lane; t < npow; t += 32) {
-    key[t] = ~0ull;
-    img[t] = ~0u;
-  }
-  __syncwarp();
-  for (int k = 2; k <= npow; k <<= 1)
-    for (int jj = k >> 1; jj > 0; jj >>= 1) {
-      for (int t = lane; t < npow; t += 32) {
-        const int p = t ^ jj;
-        if (p > t) {
-          const bool up = (t & k) == 0;
-          const unsigned long long kt = key[t], kp = key[p];
-          const bool gt = kt > kp || (kt == kp && img[t] > img[p]);
-          if (gt == up) {
-            key[t] = kp;
-            key[p] = kt;
-            const unsigned it = img[t];
-            img[t] = img[p];
-            img[p] = it;
+  if (cnt <= 64) {  // each lane ranks its two entries among all: no steps between which the warp waits
+    unsigned long long k0 = lane < cnt ? key[lane] : ~0ull, k1 = lane + 32 < cnt ? key[lane + 32] : ~0ull;
+    const unsigned i0 = lane < cnt ? img[lane] : ~0u, i1 = lane + 32 < cnt ? img[lane + 32] : ~0u;
+    int n0 = 0, n1 = 0;
+#pragma unroll 4
+    for (int t = 0; t < cnt; ++t) {
+      const unsigned long long kt = key[t];
+      const unsigned it = img[t];
+      n0 += kt < k0 || (kt == k0 && it < i0);
+      n1 += kt < k1 || (kt == k1 && it < i1);
+    }
+    __syncwarp();
+    if (lane < cnt) {
+      key[n0] = k0;
+      img[n0] = i0;
+    }
+    if (lane + 32 < cnt) {
+      key[n1] = k1;
+      img[n1] = i1;
+    }
+    __syncwarp();
+  } else {
+    int npow = 1;
+    while (npow < cnt) npow <<= 1;
+    for (int t = cnt + lane; t < npow; t += 32) {
+      key[t] = ~0ull;
+      img[t] = ~0u;
+    }
+    __syncwarp();
+    for (int k = 2; k <= npow; k <<= 1)
+      for (int jj = k >> 1; jj > 0; jj >>= 1) {
+        for (int t = lane; t < npow; t += 32) {
+          const int p = t ^ jj;
+          if (p > t) {
+            const bool up = (t & k) == 0;
+            const unsigned long long kt = key[t], kp = key[p];
+            const bool gt = kt > kp || (kt == kp && img[t] > img[p]);
+            if (gt == up) {
+              key[t] = kp;
+              key[p] = kt;
+              const unsigned it = img[t];
+              img[t] = img[p];
+              img[p] = it;
+            }
           }
         }
+        __syncwarp();
       }
-      __syncwarp();
-    }
+  }
   // the site itself first, then its sorted neighbours
   for (int e = lane - 1; e < cnt; e += 32) {
     const int k = base + 1 + e;
@@ -236,7 +401,8 @@ __global__ void __launch_bounds__(32 * kNbFillWarps) k_nb_fill(NbGeom g, const d
       const int nx = (int)(im >> 20) - kNbShift, ny = (int)((im >> 10) & 1023u) - kNbShift,
                 nz = (int)(im & 1023u) - kNbShift;
       double dx, dy, dz;
-      image_disp(g, pos, a, j, nx, ny, nz, dx, dy, dz);
+      image_disp(g, pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], pos[3 * a], pos[3 * a + 1], pos[3 * a + 2], nx, ny, nz,
+                 dx, dy, dz);
       r = sqrt(dx * dx + dy * dy + dz * dz);
       th = acos(fmin(1.0, fmax(-1.0, dz / r)));
       ph = atan2(dy, dx);
@@ -246,7 +412,7 @@ __global__ void __launch_bounds__(32 * kNbFillWarps) k_nb_fill(NbGeom g, const d
     o.phis[k] = ph;
     o.neigh_atom[k] = j;
     const unsigned bits = mask_bits(g, atom_species, atom_mult, a, j);
-    for (int s = 0; s < g.n_species; ++s) o.mask[(size_t)s * o.n_pairs + k] = (uint8_t)((bits >> s) & 1u);
+    for (int s = 0; s < g.n_species; ++s) o.mask[(size_t)s * n_pairs + k] = (uint8_t)((bits >> s) & 1u);
   }
   if (lane == 0) {
     o.n_neigh[w] = cnt + 1;
@@ -262,33 +428,42 @@ __global__ void __launch_bounds__(256) k_nb_scan(DevBatch B, int tiles, int max_
 
 }  // namespace
 
-cudaError_t launch_nb_bin(const NbGeom &g, const double *pos, int4 *atom_cell, int *cell_count,
-                          unsigned long long *err, cudaStream_t s) {
-  if (g.n_atoms > 0) k_nb_bin<<<(g.n_atoms + 255) / 256, 256, 0, s>>>(g, pos, atom_cell, cell_count, err);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_nb_place(const NbGeom &g, const int4 *atom_cell, const int *cell_start, int *cell_fill,
-                            int *cell_atoms, cudaStream_t s) {
-  if (g.n_atoms > 0) k_nb_place<<<(g.n_atoms + 255) / 256, 256, 0, s>>>(g, atom_cell, cell_start, cell_fill, cell_atoms);
+cudaError_t launch_nb_cells(const NbGeom &g, int n_cells, const double *pos, int4 *atom_cell, int *cell_count,
+                            int *cell_start, int *cell_fill, NbAtom *cells, unsigned long long *err,
+                            unsigned long long *scan_state, int *launches, cudaStream_t s) {
+  if (g.n_atoms <= kNbOneAtoms && n_cells <= kNbOneCells) {
+    k_nb_cells<<<1, kNbOneThreads, 0, s>>>(g, n_cells, pos, atom_cell, cell_start, cells, err);
+    *launches += 1;
+    return cudaGetLastError();
+  }
+  k_nb_bin<<<(g.n_atoms + 255) / 256, 256, 0, s>>>(g, pos, atom_cell, cell_count, err);
+  cudaError_t e = launch_scan(cell_count, n_cells, cell_start, scan_state, s);
+  if (e != cudaSuccess) return e;
+  k_nb_place<<<(g.n_atoms + 255) / 256, 256, 0, s>>>(g, pos, atom_cell, cell_start, cell_fill, cells);
+  *launches += 3;
   return cudaGetLastError();
 }
 
 cudaError_t launch_nb_count(const NbGeom &g, const double *pos, const int *sites, const int4 *atom_cell,
-                            const int *cell_start, const int *cell_atoms, int *counts, unsigned long long *err,
-                            cudaStream_t s) {
-  if (g.n_sites > 0)
-    k_nb_count<<<(g.n_sites + kNbWarps - 1) / kNbWarps, 32 * kNbWarps, 0, s>>>(g, pos, sites, atom_cell, cell_start,
-                                                                               cell_atoms, counts, err);
-  return cudaGetLastError();
+                            const int *cell_start, const NbAtom *cells, int *counts, int *off, int *done,
+                            unsigned long long *err, unsigned long long *scan_state, int *launches, cudaStream_t s) {
+  if (g.n_sites <= 0) return cudaSuccess;
+  const bool one = g.n_sites <= kNbOneSites;
+  k_nb_count<<<(g.n_sites + kNbWarps - 1) / kNbWarps, 32 * kNbWarps, 0, s>>>(
+      g, pos, sites, atom_cell, cell_start, cells, counts, off, one ? done : nullptr, err);
+  *launches += 1;
+  if (one) return cudaGetLastError();
+  *launches += 1;
+  return launch_scan(counts, g.n_sites, off, scan_state, s);
 }
 
 cudaError_t launch_nb_fill(const NbGeom &g, const double *pos, const int *sites, const int *atom_species,
-                           const int *atom_mult, const int4 *atom_cell, const int *cell_start, const int *cell_atoms,
-                           const int *off, const NbOut &o, unsigned long long *err, cudaStream_t s) {
-  if (g.n_sites > 0)
-    k_nb_fill<<<(g.n_sites + kNbFillWarps - 1) / kNbFillWarps, 32 * kNbFillWarps, 0, s>>>(
-        g, pos, sites, atom_species, atom_mult, atom_cell, cell_start, cell_atoms, off, o, err);
+                           const int *atom_mult, const int4 *atom_cell, const int *cell_start, const NbAtom *cells,
+                           const int *off, const NbOut &o, const unsigned long long *err, int w_cells,
+                           unsigned long long *status, cudaStream_t s) {
+  const int blocks = g.n_sites > 0 ? (g.n_sites + kNbFillWarps - 1) / kNbFillWarps : 1;
+  k_nb_fill<<<blocks, 32 * kNbFillWarps, 0, s>>>(g, pos, sites, atom_species, atom_mult, atom_cell, cell_start, cells,
+                                                 off, o, err, w_cells, status);
   return cudaGetLastError();
 }
 
