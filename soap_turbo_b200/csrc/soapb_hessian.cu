@@ -22,7 +22,6 @@ namespace soapb {
 namespace {
 
 constexpr double kPi = 3.14159265358979323846;
-constexpr int kHessThreads = 256;
 constexpr int kHessPC = 16;     // pairs per chunk of pass A
 constexpr int kHessCols = 13;   // k-sums of a unit of pass B at most (odd: the transpose buffer's row stride)
 constexpr int kHessChunk = 256; // pairs whose entries are listed at a time
@@ -394,14 +393,14 @@ struct HessSmem {
   int Z, red, ck, rad, dot, list, total;
   int rows;  // radial indices whose tables it holds
 };
-__host__ __device__ inline HessSmem hess_smem(const DevParams &P, int n_vec) {
+__host__ __device__ inline HessSmem hess_smem(const DevParams &P, int n_vec, int threads) {
   HessSmem S;
   const int N = P.n_max, K = P.k_max, AB = P.amax_t;
-  const int n_red = (kHessThreads / 32) * 32 * kHessCols, n_rad = (kHessThreads / 16) * 4 * AB;
+  const int n_red = threads * kHessCols, n_rad = (threads / 16) * 4 * AB;
   const int n_dot = 4 + 4 * n_vec, n_list = (kHessChunk * P.n_species + 3) / 4, n_ck = K + (K + 1) / 2;
   // pass B: the tables of one weight vector, of every species where two CTAs
   // then still fit an SM, and the warps' transpose buffers
-  int rows = (kHessSmemPair / 8 - n_red - n_rad - n_dot - n_list - n_ck - 4) / (8 * K);
+  int rows = (kHessSmemPair / 8 * (threads / 256) - n_red - n_rad - n_dot - n_list - n_ck - 4) / (8 * K);
   if (rows > N) rows = N;
   if (rows < AB) rows = AB;
   S.rows = rows;
@@ -502,7 +501,8 @@ __device__ __forceinline__ double second_der(const double *S, const double *g, c
 // pair (190 KB each) and Cartesian tensors of Omega formed per k; 1.81 ms with the
 // tables of a species and vector at a time in shared memory, and G beside them, the
 // barriers between them taking a quarter of the time.
-__global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, const DevBatch B, const double *rad,
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) k64_hess(const DevParams P, const DevBatch B, const double *rad,
                                                          const double *rad_der, const double *rad_der2,
                                                          const double *geo, const int *good, const double2 *cnk,
                                                          const double *norm, const double *soap, int n_vec,
@@ -514,10 +514,10 @@ __global__ void __launch_bounds__(kHessThreads, 2) k64_hess(const DevParams P, c
   const int N = P.n_max, K = P.k_max, ns = P.n_soap, nk = P.n_kept, AB = P.amax_t, nsp = P.n_species;
   const int nvh = n_vec + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = lane >> 4, hl = lane & 15;
-  constexpr int NT = kHessThreads, NW = NT / 32;
+  constexpr int NW = NT / 32;
   const size_t sp_sums = (size_t)kSumsFull * nvh + 3 * kSumsLight;
   const GeoLayout Lg(P.l_max);
-  const HessSmem Ly = hess_smem(P, n_vec);
+  const HessSmem Ly = hess_smem(P, n_vec, NT);
   const HessScratch h = carve(scratch + scratch_per_cta * blockIdx.x, P);
   double2 *G = h.G;
   const int RT = Ly.rows, NK = N * K;
@@ -907,21 +907,34 @@ size_t hess_scratch_doubles(const DevParams &P) {
   return (n + 31) / 32 * 32;
 }
 
+int hess_threads(int n_sites);
+
 size_t hess_sums_doubles(int n_vec) { return (size_t)kSumsFull * (n_vec + 1) + 3 * kSumsLight; }
 
 size_t hess_geo_doubles(const DevParams &P) { return (size_t)GeoLayout(P.l_max).size; }
 
-size_t hess_smem_bytes(const DevParams &P, int n_vec) { return sizeof(double) * (size_t)hess_smem(P, n_vec).total; }
+size_t hess_smem_bytes(const DevParams &P, int n_vec, int n_sites) {
+  return sizeof(double) * (size_t)hess_smem(P, n_vec, hess_threads(n_sites)).total;
+}
 
-int hess_grid(const DevParams &P, int n_vec) {
+// 256 threads (two CTAs to an SM) or, where those would not all be resident twice
+// over, 512, for a site's units to be done sooner: 150 sites of one species with five
+// vectors 320 and 308 us.
+int hess_threads(int n_sites) { return n_sites <= 2 * 148 ? 512 : 256; }
+
+template <int NT>
+static int hess_grid_of(const DevParams &P, int n_vec) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const size_t sm = hess_smem_bytes(P, n_vec);
-  auto kern = k64_hess;
+  const size_t sm = sizeof(double) * (size_t)hess_smem(P, n_vec, NT).total;
+  auto kern = k64_hess<NT>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return sms;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kHessThreads, sm);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, sm);
   return sms * (per_sm > 0 ? per_sm : 1);
+}
+int hess_grid(const DevParams &P, int n_vec, int n_sites) {
+  return hess_threads(n_sites) == 512 ? hess_grid_of<512>(P, n_vec) : hess_grid_of<256>(P, n_vec);
 }
 
 cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s, const Fp64Work &w,
@@ -941,12 +954,13 @@ cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s
     if (launches) *launches += 2;
   }
   if (B.n_sites > 0) {
-    const size_t sm = hess_smem_bytes(P, n_vec);
-    auto kern = k64_hess;
+    const size_t sm = hess_smem_bytes(P, n_vec, B.n_sites);
+    const int threads = hess_threads(B.n_sites);
+    auto kern = threads == 512 ? k64_hess<512> : k64_hess<256>;
     CU_RET(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int g = grid < B.n_sites ? grid : B.n_sites;
-    kern<<<g, kHessThreads, sm, s>>>(P, B, w.rad, w.rad_der, rad_der2, geo, good, (const double2 *)w.cnk, w.norm, soap,
-                                     n_vec, vecs, hess, sums, scratch, hess_scratch_doubles(P), ticket);
+    kern<<<g, threads, sm, s>>>(P, B, w.rad, w.rad_der, rad_der2, geo, good, (const double2 *)w.cnk, w.norm, soap,
+                                n_vec, vecs, hess, sums, scratch, hess_scratch_doubles(P), ticket);
     if (launches) *launches += 1;
   }
   return cudaGetLastError();

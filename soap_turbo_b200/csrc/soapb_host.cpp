@@ -1329,8 +1329,8 @@ int ctx_hessian(soapb_context *c, const soapb_batch *b, const double *d_soap, in
     int dev = 0, smem_max = 0;
     CU(cudaGetDevice(&dev));
     CU(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    while (chunk > 1 && hess_smem_bytes(c->P, chunk) > (size_t)smem_max) --chunk;
-    if (hess_smem_bytes(c->P, chunk) > (size_t)smem_max)
+    while (chunk > 1 && hess_smem_bytes(c->P, chunk, b->n_sites) > (size_t)smem_max) --chunk;
+    if (hess_smem_bytes(c->P, chunk, b->n_sites) > (size_t)smem_max)
       return fail(SOAPB_ERR_ARGUMENT, "the Hessian kernel needs more shared memory than the device has");
   }
   if (b->n_atom_pairs > 0 && !d_hess) return fail(SOAPB_ERR_ARGUMENT, "null hess");
@@ -1350,7 +1350,7 @@ int ctx_hessian(soapb_context *c, const soapb_batch *b, const double *d_soap, in
   if ((rc = c->hs_good.ensure(4 * np))) return rc;
   if ((rc = c->hs_soap.ensure(8 * ns * c->n_soap))) return rc;
   if ((rc = c->hs_ticket.ensure(16))) return rc;
-  const int grid = std::max(1, std::min(hess_grid(P, chunk), b->n_sites));
+  const int grid = std::max(1, std::min(hess_grid(P, chunk, b->n_sites), b->n_sites));
   if ((rc = c->hs_scratch.ensure(8 * (size_t)grid * hess_scratch_doubles(P)))) return rc;
   if ((rc = c->hs_sums.ensure(8 * np * hess_sums_doubles(chunk)))) return rc;
   const size_t nsv = (size_t)c->n_soap, npair = (size_t)b->n_atom_pairs, nsite = (size_t)b->n_sites;

@@ -276,8 +276,8 @@ size_t hess_scratch_doubles(const DevParams &P);
 size_t hess_sums_doubles(int n_vec);                   // per pair, of k64_hess's k-sums
 constexpr int kHessVecs = 16;                          // weight vectors of one launch at most
 size_t hess_geo_doubles(const DevParams &P);
-size_t hess_smem_bytes(const DevParams &P, int n_vec);  // dynamic shared memory of k64_hess
-int hess_grid(const DevParams &P, int n_vec);
+size_t hess_smem_bytes(const DevParams &P, int n_vec, int n_sites);  // dynamic shared memory of k64_hess
+int hess_grid(const DevParams &P, int n_vec, int n_sites);
 cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s, const Fp64Work &w,
                            double *rad_der2, double *geo, int *good, const double *soap, int n_vec,
                            const double *vecs, double *hess, double *sums, double *scratch, int grid, int *ticket,
