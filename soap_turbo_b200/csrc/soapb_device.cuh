@@ -624,16 +624,17 @@ __device__ __forceinline__ void plm_array(int lmax, T x, T sq, T (&p)[(LC + 1) *
 }
 
 // ---------------------------------------------------------------- streamed angular stage
-// The same quantities as angular_scalars, written in FP32 to `out` as each one
-// appears so that only the last two terms of each recursion are live in FP64.
-// The amplitude rcut_max^2 / sigma_t^2 is folded into i_l and its derivative:
-//   out[o_il + l] = amp i_l, out[o_ild + l] = amp d i_l / dr (DER),
-//   out[o_e + 2 m], out[o_e + 2 m + 1] = cos(m phi), -sin(m phi), out[o_sf];
-// cos(theta) and sqrt(1 - cos^2) are returned in x, sq.
+// The same quantities as angular_scalars, written in FP32 to `head` and (DER)
+// `tail`, four values at a time, as each four appear so that only the last two
+// terms of each recursion are live in FP64.  The amplitude rcut_max^2 / sigma_t^2
+// is folded into i_l and its derivative.  LC is a multiple of 4.
+//   head: amp i_l for l <= LC, 0, (cos(m phi), -sin(m phi)) for m <= LC
+//   tail: amp d i_l / dr for l <= LC, 2 sigma_t_scaling / sigma_t, cos(theta), sqrt(1 - cos^2)
+// cos(theta) and sqrt(1 - cos^2) are also returned in x, sq.
 template <int LC, bool DER>
 __device__ __forceinline__ void angular_stage(const DevParams &P, int i_sp, double rj, double theta,
-                                              double phi, float *out, int o_il, int o_ild, int o_e,
-                                              int o_sf, double &x, double &sq) {
+                                              double phi, float4 *head, float4 *tail, double &x, double &sq) {
+  static_assert(LC % 4 == 0, "the parts' last four values");
   // The pair kernel rounds everything below to FP32, so the quotients of the
   // reference's expressions are taken as products with one reciprocal each of
   // sigma, x^2 and r (an FP64 division is a long dependent sequence; these are
@@ -665,9 +666,16 @@ __device__ __forceinline__ void angular_stage(const DevParams &P, int i_sp, doub
   const bool dz = !(rj >= 1.0e-5);
   const double irj = dz ? 0.0 : 1.0 / rj;  // one division for every l below
   double fact = 1.0, il_prev = 0.0, il0 = 0.0;
+  float v[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int l = 0; l <= LC + 1; ++l) {
-    if (l > L + 1) break;
+    if (l > L + 1) {  // the four values that l = L + 1 or L is one of
+      if (l <= LC && (l & 3) == 3) {
+        head[l / 4] = make_float4(v[0], v[1], v[2], v[3]);
+        if (DER) tail[l / 4] = make_float4(d[0], d[1], d[2], d[3]);
+      }
+      continue;
+    }
     if (l > 0) fact = fact * (2.0 * (double)l + 1.0);
     double il;
     if (l == 0) {
@@ -686,25 +694,26 @@ __device__ __forceinline__ void angular_stage(const DevParams &P, int i_sp, doub
       flm1 = fl;
       il = fl;
     }
-    if (l <= LC) out[o_il + l] = (float)(amp * il);
+    if (l <= LC) v[l & 3] = (float)(amp * il);
+    if (l <= LC && (l & 3) == 3) head[l / 4] = make_float4(v[0], v[1], v[2], v[3]);
     if (DER) {
       if (l == 0) il0 = il;
-      if (l == 1 && L >= 0) out[o_ild + 0] = dz ? 0.f : (float)(amp * (c1 * (il - il0) * c2));
+      if (l == 1 && L >= 0) d[0] = dz ? 0.f : (float)(amp * (c1 * (il - il0) * c2));
       if (l >= 1 && l <= L && l <= LC)
-        out[o_ild + l] =
+        d[l & 3] =
             dz ? 0.f : (float)(amp * (((-c1 - (double)(2 * l + 2) * irj) * il + c1 * il_prev) * c2));
+      if (l < LC && (l & 3) == 3) tail[l / 4] = make_float4(d[0], d[1], d[2], d[3]);
     }
     il_prev = il;
   }
-  if (DER) out[o_sf] = (float)(2.0 * sc * isig);                         // :589
+  if (DER) tail[LC / 4] = make_float4(d[0], (float)(2.0 * sc * isig), (float)x, (float)sq);  // :589
   // e^{-i m phi}, Chebyshev recursion of get_eimphi_conjg (:284-298)
   double sphi, cphi;
   sincos(phi, &sphi, &cphi);
   double cosm2 = cphi, sinm2 = -sphi;
   const double cosphi2 = 2.0 * cosm2;
   double cosm1 = 1.0, sinm1 = 0.0;
-  out[o_e] = 1.f;
-  out[o_e + 1] = 0.f;
+  head[LC / 4] = make_float4(v[0], 0.f, 1.f, 0.f);
 #pragma unroll
   for (int l = 1; l <= LC; ++l) {
     const double cos0 = cosphi2 * cosm1 - cosm2, sin0 = cosphi2 * sinm1 - sinm2;
@@ -712,8 +721,9 @@ __device__ __forceinline__ void angular_stage(const DevParams &P, int i_sp, doub
     sinm2 = sinm1;
     cosm1 = cos0;
     sinm1 = sin0;
-    out[o_e + 2 * l] = (float)cos0;
-    out[o_e + 2 * l + 1] = (float)(-sin0);
+    v[2 * ((l - 1) & 1)] = (float)cos0;
+    v[2 * ((l - 1) & 1) + 1] = (float)(-sin0);
+    if ((l & 1) == 0) head[LC / 4 + l / 2] = make_float4(v[0], v[1], v[2], v[3]);
   }
 }
 

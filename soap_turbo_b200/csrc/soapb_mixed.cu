@@ -25,6 +25,7 @@
 // runs in an order fixed by the launch shape.
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "soapb_device.cuh"
@@ -208,7 +209,7 @@ __device__ __forceinline__ int first_species(unsigned bits) { return __ffs(bits)
 //   preflm_k P_l^m for l <= l_max (+1 with derivatives), k = l(l+1)/2 + m;
 //   amp di_l/dr, 2 sigma_t_scaling / sigma_t, cos(theta), sqrt(1 - cos^2(theta)).
 // So u_k = amp preflm_k P_k i_l of src/soap_turbo_angular.f90:590-594 is one
-// product of two row values.  LC is even: every part is a multiple of 16 bytes.
+// product of two row values.  LC is a multiple of 4: every part is one of 16 bytes.
 __host__ __device__ constexpr int row_il(int) { return 0; }
 __host__ __device__ constexpr int row_e(int LC) { return LC + 2; }
 __host__ __device__ constexpr int row_p(int LC) { return 3 * LC + 4; }
@@ -220,11 +221,12 @@ __host__ __device__ constexpr int row_sq(int LC) { return row_tail(LC) + LC + 3;
 __host__ __device__ constexpr int row_len(int LC) { return row_tail(LC) + LC + 4; }
 
 int ang_row_floats(const DevParams &P) { return row_len(P.amax_t == 8 ? 8 : 12); }
-// the pair kernel's staging stride in floats (odd): the whole row, or with TAB
-// the larger of its P_l^m values and the rest
-__host__ __device__ constexpr int pair_stage_stride(int LC, bool TAB) {
-  const int np = row_tail(LC) - row_p(LC), rest = row_len(LC) - np;
-  return TAB ? (np > rest ? np : rest) + 1 : row_len(LC) + 1;
+// The pair kernel stages a warp's rows in two parts, head and tail and then the
+// P_l^m values, as four-float pieces; the stride in pieces (odd, so that the lanes'
+// rows start in distinct banks) holds the larger of the two.
+__host__ __device__ constexpr int pair_stage_stride(int LC) {
+  const int np = (row_tail(LC) - row_p(LC)) / 4, rest = row_len(LC) / 4 - np;
+  return (np > rest ? np : rest) | 1;
 }
 
 // ------------------------------------------------------------ pair kernel
@@ -232,8 +234,17 @@ __host__ __device__ constexpr int pair_stage_stride(int LC, bool TAB) {
 //  * the radial expansion of every (pair, species) entry
 //    (src/soap_turbo_radial.f90:281-1004), rounded to FP32 with 4 pi and
 //    global_scaling folded in, into the radial buffer;
-//  * the angular row (src/soap_turbo_angular.f90:267-463, 549-607), staged in
-//    shared memory and copied out with coalesced stores.
+//  * the angular row (src/soap_turbo_angular.f90:267-463, 549-607), staged by the
+//    warp in shared memory, four values at a time, and copied out with coalesced
+//    stores.
+// Bound by instructions (half of the issue slots; 30 % of them index arithmetic)
+// and the warps' waits on tables and FP64 chains.  So a warp shares nothing but the
+// constants with its CTA and takes no barrier after theirs, the table reads of
+// one warp run under the FP64 of others, and the copies' loops are of compile-time
+// length.  Whole-step times with rows staged by value, CTA-wide copies behind
+// barriers and the tables between the two: 128.5 us at 1679 sites, 717 at 16384
+// and 75 at 777 without tables; 124.5, 707 and 72.6 now.  Eight CTAs an SM
+// (64 registers, spills) or CTA-wide copies in this form: 125 and 128.4 us at 1679.
 // The site kernels only read these rows; soap_contract reads the rows of the
 // descriptor call that kept its state, as the reference keeps the radial and
 // angular expansions between get_soap and soap_contract.
@@ -263,118 +274,105 @@ __global__ void __launch_bounds__(kPairThreads)
     order_sites<NT>(B, (int *)smem, (int *)smem + kScanTile);
     return;
   }
-  constexpr int AW = row_len(LC);
-  // odd stride in shared memory: each thread fills its own row, so lanes must
-  // not all map to one bank.  TAB stages the row in two halves (all but the
-  // P_l^m values, then those) through half the buffer, for more CTAs per SM.
-  constexpr int AWS = pair_stage_stride(LC, TAB);
-  constexpr int TO = TAB ? row_tail(LC) - row_p(LC) : 0;  // the row's tail follows its head there
+  constexpr int S4 = pair_stage_stride(LC), AW4 = row_len(LC) / 4, H4 = row_p(LC) / 4, T4 = row_tail(LC) / 4;
+  // what the descriptor alone reads ends here, rounded up to 64 bytes: a row that
+  // stops within a sector is merged with memory's (a descriptor of 32768 atoms
+  // 395 us, with whole rows 375, so 366)
+  constexpr int ND4 = (H4 + ((LC + 1) * (LC + 2) / 2 + 3) / 4 + 3) / 4 * 4;
+  static_assert(ND4 <= T4 && ND4 - H4 <= S4 && H4 + AW4 - T4 <= S4, "the staged pieces");
   const int head = (P.off_rad + P.n_species * SOAPB_RADSP_BYTES) / 16;
   for (int t = threadIdx.x; t < head; t += NT) ((uint4 *)smem)[t] = ((const uint4 *)P.blob)[t];
-  float *rows = (float *)(smem + (size_t)head * 16);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float4 *rows = (float4 *)(smem + (size_t)head * 16) + warp * 32 * S4, *row = rows + lane * S4;
   __syncthreads();
-  const int k0 = pair_lo + ((int)blockIdx.x - lead) * NT;
-  const int k = k0 + threadIdx.x;
+  const int k0 = pair_lo + ((int)blockIdx.x - lead) * NT + 32 * warp;  // the warp's pairs
+  const int k = k0 + lane, nrow = min(32, pair_hi - k0);
   bool active = false;
   double x = 0.0, sq = 0.0;
-  unsigned tab_todo = 0u;  // TAB: the species whose tables this pair is evaluated against
-  double tab_r = 0.0;
-  float *row = rows + threadIdx.x * AWS;
+  unsigned todo = 0u;  // the species whose radial expansion applies
+  double r = 0.0;
   if (k < pair_hi) {
     const unsigned bits = prep_pair(B, k, P.n_species);
-    const double r = B.rjs[k];
+    r = B.rjs[k];
     if (bits != 0u && r < P.rcut_max) {
       active = true;
       const int isp = __ffs(bits) - 1;
       if (do_der)
-        angular_stage<LC, true>(P, isp, r, B.thetas[k], B.phis[k], row, row_il(LC), row_ild(LC) - TO,
-                                row_e(LC), row_sf(LC) - TO, x, sq);
+        angular_stage<LC, true>(P, isp, r, B.thetas[k], B.phis[k], row, row + H4, x, sq);
       else
-        angular_stage<LC, false>(P, isp, r, B.thetas[k], B.phis[k], row, row_il(LC), row_ild(LC) - TO,
-                                 row_e(LC), row_sf(LC) - TO, x, sq);
-      row[row_x(LC) - TO] = (float)x;
-      row[row_sq(LC) - TO] = (float)sq;
-      if constexpr (!TAB) {
-        float *Pr = row + row_p(LC);
-        const float *kpx = (const float *)(smem + P.off_kpx);
-        plm_rows<LC + 1>(P.l_max + (do_der ? 1 : 0), (float)x, (float)sq,
-                         [&](int kk, float v) { Pr[kk] = v * kpx[kk]; });
-      }
-      // the radial expansion of each species in range, as for a neighbour: the
-      // central pair's expansion (:342-355) differs only by the factor
-      // central_weight (:638-646), which the descriptor applies to that entry
-      const double *sW = (const double *)(smem + P.off_W);
-      unsigned todo = 0u;
+        angular_stage<LC, false>(P, isp, r, B.thetas[k], B.phis[k], row, row + H4, x, sq);
       for (int s = 0; s < P.n_species; ++s) {
         const RadSp &RS = *(const RadSp *)(smem + P.off_rad + (size_t)s * SOAPB_RADSP_BYTES);
         if (((bits >> s) & 1u) && r < RS.rcut_hard) todo |= 1u << s;
       }
-      if constexpr (TAB) {
-        tab_todo = todo;
-        tab_r = r;
-        todo = 0u;
-      }
-      // species are data, not control flow: lanes of different species share
-      // one expansion call
-      while (todo) {
-        const int s = __ffs(todo) - 1;
-        todo &= todo - 1u;
-        const RadSp &RS = *(const RadSp *)(smem + P.off_rad + (size_t)s * SOAPB_RADSP_BYTES);
-        float4 *o = (float4 *)(B.rad + ((size_t)k * P.n_species + s) * 2 * AMAX);
-        double val[AMAX], der[AMAX];
-        radial_entry<AMAX, OP>(P, RS, sW + s * AMAX * AMAX, r, false, do_der != 0, val, der);
-        const double g4 = kFourPi * RS.gscale;
-#pragma unroll
-        for (int n4 = 0; n4 < AMAX / 4; ++n4)
-          o[n4] = make_float4((float)(g4 * val[4 * n4]), (float)(g4 * val[4 * n4 + 1]),
-                              (float)(g4 * val[4 * n4 + 2]), (float)(g4 * val[4 * n4 + 3]));
-        if (do_der)
-#pragma unroll
-          for (int n4 = 0; n4 < AMAX / 4; ++n4)
-            o[AMAX / 4 + n4] = make_float4((float)(g4 * der[4 * n4]), (float)(g4 * der[4 * n4 + 1]),
-                                           (float)(g4 * der[4 * n4 + 2]), (float)(g4 * der[4 * n4 + 3]));
-      }
     }
   }
-  if constexpr (TAB) {
+  // the radial expansion of each species in range, as for a neighbour: the
+  // central pair's expansion (:342-355) differs only by the factor
+  // central_weight (:638-646), which the descriptor applies to that entry
+  if constexpr (!TAB) {
+    const double *sW = (const double *)(smem + P.off_W);
+    // species are data, not control flow: lanes of different species share
+    // one expansion call
+    while (todo) {
+      const int s = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      const RadSp &RS = *(const RadSp *)(smem + P.off_rad + (size_t)s * SOAPB_RADSP_BYTES);
+      float4 *o = (float4 *)(B.rad + ((size_t)k * P.n_species + s) * 2 * AMAX);
+      double val[AMAX], der[AMAX];
+      radial_entry<AMAX, OP>(P, RS, sW + s * AMAX * AMAX, r, false, do_der != 0, val, der);
+      const double g4 = kFourPi * RS.gscale;
+#pragma unroll
+      for (int n4 = 0; n4 < AMAX / 4; ++n4)
+        o[n4] = make_float4((float)(g4 * val[4 * n4]), (float)(g4 * val[4 * n4 + 1]),
+                            (float)(g4 * val[4 * n4 + 2]), (float)(g4 * val[4 * n4 + 3]));
+      if (do_der)
+#pragma unroll
+        for (int n4 = 0; n4 < AMAX / 4; ++n4)
+          o[AMAX / 4 + n4] = make_float4((float)(g4 * der[4 * n4]), (float)(g4 * der[4 * n4 + 1]),
+                                         (float)(g4 * der[4 * n4 + 2]), (float)(g4 * der[4 * n4 + 3]));
+    }
+  } else {
     // R_n and dR_n/dr from the tables, a warp's entries of one species at a
     // time: 2 AMAX lanes per entry, lane f evaluating function f, so that the
     // segment's coefficients (stored [degree][function]) are read and the
-    // entry's radial row is written as contiguous 64-byte runs
+    // entry's radial row is written as contiguous 64-byte runs.  kTabUnroll groups
+    // of entries at a time, all their loads before the first product: an entry's
+    // eight coefficients are a round trip to L1 or L2 (one group at a time: steps
+    // of 64 and 16384 sites 37.0 and 725 us, four: 35.6 and 717)
     constexpr int G = 2 * AMAX, EPW = 32 / G;
     static_assert(32 % G == 0, "lanes per entry");
-    const int lane = threadIdx.x & 31, f = lane % G, sub = lane / G;
-    const int nf = do_der ? G : AMAX;
+    const int f = lane % G, sub = lane / G;
+    const bool want = f < (do_der ? G : AMAX);
+    __shared__ int s_who[kPairThreads];
+    int *who = s_who + 32 * warp;
     for (int s = 0; s < P.n_species; ++s) {
-      const bool mine = (tab_todo >> s) & 1u;
-      unsigned m = __ballot_sync(0xffffffffu, mine);
+      const bool mine = (todo >> s) & 1u;
+      const unsigned m = __ballot_sync(0xffffffffu, mine);
       if (!m) continue;
+      const int cnt = __popc(m);
       float t = 0.f;
       int cb = -1;
       if (mine) {
         const RadSp &RS = *(const RadSp *)(smem + P.off_rad + (size_t)s * SOAPB_RADSP_BYTES);
-        cb = radial_table_locate<AMAX>(P, RS, P.rtab_sp[s], tab_r, t);
+        cb = radial_table_locate<AMAX>(P, RS, P.rtab_sp[s], r, t);
+        who[__popc(m & ((1u << lane) - 1u))] = lane;
       }
-      // kTabUnroll groups of entries at a time, all their loads before the first
-      // product: an entry's eight coefficients are a round trip to L1 or L2 (one group at a
-      // time: steps of 64 and 16384 sites 37.0 and 725 us, four: 35.6 and 717)
-      while (m) {
+      __syncwarp();
+      const float *coef = P.rtab_coef + f;
+      float *out = B.rad + ((size_t)k0 * P.n_species + s) * G + f;
+      for (int e0 = sub; e0 - sub < cnt; e0 += kTabUnroll * EPW) {
         int src[kTabUnroll];
         float te[kTabUnroll], a[kTabUnroll][kRadTabDeg + 1];
         bool on[kTabUnroll];
 #pragma unroll
         for (int q = 0; q < kTabUnroll; ++q) {
-          unsigned mm = m;
-#pragma unroll
-          for (int i = 0; i < EPW - 1; ++i)
-            if (i < sub) mm &= mm - 1u;
-#pragma unroll
-          for (int i = 0; i < EPW; ++i) m &= m - 1u;
-          src[q] = mm ? __ffs(mm) - 1 : 0;
-          on[q] = mm && f < nf;
+          const int e = e0 + q * EPW;
+          src[q] = who[min(e, cnt - 1)];
+          on[q] = e < cnt && want;
           const int cbe = __shfl_sync(0xffffffffu, cb, src[q]);
           te[q] = __shfl_sync(0xffffffffu, t, src[q]);
-          const float *c = P.rtab_coef + cbe + f;
+          const float *c = coef + cbe;
 #pragma unroll
           for (int d = 0; d <= kRadTabDeg; ++d) a[q][d] = on[q] && cbe >= 0 ? __ldg(c + d * G) : 0.f;
         }
@@ -383,48 +381,44 @@ __global__ void __launch_bounds__(kPairThreads)
           float v = a[q][kRadTabDeg];
 #pragma unroll
           for (int d = kRadTabDeg - 1; d >= 0; --d) v = fmaf(v, te[q], a[q][d]);
-          const int ke = k0 + (threadIdx.x & ~31) + src[q];
-          if (on[q]) B.rad[((size_t)ke * P.n_species + s) * G + f] = v;
+          if (on[q]) out[src[q] * P.n_species * G] = v;
         }
       }
+      __syncwarp();  // the lanes' list is read
     }
   }
-  __syncthreads();
-  const int nrow = min(NT, pair_hi - k0);
-  if constexpr (TAB) {
-    // coalesced 16-byte stores of the rows' heads and tails, then the P_l^m
-    // values through the same buffer
-    constexpr int H4 = row_p(LC) / 4, T4 = row_tail(LC) / 4, P1 = H4 + (AW / 4 - T4), P2 = T4 - H4;
-    for (int t = threadIdx.x; t < nrow * P1; t += NT) {
-      const int i = t / P1, j = t - i * P1;
-      const float *src = rows + i * AWS + 4 * j;
-      *(float4 *)(B.ang + (size_t)(k0 + i) * AW + 4 * (j < H4 ? j : j - H4 + T4)) =
-          make_float4(src[0], src[1], src[2], src[3]);
+  // pieces 0 .. n - 1 of each of the warp's staged rows to their places in global
+  // memory, from `at` on, those from `from` on `gap` pieces farther
+  auto copy_out = [&](auto pieces, int at, int from, int gap) {
+    constexpr int n = decltype(pieces)::value;
+    float4 *dst = (float4 *)B.ang + (size_t)k0 * AW4 + at;
+#pragma unroll 4
+    for (int t = lane; t < nrow * n; t += 32) {
+      const int i = t / n, j = t - i * n;
+      dst[i * AW4 + j + (j >= from ? gap : 0)] = rows[i * S4 + j];
     }
-    __syncthreads();
-    if (active) {
-      const float *kpx = (const float *)(smem + P.off_kpx);
-      plm_rows<LC + 1>(P.l_max + (do_der ? 1 : 0), (float)x, (float)sq,
-                       [&](int kk, float v) { row[kk] = v * kpx[kk]; });
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < nrow * P2; t += NT) {
-      const int i = t / P2, j = t - i * P2;
-      const float *src = rows + i * AWS + 4 * j;
-      *(float4 *)(B.ang + (size_t)(k0 + i) * AW + row_p(LC) + 4 * j) =
-          make_float4(src[0], src[1], src[2], src[3]);
-    }
-    return;
+  };
+  __syncwarp();
+  if (do_der)
+    copy_out(std::integral_constant<int, H4 + AW4 - T4>(), 0, H4, T4 - H4);
+  else
+    copy_out(std::integral_constant<int, H4>(), 0, H4, 0);
+  __syncwarp();
+  const int l_top = P.l_max + (do_der ? 1 : 0), n_p = (l_top + 1) * (l_top + 2) / 2;
+  if (active) {
+    const float *kpx = (const float *)(smem + P.off_kpx);
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    plm_rows<LC + 1>(l_top, (float)x, (float)sq, [&](int kk, float p) {
+      v[kk & 3] = p * kpx[kk];
+      if ((kk & 3) == 3) row[kk / 4] = make_float4(v[0], v[1], v[2], v[3]);
+    });
+    if (n_p & 3) row[n_p / 4] = make_float4(v[0], v[1], v[2], v[3]);
   }
-  // coalesced 16-byte stores of the CTA's rows (AW is a multiple of 4 floats)
-  constexpr int AW4 = AW / 4;
-  const int n4 = nrow * AW4;
-  float4 *dst = (float4 *)(B.ang + (size_t)k0 * AW);
-  for (int t = threadIdx.x; t < n4; t += NT) {
-    const int i = t / AW4;
-    const float *src = rows + i * AWS + 4 * (t - i * AW4);
-    dst[t] = make_float4(src[0], src[1], src[2], src[3]);
-  }
+  __syncwarp();
+  if (do_der)
+    copy_out(std::integral_constant<int, T4 - H4>(), H4, AW4, 0);
+  else
+    copy_out(std::integral_constant<int, ND4 - H4>(), H4, AW4, 0);
 }
 
 // ------------------------------------------------------------ layouts
@@ -2489,7 +2483,7 @@ template <int AMAX, int LC, bool OP, bool TAB = false>
 static cudaError_t run_pair(const DevParams &P, const DevBatch &B, cudaStream_t s, int do_der, int pair_lo,
                             int pair_hi, bool scan) {
   size_t sm = (size_t)P.off_rad + (size_t)P.n_species * SOAPB_RADSP_BYTES +
-              (size_t)kPairThreads * pair_stage_stride(LC, TAB) * sizeof(float);
+              (size_t)kPairThreads * pair_stage_stride(LC) * sizeof(float4);
   // scan tiles reuse it: the tile's counts, then the site order's buckets
   if (sm < (kScanTile + kScanOrderBuckets) * sizeof(int)) sm = (kScanTile + kScanOrderBuckets) * sizeof(int);
   auto kern = k_pair<AMAX, LC, OP, TAB>;
