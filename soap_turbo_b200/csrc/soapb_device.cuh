@@ -441,11 +441,9 @@ __host__ __device__ __forceinline__ int radial_branch(const DevParams &P, const 
   return (keep ? 1 : 0) | (gm ? 0 : 2);
 }
 
-// R_n (out[0..AMAX)) and, with do_der, dR_n/dr (out[AMAX..2 AMAX)) of one entry
-// from its species' table, 4 pi global_scaling included: the segment and its
-// local coordinate t in FP64, the polynomial by Horner in FP32.
-// The entry's segment: the offset of its coefficients in rtab_coef (floats;
-// -1 where R_n and dR_n/dr are zero) and its local coordinate t in [-1, 1].
+// An entry's segment of its species' table, found in FP64: the offset of its
+// coefficients in rtab_coef (floats; -1 where R_n and dR_n/dr are zero) and the
+// local coordinate t in [-1, 1] of the polynomials, which k_pair takes by Horner.
 template <int AMAX>
 __device__ __forceinline__ int radial_table_locate(const DevParams &P, const RadSp &S, const RadTab &T, double r,
                                                    float &t) {
@@ -457,41 +455,6 @@ __device__ __forceinline__ int radial_table_locate(const DevParams &P, const Rad
   seg = seg < 0 ? 0 : (seg >= T.nseg[st] ? T.nseg[st] - 1 : seg);
   t = (float)(2.0 * (u - (double)seg) - 1.0);
   return (T.base[st] + seg) * (kRadTabDeg + 1) * 2 * AMAX;
-}
-
-template <int AMAX>
-__device__ __forceinline__ void radial_from_table(const DevParams &P, const RadSp &S, const RadTab &T,
-                                                  double r, bool do_der, float (&out)[2 * AMAX]) {
-  float t;
-  const int cb = radial_table_locate<AMAX>(P, S, T, r, t);
-  if (cb < 0) {
-#pragma unroll
-    for (int f = 0; f < 2 * AMAX; ++f) out[f] = 0.f;
-    return;
-  }
-  const float4 *c4 = (const float4 *)(P.rtab_coef + cb);
-  constexpr int F4 = 2 * AMAX / 4;
-  const int nf4 = do_der ? F4 : F4 / 2;
-#pragma unroll
-  for (int j = 0; j < F4; ++j) {
-    if (j < nf4) {
-      float4 a = c4[kRadTabDeg * F4 + j];
-#pragma unroll
-      for (int k = kRadTabDeg - 1; k >= 0; --k) {
-        const float4 b = c4[k * F4 + j];
-        a.x = fmaf(a.x, t, b.x);
-        a.y = fmaf(a.y, t, b.y);
-        a.z = fmaf(a.z, t, b.z);
-        a.w = fmaf(a.w, t, b.w);
-      }
-      out[4 * j] = a.x;
-      out[4 * j + 1] = a.y;
-      out[4 * j + 2] = a.z;
-      out[4 * j + 3] = a.w;
-    } else {
-      out[4 * j] = out[4 * j + 1] = out[4 * j + 2] = out[4 * j + 3] = 0.f;
-    }
-  }
 }
 
 // ---------------------------------------------------------------- angular

@@ -1,25 +1,23 @@
 // soapb_mixed.cu -- the mixed-precision descriptor and force-VJP kernels.
 //
-// One CTA per central site ("environment").  A site's CSR row of neighbour
-// pairs is walked in chunks of NT pairs; each chunk is turned into "entries",
-// one per (pair, species) the radial expansion applies to (mask set, inside
-// that species' rcut_hard, the self pair only when its central weight is
+// k_pair, one thread per pair, does the FP64 work of the path and leaves rows in
+// FP32; the site kernels, one CTA per central site ("environment"), read them.  A
+// site's CSR row of neighbour pairs is walked in chunks; each chunk is turned into
+// "entries", one per (pair, species) the radial expansion applies to (mask set,
+// inside that species' rcut_hard, the self pair only when its central weight is
 // used), sorted by species with ballot ranks so every species' entries are a
 // contiguous run.
 //
-// descriptor (get_soap, src/soap_turbo.f90:491-909):
-//   A. one thread per entry: FP64 radial expansion (R_n, alpha values), the
-//      FP64 angular scalars, FP32 P_l^m; stages 4pi*R_n, e^{-i m phi} and
-//      u_k = amp * preflm_k * P_k * ilexp_l in shared memory.
-//   B. c_nlm: one thread per (species, k) sums its species' entries in CSR
-//      order -- a fixed-order segmented reduction, no atomics.
-//   C. power spectrum of the kept components (a dot product per component),
-//      compression, norm, normalise.
-// contract (soap_contract, src/soap_turbo.f90:1723-1884):
-//   G -> Gp -> Gu -> H(n,k) in shared memory, then one thread per entry
-//   recomputes R_n, dR_n/dr and the four angular factors in registers and
-//   contracts them against H; per-pair forces are rotated to Cartesian and the
-//   self pair gets minus their sum, all in fixed order.
+// k_descriptor (get_soap, src/soap_turbo.f90:491-909): c_nlm with a thread per k
+//   and NH radial indices, each summing its species' entries in CSR order (a
+//   fixed-order segmented reduction, no atomics); the power spectrum of the kept
+//   components (a dot product per component), compression, norm, normalise.
+// k_contract (soap_contract, src/soap_turbo.f90:1723-1884): G -> Gp -> Gu -> H(n,k)
+//   in shared memory, then a half-warp per entry contracts the four angular
+//   factors and R_n, dR_n/dr of its row against H; per-pair forces are rotated to
+//   Cartesian and the self pair gets minus their sum, all in fixed order.
+// k_descriptor_tc, k_contract_tc: the same with the contractions on the tensor
+//   cores, where the caller turns them on.
 //
 // Everything is deterministic: no atomics touch results, and every reduction
 // runs in an order fixed by the launch shape.
@@ -423,11 +421,9 @@ __global__ void __launch_bounds__(kPairThreads)
 
 // ------------------------------------------------------------ layouts
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-// Staged rows are longer than the global ones and stay 16-byte aligned for the
-// asynchronous copies.  The contract (mode 1) pads by 16 floats so that its two
-// half-warps, which read neighbouring rows at the same offsets, use disjoint
-// bank halves; the descriptor reads one row per thread group and pads by 4.
-__host__ __device__ inline int stage_stride(int LC, int mode) { return row_len(LC) + (mode ? 16 : 4); }
+// Staged rows are 16 bytes longer than the global ones: consecutive rows start in
+// distinct bank groups and stay 16-byte aligned for the asynchronous copies.
+__host__ __device__ inline int stage_stride(int LC) { return row_len(LC) + 4; }
 // row stride of H: the species blocks padded to AMAX, plus 4 so that 128-bit
 // loads of consecutive k rows fall in distinct banks
 __host__ __device__ inline int h_stride(int n_species, int AMAX) { return n_species * AMAX + 4; }
@@ -456,8 +452,8 @@ __device__ __forceinline__ const RadSp &rad_of(const unsigned char *smem, const 
   return *(const RadSp *)(smem + (size_t)s * SOAPB_RADSP_BYTES);
 }
 
-// Persistent scheduling: every CTA takes sites from a counter until none are
-// left; which CTA computes a site does not change its result.  The next site
+// Persistent scheduling of the tensor-core kernels: every CTA takes sites from a
+// counter until none are left; which CTA computes a site does not change its result.  The next site
 // is fetched ahead, so that neither the ticket nor the CSR bounds are a round
 // trip between two sites: thread 0 takes the next ticket when a site starts,
 // loads that site's bounds part-way through (ahead_bounds) and hands the three
@@ -512,25 +508,22 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // Copies the rows of entries [ebase, ebase + n_round) of a chunk into the
 // staging area (the angular rows and the radial rows), every 16-byte piece an
 // independent asynchronous copy.  The caller synchronises afterwards.
-template <int NT, int AMAX, int LC, bool DER>
+template <int NT, int AMAX, int LC>
 __device__ __forceinline__ void stage_entries(const DevParams &P, const DevBatch &B, const int *sEnt,
-                                              int chunk, int ebase, int n_round, float *sA,
-                                              float *sR, float *sRd) {
+                                              int chunk, int ebase, int n_round, float *sA, float *sR) {
   constexpr int AW4 = row_len(LC) / 4;
-  const int AS = stage_stride(LC, DER ? 1 : 0);
+  const int AS = stage_stride(LC);
   for (int t = threadIdx.x; t < n_round * AW4; t += NT) {
     const int el = t / AW4, j4 = t - el * AW4;
     const int k = chunk + (sEnt[ebase + el] & 0xffffff);
     cp_async16(sA + (size_t)el * AS + 4 * j4, B.ang + (size_t)k * (4 * AW4) + 4 * j4);
   }
-  constexpr int R4 = AMAX / 4, RW4 = DER ? 2 * R4 : R4;
-  for (int t = threadIdx.x; t < n_round * RW4; t += NT) {
-    const int el = t / RW4, j4 = t - el * RW4;
+  constexpr int R4 = AMAX / 4;
+  for (int t = threadIdx.x; t < n_round * R4; t += NT) {
+    const int el = t / R4, j4 = t - el * R4;
     const int code = sEnt[ebase + el];
     const int k = chunk + (code & 0xffffff), s = code >> 24;
-    const float *src = B.rad + ((size_t)k * P.n_species + s) * 2 * AMAX + 4 * j4;
-    float *dst = (j4 < R4) ? sR + (size_t)el * AMAX + 4 * j4 : sRd + (size_t)el * AMAX + 4 * (j4 - R4);
-    cp_async16(dst, src);
+    cp_async16(sR + (size_t)el * AMAX + 4 * j4, B.rad + ((size_t)k * P.n_species + s) * 2 * AMAX + 4 * j4);
   }
   cp_async_wait_all();
 }
@@ -1113,7 +1106,7 @@ __host__ __device__ inline TdLayout make_td_layout(const DevParams &P, int NT, i
   L.X = o;
   size_t x = o;
   L.R = x; x += kTdGroup * AMAX * sizeof(float);
-  L.A = x; x += kTdGroup * (size_t)stage_stride(LC, 0) * sizeof(float);
+  L.A = x; x += kTdGroup * (size_t)stage_stride(LC) * sizeof(float);
   const size_t end_stage = x;
   x = o;
   L.C = x; x += 2 * (size_t)P.n_max * KS * sizeof(float);
@@ -1133,7 +1126,7 @@ __global__ void __launch_bounds__(NT) k_descriptor_tc(const DevParams P, const D
                                                       double *__restrict__ keep_norm, int keep) {
   static_assert(NT == 128, "one thread per TMEM lane");
   extern __shared__ __align__(16) unsigned char smem[];  // no-swizzle operand tiles need 16-byte alignment
-  const int AS = stage_stride(LC, 0);
+  const int AS = stage_stride(LC);
   const TdLayout Ly = make_td_layout(P, NT, AMAX, LC);
   const int *klm = (const int *)SBLOB(off_klm);
   const int *kept = (const int *)SBLOB(off_kept);
@@ -1200,7 +1193,7 @@ __global__ void __launch_bounds__(NT) k_descriptor_tc(const DevParams P, const D
       for (int ebase = 0; ebase < n_ent; ebase += kTdGroup) {
         const int n_g = min(kTdGroup, n_ent - ebase);
         // ---- the group's rows (angular and radial) into shared memory
-        stage_entries<NT, AMAX, LC, false>(P, B, sEnt, chunk, ebase, n_g, sA, sR, nullptr);
+        stage_entries<NT, AMAX, LC>(P, B, sEnt, chunk, ebase, n_g, sA, sR);
         __syncthreads();
         // the central pair's entries carry central_weight (:638-646)
         if (chunk == p_begin) {
