@@ -234,8 +234,10 @@ int soapb_get_basis(const soapb_context *ctx, double *W, double *S);
 int soapb_n_soap(const soapb_context *ctx, int32_t *n_soap);
 /* Work on this cudaStream_t from now on (0 = legacy default stream). */
 int soapb_set_stream(soapb_context *ctx, void *stream);
-/* Work tuning: threads per site CTA (64, 128 or 256) for both site kernels;
- * 0 returns to the autotuner's choice, or 128 before any autotuning. */
+/* Work tuning: threads per site CTA of the contract (64, 128 or 256), and the
+ * pairs whose entries the descriptor sorts and groups together (its own CTA size
+ * follows the number of sites); 0 returns to the autotuner's choice, or before any
+ * autotuning to a rule on the number of sites and 128 pairs. */
 int soapb_set_threads_per_site(soapb_context *ctx, int32_t threads);
 /* Autotuner: times the descriptor and the contract on this batch in each form
  * -- the tensor-core kernels (when allowed, see soapb_set_tensor_cores) and the
@@ -336,9 +338,9 @@ int soapb_descriptor_fp64(soapb_context *ctx, const soapb_batch *batch, double *
  * (3, 3, n_vec, n_pairs), layouts as there.  FP64; it recomputes the FP64
  * expansion state of the batch, so it needs no earlier call.  d_soap is the
  * normalised descriptor the weights were formed against (NULL: the FP64 one
- * this call computes).  Needs legacy_filter_seed = 0 (SOAPB_ERR_ARGUMENT).  More weight
- * vectors than the kernel's shared memory holds at once (about 90 for the benchmark
- * definition) are done in chunks, with two strided device copies per chunk. */
+ * this call computes).  Needs legacy_filter_seed = 0 (SOAPB_ERR_ARGUMENT).  More than
+ * 16 weight vectors (fewer where shared memory holds fewer) are done in chunks of
+ * as many, with two strided device copies per chunk. */
 int soapb_central_hessian(soapb_context *ctx, const soapb_batch *batch, const double *d_soap,
                           int32_t n_vec, const double *d_vecs, double *d_hess);
 
