@@ -26,8 +26,8 @@ namespace soapb {
 
 namespace {
 
-constexpr int kNbWarps = 4;      // warps (sites) per CTA of the count kernel
-constexpr int kNbFillWarps = 2;  // warps (sites) per CTA of the fill kernel (its rows sit in shared memory)
+constexpr int kNbWarps = 4;      // warps per CTA of the count kernel
+constexpr int kNbFillWarps = 2;  // warps per CTA of the fill kernel where each has a site (its rows sit in shared memory)
 constexpr int kNbShift = 512;    // image components are stored as n + kNbShift in 10 bits
 constexpr int kNbOneThreads = 1024;
 static_assert(kNbMaxReach + 1 + 2 * kNbMaxWrap < kNbShift, "image translations must fit 10 bits");
@@ -153,10 +153,12 @@ __global__ void k_nb_place(NbGeom g, const double *pos, const int4 *atom_cell, c
 // Visits every candidate image of a site's stencil: visit(j, nx, ny, nz, r2, ok)
 // is called by all lanes of the warp together (ok false on padding lanes), so
 // it may use warp collectives.  A run is the stencil's cells of one x, y and wrap
-// in z, contiguous in the cell order; 32 runs are laid end to end at a time.
+// in z, contiguous in the cell order; 32 runs are laid end to end at a time.  Of
+// `parts` warps that share the site, warp `part` takes every parts-th 64 candidates.
 template <typename Visit>
 __device__ __forceinline__ void for_each_neighbour(const NbGeom &g, const double *pos, const int4 *atom_cell,
-                                                   const int *cell_start, const NbAtom *cells, int a, Visit visit) {
+                                                   const int *cell_start, const NbAtom *cells, int a, int part,
+                                                   int parts, Visit visit) {
   const int lane = threadIdx.x & 31;
   const int4 ca = atom_cell[a];
   const double xi = pos[3 * a], yi = pos[3 * a + 1], zi = pos[3 * a + 2];
@@ -184,7 +186,7 @@ __device__ __forceinline__ void for_each_neighbour(const NbGeom &g, const double
     }
     const int total = __shfl_sync(0xffffffffu, incl, 31);
     // two candidates a lane at a time, so that their loads overlap
-    for (int c0 = 0; c0 < total; c0 += 64) {
+    for (int c0 = 64 * part; c0 < total; c0 += 64 * parts) {
       NbAtom b[2];
       int w[2];
 #pragma unroll
@@ -222,31 +224,36 @@ __device__ __forceinline__ void for_each_neighbour(const NbGeom &g, const double
   }
 }
 
-// ---- pass 1: neighbours of each site (the row length is one more: the site itself).
+// ---- pass 1: neighbours of each site (the row length is one more: the site itself),
+// by W warps.
 // done (may be null): the CTAs finished; the last one then scans the counts of up to
 // kNbOneSites sites into the CSR offsets.
+template <int W>
 __global__ void __launch_bounds__(32 * kNbWarps) k_nb_count(NbGeom g, const double *pos, const int *sites,
                                                             const int4 *atom_cell, const int *cell_start,
                                                             const NbAtom *cells, int *counts, int *off, int *done,
                                                             unsigned long long *err) {
   constexpr int NT = 32 * kNbWarps;
-  const int w = blockIdx.x * kNbWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (w < g.n_sites) {
-    const int a = sites[w];
-    int cnt = 0;
+  const int warp = threadIdx.x >> 5, w = blockIdx.x * (kNbWarps / W) + warp / W, lane = threadIdx.x & 31;
+  __shared__ int s_cnt[kNbWarps];
+  int cnt = 0;
+  const int a = w < g.n_sites ? sites[w] : -1;
+  if (a >= 0 && a < g.n_atoms)
+    for_each_neighbour(g, pos, atom_cell, cell_start, cells, a, warp % W, W,
+                       [&](int, int, int, int, double, bool ok) { cnt += __popc(__ballot_sync(0xffffffffu, ok)); });
+  if (W > 1) {
+    if (lane == 0) s_cnt[warp] = cnt;
+    __syncthreads();
+    if (warp % W == 0)
+#pragma unroll
+      for (int v = 1; v < W; ++v) cnt += s_cnt[warp + v];
+  }
+  if (lane == 0 && warp % W == 0 && w < g.n_sites) {
     unsigned long long bad = 0ull;
-    if (a < 0 || a >= g.n_atoms) {
-      bad = kErrTop - (unsigned long long)w;  // site index out of range
-    } else {
-      for_each_neighbour(g, pos, atom_cell, cell_start, cells, a, [&](int, int, int, int, double, bool ok) {
-        cnt += __popc(__ballot_sync(0xffffffffu, ok));
-      });
-      if (cnt > kNbCap) bad = kErrTop - ((1ull << 32) + (unsigned long long)w);  // row too long
-    }
-    if (lane == 0) {
-      counts[w] = 1 + cnt;
-      if (bad) atomicMax(err, bad);
-    }
+    if (a < 0 || a >= g.n_atoms) bad = kErrTop - (unsigned long long)w;  // site index out of range
+    else if (cnt > kNbCap) bad = kErrTop - ((1ull << 32) + (unsigned long long)w);  // row too long
+    counts[w] = 1 + cnt;
+    if (bad) atomicMax(err, bad);
   }
   if (!done) return;
   __shared__ int s_last;
@@ -293,20 +300,30 @@ __device__ __forceinline__ unsigned mask_bits(const NbGeom &g, const int *atom_s
   return bits;
 }
 
-// ---- pass 2: each site's row, sorted by (neighbour atom, distance).  The pair count
+// ---- pass 2: each site's row, sorted by (neighbour atom, distance), by W warps.
+// Bound by latency: the candidates' loads and the FP64 chain of a pair's distance and
+// angles, with few warps on an SM (40 us at 1679 sites of one warp each; the step
+// from positions 234 us so, 223 with two).  The pair count
 // comes from the offsets; nothing is written where it is above the buffers'
 // capacity, o.n_pairs (the host then makes room and launches again).  status, in
 // page-locked host memory, receives the pair count and the three error words.
-__global__ void __launch_bounds__(32 * kNbFillWarps) k_nb_fill(NbGeom g, const double *pos, const int *sites,
+template <int W>
+__global__ void __launch_bounds__(W > kNbFillWarps ? 32 * W : 32 * kNbFillWarps) k_nb_fill(NbGeom g, const double *pos, const int *sites,
                                                            const int *atom_species, const int *atom_mult,
                                                            const int4 *atom_cell, const int *cell_start,
                                                            const NbAtom *cells, const int *off, NbOut o,
                                                            const unsigned long long *err, int w_cells,
                                                            volatile unsigned long long *status) {
-  __shared__ unsigned long long s_key[kNbFillWarps][kNbCap];
-  __shared__ unsigned s_img[kNbFillWarps][kNbCap];
-  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w = blockIdx.x * kNbFillWarps + wl;
+  constexpr int S = W > 1 ? 1 : kNbFillWarps, NT = 32 * W;  // sites of the CTA, threads of a site
+  __shared__ unsigned long long s_key[S][kNbCap];
+  __shared__ unsigned s_img[S][kNbCap];
+  __shared__ int s_filled;
+  const int wl = W > 1 ? 0 : threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x % NT;
+  const int w = blockIdx.x * S + wl;
+  auto sync = [] {
+    if (W > 1) __syncthreads();
+    else __syncwarp();
+  };
   const int n_pairs = g.n_sites > 0 ? off[g.n_sites] : 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     status[0] = (unsigned long long)(long long)n_pairs;
@@ -321,9 +338,18 @@ __global__ void __launch_bounds__(32 * kNbFillWarps) k_nb_fill(NbGeom g, const d
   unsigned long long *key = s_key[wl];
   unsigned *img = s_img[wl];
   int filled = 0;
+  if (W > 1) {
+    if (tid == 0) s_filled = 0;
+    __syncthreads();
+  }
   const unsigned lt = (1u << lane) - 1u;
-  for_each_neighbour(g, pos, atom_cell, cell_start, cells, a, [&](int j, int nx, int ny, int nz, double r2, bool ok) {
+  for_each_neighbour(g, pos, atom_cell, cell_start, cells, a, tid >> 5, W,
+                     [&](int j, int nx, int ny, int nz, double r2, bool ok) {
     const unsigned bal = __ballot_sync(0xffffffffu, ok);
+    if (W > 1) {
+      if (lane == 0 && bal) filled = atomicAdd(&s_filled, __popc(bal));
+      filled = __shfl_sync(0xffffffffu, filled, 0);
+    }
     if (ok) {
       const int slot = filled + __popc(bal & lt);
       if (slot < kNbCap) {
@@ -332,45 +358,50 @@ __global__ void __launch_bounds__(32 * kNbFillWarps) k_nb_fill(NbGeom g, const d
         img[slot] = (unsigned)pack3(nx, ny, nz);
       }
     }
-    filled += __popc(bal);
+    if (W == 1) filled += __popc(bal);
   });
-  __syncwarp();
-  // bitonic sort of the row by (atom, FP32 distance, image translation in x, y, z
-  // order): every candidate differs in that triple, so the row's order does not
-  // depend on the order the cell list happened to hold the atoms in (padded with
-  // the largest key)
-  if (cnt <= 64) {  // each lane ranks its two entries among all: no steps between which the warp waits
-    unsigned long long k0 = lane < cnt ? key[lane] : ~0ull, k1 = lane + 32 < cnt ? key[lane + 32] : ~0ull;
-    const unsigned i0 = lane < cnt ? img[lane] : ~0u, i1 = lane + 32 < cnt ? img[lane + 32] : ~0u;
-    int n0 = 0, n1 = 0;
+  sync();
+  // the row sorted by (atom, FP32 distance, image translation in x, y, z order):
+  // every candidate differs in that triple, so the row's order does not depend on
+  // the order the cell list happened to hold the atoms in or the warps found them
+  if (cnt <= 64) {  // each thread ranks its entries among all: no steps between which the site waits
+    constexpr int PER = NT < 64 ? 64 / NT : 1;
+    unsigned long long k[PER];
+    unsigned im[PER];
+    int n[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      k[i] = tid + i * NT < cnt ? key[tid + i * NT] : ~0ull;
+      im[i] = tid + i * NT < cnt ? img[tid + i * NT] : ~0u;
+      n[i] = 0;
+    }
+    if (NT <= 64 || tid < 64)
 #pragma unroll 4
-    for (int t = 0; t < cnt; ++t) {
-      const unsigned long long kt = key[t];
-      const unsigned it = img[t];
-      n0 += kt < k0 || (kt == k0 && it < i0);
-      n1 += kt < k1 || (kt == k1 && it < i1);
-    }
-    __syncwarp();
-    if (lane < cnt) {
-      key[n0] = k0;
-      img[n0] = i0;
-    }
-    if (lane + 32 < cnt) {
-      key[n1] = k1;
-      img[n1] = i1;
-    }
-    __syncwarp();
-  } else {
+      for (int t = 0; t < cnt; ++t) {
+        const unsigned long long kt = key[t];
+        const unsigned it = img[t];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) n[i] += kt < k[i] || (kt == k[i] && it < im[i]);
+      }
+    sync();
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (tid + i * NT < cnt) {
+        key[n[i]] = k[i];
+        img[n[i]] = im[i];
+      }
+    sync();
+  } else {  // a bitonic sort, padded with the largest key
     int npow = 1;
     while (npow < cnt) npow <<= 1;
-    for (int t = cnt + lane; t < npow; t += 32) {
+    for (int t = cnt + tid; t < npow; t += NT) {
       key[t] = ~0ull;
       img[t] = ~0u;
     }
-    __syncwarp();
+    sync();
     for (int k = 2; k <= npow; k <<= 1)
       for (int jj = k >> 1; jj > 0; jj >>= 1) {
-        for (int t = lane; t < npow; t += 32) {
+        for (int t = tid; t < npow; t += NT) {
           const int p = t ^ jj;
           if (p > t) {
             const bool up = (t & k) == 0;
@@ -385,11 +416,11 @@ __global__ void __launch_bounds__(32 * kNbFillWarps) k_nb_fill(NbGeom g, const d
             }
           }
         }
-        __syncwarp();
+        sync();
       }
   }
   // the site itself first, then its sorted neighbours
-  for (int e = lane - 1; e < cnt; e += 32) {
+  for (int e = tid - 1; e < cnt; e += NT) {
     const int k = base + 1 + e;
     int j;
     double r = 0.0, th = 0.0, ph = 0.0;
@@ -414,11 +445,11 @@ __global__ void __launch_bounds__(32 * kNbFillWarps) k_nb_fill(NbGeom g, const d
     const unsigned bits = mask_bits(g, atom_species, atom_mult, a, j);
     for (int s = 0; s < g.n_species; ++s) o.mask[(size_t)s * n_pairs + k] = (uint8_t)((bits >> s) & 1u);
   }
-  if (lane == 0) {
+  if (tid == 0) {
     o.n_neigh[w] = cnt + 1;
     o.species_mult[w] = atom_mult[a];
   }
-  for (int m = lane; m < g.max_mult; m += 32) o.species[(size_t)w * g.max_mult + m] = atom_species[(size_t)a * g.max_mult + m];
+  for (int m = tid; m < g.max_mult; m += NT) o.species[(size_t)w * g.max_mult + m] = atom_species[(size_t)a * g.max_mult + m];
 }
 
 __global__ void __launch_bounds__(256) k_nb_scan(DevBatch B, int tiles, int max_spins) {
@@ -427,6 +458,26 @@ __global__ void __launch_bounds__(256) k_nb_scan(DevBatch B, int tiles, int max_
 }
 
 }  // namespace
+
+// Warps that share a site in the count and the fill: the number with the cheapest
+// waves of the fill (18, 14 and 7 sites fit an SM at 1, 2 and 4 warps), a site at 2
+// and 4 warps taking 0.8 and 0.7 of its time at one.  Builds at 1, 2 and 4 warps, us:
+// 64 sites 124, 106, 99; 600 96, 89, 85; 1200 98, 90, 101; 1700 101, 97, 105; 2400 107,
+// 114, 120; 8000 177, 168, 199; 32768 382, 380, 515.
+static int nb_warps(int n_sites) {
+  const int slots[3] = {148 * 18, 148 * 14, 148 * 7};
+  const double cost[3] = {1.0, 0.8, 0.7};
+  int best = 0;
+  double least = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    const double t = ((n_sites - 1) / slots[i] + 1) * cost[i];
+    if (i == 0 || t < least) {
+      least = t;
+      best = i;
+    }
+  }
+  return 1 << best;
+}
 
 cudaError_t launch_nb_cells(const NbGeom &g, int n_cells, const double *pos, int4 *atom_cell, int *cell_count,
                             int *cell_start, int *cell_fill, NbAtom *cells, unsigned long long *err,
@@ -449,8 +500,10 @@ cudaError_t launch_nb_count(const NbGeom &g, const double *pos, const int *sites
                             unsigned long long *err, unsigned long long *scan_state, int *launches, cudaStream_t s) {
   if (g.n_sites <= 0) return cudaSuccess;
   const bool one = g.n_sites <= kNbOneSites;
-  k_nb_count<<<(g.n_sites + kNbWarps - 1) / kNbWarps, 32 * kNbWarps, 0, s>>>(
-      g, pos, sites, atom_cell, cell_start, cells, counts, off, one ? done : nullptr, err);
+  const int W = nb_warps(g.n_sites), per = kNbWarps / W;
+  auto kern = W == 4 ? k_nb_count<4> : W == 2 ? k_nb_count<2> : k_nb_count<1>;
+  kern<<<(g.n_sites + per - 1) / per, 32 * kNbWarps, 0, s>>>(g, pos, sites, atom_cell, cell_start, cells, counts, off,
+                                                             one ? done : nullptr, err);
   *launches += 1;
   if (one) return cudaGetLastError();
   *launches += 1;
@@ -461,9 +514,11 @@ cudaError_t launch_nb_fill(const NbGeom &g, const double *pos, const int *sites,
                            const int *atom_mult, const int4 *atom_cell, const int *cell_start, const NbAtom *cells,
                            const int *off, const NbOut &o, const unsigned long long *err, int w_cells,
                            unsigned long long *status, cudaStream_t s) {
-  const int blocks = g.n_sites > 0 ? (g.n_sites + kNbFillWarps - 1) / kNbFillWarps : 1;
-  k_nb_fill<<<blocks, 32 * kNbFillWarps, 0, s>>>(g, pos, sites, atom_species, atom_mult, atom_cell, cell_start, cells,
-                                                 off, o, err, w_cells, status);
+  const int W = nb_warps(g.n_sites), per = W > 1 ? 1 : kNbFillWarps;
+  const int blocks = g.n_sites > 0 ? (g.n_sites + per - 1) / per : 1;
+  auto kern = W == 4 ? k_nb_fill<4> : W == 2 ? k_nb_fill<2> : k_nb_fill<1>;
+  kern<<<blocks, W > 1 ? 32 * W : 32 * kNbFillWarps, 0, s>>>(g, pos, sites, atom_species, atom_mult, atom_cell,
+                                                             cell_start, cells, off, o, err, w_cells, status);
   return cudaGetLastError();
 }
 

@@ -167,7 +167,9 @@ def test_neighbour_list_at_the_lines_of_its_rules():
     ctx = Context(syn.Hyper(alpha_max=[4, 4], l_max=4, basis="poly3"))
     for n_atoms, side, spacing, n_sites in [(343, 7, 2.0, 343), (8192, 21, 2.0, 4096), (8193, 21, 2.0, 4097),
                                             (8192, 21, 2.0, 8192), (600, 23, 5.0, 600), (343, 7, 2.0, 5),
-                                            (2744, 14, 1.9, 1)]:
+                                            (2744, 14, 1.9, 1), (4096, 16, 2.0, 1036), (4096, 16, 2.0, 1037),
+                                            (4096, 16, 2.0, 2072), (4096, 16, 2.0, 2073), (4096, 16, 2.0, 2664),
+                                            (4096, 16, 2.0, 2665)]:
         st = lattice_atoms(n_atoms, side, spacing, n_sites, seed=n_atoms + n_sites)
         nl = syn.neighbour_list(st, 5.0, 2, central_species=0)
         _, a = built(ctx, st.positions, np.eye(3) * st.box, st.species + 1, nl.site_atom)
