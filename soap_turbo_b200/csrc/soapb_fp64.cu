@@ -15,9 +15,8 @@ constexpr double kFourPi64 = 12.566370614359172954;
 
 // ---- radial, one thread per pair, every species block (:491-544)
 template <int AMAX, bool OP>
-__global__ void k64_radial(const DevParams P, const DevBatch B, int do_der, double *rad,
-                           double *rad_der) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void radial_pair64(const DevParams &P, const DevBatch &B, int k, int do_der, double *rad,
+                                              double *rad_der) {
   if (k >= B.n_pairs) return;
   // site-local index: binary search of the CSR offsets
   int lo = 0, hi = B.n_sites;
@@ -52,6 +51,11 @@ __global__ void k64_radial(const DevParams P, const DevBatch B, int do_der, doub
       if (do_der) rdo[S.nbeg + n] = der[n] * S.gscale;
     }
   }
+}
+
+template <int AMAX, bool OP>
+__global__ void k64_radial(const DevParams P, const DevBatch B, int do_der, double *rad, double *rad_der) {
+  radial_pair64<AMAX, OP>(P, B, blockIdx.x * blockDim.x + threadIdx.x, do_der, rad, rad_der);
 }
 
 // ---- angular, one thread per pair (src/soap_turbo_angular.f90:549-607)
@@ -117,9 +121,7 @@ __global__ void k64_angular(const DevParams P, const DevBatch B, int do_der, dou
 // and polar derivative), so that a pair's four planes are formed at once;
 // without, one warp writes the expansion.  Same arithmetic as k64_angular.
 template <int LC>
-__global__ void __launch_bounds__(128, 4) k64_angular2(const DevParams P, const DevBatch B, int do_der, double2 *ang) {
-  const int pl = do_der ? (int)(threadIdx.x >> 5) : 0;  // warp-uniform
-  const int k = blockIdx.x * 32 + (threadIdx.x & 31);
+__device__ __forceinline__ void angular_plane64(const DevParams &P, const DevBatch &B, int k, int pl, double2 *ang) {
   if (k >= B.n_pairs) return;
   const int K = P.k_max, L = P.l_max;
   const size_t plane = (size_t)B.n_pairs * K;
@@ -193,6 +195,24 @@ __global__ void __launch_bounds__(128, 4) k64_angular2(const DevParams P, const 
       pn[m] = nn[m];
     }
   }
+}
+
+// Both expansions in one launch, l_max <= 8: the first n_rad CTAs take 128 pairs'
+// radial ones, the others the angular planes.  Each is bound by the FP64 chain of a pair
+// (15 and 18 % of the issue slots): beside one another they take the time of the
+// longer.  One after the other: soap_cart_der with its contraction 430 us at 425
+// sites, 151 at 100; so 403 and 138.  Four CTAs an SM (128 registers, spills): 406 and 141.
+template <int AMAX, bool OP>
+__global__ void __launch_bounds__(128, 3)
+    k64_expand(const DevParams P, const DevBatch B, int n_rad, int do_der, int ang_der, double *rad, double *rad_der,
+               double2 *ang) {
+  const int b = (int)blockIdx.x - n_rad, tid = threadIdx.x;
+  if (b < 0) {
+    radial_pair64<AMAX, OP>(P, B, blockIdx.x * 128 + tid, do_der, rad, rad_der);
+    return;
+  }
+  const int pl = ang_der ? tid >> 5 : 0;  // warp-uniform
+  angular_plane64<8>(P, B, ang_der ? b * 32 + (tid & 31) : b * 128 + tid, pl, ang);
 }
 
 // ---- c_nlm, power spectrum, compression and norm, one CTA per site
@@ -1431,17 +1451,20 @@ cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaSt
   int nl = 0;
   if (np > 0) {
     const int blocks = (np + 127) / 128;
-    const bool op = P.basis == kBasisOperator;
-    if (max_alpha64(P) <= 8) {
-      if (op) k64_radial<8, true><<<blocks, 128, 0, s>>>(P, B, do_der, w.rad, w.rad_der);
-      else k64_radial<8, false><<<blocks, 128, 0, s>>>(P, B, do_der, w.rad, w.rad_der);
+    const bool op = P.basis == kBasisOperator, narrow = max_alpha64(P) <= 8;
+    if (P.l_max <= 8) {
+      auto kern = narrow ? (op ? k64_expand<8, true> : k64_expand<8, false>)
+                         : (op ? k64_expand<16, true> : k64_expand<16, false>);
+      const int n_ang = ang_der ? (np + 31) / 32 : blocks;
+      kern<<<blocks + n_ang, 128, 0, s>>>(P, B, blocks, do_der, ang_der, w.rad, w.rad_der, (double2 *)w.ang);
+      nl += 1;
     } else {
-      if (op) k64_radial<16, true><<<blocks, 128, 0, s>>>(P, B, do_der, w.rad, w.rad_der);
-      else k64_radial<16, false><<<blocks, 128, 0, s>>>(P, B, do_der, w.rad, w.rad_der);
+      auto kern = narrow ? (op ? k64_radial<8, true> : k64_radial<8, false>)
+                         : (op ? k64_radial<16, true> : k64_radial<16, false>);
+      kern<<<blocks, 128, 0, s>>>(P, B, do_der, w.rad, w.rad_der);
+      k64_angular<12><<<blocks, 128, 0, s>>>(P, B, ang_der, (double2 *)w.ang);
+      nl += 2;
     }
-    if (P.l_max <= 8) k64_angular2<8><<<(np + 31) / 32, ang_der ? 128 : 32, 0, s>>>(P, B, ang_der, (double2 *)w.ang);
-    else k64_angular<12><<<blocks, 128, 0, s>>>(P, B, ang_der, (double2 *)w.ang);
-    nl += 2;
   }
   const size_t sms = (size_t)site_smem(P).total * sizeof(double);
   const int items = (site_items(P) + kSiteThreads - 1) / kSiteThreads;
