@@ -116,10 +116,10 @@ __global__ void k64_angular(const DevParams P, const DevBatch B, int do_der, dou
 // l and l + 1 only (the recursion of get_plm_array, src/soap_turbo_angular.f90:
 // 108-160), every loop unrolled so that they stay in registers, and each (l, m)
 // written as soon as rows l and l + 1 exist (the derivative forms need
-// P_{l+1}^{m+-1}, :181-248).  With derivatives the CTA is four warps over the
-// same 32 pairs, warp w writing plane w (the expansion, its radial, azimuthal
-// and polar derivative), so that a pair's four planes are formed at once;
-// without, one warp writes the expansion.  Same arithmetic as k64_angular.
+// P_{l+1}^{m+-1}, :181-248).  A thread writes one plane of a pair: the expansion
+// or its radial, azimuthal or polar derivative.  With derivatives a CTA is four warps
+// over the same 32 pairs, warp w writing plane w, so that a pair's four planes are
+// formed at once.  Same arithmetic as k64_angular.
 template <int LC>
 __device__ __forceinline__ void angular_plane64(const DevParams &P, const DevBatch &B, int k, int pl, double2 *ang) {
   if (k >= B.n_pairs) return;

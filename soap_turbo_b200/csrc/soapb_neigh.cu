@@ -13,7 +13,7 @@
 // copied in cell order, so the cells of one (x, y) column of a site's stencil are
 // one run of them, and a warp takes a site's runs end to end, a candidate per lane.
 // Two passes: count (whose last CTA scans the counts into CSR offsets where the
-// sites are few), then fill.  One warp per site; the fill pass gathers the site's
+// sites are few), then fill.  One to four warps per site; the fill gathers the site's
 // row in shared memory and sorts it by (neighbour atom, distance) so the order
 // depends on nothing but the inputs.
 // What bounds it, at some thousand atoms: the launches and each pass's chain of
@@ -308,7 +308,8 @@ __device__ __forceinline__ unsigned mask_bits(const NbGeom &g, const int *atom_s
 // capacity, o.n_pairs (the host then makes room and launches again).  status, in
 // page-locked host memory, receives the pair count and the three error words.
 template <int W>
-__global__ void __launch_bounds__(W > kNbFillWarps ? 32 * W : 32 * kNbFillWarps) k_nb_fill(NbGeom g, const double *pos, const int *sites,
+__global__ void __launch_bounds__(W > kNbFillWarps ? 32 * W : 32 * kNbFillWarps)
+    k_nb_fill(NbGeom g, const double *pos, const int *sites,
                                                            const int *atom_species, const int *atom_mult,
                                                            const int4 *atom_cell, const int *cell_start,
                                                            const NbAtom *cells, const int *off, NbOut o,
