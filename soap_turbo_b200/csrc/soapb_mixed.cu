@@ -303,34 +303,39 @@ __global__ void __launch_bounds__(kPairThreads)
         const RadSp &RS = *(const RadSp *)(smem + P.off_rad + (size_t)s * SOAPB_RADSP_BYTES);
         if (((bits >> s) & 1u) && r < RS.rcut_hard) todo |= 1u << s;
       }
+      // the radial expansion of each species in range, as for a neighbour: the
+      // central pair's expansion (:342-355) differs only by the factor
+      // central_weight (:638-646), which the descriptor applies to that entry.  It
+      // stands inside the branch for its bits: after it, the compiler fuses other
+      // products into multiply-adds in k_pair<8, 8, false, false>, and up to 2e-4 of the
+      // values (which W's cancellation amplifies) come out one or more FP32 ulps apart
+      // from the other instantiation's
+      if constexpr (!TAB) {
+        const double *sW = (const double *)(smem + P.off_W);
+        // species are data, not control flow: lanes of different species share
+        // one expansion call
+        while (todo) {
+          const int s = __ffs(todo) - 1;
+          todo &= todo - 1u;
+          const RadSp &RS = *(const RadSp *)(smem + P.off_rad + (size_t)s * SOAPB_RADSP_BYTES);
+          float4 *o = (float4 *)(B.rad + ((size_t)k * P.n_species + s) * 2 * AMAX);
+          double val[AMAX], der[AMAX];
+          radial_entry<AMAX, OP>(P, RS, sW + s * AMAX * AMAX, r, false, do_der != 0, val, der);
+          const double g4 = kFourPi * RS.gscale;
+#pragma unroll
+          for (int n4 = 0; n4 < AMAX / 4; ++n4)
+            o[n4] = make_float4((float)(g4 * val[4 * n4]), (float)(g4 * val[4 * n4 + 1]),
+                                (float)(g4 * val[4 * n4 + 2]), (float)(g4 * val[4 * n4 + 3]));
+          if (do_der)
+#pragma unroll
+            for (int n4 = 0; n4 < AMAX / 4; ++n4)
+              o[AMAX / 4 + n4] = make_float4((float)(g4 * der[4 * n4]), (float)(g4 * der[4 * n4 + 1]),
+                                             (float)(g4 * der[4 * n4 + 2]), (float)(g4 * der[4 * n4 + 3]));
+        }
+      }
     }
   }
-  // the radial expansion of each species in range, as for a neighbour: the
-  // central pair's expansion (:342-355) differs only by the factor
-  // central_weight (:638-646), which the descriptor applies to that entry
-  if constexpr (!TAB) {
-    const double *sW = (const double *)(smem + P.off_W);
-    // species are data, not control flow: lanes of different species share
-    // one expansion call
-    while (todo) {
-      const int s = __ffs(todo) - 1;
-      todo &= todo - 1u;
-      const RadSp &RS = *(const RadSp *)(smem + P.off_rad + (size_t)s * SOAPB_RADSP_BYTES);
-      float4 *o = (float4 *)(B.rad + ((size_t)k * P.n_species + s) * 2 * AMAX);
-      double val[AMAX], der[AMAX];
-      radial_entry<AMAX, OP>(P, RS, sW + s * AMAX * AMAX, r, false, do_der != 0, val, der);
-      const double g4 = kFourPi * RS.gscale;
-#pragma unroll
-      for (int n4 = 0; n4 < AMAX / 4; ++n4)
-        o[n4] = make_float4((float)(g4 * val[4 * n4]), (float)(g4 * val[4 * n4 + 1]),
-                            (float)(g4 * val[4 * n4 + 2]), (float)(g4 * val[4 * n4 + 3]));
-      if (do_der)
-#pragma unroll
-        for (int n4 = 0; n4 < AMAX / 4; ++n4)
-          o[AMAX / 4 + n4] = make_float4((float)(g4 * der[4 * n4]), (float)(g4 * der[4 * n4 + 1]),
-                                         (float)(g4 * der[4 * n4 + 2]), (float)(g4 * der[4 * n4 + 3]));
-    }
-  } else {
+  if constexpr (TAB) {
     // R_n and dR_n/dr from the tables, a warp's entries of one species at a
     // time: 2 AMAX lanes per entry, lane f evaluating function f, so that the
     // segment's coefficients (stored [degree][function]) are read and the
