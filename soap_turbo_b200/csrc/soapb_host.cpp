@@ -1139,10 +1139,10 @@ int pick_threads(const soapb_context *c) {
 // Launch configuration of a site kernel: the caller's CTA size if set, else
 // the autotuner's choice for that kernel, else 0: the launcher's rule.
 LaunchCfg site_cfg(const soapb_context *c, bool contract) {
-  if (c->threads) return LaunchCfg{pick_threads(c), c->stream, c->max_ctas};
+  if (c->threads) return LaunchCfg{pick_threads(c), pick_threads(c), c->stream, c->max_ctas};
   const int t = contract ? c->tune_tc : c->tune_td;
-  if (t) return LaunchCfg{t, c->stream, contract ? c->tune_cc : c->tune_cd};
-  return LaunchCfg{0, c->stream, c->max_ctas};
+  if (t) return LaunchCfg{t, 128, c->stream, contract ? c->tune_cc : c->tune_cd};
+  return LaunchCfg{0, 128, c->stream, c->max_ctas};
 }
 
 // Status of the inputs from the prep error word a launch left (see soapb_scan.cuh).

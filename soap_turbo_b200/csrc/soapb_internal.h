@@ -160,8 +160,9 @@ struct DevBatch {
 // Kernel launchers (soapb_mixed.cu, soapb_fp64.cu)
 namespace soapb {
 struct LaunchCfg {
-  int threads;           // 64, 128 or 256: threads per site of the contract, and the pairs whose entries the
-                         // descriptor sorts and groups together; 0: the launcher's rule, and 128 pairs
+  int threads;           // threads per site of the contract: 64, 128 or 256; 0: the launcher's rule
+  int slots;             // 64, 128 or 256: the pairs whose entries the descriptor sorts and groups together, and
+                         // the partial sums of the norm, of q . G and of the central pair
   cudaStream_t stream;
   int max_ctas;          // grid cap (0: one CTA per site)
 };

@@ -766,6 +766,36 @@ __device__ __forceinline__ f32x2 fmul2(f32x2 a, f32x2 b) {
   return d;
 }
 
+// The site kernels' FP64 sums (the norm, q . G, the central pair) run over slots: slot
+// v of `slots` (64, 128 or 256) adds its terms v, v + slots, .. in order, 32 slots are
+// added by warp_sum and the warps' sums by slot_tree, as block_sum of so many threads
+// adds them.  So a result does not depend on the CTA size that a site was given.
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int STRIDE = 1>
+__device__ __forceinline__ double slot_tree(const double *r, int slots) {
+  constexpr int S = STRIDE;
+  if (slots == 128) return (r[0] + r[2 * S]) + (r[S] + r[3 * S]);
+  if (slots == 64) return r[0] + r[S];
+  return ((r[0] + r[4 * S]) + (r[2 * S] + r[6 * S])) + ((r[S] + r[5 * S]) + (r[3 * S] + r[7 * S]));
+}
+
+// slot_tree over the warp_sums of the four slots (lane, lane + 32, ..) that a lane
+// holds, in eight shuffles: each half of the lanes keeps half of the sums.
+__device__ __forceinline__ double slots_by_warp(const double (&v)[4]) {
+  const bool up = threadIdx.x & 16, odd = threadIdx.x & 8;
+  const double a = (up ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+  const double b = (up ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+  double t = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  t += __shfl_xor_sync(0xffffffffu, t, 16);
+  return t + __shfl_xor_sync(0xffffffffu, t, 8);
+}
+
 // ------------------------------------------------------------ descriptor
 // One CTA of a few warps per site; a thread owns one k = (l, m) and NH of the
 // radial indices of every species block (warp w: k = 32 (w % kw) + lane, radial
@@ -1039,20 +1069,36 @@ __global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AM
       }
       __syncthreads();
     }
-    // the norm (:805-809), by every warp for itself: its order then does not
-    // depend on the number of warps.  accumulate: the caller's soap row is added
-    // before the norm is taken, as the reference adds the compressed descriptor
-    // into soap (:798-802)
+    // the norm (:805-809) over `chunk` slots.  accumulate: the caller's soap row is
+    // added before the norm is taken, as the reference adds the compressed descriptor
+    // into soap (:798-802); the row may lie in host memory, so it is read here and where
+    // it is written, and not by every warp
     double *out = soap_out + (size_t)site * P.n_soap;
     const bool acc = (keep & 2) != 0;
-    double nrm2 = 0.0;
-    for (int o = lane; o < P.n_soap; o += 32) {
-      const double v = acc ? (double)sS[o] + out[o] : (double)sS[o];
-      nrm2 += v * v;
-    }
+    double nrm2;
+    if (!acc && chunk == 128) {
+      double v[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int o = lane; o < P.n_soap; o += 128)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nrm2 += __shfl_xor_sync(0xffffffffu, nrm2, o);
-    if (acc) __syncthreads();  // every warp has read the caller's row
+        for (int w = 0; w < 4; ++w) {
+          const double y = o + 32 * w < P.n_soap ? (double)sS[o + 32 * w] : 0.0;
+          v[w] = fma(y, y, v[w]);
+        }
+      nrm2 = slots_by_warp(v);
+    } else {
+      double *red = (double *)(smem + Ly.base);  // eight: the species' places are read
+      for (int w = warp; 32 * w < chunk; w += nw) {
+        double v = 0.0;
+        for (int o = 32 * w + lane; o < P.n_soap; o += chunk) {
+          const double y = acc ? (double)sS[o] + out[o] : (double)sS[o];
+          v = fma(y, y, v);
+        }
+        v = warp_sum(v);
+        if (lane == 0) red[w] = v;
+      }
+      __syncthreads();
+      nrm2 = slot_tree(red, chunk);
+    }
     double norm = sqrt(nrm2);
     if (norm < 1.0e-5) norm = 1.0;
     const double inv = 1.0 / norm;
@@ -1447,16 +1493,19 @@ constexpr int kHM = 3;  // m values per H item (the host's items must agree)
 
 template <int AMAX, int LC>
 __global__ void __launch_bounds__(256, 2)
-    k_contract(const DevParams P, const DevBatch B, const double *__restrict__ soap_in, const double *__restrict__ G,
-               int g_layout, double sgn, const float *__restrict__ keep_c, const double *__restrict__ keep_norm,
-               double *__restrict__ pair_out) {
+    k_contract(const DevParams P, const DevBatch B, int slots, const double *__restrict__ soap_in,
+               const double *__restrict__ G, int g_layout, double sgn, const float *__restrict__ keep_c,
+               const double *__restrict__ keep_norm, double *__restrict__ pair_out) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int AW = row_len(LC), ST = contract_stride(AMAX, LC);
   constexpr int KC = (LC + 1) * (LC + 2) / 2, KJ = (KC + 15) / 16;
   constexpr bool HREG = AMAX * KJ <= 24;  // the lane's H of a species fits its registers
   constexpr int GPT = 5;  // G values a thread holds while the norm dot product is reduced
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
-  const int half = lane >> 4, hl = lane & 15, n_acc = 8 / nw;
+  const int half = lane >> 4, hl = lane & 15;
+  // the first `wide` threads take the slots, two apiece where they are fewer than the slots
+  const int wide = min(nt, slots), t0 = tid < wide ? tid : P.n_soap;
+  const bool two = slots > nt;
   const ContractLayout Ly = contract_layout(P, nt, AMAX, LC);
   float2 *sH = (float2 *)(smem + Ly.H);
   double *sRed = (double *)(smem + Ly.red);
@@ -1515,7 +1564,7 @@ __global__ void __launch_bounds__(256, 2)
     double gv[GPT], qv[GPT];
 #pragma unroll
     for (int j = 0; j < GPT; ++j) {
-      const int o = tid + j * nt;
+      const int o = t0 + j * wide;
       gv[j] = qv[j] = 0.0;
       if (o < n_soap) {
         gv[j] = g[o * gs];
@@ -1528,41 +1577,34 @@ __global__ void __launch_bounds__(256, 2)
       for (int t = tid; t < n4; t += nt) cp_async16((float *)sC + 4 * t, kc + 4 * t);
       for (int t = 4 * n4 + tid; t < 2 * n_max * KS; t += nt) ((float *)sC)[t] = kc[t];
     }
-    // ---- back through the normalisation (src/soap_turbo.f90:1783-1790): q . G as 256
-    // sums over o = v, v + 256, .., a thread's 256 / nt of them apart, then added in
-    // one order: the result does not depend on the CTA size
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    // ---- back through the normalisation (src/soap_turbo.f90:1783-1790)
+    double qg0 = 0.0, qg1 = 0.0;
 #pragma unroll
     for (int j = 0; j < GPT; ++j) {
-      const double v = qv[j] * gv[j];
-      if (n_acc == 4) acc[j & 3] += v;
-      else if (n_acc == 2) acc[j & 1] += v;
-      else acc[0] += v;
+      if (two && (j & 1)) qg1 = fma(qv[j], gv[j], qg1);
+      else qg0 = fma(qv[j], gv[j], qg0);
     }
-    for (int o = tid + GPT * nt, j = GPT; o < n_soap; o += nt, ++j) {
-      const double v = q[o] * g[o * gs];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (i == (j & (n_acc - 1))) acc[i] += v;
+    for (int o = t0 + GPT * wide, j = GPT; o < n_soap; o += wide, ++j) {
+      const double gj = g[o * gs], qj = q[o];
+      if (two && (j & 1)) qg1 = fma(qj, gj, qg1);
+      else qg0 = fma(qj, gj, qg0);
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (i < n_acc) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-        if (lane == 0) sRed[warp + i * nw] = acc[i];
+    if (tid < wide) {
+      qg0 = warp_sum(qg0);
+      if (lane == 0) sRed[warp] = qg0;
+      if (two) {
+        qg1 = warp_sum(qg1);
+        if (lane == 0) sRed[warp + nw] = qg1;
       }
+    }
     __syncthreads();
-    double qg = 0.0;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) qg += sRed[w];
-    const double inv = 1.0 / knorm;
+    const double qg = slot_tree(sRed, slots), inv = 1.0 / knorm;
 #pragma unroll
     for (int j = 0; j < GPT; ++j) {
-      const int o = tid + j * nt;
+      const int o = t0 + j * wide;
       if (o < n_soap) sGp[o] = (float)((gv[j] - qv[j] * qg) * inv);
     }
-    for (int o = tid + GPT * nt; o < n_soap; o += nt) sGp[o] = (float)((g[o * gs] - q[o] * qg) * inv);
+    for (int o = t0 + GPT * wide; o < n_soap; o += wide) sGp[o] = (float)((g[o * gs] - q[o] * qg) * inv);
     cp_async_wait_all();
     __syncthreads();
     // ---- back through the compression (:1791-1798), unless it is one-to-one
@@ -1612,7 +1654,9 @@ __global__ void __launch_bounds__(256, 2)
       sH[(code >> 16) * HS + (code & 0xffff)] = make_float2(0.f, 0.f);
     }
 
-    double self = 0.0;  // threads 0..2: a component of the central pair
+    // the thread's slots of the central pair between two chunks of the row (volatile: in
+    // local memory, and not in registers while H fills them)
+    volatile double held[6];
     for (int c0 = p_begin; c0 < p_end; c0 += kContractChunk) {
       const int c1 = min(p_end, c0 + kContractChunk);
       if (c0 > p_begin) __syncthreads();  // the chunk before is read
@@ -1754,52 +1798,73 @@ __global__ void __launch_bounds__(256, 2)
       }
       __syncthreads();
       // ---- per pair: sum its entries, rotate to Cartesian (:1864-1875)
-      // and, 32 pairs at a time, their sums for the central pair
-      for (int k = tid; k < (c1 - c0 + 31) / 32 * 32; k += nt) {
+      // and add it to the central pair's slot (the pair's place in the row, modulo
+      // slots): tid's, and tid + nt's with two apiece
+      const int n_k = c1 - c0;
+      double x0 = 0.0, y0 = 0.0, z0 = 0.0, x1 = 0.0, y1 = 0.0, z1 = 0.0;
+      if (c0 > p_begin) {
+        x0 = held[0]; y0 = held[1]; z0 = held[2];
+        x1 = held[3]; y1 = held[4]; z1 = held[5];
+      }
+      for (int k = tid - (slots > kContractChunk ? (c0 - p_begin) & (slots - 1) : 0); k < n_k; k += nt) {
+        if (k < 0 || c0 + k <= p_begin) continue;
         double px = 0.0, py = 0.0, pz = 0.0, fr = 0.0, fa = 0.0, fp = 0.0;
-        if (c0 + k < c1 && c0 + k > p_begin) {
-          bool any = false;
-          for (int s = 0; s < nsp; ++s) {
-            const int e = slot[s * kContractChunk + k];
-            if (e >= 0) {
-              any = true;
-              fr += sF[3 * e];
-              fa += sF[3 * e + 1];
-              fp += sF[3 * e + 2];
-            }
+        bool any = false;
+        for (int s = 0; s < nsp; ++s) {
+          const int e = slot[s * kContractChunk + k];
+          if (e >= 0) {
+            any = true;
+            fr += sF[3 * e];
+            fa += sF[3 * e + 1];
+            fp += sF[3 * e + 2];
           }
-          if (any) {
-            const float *A = B.ang + (size_t)(c0 + k) * AW;
-            const double ct = A[row_x(LC)], st = A[row_sq(LC)], cf_ = A[row_e(LC) + 2], sf = -A[row_e(LC) + 3];
-            const double ir = 1.0 / B.rjs[c0 + k];
-            px = sgn * (st * cf_ * fr - ct * cf_ * ir * fp - sf * ir * fa);
-            py = sgn * (st * sf * fr - ct * sf * ir * fp + cf_ * ir * fa);
-            pz = sgn * (ct * fr + st * ir * fp);
-          }
-          double *po = pair_out + (size_t)3 * (c0 + k);
-          po[0] = px;
-          po[1] = py;
-          po[2] = pz;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          px += __shfl_xor_sync(0xffffffffu, px, o);
-          py += __shfl_xor_sync(0xffffffffu, py, o);
-          pz += __shfl_xor_sync(0xffffffffu, pz, o);
+        if (any) {
+          const float *A = B.ang + (size_t)(c0 + k) * AW;
+          const double ct = A[row_x(LC)], st = A[row_sq(LC)], cf_ = A[row_e(LC) + 2], sf = -A[row_e(LC) + 3];
+          const double ir = 1.0 / B.rjs[c0 + k];
+          px = sgn * (st * cf_ * fr - ct * cf_ * ir * fp - sf * ir * fa);
+          py = sgn * (st * sf * fr - ct * sf * ir * fp + cf_ * ir * fa);
+          pz = sgn * (ct * fr + st * ir * fp);
         }
-        if (lane == 0) {
-          double *r = sRed + 8 + 3 * (k >> 5);
-          r[0] = px;
-          r[1] = py;
-          r[2] = pz;
+        double *po = pair_out + (size_t)3 * (c0 + k);
+        po[0] = px;
+        po[1] = py;
+        po[2] = pz;
+        if (two && k >= nt) {
+          x1 -= px;
+          y1 -= py;
+          z1 -= pz;
+        } else {
+          x0 -= px;
+          y0 -= py;
+          z0 -= pz;
         }
       }
+      if (c1 < p_end) {
+        held[0] = x0; held[1] = y0; held[2] = z0;
+        held[3] = x1; held[4] = y1; held[5] = z1;
+        continue;
+      }
+      // the central pair is minus the sum of the others (:1875)
+      auto fold = [&](double x, double y, double z, int w) {  // the slots 32 w + lane
+        if (32 * w < p_end - p_begin) {  // the row reaches them
+          x = warp_sum(x);
+          y = warp_sum(y);
+          z = warp_sum(z);
+        }
+        if (lane == 0) {
+          double *r = sRed + 8 + 3 * w;
+          r[0] = x;
+          r[1] = y;
+          r[2] = z;
+        }
+      };
+      if (tid < slots) fold(x0, y0, z0, warp);
+      if (two) fold(x1, y1, z1, warp + nw);
       __syncthreads();
-      if (tid < 3)
-        for (int w = 0; c0 + 32 * w < c1; ++w) self -= sRed[8 + 3 * w + tid];
+      if (tid < 3) pair_out[(size_t)3 * p_begin + tid] = slot_tree<3>(sRed + 8 + tid, slots);
     }
-    // the central pair is minus the sum of the others (:1875)
-    if (tid < 3 && p_end > p_begin) pair_out[(size_t)3 * p_begin + tid] = self;
     __syncthreads();  // shared memory is free for the next site
   }
 }
@@ -2371,7 +2436,7 @@ template <int AMAX, int LC, int NH>
 static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg, int max_alpha,
                                      double *soap, float *keep_c, double *keep_norm, int keep) {
   const int kw = (P.k_max + 31) / 32, threads = 32 * kw * ((max_alpha + NH - 1) / NH);
-  const int chunk = cfg.threads ? cfg.threads : 128;  // fixes the summation groups
+  const int chunk = cfg.slots;  // fixes the summation groups
   const size_t sm = desc_layout(P, chunk, AMAX, LC).total;
   auto kern = k_descriptor<AMAX, LC, NH>;
   cudaError_t e = ensure_smem_limit(kern, sm);
@@ -2459,7 +2524,7 @@ static cudaError_t run_contract(const DevParams &P, const DevBatch &B, const Lau
   if (e != cudaSuccess) return e;
   if (n > 0) {
     const int grid = cfg.max_ctas > 0 && cfg.max_ctas < n ? cfg.max_ctas : n;
-    kern<<<grid, threads, sm, cfg.stream>>>(P, B, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
+    kern<<<grid, threads, sm, cfg.stream>>>(P, B, cfg.slots, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
   }
   return cudaGetLastError();
 }
