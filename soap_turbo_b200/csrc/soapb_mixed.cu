@@ -1594,6 +1594,7 @@ __global__ void __launch_bounds__(256, 2)
       if (two && (j & 1)) qg1 = fma(qv[j], gv[j], qg1);
       else qg0 = fma(qv[j], gv[j], qg0);
     }
+#pragma unroll 4
     for (int o = t0 + GPT * wide, j = GPT; o < n_soap; o += wide, ++j) {
       const double gj = g[o * gs], qj = q[o];
       if (two && (j & 1)) qg1 = fma(qj, gj, qg1);
@@ -1614,6 +1615,7 @@ __global__ void __launch_bounds__(256, 2)
       const int o = t0 + j * wide;
       if (o < n_soap) sGp[o] = (float)((gv[j] - qv[j] * qg) * inv);
     }
+#pragma unroll 4
     for (int o = t0 + GPT * wide; o < n_soap; o += wide) sGp[o] = (float)((g[o * gs] - q[o] * qg) * inv);
     cp_async_wait_all();
     __syncthreads();
@@ -2501,24 +2503,32 @@ static cudaError_t run_contract_tc(const DevParams &P, const DevBatch &B, const 
 }
 
 // Threads per site: with 64 a site costs the least work, with more it is done
-// sooner and the last wave wastes less (of 64, 128 and 256 threads 8, 4 and 2 CTAs
-// fit an SM).  The choice with the cheapest waves, a site at 128 and 256 threads
-// costing 1.2 and 1.6 of its share at 64.  Steps at 64, 128 and 256 threads: 64 sites
-// 47.1, 43.0, 40.8 us; 367 of two species 86, 74, 80; 727 of two 67, 71, 76; 1679 of
-// three 137, 126, 147; 16384 of one 715, 779, 941.
-static int contract_threads(int n_sites) {
-  const int slots[3] = {148 * 8, 148 * 4, 148 * 2};
+// sooner and the last wave wastes less.  Registers hold an SM to 512 threads (128
+// apiece by the launch bounds); shared memory, with many species or l_max 12, to fewer
+// CTAs of 64 or 128.  A wave of c CTAs an SM takes cost x 512 / threads, whatever c is, a
+// site at 128 and 256 threads costing 1.2 and 1.6 of its share at 64; the choice is the
+// one with the cheapest waves.  Contracts at 64, 128 and 256 threads, us: 64 sites of one
+// species 21, 15 and 13; 1000 of three 38, 39 and 53; 1679 of three 67, 60 and 79; 8000
+// of one 157, 181 and 240; of eight (three, three and two CTAs an SM) 700 89, 69 and 64,
+// 3000 324, 241 and 242.  It picks the slower of two in sites of 7 or 8 CTAs of 64 that
+// leave the L1 too little for the lists of H (l_max 12, 3000 sites: 198 for 168).
+constexpr int kSmemPerSm = 228 * 1024, kSmemReserved = 1024;  // B200; of each CTA
+template <int AMAX, int LC>
+static int contract_threads(const DevParams &P, int n_sites) {
   const double cost[3] = {1.0, 1.2, 1.6};
-  int best = 0;
+  int best = 128;
   double least = 0.0;
   for (int i = 0; i < 3; ++i) {
-    const double t = (double)((n_sites + slots[i] - 1) / slots[i]) * slots[i] * cost[i];
-    if (i == 0 || t < least) {
+    const int nt = 64 << i, by_smem = kSmemPerSm / ((int)contract_layout(P, nt, AMAX, LC).total + kSmemReserved);
+    const int slots = 148 * (by_smem < 512 / nt ? by_smem : 512 / nt);
+    if (slots == 0) continue;
+    const double t = (double)((n_sites + slots - 1) / slots) * cost[i] * (512 / nt);
+    if (least == 0.0 || t < least) {
       least = t;
-      best = i;
+      best = nt;
     }
   }
-  return 64 << best;
+  return best;
 }
 
 template <int AMAX, int LC>
@@ -2527,7 +2537,7 @@ static cudaError_t run_contract(const DevParams &P, const DevBatch &B, const Lau
                                 const float *keep_c, const double *keep_norm, double *pair) {
   if (AMAX == 8 && LC == 8 && P.tc_contract)
     return run_contract_tc(P, B, cfg, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
-  const int n = B.site_hi - B.site_lo, threads = cfg.threads ? cfg.threads : contract_threads(n);
+  const int n = B.site_hi - B.site_lo, threads = cfg.threads ? cfg.threads : contract_threads<AMAX, LC>(P, n);
   const size_t sm = contract_layout(P, threads, AMAX, LC).total;
   auto kern = k_contract<AMAX, LC>;
   cudaError_t e = ensure_smem_limit(kern, sm);
