@@ -2437,23 +2437,29 @@ static cudaError_t run_descriptor_tc(const DevParams &P, const DevBatch &B, cons
 
 // Radial indices per thread: the fewer, the more warps share a site and the more
 // loads a product takes.  Two where the sites are at most two per SM and a site's
-// latency is all; four below kDescWideSites sites, and where every k fits one
-// warp; eight from there on.  Steps of descriptor and contract with 2, 4 and 8:
-// 64 sites of one species 42.8, 45.1 and 48.7 us; with 4 and 8: 1679 sites of three
-// 127.5 and 135, 16384 of one 835 and 817; the descriptor alone at 13092 sites of
-// three 385 and 383.
+// latency is all, and where four would leave a site one or two warps or products
+// with no radial index (alpha 4, or alpha 5 and 6 with every k in one warp: the kernel at
+// 300, 1679 and 8000 sites 24.4, 55.6 and 232 us with two, 27.0, 62.6 and 286 with
+// four of eight species, alpha 4, l_max 8; 16.7, 35.2 and 133 against 18.8, 39.5 and 155
+// of five, alpha 6, l_max 6).  Else four below kDescWideSites sites, and where every k
+// fits one warp; eight from there on: 64 sites of one species of alpha 8 12.6, 13.6 and
+// 16.8 us with two, four and eight; with four and eight 29.3 and 33.0 at 1679, 47.2 and
+// 45.8 at 3000, 61.1 and 60.1 at 4000, 74.0 and 72.7 at 5000, 111 and 108 at 8000; of
+// three species 37 and 41, 64 and 64, 82 and 84, 99 and 103, 150 and 154.
 constexpr int kDescFewSites = 2 * 148, kDescWideSites = 4096;
 
 template <int AMAX, int LC, int NH>
 static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg, int max_alpha,
                                      double *soap, float *keep_c, double *keep_norm, int keep) {
-  const int kw = (P.k_max + 31) / 32, threads = 32 * kw * ((max_alpha + NH - 1) / NH);
+  const int kw = (P.k_max + 31) / 32, n = B.site_hi - B.site_lo;
+  int threads = 32 * kw * ((max_alpha + NH - 1) / NH);
+  // at few sites a small definition gets warps that only stage rows and form components
+  if (NH == 2 && n <= kDescFewSites && threads < 128) threads = 128;
   const int chunk = cfg.slots;  // fixes the summation groups
   const size_t sm = desc_layout(P, chunk, AMAX, LC).total;
   auto kern = k_descriptor<AMAX, LC, NH>;
   cudaError_t e = ensure_smem_limit(kern, sm);
   if (e != cudaSuccess) return e;
-  const int n = B.site_hi - B.site_lo;
   if (n > 0) {
     const int grid = cfg.max_ctas > 0 && cfg.max_ctas < n ? cfg.max_ctas : n;
     kern<<<grid, threads, sm, cfg.stream>>>(P, B, chunk, kw, soap, keep_c, keep_norm, keep);
@@ -2470,7 +2476,7 @@ static cudaError_t run_descriptor(const DevParams &P, const DevBatch &B, const L
   for (int s = 0; s < P.n_species; ++s) max_alpha = P.rad[s].alpha > max_alpha ? P.rad[s].alpha : max_alpha;
   if constexpr (AMAX == 8) {
     const int n = B.site_hi - B.site_lo;
-    if (n <= kDescFewSites)
+    if (n <= kDescFewSites || max_alpha <= 4 || (max_alpha <= 6 && P.k_max <= 32))
       return run_descriptor_as<AMAX, LC, 2>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
     if (n < kDescWideSites || P.k_max <= 32)
       return run_descriptor_as<AMAX, LC, 4>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
