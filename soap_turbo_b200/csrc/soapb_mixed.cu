@@ -847,13 +847,20 @@ __host__ __device__ inline DescLayout desc_layout(const DevParams &P, int chunk,
 }
 
 // resident CTAs the register count is held to (the staged round allows seven)
-__host__ __device__ constexpr int desc_min_ctas(int AMAX, int NH) {
+__host__ __device__ constexpr int desc_min_ctas(int AMAX, int NH, int groups) {
+  if (groups) return 768 / groups;
   return AMAX == 8 ? (NH == 8 ? 7 : NH == 4 ? 6 : 3) : 3;
 }
 
-template <int AMAX, int LC, int NH>
-__global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AMAX / NH), desc_min_ctas(AMAX, NH))
-    k_descriptor(const DevParams P, const DevBatch B, int chunk, int kw, double *__restrict__ soap_out,
+// Threads per site: those of one species' sums; with GROUPS more, in groups of warps
+// each of which sums another species (launch parameter groups)
+template <int AMAX, int LC, int NH, int GROUPS>
+constexpr int kDescThreads = GROUPS ? GROUPS : ((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AMAX / NH);
+
+template <int AMAX, int LC, int NH, int GROUPS>
+__global__ void __launch_bounds__(kDescThreads<AMAX, LC, NH, GROUPS>,
+                                  desc_min_ctas(AMAX, NH, GROUPS))
+    k_descriptor(const DevParams P, const DevBatch B, int chunk, int kw, int groups, double *__restrict__ soap_out,
                  float *__restrict__ keep_c, double *__restrict__ keep_norm, int keep) {
   // keep: bit 0 keeps c_nlm and the norm for the contract, bit 1 accumulates
   // into soap_out
@@ -866,7 +873,9 @@ __global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AM
   int *sBase = (int *)(smem + Ly.base);
   unsigned short *list = (unsigned short *)(smem + Ly.list);
   const int KS = P.k_max | 1, nsp = P.n_species;
-  const int k_of = 32 * (warp % kw) + lane, n0 = NH * (warp / kw);
+  if constexpr (GROUPS == 0) groups = 1;
+  const int group = GROUPS ? warp * groups / nw : 0, wg = GROUPS ? warp - group * (nw / groups) : warp;
+  const int k_of = 32 * (wg % kw) + lane, n0 = NH * (wg / kw);
   const bool own = k_of < P.k_max;
   const int kk = own ? k_of : P.k_max - 1;  // the last lanes repeat the last k and store nothing
   const int lm = __ldg((const int *)(P.blob + P.off_klm) + kk), l = lm & 0xff, m = lm >> 8;
@@ -897,7 +906,7 @@ __global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AM
     const int p_begin = B.off[site], p_end = min(B.off[site + 1], B.n_pairs);
     // the species whose sums the thread holds, its rounds so far, their sums but
     // for the last, and that of the last
-    int cs = 0, n_rounds = 0;
+    int cs = group, n_rounds = 0;
     double tr[NH], ti[NH], dr[NH], di[NH];
     float2 *kc = (float2 *)(keep_c + ((keep & 1) ? (size_t)site * keep_stride(P) : 0)) + kk;
     auto finish = [&]() {  // species cs is complete
@@ -928,13 +937,13 @@ __global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AM
         for (int n = 0; n < NH; ++n)
           if (n0 + n < a) kr[n * KS] = make_float2((float)dr[n], (float)di[n]);
       }
-      ++cs;
+      cs += groups;
       n_rounds = 0;
     };
-    // a site of one chunk takes all its species at once; else a species at a time
+    // a site of one chunk takes all its species at once; else a species per group at a time
     const bool multi = p_end - p_begin > chunk;
-    for (int s_lo = 0; s_lo < nsp; s_lo += multi ? 1 : nsp) {
-      const int s_hi = multi ? s_lo + 1 : nsp;
+    for (int s_lo = 0; s_lo < nsp; s_lo += multi ? groups : nsp) {
+      const int s_hi = multi ? min(nsp, s_lo + groups) : nsp;
       for (int c0 = p_begin; c0 < p_end; c0 += chunk) {
         const int c1 = min(p_end, c0 + chunk);
         const unsigned long long valid = valid_species(P, B, p_begin, c0, c1, false);
@@ -967,7 +976,7 @@ __global__ void __launch_bounds__(((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AM
           }
           cp_async_wait_all();
           __syncthreads();
-          for (int s = s_lo; s < s_hi; ++s) {
+          for (int s = s_lo + group; s < s_hi; s += groups) {
             const int lo = max(w0, sBase[s]), hi = min(w1, sBase[s + 1]);
             if (lo >= hi) continue;
             while (cs < s) finish();
@@ -2448,21 +2457,22 @@ static cudaError_t run_descriptor_tc(const DevParams &P, const DevBatch &B, cons
 // three species 37 and 41, 64 and 64, 82 and 84, 99 and 103, 150 and 154.
 constexpr int kDescFewSites = 2 * 148, kDescWideSites = 4096;
 
-template <int AMAX, int LC, int NH>
+template <int AMAX, int LC, int NH, int GROUPS = 0>
 static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg, int max_alpha,
                                      double *soap, float *keep_c, double *keep_norm, int keep) {
-  const int kw = (P.k_max + 31) / 32, n = B.site_hi - B.site_lo;
-  int threads = 32 * kw * ((max_alpha + NH - 1) / NH);
+  const int kw = (P.k_max + 31) / 32, n = B.site_hi - B.site_lo, own = 32 * kw * ((max_alpha + NH - 1) / NH);
+  const int room = GROUPS / own, groups = room < 1 ? 1 : room < P.n_species ? room : P.n_species;
+  int threads = own * groups;
   // at few sites a small definition gets warps that only stage rows and form components
-  if (NH == 2 && n <= kDescFewSites && threads < 128) threads = 128;
+  if (NH == 2 && GROUPS == 0 && n <= kDescFewSites && threads < 128) threads = 128;
   const int chunk = cfg.slots;  // fixes the summation groups
   const size_t sm = desc_layout(P, chunk, AMAX, LC).total;
-  auto kern = k_descriptor<AMAX, LC, NH>;
+  auto kern = k_descriptor<AMAX, LC, NH, GROUPS>;
   cudaError_t e = ensure_smem_limit(kern, sm);
   if (e != cudaSuccess) return e;
   if (n > 0) {
     const int grid = cfg.max_ctas > 0 && cfg.max_ctas < n ? cfg.max_ctas : n;
-    kern<<<grid, threads, sm, cfg.stream>>>(P, B, chunk, kw, soap, keep_c, keep_norm, keep);
+    kern<<<grid, threads, sm, cfg.stream>>>(P, B, chunk, kw, groups, soap, keep_c, keep_norm, keep);
   }
   return cudaGetLastError();
 }
@@ -2474,8 +2484,24 @@ static cudaError_t run_descriptor(const DevParams &P, const DevBatch &B, const L
     return run_descriptor_tc(P, B, cfg, soap, keep_c, keep_norm, keep);
   int max_alpha = 1;
   for (int s = 0; s < P.n_species; ++s) max_alpha = P.rad[s].alpha > max_alpha ? P.rad[s].alpha : max_alpha;
+  const int n = B.site_hi - B.site_lo;
+  // Rows of several chunks on average: one species at a time leaves a round few entries.
+  // Up to a site per SM every species gets its warps (rows of 340 pairs, 100 sites of
+  // eight species of alpha 4 103 -> 48 us, of five of alpha 6 68 -> 41); beyond, where one
+  // species' are at most two, two to four species at a time do (with the pair kernel, 290
+  // sites 127 -> 89 and 91 -> 81, 600 195 -> 158 and 135 -> 126; 450 sites of five with
+  // 256 threads 131, with 128 111, without groups 117).
+  if constexpr (AMAX == 8)
+    if (P.n_species > 1 && max_alpha > 2 && (long)B.n_pairs > (long)cfg.slots * B.n_sites) {
+      if (n <= kDescFewSites / 2)
+        return run_descriptor_as<AMAX, LC, 4, 512>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
+      if (32 * ((P.k_max + 31) / 32) * ((max_alpha + 3) / 4) <= 64) {
+        if (n <= kDescFewSites / 2 * 3)  // its resident CTAs
+          return run_descriptor_as<AMAX, LC, 4, 256>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
+        return run_descriptor_as<AMAX, LC, 4, 128>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
+      }
+    }
   if constexpr (AMAX == 8) {
-    const int n = B.site_hi - B.site_lo;
     if (n <= kDescFewSites || max_alpha <= 4 || (max_alpha <= 6 && P.k_max <= 32))
       return run_descriptor_as<AMAX, LC, 2>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
     if (n < kDescWideSites || P.k_max <= 32)

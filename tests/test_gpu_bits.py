@@ -142,3 +142,26 @@ def test_a_sites_bits_do_not_depend_on_the_batch(name):
         want = want or got
         np.testing.assert_array_equal(got[0], want[0][site])
         np.testing.assert_array_equal(got[1], want[1][pair])
+
+
+LONG = {"8sp_a4": syn.Hyper(alpha_max=[4] * 8, l_max=8, basis="poly3gauss", compress_mode="trivial"),
+        "5sp_a6": syn.Hyper(alpha_max=[6, 5, 6, 4, 6], l_max=6, basis="poly3", compress_mode="trivial"),
+        "3sp_a8": syn.Hyper(alpha_max=[8, 8, 8], l_max=8, basis="poly3gauss", compress_mode="trivial")}
+
+
+@pytest.mark.parametrize("threads", [0, 64, 256])
+@pytest.mark.parametrize("name", list(LONG))
+def test_groups_of_warps_give_the_same_sums(name, threads):
+    """Batches whose rows are several chunks on average give every species its own
+    warps, or some at a time, by the number of sites: each site's bits are those of a
+    batch of short rows, which the sites' species take in turn."""
+    hp = LONG[name]
+    base = edge_sites([64, 129, 256, 257, 300, 600], hp.n_species, seed=41)
+    ctx = Context(hp)
+    ctx.set_threads_per_site(threads)
+    short = edge_sites([1], hp.n_species, seed=1)
+    mixed = syn.concatenate([base] + [short] * 400)  # under a chunk on average
+    want = ctx.descriptor(ctx.batch(mixed)).cpu().numpy()[:base.n_sites]
+    for n_sites in (base.n_sites, 148, 149, 444, 445):
+        nl, site, _ = repeated(base, n_sites)
+        np.testing.assert_array_equal(ctx.descriptor(ctx.batch(nl)).cpu().numpy(), want[site])
