@@ -1468,9 +1468,10 @@ cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaSt
   }
   const size_t sms = (size_t)site_smem(P).total * sizeof(double);
   const int items = (site_items(P) + kSiteThreads - 1) / kSiteThreads;
-  const bool one = items <= 2 && sms <= kCartSmemCap;
+  // up to four items a thread (every definition with n_max k_max <= 2048 has at most 1001 items)
+  const bool one = items <= 4 && sms + 64 <= kCartSmemCap;  // beside the warps' sums
   if (nsites > 0 && one) {
-    auto kern = items == 1 ? k64_site<1> : k64_site<2>;
+    auto kern = items == 1 ? k64_site<1> : items == 2 ? k64_site<2> : items == 3 ? k64_site<3> : k64_site<4>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms);
     if (e != cudaSuccess) return e;
     kern<<<nsites, kSiteThreads, sms, s>>>(P, B, w.rad, (const double2 *)w.ang, (double2 *)w.cnk, soap_acc,
