@@ -1426,11 +1426,20 @@ size_t fp64_cart_smem(const DevParams &P) {
   return staged <= kCartSmemCap ? staged : (size_t)cart_smem(P, false).total * sizeof(double);
 }
 
-// CTAs per site of k64_cart_site4 (two of which fit an SM): the share that leaves
-// the fewest pairs to the last wave, every further CTA of a site costing it about a
-// twelfth (the site's c_nlm and z again).
+// Whether k64_cart_site4 takes a definition.
+static bool cart4_fits(const DevParams &P) {
+  return P.cmap_identity && P.n_max <= 32 && P.l_max <= 8 && P.n_soap <= 3 * kC4Threads &&
+         (size_t)cart4_smem(P).total * sizeof(double) <= kCartSmemCap;
+}
+
+// CTAs per site of k64_cart_site4: the share that leaves the fewest pairs to the last
+// wave, every further CTA of a site costing it about a twelfth (the site's c_nlm and z
+// again).  Two CTAs fit an SM by registers, one where n_max is so large that shared
+// memory holds no more (n_max above 30 with l_max 8).  1 where another kernel takes the
+// definition: the others have no use for the parts and their counters.
 int fp64_cart_split(const DevParams &P, int n_sites) {
-  const int slots = 2 * 148;
+  if (!cart4_fits(P)) return 1;
+  const int slots = 148 * ((size_t)cart4_smem(P).total * sizeof(double) <= 113 * 1024 ? 2 : 1);
   int best = 1;
   double cost = 1e30;
   for (int s = 1; s <= 4; ++s) {
@@ -1440,7 +1449,7 @@ int fp64_cart_split(const DevParams &P, int n_sites) {
       best = s;
     }
   }
-  return P.cmap_identity ? best : 1;
+  return best;
 }
 
 cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaStream_t s,
@@ -1488,7 +1497,7 @@ cudaError_t launch_fp64_descriptor(const DevParams &P, const DevBatch &B, cudaSt
     const size_t sm2 = (size_t)cart2_smem(P).total * sizeof(double);
     const size_t sm3 = (size_t)cart3_smem(P).total * sizeof(double);
     const size_t sm4 = (size_t)cart4_smem(P).total * sizeof(double);
-    if (P.cmap_identity && P.n_max <= 32 && P.l_max <= 8 && P.n_soap <= 3 * kC4Threads && sm4 <= kCartSmemCap) {
+    if (cart4_fits(P)) {
       auto kern = k64_cart_site4<8>;
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm4);
       if (e != cudaSuccess) return e;

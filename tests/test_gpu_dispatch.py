@@ -9,6 +9,7 @@ import torch
 
 import oracle as O
 from conftest import FP64_TOL, SOAP_TOL, VJP_TOL, max_rel_err, site_rel_err
+from soap_turbo_b200 import _lib
 from soap_turbo_b200 import synthetic as syn
 from soap_turbo_b200.context import Context
 from test_gpu_size_rules import edge_sites, repeated
@@ -34,3 +35,22 @@ def test_fp64_site_kernel_at_each_number_of_items(items):
     ctx.check_inputs()
     ok = np.abs(ref).max(axis=1)[site] > 0
     assert site_rel_err(soap[ok], ref[site][ok]) <= FP64_TOL
+
+
+def test_soap_cart_der_takes_no_workspace_of_another_form():
+    """An uncompressed definition of 2700 components is beyond the form that shares a
+    site among CTAs: its call does not take that form's (n_sites, split, 3 n_soap) sums."""
+    hp = syn.Hyper(alpha_max=[8, 8, 8], basis="poly3")
+    nl, _, _ = repeated(edge_sites([2], 3, seed=1), 445)  # a count that the form splits
+    ctx = Context(hp)
+    b = ctx.batch(nl)
+    soap = torch.empty(b.n_sites, ctx.n_soap, dtype=torch.float64, device="cuda")
+    cart = torch.empty(b.n_pairs, ctx.n_soap, 3, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    _lib.check(ctx._lib.soapb_descriptor_fp64(ctx._h, b.c, soap.data_ptr(), cart.data_ptr()))
+    torch.cuda.synchronize()
+    k_max, pairs, sites = 45, b.n_pairs + 1, b.n_sites + 1
+    need = (2 * 8 * 24 + 4 * 16 * k_max) * pairs + (16 * 24 * k_max + 8 * ctx.n_soap) * sites
+    # each of some twenty buffers is rounded up to the allocator's 2 MB
+    assert free - torch.cuda.mem_get_info()[0] <= need + 20 * 2 ** 21
