@@ -1439,7 +1439,7 @@ static bool cart4_fits(const DevParams &P) {
 // definition: the others have no use for the parts and their counters.
 int fp64_cart_split(const DevParams &P, int n_sites) {
   if (!cart4_fits(P)) return 1;
-  const int slots = 148 * ((size_t)cart4_smem(P).total * sizeof(double) <= 113 * 1024 ? 2 : 1);
+  const int slots = sm_count() * ((size_t)cart4_smem(P).total * sizeof(double) <= 113 * 1024 ? 2 : 1);
   int best = 1;
   double cost = 1e30;
   for (int s = 1; s <= 4; ++s) {
@@ -1546,7 +1546,7 @@ cudaError_t launch_fp64_contract(const DevParams &P, const DevBatch &B, cudaStre
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   // CTAs per site: the chip full, at 2048 threads per SM, where the sites are few
-  const int split = B.n_sites >= 148 * 4 ? 1 : (B.n_sites >= 148 * 2 ? 2 : 4);
+  const int sms = sm_count(), split = B.n_sites >= 4 * sms ? 1 : (B.n_sites >= 2 * sms ? 2 : 4);
   kern<<<B.n_sites * split, 256, sm, s>>>(P, B, cart, G, g_layout, sgn, split, pair);
   if (launches) *launches += 1;
   return cudaGetLastError();

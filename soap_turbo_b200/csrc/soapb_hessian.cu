@@ -920,7 +920,7 @@ size_t hess_smem_bytes(const DevParams &P, int n_vec, int n_sites) {
 // 256 threads (two CTAs to an SM) or, where those would not all be resident twice
 // over, 512, for a site's units to be done sooner: 150 sites of one species with five
 // vectors 320 and 308 us.
-int hess_threads(int n_sites) { return n_sites <= 2 * 148 ? 512 : 256; }
+int hess_threads(int n_sites) { return n_sites <= 2 * sm_count() ? 512 : 256; }
 
 template <int NT>
 static int hess_grid_of(const DevParams &P, int n_vec) {

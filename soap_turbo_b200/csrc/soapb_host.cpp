@@ -1198,8 +1198,8 @@ int ctx_descriptor(soapb_context *c, const soapb_batch *b, double *d_soap, int k
   // a batch one scan tile covers, run whole: the scan orders its sites
   // heaviest first for the site kernels (and the contract that follows)
   c->order_sites = -1;
-  // (592 and fewer are all resident at once: the order cost 64 sites 2 of 39 us)
-  if (!ch && b->n_sites > 4 * 148 && b->n_sites <= kScanTileSites) {
+  // (592 and fewer, four per SM, are all resident at once: the order cost 64 sites 2 of 39 us)
+  if (!ch && b->n_sites > 4 * sm_count() && b->n_sites <= kScanTileSites) {
     if ((rc = c->order.ensure(sizeof(int) * (size_t)b->n_sites))) return rc;
     B.order = c->order.as<int>();
   }

@@ -166,6 +166,7 @@ struct LaunchCfg {
   cudaStream_t stream;
   int max_ctas;          // grid cap (0: one CTA per site)
 };
+int sm_count();  // SMs of the current device, asked once (the launchers' rules are in waves of its CTAs)
 cudaError_t launch_prep(const DevParams &P, const DevBatch &B, cudaStream_t s);
 // sites per tile of the CSR offset scan (soapb_scan.cuh)
 constexpr int kScanTileSites = 2048;

@@ -21,6 +21,7 @@
 //
 // Everything is deterministic: no atomics touch results, and every reduction
 // runs in an order fixed by the launch shape.
+#include <atomic>
 #include <cstdio>
 #include <mutex>
 #include <type_traits>
@@ -2366,6 +2367,17 @@ static cudaError_t ensure_smem_limit(K kernel, size_t smem) {
   return e;
 }
 
+int sm_count() {
+  static std::atomic<int> known[32];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int n = dev < 32 ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
+  if (dev < 32) known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 template <typename K>
 static int persistent_grid_query(K kernel, int threads, size_t smem, int dev, int &sms);
 
@@ -2455,7 +2467,7 @@ static cudaError_t run_descriptor_tc(const DevParams &P, const DevBatch &B, cons
 // 16.8 us with two, four and eight; with four and eight 29.3 and 33.0 at 1679, 47.2 and
 // 45.8 at 3000, 61.1 and 60.1 at 4000, 74.0 and 72.7 at 5000, 111 and 108 at 8000; of
 // three species 37 and 41, 64 and 64, 82 and 84, 99 and 103, 150 and 154.
-constexpr int kDescFewSites = 2 * 148, kDescWideSites = 4096;
+constexpr int kDescFewPerSm = 2, kDescWideSites = 4096;
 
 template <int AMAX, int LC, int NH, int GROUPS = 0>
 static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg, int max_alpha,
@@ -2464,7 +2476,7 @@ static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, cons
   const int room = GROUPS / own, groups = room < 1 ? 1 : room < P.n_species ? room : P.n_species;
   int threads = own * groups;
   // at few sites a small definition gets warps that only stage rows and form components
-  if (NH == 2 && GROUPS == 0 && n <= kDescFewSites && threads < 128) threads = 128;
+  if (NH == 2 && GROUPS == 0 && n <= kDescFewPerSm * sm_count() && threads < 128) threads = 128;
   const int chunk = cfg.slots;  // fixes the summation groups
   const size_t sm = desc_layout(P, chunk, AMAX, LC).total;
   auto kern = k_descriptor<AMAX, LC, NH, GROUPS>;
@@ -2484,7 +2496,7 @@ static cudaError_t run_descriptor(const DevParams &P, const DevBatch &B, const L
     return run_descriptor_tc(P, B, cfg, soap, keep_c, keep_norm, keep);
   int max_alpha = 1;
   for (int s = 0; s < P.n_species; ++s) max_alpha = P.rad[s].alpha > max_alpha ? P.rad[s].alpha : max_alpha;
-  const int n = B.site_hi - B.site_lo;
+  const int n = B.site_hi - B.site_lo, sms = sm_count();
   // Rows of several chunks on average: one species at a time leaves a round few entries.
   // Up to a site per SM every species gets its warps (rows of 340 pairs, 100 sites of
   // eight species of alpha 4 103 -> 48 us, of five of alpha 6 68 -> 41); beyond, where one
@@ -2493,16 +2505,16 @@ static cudaError_t run_descriptor(const DevParams &P, const DevBatch &B, const L
   // 256 threads 131, with 128 111, without groups 117).
   if constexpr (AMAX == 8)
     if (P.n_species > 1 && max_alpha > 2 && (long)B.n_pairs > (long)cfg.slots * B.n_sites) {
-      if (n <= kDescFewSites / 2)
+      if (n <= sms)
         return run_descriptor_as<AMAX, LC, 4, 512>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
       if (32 * ((P.k_max + 31) / 32) * ((max_alpha + 3) / 4) <= 64) {
-        if (n <= kDescFewSites / 2 * 3)  // its resident CTAs
+        if (n <= 3 * sms)  // its resident CTAs
           return run_descriptor_as<AMAX, LC, 4, 256>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
         return run_descriptor_as<AMAX, LC, 4, 128>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
       }
     }
   if constexpr (AMAX == 8) {
-    if (n <= kDescFewSites || max_alpha <= 4 || (max_alpha <= 6 && P.k_max <= 32))
+    if (n <= kDescFewPerSm * sms || max_alpha <= 4 || (max_alpha <= 6 && P.k_max <= 32))
       return run_descriptor_as<AMAX, LC, 2>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
     if (n < kDescWideSites || P.k_max <= 32)
       return run_descriptor_as<AMAX, LC, 4>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
@@ -2552,7 +2564,7 @@ static int contract_threads(const DevParams &P, int n_sites) {
   double least = 0.0;
   for (int i = 0; i < 3; ++i) {
     const int nt = 64 << i, by_smem = kSmemPerSm / ((int)contract_layout(P, nt, AMAX, LC).total + kSmemReserved);
-    const int slots = 148 * (by_smem < 512 / nt ? by_smem : 512 / nt);
+    const int slots = sm_count() * (by_smem < 512 / nt ? by_smem : 512 / nt);
     if (slots == 0) continue;
     const double t = (double)((n_sites + slots - 1) / slots) * cost[i] * (512 / nt);
     if (least == 0.0 || t < least) {

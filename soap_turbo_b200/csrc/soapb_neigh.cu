@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(256) k_nb_scan(DevBatch B, int tiles, int max_
 // 64 sites 124, 106, 99; 600 96, 89, 85; 1200 98, 90, 101; 1700 101, 97, 105; 2400 107,
 // 114, 120; 8000 177, 168, 199; 32768 382, 380, 515.
 static int nb_warps(int n_sites) {
-  const int slots[3] = {148 * 18, 148 * 14, 148 * 7};
+  const int sms = sm_count(), slots[3] = {18 * sms, 14 * sms, 7 * sms};
   const double cost[3] = {1.0, 0.8, 0.7};
   int best = 0;
   double least = 0.0;
