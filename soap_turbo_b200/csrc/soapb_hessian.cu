@@ -939,10 +939,11 @@ int hess_grid(const DevParams &P, int n_vec, int n_sites) {
 
 cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s, const Fp64Work &w,
                            double *rad_der2, double *geo, int *good, const double *soap, int n_vec,
-                           const double *vecs, double *hess, double *sums, double *scratch, int grid, int *ticket, int *launches) {
+                           const double *vecs, double *hess, double *sums, double *scratch, int grid, int *ticket,
+                           int *launches, bool pair_state) {
   CU_RET(cudaMemsetAsync(hess, 0, sizeof(double) * 9 * (size_t)n_vec * B.n_pairs, s));
   CU_RET(cudaMemsetAsync(ticket, 0, sizeof(int), s));
-  if (B.n_pairs > 0) {
+  if (B.n_pairs > 0 && pair_state) {
     const int blocks = (B.n_pairs + 127) / 128;
     int amax = 0;
     for (int sp = 0; sp < P.n_species; ++sp) amax = amax > P.rad[sp].alpha ? amax : P.rad[sp].alpha;

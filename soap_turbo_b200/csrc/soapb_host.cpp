@@ -1375,7 +1375,7 @@ int ctx_hessian(soapb_context *c, const soapb_batch *b, const double *d_soap, in
     }
     CU(launch_hessian(P, B, c->stream, w, c->hs_rad_der2.as<double>(), c->hs_geo.as<double>(),
                       c->hs_good.as<int>(), d_soap ? d_soap : c->hs_soap.as<double>(), nc, vecs, hess,
-                      c->hs_sums.as<double>(), c->hs_scratch.as<double>(), grid, c->hs_ticket.as<int>(), &nl));
+                      c->hs_sums.as<double>(), c->hs_scratch.as<double>(), grid, c->hs_ticket.as<int>(), &nl, v0 == 0));
     if (chunk < n_vec && npair > 0)
       CU(cudaMemcpy2DAsync(d_hess + (size_t)v0 * 9, 72 * (size_t)n_vec, c->hs_hchunk.p, 72 * (size_t)nc,
                            72 * (size_t)nc, npair, cudaMemcpyDeviceToDevice, c->stream));

@@ -271,9 +271,10 @@ cudaError_t launch_fp64_contract(const DevParams &P, const DevBatch &B, cudaStre
 // Central-atom Hessian (soapb_hessian.cu), on the state launch_fp64_descriptor
 // left with do_der: second radial derivatives into rad_der2 (n_pairs, n_max),
 // per-pair geometry records into geo (n_pairs * hess_geo_doubles) and good
-// (n_pairs ints), then hess (n_pairs, n_vec, 3, 3) = 9 n_vec doubles per pair,
-// cleared first.  sums: n_pairs * hess_sums_doubles doubles; scratch: grid *
-// hess_scratch_doubles doubles; ticket: one int.
+// (n_pairs ints) -- unless an earlier launch of the call left them (pair_state false)
+// -- then hess (n_pairs, n_vec, 3, 3) = 9 n_vec doubles per pair, cleared first.
+// sums: n_pairs * hess_sums_doubles doubles; scratch: grid * hess_scratch_doubles
+// doubles; ticket: one int.
 size_t hess_scratch_doubles(const DevParams &P);
 size_t hess_sums_doubles(int n_vec);                   // per pair, of k64_hess's k-sums
 constexpr int kHessVecs = 16;                          // weight vectors of one launch at most
@@ -283,5 +284,5 @@ int hess_grid(const DevParams &P, int n_vec, int n_sites);
 cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s, const Fp64Work &w,
                            double *rad_der2, double *geo, int *good, const double *soap, int n_vec,
                            const double *vecs, double *hess, double *sums, double *scratch, int grid, int *ticket,
-                           int *launches);
+                           int *launches, bool pair_state = true);
 }  // namespace soapb

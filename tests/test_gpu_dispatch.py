@@ -54,3 +54,18 @@ def test_soap_cart_der_takes_no_workspace_of_another_form():
     need = (2 * 8 * 24 + 4 * 16 * k_max) * pairs + (16 * 24 * k_max + 8 * ctx.n_soap) * sites
     # each of some twenty buffers is rounded up to the allocator's 2 MB
     assert free - torch.cuda.mem_get_info()[0] <= need + 20 * 2 ** 21
+
+
+def test_hessian_forms_the_pairs_once_per_call():
+    """17 weight vectors are two launches of the Hessian kernel, and one more launch
+    than one vector: the pairs' second derivatives and records serve both."""
+    hp = syn.Hyper(alpha_max=[4, 4], l_max=4, basis="poly3gauss")
+    base = edge_sites([2, 33, 60], 2, seed=29)
+    ctx = Context(hp, legacy_filter_seed=False)
+    b = ctx.batch(base)
+    count = []
+    for n_vec in (1, 17):
+        before = ctx.launch_count
+        ctx.central_hessian(b, torch.ones(base.n_sites, n_vec, ctx.n_soap, dtype=torch.float64, device="cuda"))
+        count.append(ctx.launch_count - before)
+    assert count[1] == count[0] + 1
