@@ -339,8 +339,9 @@ int soapb_descriptor_fp64(soapb_context *ctx, const soapb_batch *batch, double *
  * expansion state of the batch, so it needs no earlier call.  d_soap is the
  * normalised descriptor the weights were formed against (NULL: the FP64 one
  * this call computes).  Needs legacy_filter_seed = 0 (SOAPB_ERR_ARGUMENT).  More than
- * 16 weight vectors (fewer where shared memory holds fewer) are done in chunks of
- * as many, with two strided device copies per chunk. */
+ * 16 weight vectors (fewer for so many pairs that their sums would take over 4 GB,
+ * or where shared memory holds fewer) are done in even chunks, with two strided
+ * device copies per chunk. */
 int soapb_central_hessian(soapb_context *ctx, const soapb_batch *batch, const double *d_soap,
                           int32_t n_vec, const double *d_vecs, double *d_hess);
 

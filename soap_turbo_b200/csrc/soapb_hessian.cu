@@ -911,6 +911,17 @@ int hess_threads(int n_sites);
 
 size_t hess_sums_doubles(int n_vec) { return (size_t)kSumsFull * (n_vec + 1) + 3 * kSumsLight; }
 
+// At most 16 vectors in a launch, and no more than keep the pairs' sums within 4 GB
+// (16 at 1.2 M pairs, 7 at 2.4 M), in chunks as even as they come.  A chunk forms a site's
+// G and dp1 again: 17 vectors at 100 sites of one species take 1.2 times 16's time.
+int hess_vecs(int n_vec, long long n_pairs) {
+  constexpr size_t kBytes = (size_t)4 << 30;
+  int most = 16;
+  while (most > 1 && sizeof(double) * hess_sums_doubles(most) * (size_t)n_pairs > kBytes) --most;
+  const int chunks = (n_vec + most - 1) / most;
+  return (n_vec + chunks - 1) / chunks;
+}
+
 size_t hess_geo_doubles(const DevParams &P) { return (size_t)GeoLayout(P.l_max).size; }
 
 size_t hess_smem_bytes(const DevParams &P, int n_vec, int n_sites) {

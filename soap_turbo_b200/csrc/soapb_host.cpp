@@ -1322,9 +1322,9 @@ int ctx_hessian(soapb_context *c, const soapb_batch *b, const double *d_soap, in
   if (n_vec == 0) return SOAPB_OK;
   if (b->n_sites > 0 && !d_vecs) return fail(SOAPB_ERR_ARGUMENT, "null vecs");
   // The kernel keeps the pairs' k-sums for every weight vector of a launch: more
-  // than kHessVecs are done in chunks (each vector's block depends on that vector
-  // alone, so the chunking changes no bits).
-  int chunk = std::min(n_vec, kHessVecs);
+  // vectors than hess_vecs allows are done in chunks of about the same size (each
+  // vector's block depends on that vector alone, so the chunking changes no bits).
+  int chunk = hess_vecs(n_vec, b->n_atom_pairs);
   {
     int dev = 0, smem_max = 0;
     CU(cudaGetDevice(&dev));

@@ -277,7 +277,7 @@ cudaError_t launch_fp64_contract(const DevParams &P, const DevBatch &B, cudaStre
 // doubles; ticket: one int.
 size_t hess_scratch_doubles(const DevParams &P);
 size_t hess_sums_doubles(int n_vec);                   // per pair, of k64_hess's k-sums
-constexpr int kHessVecs = 16;                          // weight vectors of one launch at most
+int hess_vecs(int n_vec, long long n_pairs);           // weight vectors of one launch
 size_t hess_geo_doubles(const DevParams &P);
 size_t hess_smem_bytes(const DevParams &P, int n_vec, int n_sites);  // dynamic shared memory of k64_hess
 int hess_grid(const DevParams &P, int n_vec, int n_sites);
