@@ -907,7 +907,7 @@ size_t hess_scratch_doubles(const DevParams &P) {
   return (n + 31) / 32 * 32;
 }
 
-int hess_threads(int n_sites);
+int hess_threads(const DevParams &P, int n_vec, int n_sites);
 
 size_t hess_sums_doubles(int n_vec) { return (size_t)kSumsFull * (n_vec + 1) + 3 * kSumsLight; }
 
@@ -925,13 +925,22 @@ int hess_vecs(int n_vec, long long n_pairs) {
 size_t hess_geo_doubles(const DevParams &P) { return (size_t)GeoLayout(P.l_max).size; }
 
 size_t hess_smem_bytes(const DevParams &P, int n_vec, int n_sites) {
-  return sizeof(double) * (size_t)hess_smem(P, n_vec, hess_threads(n_sites)).total;
+  return sizeof(double) * (size_t)hess_smem(P, n_vec, hess_threads(P, n_vec, n_sites)).total;
 }
 
-// 256 threads (two CTAs to an SM) or, where those would not all be resident twice
-// over, 512, for a site's units to be done sooner: 150 sites of one species with five
-// vectors 320 and 308 us.
-int hess_threads(int n_sites) { return n_sites <= 2 * sm_count() ? 512 : 256; }
+// One CTA of 512 threads an SM or two of 256.  512 where shared memory holds one CTA
+// of 256 only; else where the sites are one wave of 512, or three against two of 256,
+// each of which takes 1.6 (small definitions) to 1.9 of the time of a wave of 512.  Calls
+// of three vectors with 512 and 256 threads, us: one species, l_max 8, 148 sites 225 and
+// 281, 149 317 and 315, 296 353 and 348, 297 419 and 456, 444 485 and 561, 445 527 and
+// 561, 600 697 and 715; two species of alpha 4, l_max 4 145 and 162, 193 and 175, 211 and
+// 189, 250 and 239, 277 and 290, 305 and 291, 384 and 349; one of alpha 10, l_max 12 (one
+// CTA of either) 403 and 492 at 148, 666 and 851 at 296, 1376 and 1769 at 600.
+int hess_threads(const DevParams &P, int n_vec, int n_sites) {
+  if (sizeof(double) * (size_t)hess_smem(P, n_vec, 256).total > kHessSmemPair) return 512;
+  const int sms = sm_count(), waves = (n_sites + sms - 1) / sms;
+  return waves <= 1 || waves == 3 ? 512 : 256;
+}
 
 template <int NT>
 static int hess_grid_of(const DevParams &P, int n_vec) {
@@ -945,7 +954,7 @@ static int hess_grid_of(const DevParams &P, int n_vec) {
   return sms * (per_sm > 0 ? per_sm : 1);
 }
 int hess_grid(const DevParams &P, int n_vec, int n_sites) {
-  return hess_threads(n_sites) == 512 ? hess_grid_of<512>(P, n_vec) : hess_grid_of<256>(P, n_vec);
+  return hess_threads(P, n_vec, n_sites) == 512 ? hess_grid_of<512>(P, n_vec) : hess_grid_of<256>(P, n_vec);
 }
 
 cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s, const Fp64Work &w,
@@ -967,7 +976,7 @@ cudaError_t launch_hessian(const DevParams &P, const DevBatch &B, cudaStream_t s
   }
   if (B.n_sites > 0) {
     const size_t sm = hess_smem_bytes(P, n_vec, B.n_sites);
-    const int threads = hess_threads(B.n_sites);
+    const int threads = hess_threads(P, n_vec, B.n_sites);
     auto kern = threads == 512 ? k64_hess<512> : k64_hess<256>;
     CU_RET(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int g = grid < B.n_sites ? grid : B.n_sites;

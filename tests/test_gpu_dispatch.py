@@ -69,3 +69,23 @@ def test_hessian_forms_the_pairs_once_per_call():
         ctx.central_hessian(b, torch.ones(base.n_sites, n_vec, ctx.n_soap, dtype=torch.float64, device="cuda"))
         count.append(ctx.launch_count - before)
     assert count[1] == count[0] + 1
+
+
+@pytest.mark.parametrize("alpha,l_max", [([4, 4], 4), ([10], 12)])
+def test_hessian_bits_do_not_depend_on_the_batch(alpha, l_max):
+    """The site count picks 256 or 512 threads per site (l_max 12: always 512); every
+    sum keeps its order.  (Against the oracle: test_gpu_hessian and test_gpu_size_rules;
+    alpha 10 is beyond their gate, W's conditioning amplifies the radial expansion's
+    last bits to 4.5e-7.)"""
+    hp = syn.Hyper(alpha_max=alpha, l_max=l_max, basis="poly3gauss" if l_max == 4 else "poly3")
+    base = edge_sites([2, 33, 60], hp.n_species, seed=37)
+    ctx = Context(hp, legacy_filter_seed=False)
+    vecs = np.random.default_rng(5).standard_normal((base.n_sites, 2, ctx.n_soap))
+    first = None
+    for n_sites in (3, 148, 149, 296, 297, 444, 445):
+        nl, site, pair = repeated(base, n_sites)
+        v = torch.as_tensor(np.ascontiguousarray(vecs[site])).cuda()
+        got = ctx.central_hessian(ctx.batch(nl), v).cpu().numpy()
+        first = got if first is None else first
+        np.testing.assert_array_equal(got, first[pair])
+    assert np.isfinite(first).all() and np.abs(first).max() > 0
