@@ -342,8 +342,8 @@ def run_ours(args):
         p = ctx.contract(b, s, G)
         return s, p
 
-    # the project's autotuner picks the form (tensor or CUDA cores), CTA size and
-    # persistent grid cap per site kernel; --tensor-cores on forces the tensor cores
+    # the project's autotuner picks the form (tensor or CUDA cores) per site kernel and
+    # the contract's CTA size; --tensor-cores on forces the tensor cores
     tune = ctx.autotune(b)
     if args.tensor_cores == "on":
         ctx.set_tensor_cores(True)

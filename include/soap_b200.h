@@ -234,22 +234,25 @@ int soapb_get_basis(const soapb_context *ctx, double *W, double *S);
 int soapb_n_soap(const soapb_context *ctx, int32_t *n_soap);
 /* Work on this cudaStream_t from now on (0 = legacy default stream). */
 int soapb_set_stream(soapb_context *ctx, void *stream);
-/* Work tuning: threads per site CTA of the contract (64, 128 or 256), and the
- * pairs whose entries the descriptor sorts and groups together (its own CTA size
- * follows the number of sites); 0 returns to the autotuner's choice, or before any
- * autotuning to a rule on the number of sites and 128 pairs. */
+/* Work tuning: threads per site CTA of the contract (64, 128 or 256); the pairs whose
+ * entries the descriptor sorts and groups together, and the partial sums of the norm, of
+ * q . G and of the central pair's force, are then as many (so that the choice changes
+ * the summation grouping, within FP32 rounding).  0 returns to the autotuner's choice,
+ * or before any autotuning to a rule on the number of sites and the shared memory, and
+ * to 128 pairs and sums.  The descriptor's own CTA size follows the number of sites. */
 int soapb_set_threads_per_site(soapb_context *ctx, int32_t threads);
 /* Autotuner: times the descriptor and the contract on this batch in each form
- * -- the tensor-core kernels (when allowed, see soapb_set_tensor_cores) and the
- * CUDA-core kernels at every CTA size (64, 128, 256 threads per site) -- and
- * each persistent grid cap (the occupancy limit, 2 and 1 CTAs per SM), and
- * keeps the fastest per kernel in the context.  choice (4, may be NULL)
- * receives {descriptor threads, descriptor grid cap, contract threads,
- * contract grid cap}: threads 0 means the tensor-core kernel, a grid cap of 0
- * the occupancy limit.  A set-up call: it allocates and frees work buffers,
- * synchronises the context's stream and discards the state kept for
- * soapb_contract.  Results are bit-reproducible for a fixed choice; another
- * CTA size changes the summation grouping within FP32 rounding. */
+ * -- the CUDA-core kernels, the contract at every CTA size (64, 128, 256 threads
+ * per site), and the tensor-core kernels (when allowed, see
+ * soapb_set_tensor_cores) at each cap of their persistent grids (the occupancy limit, 2
+ * and 1 CTAs per SM) -- and keeps the fastest per kernel in the context: the form for
+ * every later batch, the contract's CTA size for batches of this number of sites (others
+ * take the rule).  choice (4, may be NULL) receives {descriptor threads, descriptor grid
+ * cap, contract threads, contract grid cap}: threads 0 means the tensor-core kernel, 128
+ * the CUDA-core descriptor; a grid cap of 0 the occupancy limit or a CTA per site.  A
+ * set-up call: it allocates and frees work buffers, synchronises the context's stream
+ * and discards the state kept for soapb_contract.  Results are bit-reproducible for a
+ * fixed form; the CTA size changes no bits. */
 int soapb_autotune(soapb_context *ctx, const soapb_batch *batch, int32_t *choice);
 
 /* Radial expansion of the mixed path.  With atom_sigma_r_scaling = 0 (poly3,

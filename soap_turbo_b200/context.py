@@ -256,9 +256,10 @@ class Context:
         return out
 
     def autotune(self, b: DeviceBatch) -> dict:
-        """soapb_autotune: time both site kernels on this batch in each form
-        (tensor cores, CUDA cores at every CTA size) and grid cap, and keep the
-        fastest; returns the choice (threads 0: the tensor-core kernel)."""
+        """soapb_autotune: time both site kernels on this batch in each form (CUDA
+        cores, the contract at every CTA size; tensor cores at every grid cap) and keep
+        the fastest, the CTA size for batches of this many sites; returns the choice
+        (threads 0: the tensor-core kernel)."""
         ch = (C.c_int32 * 4)()
         _lib.check(self._lib.soapb_autotune(self._h, b.c, ch))
         return {"descriptor_threads": ch[0], "descriptor_max_ctas": ch[1],

@@ -312,9 +312,9 @@ struct soapb_context {
   DBuf nb_rjs, nb_th, nb_ph, nb_mask, nb_natom, nb_nneigh, nb_species, nb_smult;
   cudaStream_t stream = 0;
   int threads = 0;   // threads per site CTA chosen by the caller (0 = tuned or default)
-  int max_ctas = 0;
-  // the autotuner's choice per site kernel: CTA size and persistent grid cap
-  int tune_td = 0, tune_cd = 0, tune_tc = 0, tune_cc = 0;
+  // the autotuner's choice: the grid caps of the tensor-core kernels, and the threads per
+  // site of the CUDA-core contract for batches of tune_sites sites (0: the launcher's rule)
+  int tune_cd = 0, tune_cc = 0, tune_tc = 0, tune_sites = -1;
   int64_t launches = 0;
   int keep_valid = 0, keep_sites = 0, keep_pairs = 0;
   DBuf order;           // the last whole-batch descriptor call's site order
@@ -1136,13 +1136,13 @@ int pick_threads(const soapb_context *c) {
   return 128;
 }
 
-// Launch configuration of a site kernel: the caller's CTA size if set, else
-// the autotuner's choice for that kernel, else 0: the launcher's rule.
-LaunchCfg site_cfg(const soapb_context *c, bool contract) {
-  if (c->threads) return LaunchCfg{pick_threads(c), pick_threads(c), c->stream, c->max_ctas};
-  const int t = contract ? c->tune_tc : c->tune_td;
-  if (t) return LaunchCfg{t, 128, c->stream, contract ? c->tune_cc : c->tune_cd};
-  return LaunchCfg{0, 128, c->stream, c->max_ctas};
+// Launch configuration of a site kernel on a batch of n_sites: the caller's CTA size if
+// set, else the autotuner's for a batch of that size, else 0: the launcher's rule.  The
+// caller's size also fixes the sums' slots; the autotuner's leaves every bit as it is.
+LaunchCfg site_cfg(const soapb_context *c, bool contract, int n_sites) {
+  if (c->threads) return LaunchCfg{pick_threads(c), pick_threads(c), c->stream, contract ? c->tune_cc : c->tune_cd};
+  const int t = contract && n_sites == c->tune_sites ? c->tune_tc : 0;
+  return LaunchCfg{t, 128, c->stream, contract ? c->tune_cc : c->tune_cd};
 }
 
 // Status of the inputs from the prep error word a launch left (see soapb_scan.cuh).
@@ -1191,7 +1191,7 @@ int ctx_descriptor(soapb_context *c, const soapb_batch *b, double *d_soap, int k
     if ((rc = c->keep_c.ensure(sizeof(float) * keep_floats_per_site(P) * ((size_t)b->n_sites + 1)))) return rc;
     if ((rc = c->keep_norm.ensure(sizeof(double) * ((size_t)b->n_sites + 1)))) return rc;
   }
-  LaunchCfg cfg = site_cfg(c, false);
+  LaunchCfg cfg = site_cfg(c, false, b->n_sites);
   // the pair kernel also scans n_neigh into the CSR offsets, packs the mask
   // and checks the inputs (its first launch scans, when it runs per chunk)
   const bool pair_chunks = ch && ch->site_off && b->n_sites > 0;
@@ -1249,7 +1249,7 @@ int ctx_contract(soapb_context *c, const soapb_batch *b, const double *d_soap, c
   DevParams P = c->P;
   P.n_pairs = B.n_pairs;
   P.n_sites = B.n_sites;
-  LaunchCfg cfg = site_cfg(c, true);
+  LaunchCfg cfg = site_cfg(c, true, ch ? -1 : b->n_sites);
   // the descriptor call's site order (a permutation of the batch's sites)
   if (!ch && c->order_sites == b->n_sites && b->n_sites > 0) B.order = c->order.as<int>();
   const int nch = (ch && b->n_sites > 0) ? ch->n : 1;
@@ -1583,7 +1583,7 @@ int soapb_descriptor_noalloc(soapb_context *c, const soapb_batch *b, double *d_s
   DevParams P = c->P;
   P.n_pairs = B.n_pairs;
   P.n_sites = B.n_sites;
-  LaunchCfg cfg = site_cfg(c, false);
+  LaunchCfg cfg = site_cfg(c, false, b->n_sites);
   if (b->n_atom_pairs > 0 || b->n_sites > 0) {
     TimedLaunch tl(c, SOAPB_KERNEL_PAIR);
     CU(launch_pair(P, B, c->stream, 0));
@@ -1851,74 +1851,77 @@ int soapb_autotune(soapb_context *c, const soapb_batch *b, int32_t *choice) {
       (rc = pair.ensure(sizeof(double) * 3 * ((size_t)b->n_atom_pairs + 1))))
     return rc;
   CU(cudaMemsetAsync(G.p, 0, sizeof(double) * (size_t)b->n_sites * c->n_soap, c->stream));
-  const int saved_threads = c->threads, saved_ctas = c->max_ctas;
+  const int saved_threads = c->threads, saved[6] = {c->tune_tcd, c->tune_tcc, c->tune_cd,
+                                                    c->tune_cc,  c->tune_tc,  c->tune_sites};
+  auto choose = [&](int tcd, int tcc, int cd, int cc, int tc, int sites) {
+    c->tune_tcd = tcd;
+    c->tune_tcc = tcc;
+    c->tune_cd = cd;
+    c->tune_cc = cc;
+    c->tune_tc = tc;
+    c->tune_sites = sites;
+    c->P.tc_descriptor = c->tc_enable && tcd;
+    c->P.tc_contract = c->tc_enable && tcc;
+  };
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
-  // candidates: the tensor-core kernels (one CTA size) when the caller allows
-  // them, then the CUDA-core kernels at each CTA size; each with three grid caps
-  const int tcand[4] = {0, 64, 128, 256};  // 0: the tensor-core kernel
-  const int ccand[3] = {0, 2 * sms, sms};
-  const int saved_tcd = c->tune_tcd, saved_tcc = c->tune_tcc;
-  float best_d = 1e30f, best_c = 1e30f;
-  int td = 128, cd = 0, tc = 128, cc = 0;
+  // candidates: the CUDA-core kernels, the contract as its launcher's rule has it and at
+  // each CTA size, then the tensor-core kernels, when the caller allows them, at three caps
+  // of their persistent grids
+  struct Form {
+    int tensor, cap, threads;
+  };
+  std::vector<Form> forms = {{0, 0, 0}, {0, 0, 64}, {0, 0, 128}, {0, 0, 256}};
+  if (c->tc_enable) forms.insert(forms.end(), {{1, 0, 0}, {1, 2 * sms, 0}, {1, sms, 0}});
+  Form best_d{}, best_c{};
+  float least_d = 1e30f, least_c = 1e30f;
+  c->threads = 0;
   rc = SOAPB_OK;
-  for (int it = c->tc_enable ? 0 : 1; it < 4 && !rc; ++it)
-    for (int ic = 0; ic < 3 && !rc; ++ic) {
-      c->threads = tcand[it] ? tcand[it] : 128;
-      c->max_ctas = ccand[ic];
-      c->tune_tcd = c->tune_tcc = tcand[it] == 0;
-      c->P.tc_descriptor = c->P.tc_contract = tcand[it] == 0;
-      float md = 1e30f, mc = 1e30f;
-      for (int rep = 0; rep < 4 && !rc; ++rep) {
-        float t1 = 0.f, t2 = 0.f;
-        if (cudaEventRecord(e0, c->stream) != cudaSuccess) { rc = fail(SOAPB_ERR_CUDA, "event"); break; }
-        if ((rc = ctx_descriptor(c, b, soap.as<double>(), 1))) break;
-        if (cudaEventRecord(e1, c->stream) != cudaSuccess) { rc = fail(SOAPB_ERR_CUDA, "event"); break; }
-        if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&t1, e0, e1) != cudaSuccess) {
-          rc = fail(SOAPB_ERR_CUDA, "event timing");
-          break;
-        }
-        cudaEventRecord(e0, c->stream);
-        if ((rc = ctx_contract(c, b, soap.as<double>(), G.as<double>(), 0, 1.0, pair.as<double>()))) break;
-        cudaEventRecord(e1, c->stream);
-        if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&t2, e0, e1) != cudaSuccess) {
-          rc = fail(SOAPB_ERR_CUDA, "event timing");
-          break;
-        }
-        if (rep > 0) {  // the first call of a configuration is a warm-up
-          md = std::min(md, t1);
-          mc = std::min(mc, t2);
-        }
+  for (const Form &f : forms) {
+    if (rc) break;
+    choose(f.tensor, f.tensor, f.cap, f.cap, f.threads, b->n_sites);
+    float md = 1e30f, mc = 1e30f;
+    for (int rep = 0; rep < 4 && !rc; ++rep) {
+      float t1 = 0.f, t2 = 0.f;
+      if (cudaEventRecord(e0, c->stream) != cudaSuccess) { rc = fail(SOAPB_ERR_CUDA, "event"); break; }
+      if ((rc = ctx_descriptor(c, b, soap.as<double>(), 1))) break;
+      if (cudaEventRecord(e1, c->stream) != cudaSuccess) { rc = fail(SOAPB_ERR_CUDA, "event"); break; }
+      if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&t1, e0, e1) != cudaSuccess) {
+        rc = fail(SOAPB_ERR_CUDA, "event timing");
+        break;
       }
-      if (!rc && md < best_d) { best_d = md; td = tcand[it]; cd = ccand[ic]; }
-      if (!rc && mc < best_c) { best_c = mc; tc = tcand[it]; cc = ccand[ic]; }
+      cudaEventRecord(e0, c->stream);
+      if ((rc = ctx_contract(c, b, soap.as<double>(), G.as<double>(), 0, 1.0, pair.as<double>()))) break;
+      cudaEventRecord(e1, c->stream);
+      if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&t2, e0, e1) != cudaSuccess) {
+        rc = fail(SOAPB_ERR_CUDA, "event timing");
+        break;
+      }
+      if (rep > 0) {  // the first call of a configuration is a warm-up
+        md = std::min(md, t1);
+        mc = std::min(mc, t2);
+      }
     }
+    // a later candidate has to win by more than the timings' noise; the CUDA-core
+    // descriptor is one form, whatever the contract's threads
+    if (!rc && (f.tensor || &f == &forms[0]) && md < 0.98f * least_d) { least_d = md; best_d = f; }
+    if (!rc && mc < 0.98f * least_c) { least_c = mc; best_c = f; }
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   c->threads = saved_threads;
-  c->max_ctas = saved_ctas;
   c->keep_valid = 0;  // the timed calls replaced the kept state
   if (rc) {
-    c->tune_tcd = saved_tcd;
-    c->tune_tcc = saved_tcc;
-    c->P.tc_descriptor = c->tc_enable && c->tune_tcd;
-    c->P.tc_contract = c->tc_enable && c->tune_tcc;
+    choose(saved[0], saved[1], saved[2], saved[3], saved[4], saved[5]);
     return rc;
   }
-  c->tune_tcd = td == 0;
-  c->tune_tcc = tc == 0;
-  c->P.tc_descriptor = c->tc_enable && c->tune_tcd;
-  c->P.tc_contract = c->tc_enable && c->tune_tcc;
-  c->tune_td = td ? td : 128;
-  c->tune_cd = cd;
-  c->tune_tc = tc ? tc : 128;
-  c->tune_cc = cc;
+  choose(best_d.tensor, best_c.tensor, best_d.cap, best_c.cap, best_c.threads, b->n_sites);
   if (choice) {
-    choice[0] = td;
-    choice[1] = cd;
-    choice[2] = tc;
-    choice[3] = cc;
+    choice[0] = best_d.tensor ? 0 : 128;
+    choice[1] = best_d.cap;
+    choice[2] = best_c.tensor ? 0 : best_c.threads ? best_c.threads : contract_rule_threads(c->P, b->n_sites);
+    choice[3] = best_c.cap;
   }
   return SOAPB_OK;
 }

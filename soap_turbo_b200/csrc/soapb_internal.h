@@ -164,7 +164,7 @@ struct LaunchCfg {
   int slots;             // 64, 128 or 256: the pairs whose entries the descriptor sorts and groups together, and
                          // the partial sums of the norm, of q . G and of the central pair
   cudaStream_t stream;
-  int max_ctas;          // grid cap (0: one CTA per site)
+  int max_ctas;          // cap of the tensor-core kernels' persistent grids (0: what is resident)
 };
 int sm_count();  // SMs of the current device, asked once (the launchers' rules are in waves of its CTAs)
 cudaError_t launch_prep(const DevParams &P, const DevBatch &B, cudaStream_t s);
@@ -187,6 +187,7 @@ cudaError_t launch_descriptor(const DevParams &P, const DevBatch &B, const Launc
 cudaError_t launch_contract(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
                             const double *soap, const double *G, int g_layout, double sgn,
                             const float *keep_c, const double *keep_norm, double *pair);
+int contract_rule_threads(const DevParams &P, int n_sites);  // of the CUDA-core contract, LaunchCfg::threads 0
 // Device address and size of the static scratch array (soapb_noalloc.cu);
 // `device` must be current.
 cudaError_t noalloc_scratch(int device, unsigned char **addr, size_t *bytes);

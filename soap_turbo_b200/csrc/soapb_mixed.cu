@@ -881,7 +881,6 @@ __global__ void __launch_bounds__(kDescThreads<AMAX, LC, NH, GROUPS>,
   const int kk = own ? k_of : P.k_max - 1;  // the last lanes repeat the last k and store nothing
   const int lm = __ldg((const int *)(P.blob + P.off_klm) + kk), l = lm & 0xff, m = lm >> 8;
   const int rounds = min(chunk / 2, 64);
-  const int n_run = B.site_hi - B.site_lo;
   const int4 it0 = tid < P.n_kept ? __ldg(P.ps_order + tid) : make_int4(0, 0, 0, 0);
   // the 16-byte pieces of an entry that the lane stages: of the row's head, then of R_n
   constexpr int NC = (HD / 4 + AMAX / 4 + 31) / 32;
@@ -902,233 +901,230 @@ __global__ void __launch_bounds__(kDescThreads<AMAX, LC, NH, GROUPS>,
     piece[c].per_species = r >= 0 ? 2 * AMAX : 0;
   }
 
-  for (int b = blockIdx.x; b < n_run; b += gridDim.x) {
-    const int site = B.order ? B.order[b] : B.site_lo + b;
-    const int p_begin = B.off[site], p_end = min(B.off[site + 1], B.n_pairs);
-    // the species whose sums the thread holds, its rounds so far, their sums but
-    // for the last, and that of the last
-    int cs = group, n_rounds = 0;
-    double tr[NH], ti[NH], dr[NH], di[NH];
-    float2 *kc = (float2 *)(keep_c + ((keep & 1) ? (size_t)site * keep_stride(P) : 0)) + kk;
-    auto finish = [&]() {  // species cs is complete
-      const int a = P.rad[cs].alpha, nb = P.rad[cs].nbeg;
-      if (n_rounds != 1)
+  const int site = B.order ? B.order[blockIdx.x] : B.site_lo + (int)blockIdx.x;
+  const int p_begin = B.off[site], p_end = min(B.off[site + 1], B.n_pairs);
+  // the species whose sums the thread holds, its rounds so far, their sums but
+  // for the last, and that of the last
+  int cs = group, n_rounds = 0;
+  double tr[NH], ti[NH], dr[NH], di[NH];
+  float2 *kc = (float2 *)(keep_c + ((keep & 1) ? (size_t)site * keep_stride(P) : 0)) + kk;
+  auto finish = [&]() {  // species cs is complete
+    const int a = P.rad[cs].alpha, nb = P.rad[cs].nbeg;
+    if (n_rounds != 1)
 #pragma unroll
-        for (int n = 0; n < NH; ++n) {
-          dr[n] = n_rounds ? tr[n] + dr[n] : 0.0;
-          di[n] = n_rounds ? ti[n] + di[n] : 0.0;
-        }
-      // poly3gauss central-atom term (src/soap_turbo.f90:646-662)
-      if (P.basis == 1 && kk == 0) {
-        const int mult = B.species_mult[site];
-        for (int mm = 0; mm < mult; ++mm)
-          if (B.species[(size_t)site * B.max_mult + mm] - 1 == cs)
-#pragma unroll
-            for (int n = 0; n < NH; ++n)
-              if (n0 + n < a) dr[n] += P.central[nb + n0 + n];
+      for (int n = 0; n < NH; ++n) {
+        dr[n] = n_rounds ? tr[n] + dr[n] : 0.0;
+        di[n] = n_rounds ? ti[n] + di[n] : 0.0;
       }
-      float2 *cc = sC + (nb + n0) * KS + kk;
-      if (own)
+    // poly3gauss central-atom term (src/soap_turbo.f90:646-662)
+    if (P.basis == 1 && kk == 0) {
+      const int mult = B.species_mult[site];
+      for (int mm = 0; mm < mult; ++mm)
+        if (B.species[(size_t)site * B.max_mult + mm] - 1 == cs)
 #pragma unroll
-        for (int n = 0; n < NH; ++n)
-          if (n0 + n < a) cc[n * KS] = make_float2((float)dr[n], (float)di[n]);
-      if (own && (keep & 1)) {
-        float2 *kr = kc + (nb + n0) * KS;
+          for (int n = 0; n < NH; ++n)
+            if (n0 + n < a) dr[n] += P.central[nb + n0 + n];
+    }
+    float2 *cc = sC + (nb + n0) * KS + kk;
+    if (own)
 #pragma unroll
-        for (int n = 0; n < NH; ++n)
-          if (n0 + n < a) kr[n * KS] = make_float2((float)dr[n], (float)di[n]);
+      for (int n = 0; n < NH; ++n)
+        if (n0 + n < a) cc[n * KS] = make_float2((float)dr[n], (float)di[n]);
+    if (own && (keep & 1)) {
+      float2 *kr = kc + (nb + n0) * KS;
+#pragma unroll
+      for (int n = 0; n < NH; ++n)
+        if (n0 + n < a) kr[n * KS] = make_float2((float)dr[n], (float)di[n]);
+    }
+    cs += groups;
+    n_rounds = 0;
+  };
+  // a site of one chunk takes all its species at once; else a species per group at a time
+  const bool multi = p_end - p_begin > chunk;
+  for (int s_lo = 0; s_lo < nsp; s_lo += multi ? groups : nsp) {
+    const int s_hi = multi ? min(nsp, s_lo + groups) : nsp;
+    for (int c0 = p_begin; c0 < p_end; c0 += chunk) {
+      const int c1 = min(p_end, c0 + chunk);
+      const unsigned long long valid = valid_species(P, B, p_begin, c0, c1, false);
+      // the place of species s_lo among the chunk's entries, which fixes the rounds
+      const int e0 = __reduce_add_sync(0xffffffffu, __popcll(valid & (0x0101010101010101ull * ((1u << s_lo) - 1u))));
+      if (multi) __syncthreads();  // the previous chunk's list is read
+      int e = e0;
+      for (int s = s_lo; s < s_hi; ++s) {
+        if (lane == 0) sBase[s] = e;
+        e = list_species(valid, s, c1 - c0, e, list - e0);
       }
-      cs += groups;
-      n_rounds = 0;
-    };
-    // a site of one chunk takes all its species at once; else a species per group at a time
-    const bool multi = p_end - p_begin > chunk;
-    for (int s_lo = 0; s_lo < nsp; s_lo += multi ? groups : nsp) {
-      const int s_hi = multi ? min(nsp, s_lo + groups) : nsp;
-      for (int c0 = p_begin; c0 < p_end; c0 += chunk) {
-        const int c1 = min(p_end, c0 + chunk);
-        const unsigned long long valid = valid_species(P, B, p_begin, c0, c1, false);
-        // the place of species s_lo among the chunk's entries, which fixes the rounds
-        const int e0 = __reduce_add_sync(0xffffffffu, __popcll(valid & (0x0101010101010101ull * ((1u << s_lo) - 1u))));
-        if (multi) __syncthreads();  // the previous chunk's list is read
-        int e = e0;
-        for (int s = s_lo; s < s_hi; ++s) {
-          if (lane == 0) sBase[s] = e;
-          e = list_species(valid, s, c1 - c0, e, list - e0);
-        }
-        if (lane == 0) sBase[s_hi] = e;
-        __syncwarp();
-        const int e1 = e;
-        const float *src[NC];
+      if (lane == 0) sBase[s_hi] = e;
+      __syncwarp();
+      const int e1 = e;
+      const float *src[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
-          src[c] = piece[c].rad ? B.rad + (size_t)c0 * nsp * 2 * AMAX + piece[c].first
-                                : B.ang + (size_t)c0 * AW + piece[c].first;
-        for (int w0 = e0, w1; w0 < e1; w0 = w1) {
-          w1 = min(e1, w0 + rounds - (w0 & (rounds - 1)));
-          float *dst = sX + warp * ST;
+      for (int c = 0; c < NC; ++c)
+        src[c] = piece[c].rad ? B.rad + (size_t)c0 * nsp * 2 * AMAX + piece[c].first
+                              : B.ang + (size_t)c0 * AW + piece[c].first;
+      for (int w0 = e0, w1; w0 < e1; w0 = w1) {
+        w1 = min(e1, w0 + rounds - (w0 & (rounds - 1)));
+        float *dst = sX + warp * ST;
 #pragma unroll 4
-          for (int q = w0 + warp; q < w1; q += nw, dst += nw * ST) {
-            const unsigned code = list[q - e0], j = code & 0xffu, sp = code >> 8;
+        for (int q = w0 + warp; q < w1; q += nw, dst += nw * ST) {
+          const unsigned code = list[q - e0], j = code & 0xffu, sp = code >> 8;
 #pragma unroll
-            for (int c = 0; c < NC; ++c)
-              if (piece[c].on)
-                cp_async16(dst + piece[c].dst, src[c] + (j * piece[c].per_pair + sp * piece[c].per_species));
-          }
-          cp_async_wait_all();
-          __syncthreads();
-          for (int s = s_lo + group; s < s_hi; s += groups) {
-            const int lo = max(w0, sBase[s]), hi = min(w1, sBase[s + 1]);
-            if (lo >= hi) continue;
-            while (cs < s) finish();
-            if (n0 >= P.rad[s].alpha) continue;
-            // the central pair carries central_weight (:638-646): the pair kernel
-            // expanded every pair as a neighbour
-            const bool weighted = P.rad[s].cw != 1.0 && c0 == p_begin && lo == sBase[s] && (list[lo - e0] & 0xff) == 0;
-            const float cw = (float)P.rad[s].cw;
-            if (n_rounds > 0)
+          for (int c = 0; c < NC; ++c)
+            if (piece[c].on)
+              cp_async16(dst + piece[c].dst, src[c] + (j * piece[c].per_pair + sp * piece[c].per_species));
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        for (int s = s_lo + group; s < s_hi; s += groups) {
+          const int lo = max(w0, sBase[s]), hi = min(w1, sBase[s + 1]);
+          if (lo >= hi) continue;
+          while (cs < s) finish();
+          if (n0 >= P.rad[s].alpha) continue;
+          // the central pair carries central_weight (:638-646): the pair kernel
+          // expanded every pair as a neighbour
+          const bool weighted = P.rad[s].cw != 1.0 && c0 == p_begin && lo == sBase[s] && (list[lo - e0] & 0xff) == 0;
+          const float cw = (float)P.rad[s].cw;
+          if (n_rounds > 0)
 #pragma unroll
-              for (int n = 0; n < NH; ++n) {
-                tr[n] = n_rounds > 1 ? tr[n] + dr[n] : dr[n];
-                ti[n] = n_rounds > 1 ? ti[n] + di[n] : di[n];
+            for (int n = 0; n < NH; ++n) {
+              tr[n] = n_rounds > 1 ? tr[n] + dr[n] : dr[n];
+              ti[n] = n_rounds > 1 ? ti[n] + di[n] : di[n];
+            }
+          ++n_rounds;
+          f32x2 pr[NH / 2], pi[NH / 2];
+          const float *A = sX + (lo - w0) * ST;
+          const float *aP = A + row_p(LC) + kk, *aL = A + row_il(LC) + l, *aE = A + row_e(LC) + 2 * m,
+                      *aR = A + HD + n0;
+          auto add = [&](int o, bool first, bool opens) {  // the round's first entry, its group's first
+            // u_k = (preflm_k P_k) (amp i_l) (src/soap_turbo_angular.f90:590-594)
+            const float u = aP[o] * aL[o];
+            const float2 e2 = *(const float2 *)(aE + o);
+            const float ar = u * e2.x, ai = u * e2.y;
+            const f32x2 ar2 = pack2(ar, ar), ai2 = pack2(ai, ai);
+            f32x2 r[NH / 2];
+            if constexpr (NH % 4 == 0) {
+#pragma unroll
+              for (int n = 0; n < NH / 4; ++n) {
+                const ulonglong2 v = *(const ulonglong2 *)(aR + o + 4 * n);
+                r[2 * n] = v.x;
+                r[2 * n + 1] = v.y;
               }
-            ++n_rounds;
-            f32x2 pr[NH / 2], pi[NH / 2];
-            const float *A = sX + (lo - w0) * ST;
-            const float *aP = A + row_p(LC) + kk, *aL = A + row_il(LC) + l, *aE = A + row_e(LC) + 2 * m,
-                        *aR = A + HD + n0;
-            auto add = [&](int o, bool first, bool opens) {  // the round's first entry, its group's first
-              // u_k = (preflm_k P_k) (amp i_l) (src/soap_turbo_angular.f90:590-594)
-              const float u = aP[o] * aL[o];
-              const float2 e2 = *(const float2 *)(aE + o);
-              const float ar = u * e2.x, ai = u * e2.y;
-              const f32x2 ar2 = pack2(ar, ar), ai2 = pack2(ai, ai);
-              f32x2 r[NH / 2];
-              if constexpr (NH % 4 == 0) {
+            } else {
 #pragma unroll
-                for (int n = 0; n < NH / 4; ++n) {
-                  const ulonglong2 v = *(const ulonglong2 *)(aR + o + 4 * n);
-                  r[2 * n] = v.x;
-                  r[2 * n + 1] = v.y;
-                }
-              } else {
-#pragma unroll
-                for (int n = 0; n < NH / 2; ++n) r[n] = *(const f32x2 *)(aR + o + 2 * n);
-              }
-              if (first && weighted)
-#pragma unroll
-                for (int n = 0; n < NH / 2; ++n) {
-                  const float2 v = unpack2(r[n]);
-                  r[n] = pack2(v.x * cw, v.y * cw);
-                }
+              for (int n = 0; n < NH / 2; ++n) r[n] = *(const f32x2 *)(aR + o + 2 * n);
+            }
+            if (first && weighted)
 #pragma unroll
               for (int n = 0; n < NH / 2; ++n) {
-                pr[n] = opens ? fmul2(r[n], ar2) : ffma2(r[n], ar2, pr[n]);
-                pi[n] = opens ? fmul2(r[n], ai2) : ffma2(r[n], ai2, pi[n]);
+                const float2 v = unpack2(r[n]);
+                r[n] = pack2(v.x * cw, v.y * cw);
               }
-            };
-            auto flush = [&](bool first) {  // the round's first group
 #pragma unroll
-              for (int n = 0; n < NH / 2; ++n) {
-                const float2 vr = unpack2(pr[n]), vi = unpack2(pi[n]);
-                dr[2 * n] = first ? (double)vr.x : dr[2 * n] + (double)vr.x;
-                dr[2 * n + 1] = first ? (double)vr.y : dr[2 * n + 1] + (double)vr.y;
-                di[2 * n] = first ? (double)vi.x : di[2 * n] + (double)vi.x;
-                di[2 * n + 1] = first ? (double)vi.y : di[2 * n + 1] + (double)vi.y;
-              }
-            };
-            int i = lo;
-            for (; i + 4 <= hi; i += 4) {
+            for (int n = 0; n < NH / 2; ++n) {
+              pr[n] = opens ? fmul2(r[n], ar2) : ffma2(r[n], ar2, pr[n]);
+              pi[n] = opens ? fmul2(r[n], ai2) : ffma2(r[n], ai2, pi[n]);
+            }
+          };
+          auto flush = [&](bool first) {  // the round's first group
 #pragma unroll
-              for (int q = 0; q < 4; ++q) add(q * ST, q == 0 && i == lo, q == 0);
-              if (i == lo) flush(true);
-              else flush(false);
-              aP += 4 * ST;
-              aL += 4 * ST;
-              aE += 4 * ST;
-              aR += 4 * ST;
+            for (int n = 0; n < NH / 2; ++n) {
+              const float2 vr = unpack2(pr[n]), vi = unpack2(pi[n]);
+              dr[2 * n] = first ? (double)vr.x : dr[2 * n] + (double)vr.x;
+              dr[2 * n + 1] = first ? (double)vr.y : dr[2 * n + 1] + (double)vr.y;
+              di[2 * n] = first ? (double)vi.x : di[2 * n] + (double)vi.x;
+              di[2 * n + 1] = first ? (double)vi.y : di[2 * n + 1] + (double)vi.y;
             }
-            if (i < hi) {
-              const int n_last = hi - i;
-              add(0, i == lo, true);
-              if (n_last > 1) add(ST, false, false);
-              if (n_last > 2) add(2 * ST, false, false);
-              if (i == lo) flush(true);
-              else flush(false);
-            }
+          };
+          int i = lo;
+          for (; i + 4 <= hi; i += 4) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) add(q * ST, q == 0 && i == lo, q == 0);
+            if (i == lo) flush(true);
+            else flush(false);
+            aP += 4 * ST;
+            aL += 4 * ST;
+            aE += 4 * ST;
+            aR += 4 * ST;
           }
-          __syncthreads();  // the round's rows are read
+          if (i < hi) {
+            const int n_last = hi - i;
+            add(0, i == lo, true);
+            if (n_last > 1) add(ST, false, false);
+            if (n_last > 2) add(2 * ST, false, false);
+            if (i == lo) flush(true);
+            else flush(false);
+          }
         }
+        __syncthreads();  // the round's rows are read
       }
     }
-    while (cs < nsp) finish();
-    __syncthreads();
-    // power spectrum of the kept components (src/soap_turbo.f90:750-795)
-    float *pout = P.cmap_identity ? sS : sP;
-    int4 it = it0;
-    for (int t = tid; t < P.n_kept; t += nt) {
-      const int4 nx = t + nt < P.n_kept ? __ldg(P.ps_order + t + nt) : it;  // a round trip ahead
-      const float2 *cn = sC + it.x, *cp = sC + it.y;
-      const int lq = it.w & 0xff;
-      const float acc0 = cn[0].x * cp[0].x + cn[0].y * cp[0].y;
-      float acc = 0.f;
-#pragma unroll 4
-      for (int q = 1; q <= lq; ++q) acc += cn[q].x * cp[q].x + cn[q].y * cp[q].y;
-      const float base = it.w < 0 ? 1.41421356237309504880f : 1.f;
-      const float v = base * (acc0 + 2.f * acc);
-      pout[it.z] = v;
-      it = nx;
-    }
-    __syncthreads();
-    if (!P.cmap_identity) {
-      // compression through the map (:798-802)
-      for (int o = tid; o < P.n_soap; o += nt) {
-        float v = 0.f;
-        for (int t = P.pi_off[o]; t < P.pi_off[o + 1]; ++t) v += P.pi_el[t] * sP[P.pi_q[t]];
-        sS[o] = v;
-      }
-      __syncthreads();
-    }
-    // the norm (:805-809) over `chunk` slots.  accumulate: the caller's soap row is
-    // added before the norm is taken, as the reference adds the compressed descriptor
-    // into soap (:798-802); the row may lie in host memory, so it is read here and where
-    // it is written, and not by every warp
-    double *out = soap_out + (size_t)site * P.n_soap;
-    const bool acc = (keep & 2) != 0;
-    double nrm2;
-    if (!acc && chunk == 128) {
-      double v[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int o = lane; o < P.n_soap; o += 128)
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const double y = o + 32 * w < P.n_soap ? (double)sS[o + 32 * w] : 0.0;
-          v[w] = fma(y, y, v[w]);
-        }
-      nrm2 = slots_by_warp(v);
-    } else {
-      double *red = (double *)(smem + Ly.base);  // eight: the species' places are read
-      for (int w = warp; 32 * w < chunk; w += nw) {
-        double v = 0.0;
-        for (int o = 32 * w + lane; o < P.n_soap; o += chunk) {
-          const double y = acc ? (double)sS[o] + out[o] : (double)sS[o];
-          v = fma(y, y, v);
-        }
-        v = warp_sum(v);
-        if (lane == 0) red[w] = v;
-      }
-      __syncthreads();
-      nrm2 = slot_tree(red, chunk);
-    }
-    double norm = sqrt(nrm2);
-    if (norm < 1.0e-5) norm = 1.0;
-    const double inv = 1.0 / norm;
-    if (acc)
-      for (int o = tid; o < P.n_soap; o += nt) out[o] = ((double)sS[o] + out[o]) * inv;
-    else
-      for (int o = tid; o < P.n_soap; o += nt) out[o] = (double)sS[o] * inv;
-    if ((keep & 1) && tid == 0) keep_norm[site] = norm;
-    __syncthreads();  // sC and sS are free for the next site
   }
+  while (cs < nsp) finish();
+  __syncthreads();
+  // power spectrum of the kept components (src/soap_turbo.f90:750-795)
+  float *pout = P.cmap_identity ? sS : sP;
+  int4 it = it0;
+  for (int t = tid; t < P.n_kept; t += nt) {
+    const int4 nx = t + nt < P.n_kept ? __ldg(P.ps_order + t + nt) : it;  // a round trip ahead
+    const float2 *cn = sC + it.x, *cp = sC + it.y;
+    const int lq = it.w & 0xff;
+    const float acc0 = cn[0].x * cp[0].x + cn[0].y * cp[0].y;
+    float acc = 0.f;
+#pragma unroll 4
+    for (int q = 1; q <= lq; ++q) acc += cn[q].x * cp[q].x + cn[q].y * cp[q].y;
+    const float base = it.w < 0 ? 1.41421356237309504880f : 1.f;
+    const float v = base * (acc0 + 2.f * acc);
+    pout[it.z] = v;
+    it = nx;
+  }
+  __syncthreads();
+  if (!P.cmap_identity) {
+    // compression through the map (:798-802)
+    for (int o = tid; o < P.n_soap; o += nt) {
+      float v = 0.f;
+      for (int t = P.pi_off[o]; t < P.pi_off[o + 1]; ++t) v += P.pi_el[t] * sP[P.pi_q[t]];
+      sS[o] = v;
+    }
+    __syncthreads();
+  }
+  // the norm (:805-809) over `chunk` slots.  accumulate: the caller's soap row is
+  // added before the norm is taken, as the reference adds the compressed descriptor
+  // into soap (:798-802); the row may lie in host memory, so it is read here and where
+  // it is written, and not by every warp
+  double *out = soap_out + (size_t)site * P.n_soap;
+  const bool acc = (keep & 2) != 0;
+  double nrm2;
+  if (!acc && chunk == 128) {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int o = lane; o < P.n_soap; o += 128)
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const double y = o + 32 * w < P.n_soap ? (double)sS[o + 32 * w] : 0.0;
+        v[w] = fma(y, y, v[w]);
+      }
+    nrm2 = slots_by_warp(v);
+  } else {
+    double *red = (double *)(smem + Ly.base);  // eight: the species' places are read
+    for (int w = warp; 32 * w < chunk; w += nw) {
+      double v = 0.0;
+      for (int o = 32 * w + lane; o < P.n_soap; o += chunk) {
+        const double y = acc ? (double)sS[o] + out[o] : (double)sS[o];
+        v = fma(y, y, v);
+      }
+      v = warp_sum(v);
+      if (lane == 0) red[w] = v;
+    }
+    __syncthreads();
+    nrm2 = slot_tree(red, chunk);
+  }
+  double norm = sqrt(nrm2);
+  if (norm < 1.0e-5) norm = 1.0;
+  const double inv = 1.0 / norm;
+  if (acc)
+    for (int o = tid; o < P.n_soap; o += nt) out[o] = ((double)sS[o] + out[o]) * inv;
+  else
+    for (int o = tid; o < P.n_soap; o += nt) out[o] = (double)sS[o] * inv;
+  if ((keep & 1) && tid == 0) keep_norm[site] = norm;
 }
 
 // ------------------------------------------------------------ descriptor on tensor cores
@@ -1539,7 +1535,6 @@ __global__ void __launch_bounds__(256, 2)
   const int n_max = P.n_max, k_max = P.k_max, n_soap = P.n_soap, nsp = P.n_species, n_sites = B.n_sites;
   const int *klm = (const int *)(P.blob + P.off_klm);
   const int *hitem = (const int *)(P.blob_c + P.off_hitem), *nmap = (const int *)(P.blob_c + P.off_nmap);
-  const int n_run = B.site_hi - B.site_lo;
 
   // the lane's k: where its values stand in a row, and the derivative forms'
   // coefficients (src/soap_turbo_angular.f90:194-246; a form that an (l, m) lacks has
@@ -1574,320 +1569,317 @@ __global__ void __launch_bounds__(256, 2)
     piece[c].per_species = p >= AW / 4 ? 2 * AMAX : 0;
   }
 
-  for (int b = blockIdx.x; b < n_run; b += gridDim.x) {
-    const int site = B.order ? B.order[b] : B.site_lo + b;
-    const int p_begin = B.off[site], p_end = min(B.off[site + 1], B.n_pairs);
-    const double knorm = keep_norm[site];
-    const double *q = soap_in + (size_t)site * n_soap;
-    const double *g = g_layout == 0 ? G + site : G + (size_t)site * n_soap;
-    const size_t gs = g_layout == 0 ? (size_t)n_sites : 1;
-    double gv[GPT], qv[GPT];
+  const int site = B.order ? B.order[blockIdx.x] : B.site_lo + (int)blockIdx.x;
+  const int p_begin = B.off[site], p_end = min(B.off[site + 1], B.n_pairs);
+  const double knorm = keep_norm[site];
+  const double *q = soap_in + (size_t)site * n_soap;
+  const double *g = g_layout == 0 ? G + site : G + (size_t)site * n_soap;
+  const size_t gs = g_layout == 0 ? (size_t)n_sites : 1;
+  double gv[GPT], qv[GPT];
 #pragma unroll
-    for (int j = 0; j < GPT; ++j) {
-      const int o = t0 + j * wide;
-      gv[j] = qv[j] = 0.0;
-      if (o < n_soap) {
-        gv[j] = g[o * gs];
-        qv[j] = q[o];
-      }
+  for (int j = 0; j < GPT; ++j) {
+    const int o = t0 + j * wide;
+    gv[j] = qv[j] = 0.0;
+    if (o < n_soap) {
+      gv[j] = g[o * gs];
+      qv[j] = q[o];
     }
-    {
-      const float *kc = keep_c + (size_t)site * keep_stride(P);
-      const int n4 = (2 * n_max * KS) / 4;
-      for (int t = tid; t < n4; t += nt) cp_async16((float *)sC + 4 * t, kc + 4 * t);
-      for (int t = 4 * n4 + tid; t < 2 * n_max * KS; t += nt) ((float *)sC)[t] = kc[t];
-    }
-    // ---- back through the normalisation (src/soap_turbo.f90:1783-1790)
-    double qg0 = 0.0, qg1 = 0.0;
+  }
+  {
+    const float *kc = keep_c + (size_t)site * keep_stride(P);
+    const int n4 = (2 * n_max * KS) / 4;
+    for (int t = tid; t < n4; t += nt) cp_async16((float *)sC + 4 * t, kc + 4 * t);
+    for (int t = 4 * n4 + tid; t < 2 * n_max * KS; t += nt) ((float *)sC)[t] = kc[t];
+  }
+  // ---- back through the normalisation (src/soap_turbo.f90:1783-1790)
+  double qg0 = 0.0, qg1 = 0.0;
 #pragma unroll
-    for (int j = 0; j < GPT; ++j) {
-      if (two && (j & 1)) qg1 = fma(qv[j], gv[j], qg1);
-      else qg0 = fma(qv[j], gv[j], qg0);
-    }
+  for (int j = 0; j < GPT; ++j) {
+    if (two && (j & 1)) qg1 = fma(qv[j], gv[j], qg1);
+    else qg0 = fma(qv[j], gv[j], qg0);
+  }
 #pragma unroll 4
-    for (int o = t0 + GPT * wide, j = GPT; o < n_soap; o += wide, ++j) {
-      const double gj = g[o * gs], qj = q[o];
-      if (two && (j & 1)) qg1 = fma(qj, gj, qg1);
-      else qg0 = fma(qj, gj, qg0);
+  for (int o = t0 + GPT * wide, j = GPT; o < n_soap; o += wide, ++j) {
+    const double gj = g[o * gs], qj = q[o];
+    if (two && (j & 1)) qg1 = fma(qj, gj, qg1);
+    else qg0 = fma(qj, gj, qg0);
+  }
+  if (tid < wide) {
+    qg0 = warp_sum(qg0);
+    if (lane == 0) sRed[warp] = qg0;
+    if (two) {
+      qg1 = warp_sum(qg1);
+      if (lane == 0) sRed[warp + nw] = qg1;
     }
-    if (tid < wide) {
-      qg0 = warp_sum(qg0);
-      if (lane == 0) sRed[warp] = qg0;
-      if (two) {
-        qg1 = warp_sum(qg1);
-        if (lane == 0) sRed[warp + nw] = qg1;
-      }
+  }
+  __syncthreads();
+  const double qg = slot_tree(sRed, slots), inv = 1.0 / knorm;
+#pragma unroll
+  for (int j = 0; j < GPT; ++j) {
+    const int o = t0 + j * wide;
+    if (o < n_soap) sGp[o] = (float)((gv[j] - qv[j] * qg) * inv);
+  }
+#pragma unroll 4
+  for (int o = t0 + GPT * wide; o < n_soap; o += wide) sGp[o] = (float)((g[o * gs] - q[o] * qg) * inv);
+  cp_async_wait_all();
+  __syncthreads();
+  // ---- back through the compression (:1791-1798), unless it is one-to-one
+  if (!P.cmap_identity) {
+    for (int t = tid; t < P.n_kept; t += nt) {
+      float v = 0.f;
+      for (int e = P.pj_off[t]; e < P.pj_off[t + 1]; ++e) v += P.pj_el[e] * sGp[P.pj_o[e]];
+      sGu[t] = v;
     }
     __syncthreads();
-    const double qg = slot_tree(sRed, slots), inv = 1.0 / knorm;
+  }
+  // ---- H(k,n) = w(m) sum_np Y(n,np,l) c(k,np) over the non-zero Y (:1800-1835); an
+  // item per (n, l, m0) walks its Y list once for up to kHM values of m, the
+  // longest lists first
+  for (int it = tid; it < P.n_hitem; it += nt) {
+    const int code = __ldg(hitem + it), n = code & 0xff, l = (code >> 8) & 0xff, m0 = code >> 16;
+    const int kb = l * (l + 1) / 2 + m0, mn = min(kHM, l + 1 - m0), li = l * n_max + n;
+    const int t1 = __ldg(P.hl_off + li + 1);
+    float2 h[kHM];
 #pragma unroll
-    for (int j = 0; j < GPT; ++j) {
-      const int o = t0 + j * wide;
-      if (o < n_soap) sGp[o] = (float)((gv[j] - qv[j] * qg) * inv);
-    }
-#pragma unroll 4
-    for (int o = t0 + GPT * wide; o < n_soap; o += wide) sGp[o] = (float)((g[o * gs] - q[o] * qg) * inv);
-    cp_async_wait_all();
-    __syncthreads();
-    // ---- back through the compression (:1791-1798), unless it is one-to-one
-    if (!P.cmap_identity) {
-      for (int t = tid; t < P.n_kept; t += nt) {
-        float v = 0.f;
-        for (int e = P.pj_off[t]; e < P.pj_off[t + 1]; ++e) v += P.pj_el[e] * sGp[P.pj_o[e]];
-        sGu[t] = v;
-      }
-      __syncthreads();
-    }
-    // ---- H(k,n) = w(m) sum_np Y(n,np,l) c(k,np) over the non-zero Y (:1800-1835); an
-    // item per (n, l, m0) walks its Y list once for up to kHM values of m, the
-    // longest lists first
-    for (int it = tid; it < P.n_hitem; it += nt) {
-      const int code = __ldg(hitem + it), n = code & 0xff, l = (code >> 8) & 0xff, m0 = code >> 16;
-      const int kb = l * (l + 1) / 2 + m0, mn = min(kHM, l + 1 - m0), li = l * n_max + n;
-      const int t1 = __ldg(P.hl_off + li + 1);
-      float2 h[kHM];
-#pragma unroll
-      for (int j = 0; j < kHM; ++j) h[j] = make_float2(0.f, 0.f);
-      const float2 *cb = sC + kb;
+    for (int j = 0; j < kHM; ++j) h[j] = make_float2(0.f, 0.f);
+    const float2 *cb = sC + kb;
 #pragma unroll 2
-      for (int t = __ldg(P.hl_off + li); t < t1; ++t) {
-        const int e = __ldg(P.hl_packed + t);
-        const float y = (e < 0 ? 2.f : 1.41421356237309504880f) * sGu[(e >> 8) & 0xffff];
-        // past the last m the values belong to the next l, or to the next array: read, not stored
-        const float2 *c = cb + (e & 0xff) * KS;
+    for (int t = __ldg(P.hl_off + li); t < t1; ++t) {
+      const int e = __ldg(P.hl_packed + t);
+      const float y = (e < 0 ? 2.f : 1.41421356237309504880f) * sGu[(e >> 8) & 0xffff];
+      // past the last m the values belong to the next l, or to the next array: read, not stored
+      const float2 *c = cb + (e & 0xff) * KS;
 #pragma unroll
-        for (int j = 0; j < kHM; ++j) {
-          h[j].x = fmaf(y, c[j].x, h[j].x);
-          h[j].y = fmaf(y, c[j].y, h[j].y);
-        }
+      for (int j = 0; j < kHM; ++j) {
+        h[j].x = fmaf(y, c[j].x, h[j].x);
+        h[j].y = fmaf(y, c[j].y, h[j].y);
       }
-      const int nm = __ldg(nmap + n);
-      float2 *o = sH + kb * HS + (nm & 0xff) * AMAX + (nm >> 8);
+    }
+    const int nm = __ldg(nmap + n);
+    float2 *o = sH + kb * HS + (nm & 0xff) * AMAX + (nm >> 8);
 #pragma unroll
-      for (int j = 0; j < kHM; ++j)
-        if (j < mn) {
-          const float w = (m0 + j == 0) ? 1.f : 2.f;
-          o[j * HS] = make_float2(w * h[j].x, w * h[j].y);
-        }
-    }
-    // what no item writes: the columns past a species' alpha, and of empty lists
-    for (int t = tid; t < P.n_hzero; t += nt) {
-      const int code = __ldg(P.h_zero + t);
-      sH[(code >> 16) * HS + (code & 0xffff)] = make_float2(0.f, 0.f);
-    }
+    for (int j = 0; j < kHM; ++j)
+      if (j < mn) {
+        const float w = (m0 + j == 0) ? 1.f : 2.f;
+        o[j * HS] = make_float2(w * h[j].x, w * h[j].y);
+      }
+  }
+  // what no item writes: the columns past a species' alpha, and of empty lists
+  for (int t = tid; t < P.n_hzero; t += nt) {
+    const int code = __ldg(P.h_zero + t);
+    sH[(code >> 16) * HS + (code & 0xffff)] = make_float2(0.f, 0.f);
+  }
 
-    // the thread's slots of the central pair between two chunks of the row (volatile: in
-    // local memory, and not in registers while H fills them)
-    volatile double held[6];
-    for (int c0 = p_begin; c0 < p_end; c0 += kContractChunk) {
-      const int c1 = min(p_end, c0 + kContractChunk);
-      if (c0 > p_begin) __syncthreads();  // the chunk before is read
-      // entries by species, and per (pair, species) its entry or -1, by the last warp
-      // (which has the shortest of H's lists)
-      if (warp == nw - 1) {
-        const unsigned long long valid = valid_species(P, B, p_begin, c0, c1, true);
-        const unsigned lt = (1u << lane) - 1u;
-        int e = 0;
-        for (int s = 0; s < nsp; ++s) {
-          if (lane == 0) sBase[s] = e;
-          for (int c = 0; c0 + 32 * c < c1; ++c) {
-            const bool on = (valid >> (8 * c + s)) & 1ull;
-            const unsigned m = __ballot_sync(0xffffffffu, on);
-            const int at = e + __popc(m & lt);
-            if (on) list[at] = (unsigned short)(32 * c + lane);
-            slot[s * kContractChunk + 32 * c + lane] = (short)(on ? at : -1);
-            e += __popc(m);
-          }
+  // the thread's slots of the central pair between two chunks of the row (volatile: in
+  // local memory, and not in registers while H fills them)
+  volatile double held[6];
+  for (int c0 = p_begin; c0 < p_end; c0 += kContractChunk) {
+    const int c1 = min(p_end, c0 + kContractChunk);
+    if (c0 > p_begin) __syncthreads();  // the chunk before is read
+    // entries by species, and per (pair, species) its entry or -1, by the last warp
+    // (which has the shortest of H's lists)
+    if (warp == nw - 1) {
+      const unsigned long long valid = valid_species(P, B, p_begin, c0, c1, true);
+      const unsigned lt = (1u << lane) - 1u;
+      int e = 0;
+      for (int s = 0; s < nsp; ++s) {
+        if (lane == 0) sBase[s] = e;
+        for (int c = 0; c0 + 32 * c < c1; ++c) {
+          const bool on = (valid >> (8 * c + s)) & 1ull;
+          const unsigned m = __ballot_sync(0xffffffffu, on);
+          const int at = e + __popc(m & lt);
+          if (on) list[at] = (unsigned short)(32 * c + lane);
+          slot[s * kContractChunk + 32 * c + lane] = (short)(on ? at : -1);
+          e += __popc(m);
         }
-        if (lane == 0) sBase[nsp] = e;
       }
-      __syncthreads();  // H and the lists are complete; c_nlm and Gp under the rows are read
-      const float *src[NC];
+      if (lane == 0) sBase[nsp] = e;
+    }
+    __syncthreads();  // H and the lists are complete; c_nlm and Gp under the rows are read
+    const float *src[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+      src[c] = piece[c].rad ? B.rad + (size_t)c0 * nsp * 2 * AMAX + piece[c].first
+                            : B.ang + (size_t)c0 * AW + piece[c].first;
+    // a unit: two entries of a species.  The units go round the warps, from one
+    // species on to the next; s, e: this warp's next unit, turn: the warp to which
+    // the species' first unit falls
+    int s = 0, turn = 0, e = sBase[0] + 2 * warp;
+    auto settle = [&]() {  // past the species' last unit: on to the next species
+      while (s < nsp && e >= sBase[s + 1]) {
+        turn = (turn + ((sBase[s + 1] - sBase[s] + 1) >> 1)) & (nw - 1);
+        ++s;
+        if (s < nsp) e = sBase[s] + 2 * ((warp - turn) & (nw - 1));
+      }
+    };
+    auto copy = [&](float *dst) {
+      const int last = sBase[s + 1] - 1;
+      const unsigned j0 = list[e], j1 = list[min(e + 1, last)];
 #pragma unroll
       for (int c = 0; c < NC; ++c)
-        src[c] = piece[c].rad ? B.rad + (size_t)c0 * nsp * 2 * AMAX + piece[c].first
-                              : B.ang + (size_t)c0 * AW + piece[c].first;
-      // a unit: two entries of a species.  The units go round the warps, from one
-      // species on to the next; s, e: this warp's next unit, turn: the warp to which
-      // the species' first unit falls
-      int s = 0, turn = 0, e = sBase[0] + 2 * warp;
-      auto settle = [&]() {  // past the species' last unit: on to the next species
-        while (s < nsp && e >= sBase[s + 1]) {
-          turn = (turn + ((sBase[s + 1] - sBase[s] + 1) >> 1)) & (nw - 1);
-          ++s;
-          if (s < nsp) e = sBase[s] + 2 * ((warp - turn) & (nw - 1));
-        }
-      };
-      auto copy = [&](float *dst) {
-        const int last = sBase[s + 1] - 1;
-        const unsigned j0 = list[e], j1 = list[min(e + 1, last)];
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-          if (piece[c].on)
-            cp_async16(dst + piece[c].dst,
-                       src[c] + ((piece[c].second ? j1 : j0) * piece[c].per_pair + s * piece[c].per_species));
-      };
-      float2 H[HREG ? KJ * AMAX : 1];
-      int hs = -1;  // the species H holds
+        if (piece[c].on)
+          cp_async16(dst + piece[c].dst,
+                     src[c] + ((piece[c].second ? j1 : j0) * piece[c].per_pair + s * piece[c].per_species));
+    };
+    float2 H[HREG ? KJ * AMAX : 1];
+    int hs = -1;  // the species H holds
+    settle();
+    if (s < nsp) copy(stage);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    for (int buf = 0; s < nsp; buf ^= 1) {
+      const int us = s, ue = e, u_end = sBase[s + 1];
+      e += 2 * nw;
       settle();
-      if (s < nsp) copy(stage);
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-      for (int buf = 0; s < nsp; buf ^= 1) {
-        const int us = s, ue = e, u_end = sBase[s + 1];
-        e += 2 * nw;
-        settle();
-        if (s < nsp) copy(stage + (buf ^ 1) * 2 * ST);
-        asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
-        const float2 *Hs = sH + us * AMAX;
-        if constexpr (HREG)
-          if (us != hs) {
-            hs = us;
+      if (s < nsp) copy(stage + (buf ^ 1) * 2 * ST);
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
+      const float2 *Hs = sH + us * AMAX;
+      if constexpr (HREG)
+        if (us != hs) {
+          hs = us;
 #pragma unroll
-            for (int j = 0; j < KJ; ++j) {
-              const int k = hl + 16 * j;
+          for (int j = 0; j < KJ; ++j) {
+            const int k = hl + 16 * j;
 #pragma unroll
-              for (int n = 0; n < AMAX; n += 2) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (k < k_max) v = *(const float4 *)(Hs + k * HS + n);
-                H[j * AMAX + n] = make_float2(v.x, v.y);
-                H[j * AMAX + n + 1] = make_float2(v.z, v.w);
-              }
+            for (int n = 0; n < AMAX; n += 2) {
+              float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (k < k_max) v = *(const float4 *)(Hs + k * HS + n);
+              H[j * AMAX + n] = make_float2(v.x, v.y);
+              H[j * AMAX + n + 1] = make_float2(v.z, v.w);
             }
           }
-        __syncwarp();
-        const float *A = stage + (2 * buf + half) * ST;
-        const bool act = ue + half < u_end;
-        float R[AMAX], Rd[AMAX];
+        }
+      __syncwarp();
+      const float *A = stage + (2 * buf + half) * ST;
+      const bool act = ue + half < u_end;
+      float R[AMAX], Rd[AMAX];
 #pragma unroll
-        for (int n4 = 0; n4 < AMAX / 4; ++n4) {
-          const float4 a = ((const float4 *)(A + AW))[n4], d = ((const float4 *)(A + AW + AMAX))[n4];
-          R[4 * n4] = a.x; R[4 * n4 + 1] = a.y; R[4 * n4 + 2] = a.z; R[4 * n4 + 3] = a.w;
-          Rd[4 * n4] = d.x; Rd[4 * n4 + 1] = d.y; Rd[4 * n4 + 2] = d.z; Rd[4 * n4 + 3] = d.w;
-        }
-        const float sfac = A[row_sf(LC)];
-        float f_rad = 0.f, f_azi = 0.f, f_pol = 0.f;
+      for (int n4 = 0; n4 < AMAX / 4; ++n4) {
+        const float4 a = ((const float4 *)(A + AW))[n4], d = ((const float4 *)(A + AW + AMAX))[n4];
+        R[4 * n4] = a.x; R[4 * n4 + 1] = a.y; R[4 * n4 + 2] = a.z; R[4 * n4 + 3] = a.w;
+        Rd[4 * n4] = d.x; Rd[4 * n4 + 1] = d.y; Rd[4 * n4 + 2] = d.z; Rd[4 * n4 + 3] = d.w;
+      }
+      const float sfac = A[row_sf(LC)];
+      float f_rad = 0.f, f_azi = 0.f, f_pol = 0.f;
 #pragma unroll
-        for (int j = 0; j < KJ; ++j) {
-          if (16 * j >= k_max) break;
-          float Ur = 0.f, Ui = 0.f, Vr = 0.f, Vi = 0.f;
-          const int kj = hl + 16 * j;
-          const float2 *h = Hs + (kj < k_max ? kj : 0) * HS;
+      for (int j = 0; j < KJ; ++j) {
+        if (16 * j >= k_max) break;
+        float Ur = 0.f, Ui = 0.f, Vr = 0.f, Vi = 0.f;
+        const int kj = hl + 16 * j;
+        const float2 *h = Hs + (kj < k_max ? kj : 0) * HS;
 #pragma unroll
-          for (int n = 0; n < AMAX; n += 2) {
-            float4 v;
-            if constexpr (HREG)
-              v = make_float4(H[j * AMAX + n].x, H[j * AMAX + n].y, H[j * AMAX + n + 1].x, H[j * AMAX + n + 1].y);
-            else
-              v = *(const float4 *)(h + n);
-            Ur = fmaf(Rd[n], v.x, Ur); Ui = fmaf(Rd[n], v.y, Ui);
-            Vr = fmaf(R[n], v.x, Vr); Vi = fmaf(R[n], v.y, Vi);
-            Ur = fmaf(Rd[n + 1], v.z, Ur); Ui = fmaf(Rd[n + 1], v.w, Ui);
-            Vr = fmaf(R[n + 1], v.z, Vr); Vi = fmaf(R[n + 1], v.w, Vi);
-          }
-          if (!HREG && kj >= k_max) Ur = Ui = Vr = Vi = 0.f;
-          // rows hold amp i_l, amp di_l/dr and preflm_k P_k; cf carries the
-          // preflm ratios of the derivative combinations
-          const float Pk = A[oP[j]], il = A[row_il(LC) + oL[j]], ild = A[row_ild(LC) + oL[j]];
-          const float2 ee = *(const float2 *)(A + oE[j]);
-          const float *Pl = A + oP[j] + oL[j];
-          const float dms = cf[j].x * A[oX[j]] + cf[j].y * A[oP[j] + 1];
-          const float dvs = cf[j].z * Pl[0] + cf[j].w * Pl[2];
-          const float er = ee.x, ei = ee.y;
-          const float uu = Pk * il;
-          const float ur = Pk * ild - sfac * uu;
-          const float ua = dvs * il;
-          const float up = dms * il;
-          const float reU = er * Ur + ei * Ui;
-          const float reV = er * Vr + ei * Vi;
-          const float imV = ei * Vr - er * Vi;
-          f_rad = fmaf(uu, reU, fmaf(ur, reV, f_rad));
-          f_azi = fmaf(-ua, imV, f_azi);
-          f_pol = fmaf(up, reV, f_pol);
+        for (int n = 0; n < AMAX; n += 2) {
+          float4 v;
+          if constexpr (HREG)
+            v = make_float4(H[j * AMAX + n].x, H[j * AMAX + n].y, H[j * AMAX + n + 1].x, H[j * AMAX + n + 1].y);
+          else
+            v = *(const float4 *)(h + n);
+          Ur = fmaf(Rd[n], v.x, Ur); Ui = fmaf(Rd[n], v.y, Ui);
+          Vr = fmaf(R[n], v.x, Vr); Vi = fmaf(R[n], v.y, Vi);
+          Ur = fmaf(Rd[n + 1], v.z, Ur); Ui = fmaf(Rd[n + 1], v.w, Ui);
+          Vr = fmaf(R[n + 1], v.z, Vr); Vi = fmaf(R[n + 1], v.w, Vi);
         }
+        if (!HREG && kj >= k_max) Ur = Ui = Vr = Vi = 0.f;
+        // rows hold amp i_l, amp di_l/dr and preflm_k P_k; cf carries the
+        // preflm ratios of the derivative combinations
+        const float Pk = A[oP[j]], il = A[row_il(LC) + oL[j]], ild = A[row_ild(LC) + oL[j]];
+        const float2 ee = *(const float2 *)(A + oE[j]);
+        const float *Pl = A + oP[j] + oL[j];
+        const float dms = cf[j].x * A[oX[j]] + cf[j].y * A[oP[j] + 1];
+        const float dvs = cf[j].z * Pl[0] + cf[j].w * Pl[2];
+        const float er = ee.x, ei = ee.y;
+        const float uu = Pk * il;
+        const float ur = Pk * ild - sfac * uu;
+        const float ua = dvs * il;
+        const float up = dms * il;
+        const float reU = er * Ur + ei * Ui;
+        const float reV = er * Vr + ei * Vi;
+        const float imV = ei * Vr - er * Vi;
+        f_rad = fmaf(uu, reU, fmaf(ur, reV, f_rad));
+        f_azi = fmaf(-ua, imV, f_azi);
+        f_pol = fmaf(up, reV, f_pol);
+      }
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-          f_rad += __shfl_xor_sync(0xffffffffu, f_rad, o);
-          f_azi += __shfl_xor_sync(0xffffffffu, f_azi, o);
-          f_pol += __shfl_xor_sync(0xffffffffu, f_pol, o);
-        }
-        if (act && hl == 0) {
-          float *F = sF + 3 * (ue + half);
-          F[0] = f_rad;
-          F[1] = f_azi;
-          F[2] = f_pol;
-        }
-        __syncwarp();  // the rows are read: the buffer is free for the unit after next
+      for (int o = 8; o > 0; o >>= 1) {
+        f_rad += __shfl_xor_sync(0xffffffffu, f_rad, o);
+        f_azi += __shfl_xor_sync(0xffffffffu, f_azi, o);
+        f_pol += __shfl_xor_sync(0xffffffffu, f_pol, o);
       }
-      __syncthreads();
-      // ---- per pair: sum its entries, rotate to Cartesian (:1864-1875)
-      // and add it to the central pair's slot (the pair's place in the row, modulo
-      // slots): tid's, and tid + nt's with two apiece
-      const int n_k = c1 - c0;
-      double x0 = 0.0, y0 = 0.0, z0 = 0.0, x1 = 0.0, y1 = 0.0, z1 = 0.0;
-      if (c0 > p_begin) {
-        x0 = held[0]; y0 = held[1]; z0 = held[2];
-        x1 = held[3]; y1 = held[4]; z1 = held[5];
+      if (act && hl == 0) {
+        float *F = sF + 3 * (ue + half);
+        F[0] = f_rad;
+        F[1] = f_azi;
+        F[2] = f_pol;
       }
-      for (int k = tid - (slots > kContractChunk ? (c0 - p_begin) & (slots - 1) : 0); k < n_k; k += nt) {
-        if (k < 0 || c0 + k <= p_begin) continue;
-        double px = 0.0, py = 0.0, pz = 0.0, fr = 0.0, fa = 0.0, fp = 0.0;
-        bool any = false;
-        for (int s = 0; s < nsp; ++s) {
-          const int e = slot[s * kContractChunk + k];
-          if (e >= 0) {
-            any = true;
-            fr += sF[3 * e];
-            fa += sF[3 * e + 1];
-            fp += sF[3 * e + 2];
-          }
-        }
-        if (any) {
-          const float *A = B.ang + (size_t)(c0 + k) * AW;
-          const double ct = A[row_x(LC)], st = A[row_sq(LC)], cf_ = A[row_e(LC) + 2], sf = -A[row_e(LC) + 3];
-          const double ir = 1.0 / B.rjs[c0 + k];
-          px = sgn * (st * cf_ * fr - ct * cf_ * ir * fp - sf * ir * fa);
-          py = sgn * (st * sf * fr - ct * sf * ir * fp + cf_ * ir * fa);
-          pz = sgn * (ct * fr + st * ir * fp);
-        }
-        double *po = pair_out + (size_t)3 * (c0 + k);
-        po[0] = px;
-        po[1] = py;
-        po[2] = pz;
-        if (two && k >= nt) {
-          x1 -= px;
-          y1 -= py;
-          z1 -= pz;
-        } else {
-          x0 -= px;
-          y0 -= py;
-          z0 -= pz;
-        }
-      }
-      if (c1 < p_end) {
-        held[0] = x0; held[1] = y0; held[2] = z0;
-        held[3] = x1; held[4] = y1; held[5] = z1;
-        continue;
-      }
-      // the central pair is minus the sum of the others (:1875)
-      auto fold = [&](double x, double y, double z, int w) {  // the slots 32 w + lane
-        if (32 * w < p_end - p_begin) {  // the row reaches them
-          x = warp_sum(x);
-          y = warp_sum(y);
-          z = warp_sum(z);
-        }
-        if (lane == 0) {
-          double *r = sRed + 8 + 3 * w;
-          r[0] = x;
-          r[1] = y;
-          r[2] = z;
-        }
-      };
-      if (tid < slots) fold(x0, y0, z0, warp);
-      if (two) fold(x1, y1, z1, warp + nw);
-      __syncthreads();
-      if (tid < 3) pair_out[(size_t)3 * p_begin + tid] = slot_tree<3>(sRed + 8 + tid, slots);
+      __syncwarp();  // the rows are read: the buffer is free for the unit after next
     }
-    __syncthreads();  // shared memory is free for the next site
+    __syncthreads();
+    // ---- per pair: sum its entries, rotate to Cartesian (:1864-1875)
+    // and add it to the central pair's slot (the pair's place in the row, modulo
+    // slots): tid's, and tid + nt's with two apiece
+    const int n_k = c1 - c0;
+    double x0 = 0.0, y0 = 0.0, z0 = 0.0, x1 = 0.0, y1 = 0.0, z1 = 0.0;
+    if (c0 > p_begin) {
+      x0 = held[0]; y0 = held[1]; z0 = held[2];
+      x1 = held[3]; y1 = held[4]; z1 = held[5];
+    }
+    for (int k = tid - (slots > kContractChunk ? (c0 - p_begin) & (slots - 1) : 0); k < n_k; k += nt) {
+      if (k < 0 || c0 + k <= p_begin) continue;
+      double px = 0.0, py = 0.0, pz = 0.0, fr = 0.0, fa = 0.0, fp = 0.0;
+      bool any = false;
+      for (int s = 0; s < nsp; ++s) {
+        const int e = slot[s * kContractChunk + k];
+        if (e >= 0) {
+          any = true;
+          fr += sF[3 * e];
+          fa += sF[3 * e + 1];
+          fp += sF[3 * e + 2];
+        }
+      }
+      if (any) {
+        const float *A = B.ang + (size_t)(c0 + k) * AW;
+        const double ct = A[row_x(LC)], st = A[row_sq(LC)], cf_ = A[row_e(LC) + 2], sf = -A[row_e(LC) + 3];
+        const double ir = 1.0 / B.rjs[c0 + k];
+        px = sgn * (st * cf_ * fr - ct * cf_ * ir * fp - sf * ir * fa);
+        py = sgn * (st * sf * fr - ct * sf * ir * fp + cf_ * ir * fa);
+        pz = sgn * (ct * fr + st * ir * fp);
+      }
+      double *po = pair_out + (size_t)3 * (c0 + k);
+      po[0] = px;
+      po[1] = py;
+      po[2] = pz;
+      if (two && k >= nt) {
+        x1 -= px;
+        y1 -= py;
+        z1 -= pz;
+      } else {
+        x0 -= px;
+        y0 -= py;
+        z0 -= pz;
+      }
+    }
+    if (c1 < p_end) {
+      held[0] = x0; held[1] = y0; held[2] = z0;
+      held[3] = x1; held[4] = y1; held[5] = z1;
+      continue;
+    }
+    // the central pair is minus the sum of the others (:1875)
+    auto fold = [&](double x, double y, double z, int w) {  // the slots 32 w + lane
+      if (32 * w < p_end - p_begin) {  // the row reaches them
+        x = warp_sum(x);
+        y = warp_sum(y);
+        z = warp_sum(z);
+      }
+      if (lane == 0) {
+        double *r = sRed + 8 + 3 * w;
+        r[0] = x;
+        r[1] = y;
+        r[2] = z;
+      }
+    };
+    if (tid < slots) fold(x0, y0, z0, warp);
+    if (two) fold(x1, y1, z1, warp + nw);
+    __syncthreads();
+    if (tid < 3) pair_out[(size_t)3 * p_begin + tid] = slot_tree<3>(sRed + 8 + tid, slots);
   }
 }
 
@@ -2483,8 +2475,7 @@ static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, cons
   cudaError_t e = ensure_smem_limit(kern, sm);
   if (e != cudaSuccess) return e;
   if (n > 0) {
-    const int grid = cfg.max_ctas > 0 && cfg.max_ctas < n ? cfg.max_ctas : n;
-    kern<<<grid, threads, sm, cfg.stream>>>(P, B, chunk, kw, groups, soap, keep_c, keep_norm, keep);
+    kern<<<n, threads, sm, cfg.stream>>>(P, B, chunk, kw, groups, soap, keep_c, keep_norm, keep);
   }
   return cudaGetLastError();
 }
@@ -2575,6 +2566,10 @@ static int contract_threads(const DevParams &P, int n_sites) {
   return best;
 }
 
+int contract_rule_threads(const DevParams &P, int n_sites) {
+  return P.amax_t == 8 ? contract_threads<8, 8>(P, n_sites) : contract_threads<16, 12>(P, n_sites);
+}
+
 template <int AMAX, int LC>
 static cudaError_t run_contract(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg,
                                 const double *soap, const double *G, int g_layout, double sgn,
@@ -2587,8 +2582,7 @@ static cudaError_t run_contract(const DevParams &P, const DevBatch &B, const Lau
   cudaError_t e = ensure_smem_limit(kern, sm);
   if (e != cudaSuccess) return e;
   if (n > 0) {
-    const int grid = cfg.max_ctas > 0 && cfg.max_ctas < n ? cfg.max_ctas : n;
-    kern<<<grid, threads, sm, cfg.stream>>>(P, B, cfg.slots, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
+    kern<<<n, threads, sm, cfg.stream>>>(P, B, cfg.slots, soap, G, g_layout, sgn, keep_c, keep_norm, pair);
   }
   return cudaGetLastError();
 }

@@ -165,3 +165,27 @@ def test_groups_of_warps_give_the_same_sums(name, threads):
     for n_sites in (base.n_sites, 148, 149, 444, 445):
         nl, site, _ = repeated(base, n_sites)
         np.testing.assert_array_equal(ctx.descriptor(ctx.batch(nl)).cpu().numpy(), want[site])
+
+
+@pytest.mark.parametrize("name", ["3sp", "wide"])
+def test_the_autotuner_changes_no_bits(name):
+    """It times the contract's CTA sizes, which share their sums' slots, and leaves the
+    descriptor's chunks as they are; a batch of another size takes the rule again."""
+    hp = DEFS[name]
+    base = edge_sites([64, 129, 256, 257, 300], hp.n_species, seed=43)
+    ctx = Context(hp)
+    ctx.set_tensor_cores(False)
+    G = np.random.default_rng(6).standard_normal((ctx.n_soap, base.n_sites))
+
+    def both(n_sites):
+        nl, site, _ = repeated(base, n_sites)
+        b = ctx.batch(nl)
+        soap = ctx.descriptor(b)
+        force = ctx.contract(b, soap, torch.as_tensor(np.ascontiguousarray(G[:, site])).cuda())
+        return b, soap, force
+    before = {n: both(n)[1:] for n in (5, 700)}
+    for tuned in (5, 700, 200, 5):
+        ctx.autotune(both(tuned)[0])
+        for n, (soap, force) in before.items():
+            _, s, f = both(n)
+            assert torch.equal(s, soap) and torch.equal(f, force)
