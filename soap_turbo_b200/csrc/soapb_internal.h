@@ -149,10 +149,10 @@ struct DevBatch {
                             // word) the site kernels' work counters
   float *rad;            // (n_pairs, n_species, 2, amax_t): 4 pi R_n and its r-derivative
   float *ang;            // (n_pairs, ang_row): the pair's angular row (see soapb_mixed.cu)
-  int *ticket;           // work counters of the persistent site kernels, in the last word
+  int *ticket;           // work counters of the tensor-core site kernels, in the last word
                          // of err (the kernels put them back to 0 when they finish)
   int site_lo, site_hi;  // the sites a site-kernel launch processes (all: 0, n_sites)
-  int *order = nullptr;  // n_sites: the order in which the persistent site kernels take the
+  int *order = nullptr;  // n_sites: the order in which the site kernels take the
                          // sites, heaviest rows first (written by the pair kernel's scan when
                          // one scan tile covers the batch), or null: index order
 };

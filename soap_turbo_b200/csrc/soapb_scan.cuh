@@ -15,7 +15,7 @@ namespace soapb {
 //   err[1]     the scan's tile counter (low 32 bits);
 //   err[2 + t] scan tile t's status: flag << 32 | sum, flag 1 = the tile's own
 //              sum, 2 = the inclusive prefix up to the tile (0 = not yet);
-//   the last word: the two work counters of the persistent site kernels.
+//   the last word: the two work counters of the tensor-core site kernels.
 // n_neigh is scanned in tiles of 2048 sites with a decoupled look-back: each
 // tile publishes its sum, then walks back over its predecessors until it meets
 // an inclusive prefix.  A tile takes its index from the counter, so every
@@ -127,7 +127,7 @@ __device__ __forceinline__ void prep_scan_tile(const DevBatch &B, int scan_tiles
 }
 
 // The sites of a batch one scan tile covers, heaviest row first, into
-// B.order for the persistent site kernels (a counting sort on min(n_neigh, 255);
+// B.order for the site kernels (a counting sort on min(n_neigh, 255);
 // the order within a count is whatever the atomics give, which changes only
 // which CTA computes a site, not its result), so that their last sites are the
 // lightest.  One CTA of NTH threads, beside the scan CTA; sv: kScanTile ints

@@ -89,3 +89,28 @@ def test_hessian_bits_do_not_depend_on_the_batch(alpha, l_max):
         first = got if first is None else first
         np.testing.assert_array_equal(got, first[pair])
     assert np.isfinite(first).all() and np.abs(first).max() > 0
+
+
+@pytest.mark.parametrize("threads", [0, 64, 256])
+@pytest.mark.parametrize("n_sites", [1, 6, 297, 1185])
+def test_wide_instantiation_over_rows_of_several_chunks(n_sites, threads):
+    """alpha above 8 and l_max above 8: two groups of radial indices, of which the second
+    species' last is partly past its alpha, three warps of k, H read from shared memory.
+    The first site's row is several chunks long, so that a batch of one has one too."""
+    hp = syn.Hyper(alpha_max=[10, 7], l_max=10, basis="poly3gauss", compress_mode="trivial")
+    base = edge_sites([290, 64, 129, 256, 33, 1], 2, seed=47)
+    ctx = Context(hp)
+    ctx.set_threads_per_site(threads)
+    W, S = ctx.basis()
+    ref = O.get_soap(hp, base, W, S, do_derivatives=True)
+    G = np.random.default_rng(8).standard_normal((ctx.n_soap, base.n_sites))
+    pref = ref.contract(G, 1.0)
+    nl, site, pair = repeated(base, n_sites)
+    b = ctx.batch(nl)
+    soap = ctx.descriptor(b)
+    force = ctx.contract(b, soap, torch.as_tensor(np.ascontiguousarray(G[:, site])).cuda()).cpu().numpy()
+    ctx.check_inputs()
+    ok = np.abs(ref.soap).max(axis=1)[site] > 0
+    assert ok.any()
+    assert site_rel_err(soap.cpu().numpy()[ok], ref.soap[site][ok]) <= SOAP_TOL
+    assert max_rel_err(force, pref[pair]) <= VJP_TOL
