@@ -929,17 +929,18 @@ size_t hess_smem_bytes(const DevParams &P, int n_vec, int n_sites) {
 }
 
 // One CTA of 512 threads an SM or two of 256.  512 where shared memory holds one CTA
-// of 256 only; else where the sites are one wave of 512, or three against two of 256,
-// each of which takes 1.6 (small definitions) to 1.9 of the time of a wave of 512.  Calls
-// of three vectors with 512 and 256 threads, us: one species, l_max 8, 148 sites 225 and
-// 281, 149 317 and 315, 296 353 and 348, 297 419 and 456, 444 485 and 561, 445 527 and
-// 561, 600 697 and 715; two species of alpha 4, l_max 4 145 and 162, 193 and 175, 211 and
-// 189, 250 and 239, 277 and 290, 305 and 291, 384 and 349; one of alpha 10, l_max 12 (one
-// CTA of either) 403 and 492 at 148, 666 and 851 at 296, 1376 and 1769 at 600.
+// of 256 only; else up to one site per SM, and up to three where a site is some work
+// (beyond, two CTAs of 256 have less of a last wave).  Calls of three vectors with 512 and
+// 256 threads, us, at 148, 149, 296, 297, 444, 445 and 600 sites: one species, l_max 8 225
+// and 281, 317 and 315, 353 and 348, 419 and 456, 485 and 561, 527 and 561, 697 and 715;
+// two species of alpha 4, l_max 4 145 and 162, 193 and 175, 211 and 189, 250 and 239, 277
+// and 290, 305 and 291, 384 and 349.  One species of alpha 10, l_max 12 (one CTA of
+// either) 403 and 492 at 148, 666 and 851 at 296, 1376 and 1769 at 600.  150 sites of one
+// species, l_max 6, with five vectors 300 and 313.
 int hess_threads(const DevParams &P, int n_vec, int n_sites) {
   if (sizeof(double) * (size_t)hess_smem(P, n_vec, 256).total > kHessSmemPair) return 512;
-  const int sms = sm_count(), waves = (n_sites + sms - 1) / sms;
-  return waves <= 1 || waves == 3 ? 512 : 256;
+  const int sms = sm_count(), most = P.n_max * P.k_max > 128 ? 3 * sms : sms;
+  return n_sites <= most ? 512 : 256;
 }
 
 template <int NT>
