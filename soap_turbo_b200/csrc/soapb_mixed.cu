@@ -807,6 +807,55 @@ __device__ __forceinline__ double slots_by_warp(const double (&v)[4]) {
   return t + __shfl_xor_sync(0xffffffffu, t, 8);
 }
 
+// The norm of a site's components (:805-809), squared: over 128 slots by every warp for
+// itself, or over `slots` of them by the CTA through red (slots / 32 doubles).
+__device__ __forceinline__ double norm2_by_warp(const float *s, int n) {
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int o = threadIdx.x & 31; o < n; o += 128)
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const double y = o + 32 * w < n ? (double)s[o + 32 * w] : 0.0;
+      v[w] = fma(y, y, v[w]);
+    }
+  return slots_by_warp(v);
+}
+template <typename Value>
+__device__ __forceinline__ double norm2_by_slots(int n, int slots, double *red, Value value) {
+  const int lane = threadIdx.x & 31;
+  for (int w = threadIdx.x >> 5; 32 * w < slots; w += blockDim.x >> 5) {
+    double v = 0.0;
+    for (int o = 32 * w + lane; o < n; o += slots) {
+      const double y = value(o);
+      v = fma(y, y, v);
+    }
+    v = warp_sum(v);
+    if (lane == 0) red[w] = v;
+  }
+  __syncthreads();
+  return slot_tree(red, slots);
+}
+
+// A site's components s added to the caller's row before the norm is taken, as the
+// reference adds the compressed descriptor into soap (:798-802); returns the norm.  The row
+// may lie in host memory, a round trip over the link away: with room for the sums (sum)
+// it is read once, by loads that overlap (page-locked soap of 5000 and 1679 sites, both
+// calls: 5163 -> 4743 and 1605 -> 1560 us).  An instantiation of its own: beside the other
+// outcome in one kernel it took that 1 to 4 % more time.
+__device__ __forceinline__ double add_and_normalise(const float *s, int n, int slots, double *red, double *sum,
+                                                 double *out) {
+  if (sum) {
+#pragma unroll 4
+    for (int o = threadIdx.x; o < n; o += blockDim.x) sum[o] = (double)s[o] + out[o];
+    __syncthreads();
+  }
+  auto value = [&](int o) { return sum ? sum[o] : (double)s[o] + out[o]; };
+  double norm = sqrt(norm2_by_slots(n, slots, red, value));
+  if (norm < 1.0e-5) norm = 1.0;
+  const double inv = 1.0 / norm;
+  for (int o = threadIdx.x; o < n; o += blockDim.x) out[o] = value(o) * inv;
+  return norm;
+}
+
 // ------------------------------------------------------------ descriptor
 // One CTA of a few warps per site; a thread owns one k = (l, m) and NH of the
 // radial indices of every species block (warp w: k = 32 (w % kw) + lane, radial
@@ -858,13 +907,13 @@ __host__ __device__ constexpr int desc_min_ctas(int AMAX, int NH, int groups) {
 template <int AMAX, int LC, int NH, int GROUPS>
 constexpr int kDescThreads = GROUPS ? GROUPS : ((LC + 1) * (LC + 2) / 2 + 31) / 32 * 32 * (AMAX / NH);
 
-template <int AMAX, int LC, int NH, int GROUPS>
+// ACC: the components are added to the caller's rows
+template <int AMAX, int LC, int NH, int GROUPS, bool ACC>
 __global__ void __launch_bounds__(kDescThreads<AMAX, LC, NH, GROUPS>,
                                   desc_min_ctas(AMAX, NH, GROUPS))
     k_descriptor(const DevParams P, const DevBatch B, int chunk, int kw, int groups, double *__restrict__ soap_out,
                  float *__restrict__ keep_c, double *__restrict__ keep_norm, int keep) {
-  // keep: bit 0 keeps c_nlm and the norm for the contract, bit 1 accumulates
-  // into soap_out
+  // keep: whether c_nlm and the norm are kept for the contract
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int AW = row_len(LC), ST = desc_stride(AMAX, LC), HD = desc_head(LC);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
@@ -907,7 +956,7 @@ __global__ void __launch_bounds__(kDescThreads<AMAX, LC, NH, GROUPS>,
   // for the last, and that of the last
   int cs = group, n_rounds = 0;
   double tr[NH], ti[NH], dr[NH], di[NH];
-  float2 *kc = (float2 *)(keep_c + ((keep & 1) ? (size_t)site * keep_stride(P) : 0)) + kk;
+  float2 *kc = (float2 *)(keep_c + (keep ? (size_t)site * keep_stride(P) : 0)) + kk;
   auto finish = [&]() {  // species cs is complete
     const int a = P.rad[cs].alpha, nb = P.rad[cs].nbeg;
     if (n_rounds != 1)
@@ -930,7 +979,7 @@ __global__ void __launch_bounds__(kDescThreads<AMAX, LC, NH, GROUPS>,
 #pragma unroll
       for (int n = 0; n < NH; ++n)
         if (n0 + n < a) cc[n * KS] = make_float2((float)dr[n], (float)di[n]);
-    if (own && (keep & 1)) {
+    if (own && keep) {
       float2 *kr = kc + (nb + n0) * KS;
 #pragma unroll
       for (int n = 0; n < NH; ++n)
@@ -1087,44 +1136,19 @@ __global__ void __launch_bounds__(kDescThreads<AMAX, LC, NH, GROUPS>,
     }
     __syncthreads();
   }
-  // the norm (:805-809) over `chunk` slots.  accumulate: the caller's soap row is
-  // added before the norm is taken, as the reference adds the compressed descriptor
-  // into soap (:798-802); the row may lie in host memory, so it is read here and where
-  // it is written, and not by every warp
-  double *out = soap_out + (size_t)site * P.n_soap;
-  const bool acc = (keep & 2) != 0;
-  double nrm2;
-  if (!acc && chunk == 128) {
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int o = lane; o < P.n_soap; o += 128)
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const double y = o + 32 * w < P.n_soap ? (double)sS[o + 32 * w] : 0.0;
-        v[w] = fma(y, y, v[w]);
-      }
-    nrm2 = slots_by_warp(v);
+  double *out = soap_out + (size_t)site * P.n_soap, norm;
+  if constexpr (ACC) {
+    const size_t at = align_up(Ly.S + (size_t)P.n_soap * sizeof(float), 8);
+    const bool room = at + (size_t)P.n_soap * sizeof(double) <= Ly.total;
+    norm = add_and_normalise(sS, P.n_soap, chunk, (double *)(smem + Ly.base), room ? (double *)(smem + at) : nullptr, out);
   } else {
-    double *red = (double *)(smem + Ly.base);  // eight: the species' places are read
-    for (int w = warp; 32 * w < chunk; w += nw) {
-      double v = 0.0;
-      for (int o = 32 * w + lane; o < P.n_soap; o += chunk) {
-        const double y = acc ? (double)sS[o] + out[o] : (double)sS[o];
-        v = fma(y, y, v);
-      }
-      v = warp_sum(v);
-      if (lane == 0) red[w] = v;
-    }
-    __syncthreads();
-    nrm2 = slot_tree(red, chunk);
-  }
-  double norm = sqrt(nrm2);
-  if (norm < 1.0e-5) norm = 1.0;
-  const double inv = 1.0 / norm;
-  if (acc)
-    for (int o = tid; o < P.n_soap; o += nt) out[o] = ((double)sS[o] + out[o]) * inv;
-  else
+    norm = sqrt(chunk == 128 ? norm2_by_warp(sS, P.n_soap)
+                             : norm2_by_slots(P.n_soap, chunk, (double *)(smem + Ly.base), [&](int o) { return (double)sS[o]; }));
+    if (norm < 1.0e-5) norm = 1.0;
+    const double inv = 1.0 / norm;
     for (int o = tid; o < P.n_soap; o += nt) out[o] = (double)sS[o] * inv;
-  if ((keep & 1) && tid == 0) keep_norm[site] = norm;
+  }
+  if (keep && tid == 0) keep_norm[site] = norm;
 }
 
 // ------------------------------------------------------------ descriptor on tensor cores
@@ -2461,7 +2485,7 @@ static cudaError_t run_descriptor_tc(const DevParams &P, const DevBatch &B, cons
 // three species 37 and 41, 64 and 64, 82 and 84, 99 and 103, 150 and 154.
 constexpr int kDescFewPerSm = 2, kDescWideSites = 4096;
 
-template <int AMAX, int LC, int NH, int GROUPS = 0>
+template <int AMAX, int LC, int NH, int GROUPS = 0, bool ACC = false>
 static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, const LaunchCfg &cfg, int max_alpha,
                                      double *soap, float *keep_c, double *keep_norm, int keep) {
   const int kw = (P.k_max + 31) / 32, n = B.site_hi - B.site_lo, own = 32 * kw * ((max_alpha + NH - 1) / NH);
@@ -2471,11 +2495,11 @@ static cudaError_t run_descriptor_as(const DevParams &P, const DevBatch &B, cons
   if (NH == 2 && GROUPS == 0 && n <= kDescFewPerSm * sm_count() && threads < 128) threads = 128;
   const int chunk = cfg.slots;  // fixes the summation groups
   const size_t sm = desc_layout(P, chunk, AMAX, LC).total;
-  auto kern = k_descriptor<AMAX, LC, NH, GROUPS>;
+  auto kern = k_descriptor<AMAX, LC, NH, GROUPS, ACC>;
   cudaError_t e = ensure_smem_limit(kern, sm);
   if (e != cudaSuccess) return e;
   if (n > 0) {
-    kern<<<n, threads, sm, cfg.stream>>>(P, B, chunk, kw, groups, soap, keep_c, keep_norm, keep);
+    kern<<<n, threads, sm, cfg.stream>>>(P, B, chunk, kw, groups, soap, keep_c, keep_norm, keep & 1);
   }
   return cudaGetLastError();
 }
@@ -2488,6 +2512,10 @@ static cudaError_t run_descriptor(const DevParams &P, const DevBatch &B, const L
   int max_alpha = 1;
   for (int s = 0; s < P.n_species; ++s) max_alpha = P.rad[s].alpha > max_alpha ? P.rad[s].alpha : max_alpha;
   const int n = B.site_hi - B.site_lo, sms = sm_count();
+  // Sums into the caller's rows are the drop-in call's alone, which the copies around
+  // bound: one form.
+  if (keep & 2)
+    return run_descriptor_as<AMAX, LC, AMAX == 8 ? 4 : 8, 0, true>(P, B, cfg, max_alpha, soap, keep_c, keep_norm, keep);
   // Rows of several chunks on average: one species at a time leaves a round few entries.
   // Up to a site per SM every species gets its warps (rows of 340 pairs, 100 sites of
   // eight species of alpha 4 103 -> 48 us, of five of alpha 6 68 -> 41); beyond, where one
