@@ -236,14 +236,17 @@ __host__ __device__ constexpr int pair_stage_stride(int LC) {
 //  * the angular row (src/soap_turbo_angular.f90:267-463, 549-607), staged by the
 //    warp in shared memory, four values at a time, and copied out with coalesced
 //    stores.
-// Bound by instructions (half of the issue slots; 30 % of them index arithmetic)
-// and the warps' waits on tables and FP64 chains.  So a warp shares nothing but the
+// Bound by instructions (44 % of the issue slots at 1679 sites, 55 % at 16384; 30 % of
+// them index arithmetic) and the warps' waits on tables and FP64 chains; without tables by
+// the FP64 chain of a pair alone (12 and 20 % of the slots, 179 and 122 registers: sigma
+// scaling at l_max 12, poly3operator).  So a warp shares nothing but the
 // constants with its CTA and takes no barrier after theirs, the table reads of
 // one warp run under the FP64 of others, and the copies' loops are of compile-time
 // length.  Whole-step times with rows staged by value, CTA-wide copies behind
 // barriers and the tables between the two: 128.5 us at 1679 sites, 717 at 16384
-// and 75 at 777 without tables; 124.5, 707 and 72.6 now.  Eight CTAs an SM
-// (64 registers, spills) or CTA-wide copies in this form: 125 and 128.4 us at 1679.
+// and 75 at 777 without tables; in this form, beside the same site kernels, 124.5, 707
+// and 72.6.  Eight CTAs an SM (64 registers, spills) or CTA-wide copies in this form: 125
+// and 128.4 us at 1679.
 // The site kernels only read these rows; soap_contract reads the rows of the
 // descriptor call that kept its state, as the reference keeps the radial and
 // angular expansions between get_soap and soap_contract.
@@ -871,11 +874,11 @@ __device__ __forceinline__ double add_and_normalise(const float *s, int n, int s
 //             groups do not depend on the launch shape.
 //  spectrum   one dot product per kept component, the components ordered by
 //             l (P.ps_order) so that a warp's dot products are equally long
-// What bounds it: instructions (8.3 k per site of 52 pairs and three species, of
-// which the products are a tenth) issued at 43 % of the rate with 14 warps per SM,
-// by the latency of a warp's chain.  One CTA of 128 threads that staged, sorted and
-// summed behind barriers took 15 k: 338 against 251 us at 13092 sites of three
-// species, 55 against 43 us at 1679.
+// What bounds it: instructions, and the latency of a warp's chain: per site of 52 pairs and
+// three species 14.0 k with four radial indices a thread, issued at 60 % of the rate (39.6
+// us at 1679 sites), 8.7 k with eight, at 46 % (227 us at 13092); the products are a tenth
+// of them.  One CTA of 128 threads that staged, sorted and summed behind barriers took
+// 15 k: 55 and 338 us.
 struct DescLayout {
   size_t list, base, X, P, S, total;
 };
@@ -1491,10 +1494,11 @@ __global__ void __launch_bounds__(NT) k_descriptor_tc(const DevParams P, const D
 //             species' first entry to its last where they hold it (AMAX 8, three k a
 //             lane); the k summed over the lanes
 //  pairs      their entries added, rotated to Cartesian; the self pair minus their sum
-// What bounds it: instructions (16 k per site of 58 pairs and one species), issued at
-// 59 % of the rate by 16 warps per SM.  The kernel before (one CTA of 128 threads,
-// 32 staged entries behind barriers, H read from shared memory for every entry)
-// took 439 us at 16384 sites of one species and 66 at 1679 of three; this one 313 and 62.
+// What bounds it: instructions (13.7 k per site of 58 pairs and one species, 16.7 k of
+// three species), issued at 66 and 48 % of the rate by 16 warps per SM.  One CTA of 128
+// threads with 32 staged entries behind barriers and H read from shared memory for every
+// entry took 439 us at 16384 sites of one species and 66 at 1679 of three; this one 313
+// and 57.
 struct ContractLayout {
   size_t H, base, list, slot, red, X, C, Gu, Gp, F, stage, total;
 };
